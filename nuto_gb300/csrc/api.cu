@@ -489,8 +489,12 @@ static void SetupLaw(Ctx& c)
     L.alpha = p.alpha;
     // ModifiedMisesStrainNorm (ModifiedMisesStrainNorm.h:70-78)
     L.k = p.k;
+    L.lamD = (L.m3K - L.m2G) * L.d2 / 3;
+    L.muD = L.m2G / 2;
     L.K1 = (p.k - 1.) / (2. * p.k * (1 - 2 * p.nu));
     L.K2 = 3. / (p.k * (1. + p.nu) * (1. + p.nu));
+    L.K2o6 = L.K2 / 6.;
+    L.K2o4 = L.K2 / 4.;
     L.c = p.c;
     L.R = p.R;
     L.eta = p.eta;

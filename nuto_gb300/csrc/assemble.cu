@@ -8,6 +8,7 @@
 // integrates over the points and scatters. Geometry (w * det J and dN/dX per integration point) is computed once
 // per mesh and cached planar ([field][cell]) so that every per-cell load is coalesced.
 #include "internal.cuh"
+#include "sumfac.cuh"
 
 #include <algorithm>
 #include <mutex>
@@ -85,7 +86,7 @@ __global__ void __launch_bounds__(128) k_geometry(int64_t nCells, int64_t nCoord
                                                   const int32_t* __restrict__ geoConnT,
                                                   const double* __restrict__ tables, int tabW, int tabDNg,
                                                   int tabDNd, int stride, double* __restrict__ geo64,
-                                                  float* __restrict__ geo32)
+                                                  double* __restrict__ jac, double jacScale)
 {
     const int64_t it = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
     if (it >= nCells * NIP)
@@ -143,7 +144,16 @@ __global__ void __launch_bounds__(128) k_geometry(int64_t nCells, int64_t nCoord
     const int64_t base = static_cast<int64_t>(q) * stride;
     const double wdj = tables[tabW + q] * det;
     geo64[base * nCells + e] = wdj;
-    geo32[base * nCells + e] = static_cast<float>(wdj);
+    if (jac)
+    {
+        const int64_t jb = static_cast<int64_t>(q) * (1 + DIM * DIM);
+        jac[jb * nCells + e] = wdj;
+#pragma unroll
+        for (int j = 0; j < DIM; ++j)
+#pragma unroll
+            for (int k = 0; k < DIM; ++k)
+                jac[(jb + 1 + j * DIM + k) * nCells + e] = jacScale * inv[j][k];
+    }
     const double* dNd = tables + tabDNd + q * ND * 3;
     for (int n = 0; n < ND; ++n)
 #pragma unroll
@@ -153,10 +163,16 @@ __global__ void __launch_bounds__(128) k_geometry(int64_t nCells, int64_t nCoord
 #pragma unroll
             for (int j = 0; j < DIM; ++j)
                 s += dNd[n * 3 + j] * inv[j][k];
-            const int64_t idx = (base + 1 + n * DIM + k) * nCells + e;
-            geo64[idx] = s;
-            geo32[idx] = static_cast<float>(s);
+            geo64[(base + 1 + n * DIM + k) * nCells + e] = s;
         }
+}
+
+// Quad4 / Hex8 displacement and coordinate cells with the two-point rule: the configurations of sumfac.cuh
+bool LinearTwoPoint(const Ctx& c)
+{
+    const Slot& D = c.slots[c.prm.disp_slot];
+    return (c.dim == 2 && c.nge == 4 && D.nen == 4 && c.ip.nIp == 4) ||
+           (c.dim == 3 && c.nge == 8 && D.nen == 8 && c.ip.nIp == 8);
 }
 
 void BuildGeometryCache(Ctx& c)
@@ -165,17 +181,41 @@ void BuildGeometryCache(Ctx& c)
     c.geoStride = 1 + D.nen * c.dim;
     const size_t total = static_cast<size_t>(c.geoStride) * c.ip.nIp * c.nCells;
     c.dGeo64.alloc(total);
-    c.dGeo32.alloc(total);
+    const bool linear = LinearTwoPoint(c);
+    if (linear)
+        c.dJac.alloc(static_cast<size_t>(1 + c.dim * c.dim) * c.ip.nIp * c.nCells);
+    else
+        c.dJac.free();
     const int64_t items = c.nCells * c.ip.nIp;
     const int blocks = static_cast<int>((items + 127) / 128);
     DispatchCfg(c, [&](auto cfg) {
         using C = decltype(cfg);
         k_geometry<C::dim, C::ng, C::nd, C::nip><<<blocks, 128, 0, c.stream>>>(
                 c.nCells, static_cast<int64_t>(c.dCoords.n), c.dCoords.p, c.dGeoConnT.p, c.dTables.p, c.tabW, c.tabDN[c.geoInterp], c.tabDN[D.interp],
-                c.geoStride, c.dGeo64.p, c.dGeo32.p);
+                c.geoStride, c.dGeo64.p, linear ? c.dJac.p : nullptr, SumFac<C::dim>::gradScale);
     });
     AfterLaunch(c, "k_geometry");
+    c.dGeo32.free(); // FP32 copy: made by EnsureGeo32 where a kernel reads it
     c.haveGeo = true;
+}
+
+// FP32 copy of the geometry cache, made the first time the FP32 element kernel (atomics) runs on this geometry
+__global__ void __launch_bounds__(256) k_geometry32(int64_t n, const double* __restrict__ geo64,
+                                                    float* __restrict__ geo32)
+{
+    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
+         i += static_cast<int64_t>(gridDim.x) * blockDim.x)
+        geo32[i] = static_cast<float>(geo64[i]);
+}
+
+static void EnsureGeo32(Ctx& c)
+{
+    if (c.dGeo32.n == c.dGeo64.n)
+        return;
+    c.dGeo32.alloc(c.dGeo64.n);
+    k_geometry32<<<static_cast<unsigned>(std::max(c.smCount, 1) * 8), 256, 0, c.stream>>>(
+            static_cast<int64_t>(c.dGeo64.n), c.dGeo64.p, c.dGeo32.p);
+    AfterLaunch(c, "k_geometry32");
 }
 
 static CellArgs MakeCellArgs(Ctx& c);
@@ -208,10 +248,35 @@ static CellArgs MakeCellArgs(Ctx& c)
     }
     a.geo64 = c.dGeo64.p;
     a.geo32 = c.dGeo32.p;
+    a.jac = c.dJac.n ? c.dJac.p : nullptr;
+    a.jacSize = static_cast<int64_t>(c.dJac.n);
     a.geoStride = c.geoStride;
     a.kappa = c.dKappa.p;
     a.escale = c.dEScale.n ? c.dEScale.p : nullptr;
     return a;
+}
+
+// engineering strain from the natural gradients G[c][j] = du_c/dxi_j and the inverse Jacobian J[j][d] = dxi_j/dx_d
+template <typename T, int DIM>
+__device__ __forceinline__ void StrainFromNatural(const T (&G)[DIM][DIM], const T (&J)[DIM][DIM], T* e)
+{
+    auto dot = [&](int c, int d, T s) {
+#pragma unroll
+        for (int j = 0; j < DIM; ++j)
+            s += G[c][j] * J[j][d];
+        return s;
+    };
+#pragma unroll
+    for (int c = 0; c < DIM; ++c)
+        e[c] = dot(c, c, T(0));
+    if (DIM == 2)
+        e[2] = dot(0, 1, dot(1, 0, T(0)));
+    else
+    {
+        e[3] = dot(1, 2, dot(2, 1, T(0)));
+        e[4] = dot(0, 2, dot(2, 0, T(0)));
+        e[5] = dot(0, 1, dot(1, 0, T(0)));
+    }
 }
 
 // ---- FP64 internal-force residual --------------------------------------------------------------------------
@@ -399,6 +464,222 @@ void GatherCellVectors(Ctx& c, const Slot& S, int ncomp, int off, int64_t nLocal
     AfterLaunch(c, "k_gather_cell_vectors");
 }
 
+// The same residual for Quad4 / Hex8 cells with the two-point rule, with the fields' gradients and the transposed sums
+// sum-factorised (sumfac.cuh). A warp takes CPB cells (one warp per block, so that nothing but the warp itself waits
+// and a mesh of a few thousand cells still spreads over the SMs):
+//   (1) lane (cell, field): the gradient of one displacement component (or of eeq, with its values) at all points;
+//   (2) lane (cell, point): H = G J^-1, the law, and the stress carried back to natural coordinates, T = w sigma J^-T;
+//   (3) lane (cell, field): the field's entries of the cell vector from T.
+// Bound by the FP64 pipe (2 lanes per clock and SM, 87 % busy): 220 FP64 instructions per Hex8 gradient-damage point, half
+// of them the law, against 352 with the gradients of all nodes read from the cache (k_residual), and 80 bytes of geometry
+// per point instead of 200. 64^3: 1345 -> 881 us with the gathers; 17^3: 56 -> 31 us; 200^2 Quad4 elastic: 26 -> 19 us.
+// (Two warps per 8 cells left one of them idle in phases 1 and 3: 922 us at 64^3.)
+template <int DIM, int KIND>
+struct ResShape
+{
+    static constexpr bool GD = KIND == NUTO_GPU_GRADIENT_DAMAGE;
+    static constexpr int nip = SumFac<DIM>::nd;
+    static constexpr int nf = DIM + (GD ? 1 : 0);
+    static constexpr int threads = 32;
+};
+
+
+template <int DIM, int KIND, int CPB>
+__global__ void __launch_bounds__(32, 16) k_residual_sf(CellArgs a, LawParams L, const double* __restrict__ u,
+                                                    double* __restrict__ fcell)
+{
+    using R = ResShape<DIM, KIND>;
+    using S = SumFac<DIM>;
+    constexpr bool GD = R::GD;
+    constexpr int VD = DIM == 2 ? 3 : 6;
+    constexpr int ND = S::nd, NIP = S::nd, NF = R::nf;
+    __shared__ double sG[NF][S::ng][CPB];
+    __shared__ double sV[GD ? NIP : 1][CPB];
+    __shared__ double sT[NF][NIP][DIM][CPB];
+    __shared__ double sTV[GD ? NIP : 1][CPB];
+    const int64_t n = a.nCells;
+    for (int64_t cell0 = static_cast<int64_t>(blockIdx.x) * CPB; cell0 < n;
+         cell0 += static_cast<int64_t>(gridDim.x) * CPB)
+    {
+        for (int it = threadIdx.x; it < CPB * NF; it += R::threads)
+        {
+            const int cl = it % CPB, fl = it / CPB;
+            const int64_t e = cell0 + cl;
+            if (e >= n)
+                continue;
+            // one code path for all fields (a warp holds all of them): the displacements' values are not used
+            const bool eq = GD && fl == DIM;
+            const int32_t* conn = eq ? a.connE : a.connD;
+            const int64_t* gdof = eq ? a.gdofE : a.gdofD;
+            const int comp = eq ? 0 : fl;
+            double v[ND], g[S::ng], val[NIP];
+#pragma unroll
+            for (int nd = 0; nd < ND; ++nd)
+            {
+                const int64_t gd = gdof[NG_IDX(conn[static_cast<int64_t>(nd) * n + e], eq ? a.nNodesE : a.nNodesD, 2)];
+                v[nd] = u[NG_IDX(gd + comp, a.nDofs, 3)];
+            }
+            SfForward<double, DIM, GD>(v, g, val);
+            if (eq)
+            {
+#pragma unroll
+                for (int q = 0; q < NIP; ++q)
+                    sV[q][cl] = val[q];
+            }
+#pragma unroll
+            for (int k = 0; k < S::ng; ++k)
+                sG[fl][k][cl] = g[k];
+        }
+        __syncwarp();
+#pragma unroll 1
+        for (int it = threadIdx.x; it < CPB * NIP; it += R::threads)
+        {
+            const int cl = it % CPB, q = it / CPB;
+            const int64_t e = cell0 + cl;
+            if (e < n)
+            {
+                const int64_t jb = static_cast<int64_t>(q) * (1 + DIM * DIM) * n + e;
+                const double* Jq = a.jac + NG_IDX(jb, a.jacSize, 6);
+                const double wdj = Jq[0];
+                // per-cell Young's modulus factor: scales the stress, i.e. the displacement rows
+                const double wdjE = a.escale ? wdj * a.escale[e] : wdj;
+                double J[DIM][DIM];
+#pragma unroll
+                for (int j = 0; j < DIM; ++j)
+#pragma unroll
+                    for (int d = 0; d < DIM; ++d)
+                        J[j][d] = Jq[(1 + j * DIM + d) * n];
+                const double kh = KIND == NUTO_GPU_MB_LINEAR_ELASTIC ? 0. : a.kappa[NG_IDX(e * NIP + q, n * NIP, 7)];
+                int gi[DIM];
+#pragma unroll
+                for (int j = 0; j < DIM; ++j)
+                    gi[j] = SfGradIndex<DIM>(j, q);
+                double G[DIM][DIM], eps[VD], sig[VD];
+#pragma unroll
+                for (int c = 0; c < DIM; ++c)
+#pragma unroll
+                    for (int j = 0; j < DIM; ++j)
+                        G[c][j] = sG[c][gi[j]][cl];
+                StrainFromNatural<double, DIM>(G, J, eps);
+                if (KIND == NUTO_GPU_MB_LINEAR_ELASTIC)
+                {
+                    ElasticStress<double, DIM>(L, eps, sig);
+#pragma unroll
+                    for (int v = 0; v < VD; ++v)
+                        sig[v] *= wdjE;
+                }
+                else if (KIND == NUTO_GPU_MB_LOCAL_DAMAGE)
+                {
+                    const double kap = fmax(MisesNorm<double, DIM>(L, eps), kh);
+                    LedStressWeighted<double, DIM>(L, eps, DamageIntegrity<double>(L, kap), wdjE, sig);
+                }
+                else
+                {
+                    const double eeq = S::valScale * sV[q][cl];
+                    const double kap = fmax(kh, eeq); // GradientDamage::Kappa (GradientDamage.h:127-130)
+                    const double phi = DamageIntegrity<double>(L, kap);
+                    LedStressWeighted<double, DIM>(L, eps, phi, wdjE, sig);
+                    double cg = L.c * wdj;
+                    if (L.interaction != NUTO_GPU_INTERACTION_CONSTANT)
+                        cg *= InteractionFactor<double>(L, 1. - phi);
+                    sTV[q][cl] = (eeq - MisesNorm<double, DIM>(L, eps)) * (S::valScale * wdj);
+                    double g[DIM], ge[DIM];
+#pragma unroll
+                    for (int j = 0; j < DIM; ++j)
+                        g[j] = cg * sG[DIM][gi[j]][cl];
+#pragma unroll
+                    for (int d = 0; d < DIM; ++d)
+                    {
+                        double s = g[0] * J[0][d];
+#pragma unroll
+                        for (int j = 1; j < DIM; ++j)
+                            s += g[j] * J[j][d];
+                        ge[d] = s;
+                    }
+#pragma unroll
+                    for (int j = 0; j < DIM; ++j)
+                    {
+                        double s = ge[0] * J[j][0];
+#pragma unroll
+                        for (int d = 1; d < DIM; ++d)
+                            s += ge[d] * J[j][d];
+                        sT[DIM][q][j][cl] = s;
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < DIM; ++j)
+                {
+                    double b[DIM];
+                    BtS<double, DIM>(J[j], sig, b); // row j of J^-1 in the place of a node gradient
+#pragma unroll
+                    for (int c = 0; c < DIM; ++c)
+                        sT[c][q][j][cl] = b[c];
+                }
+            }
+        }
+        __syncwarp();
+        const int64_t nLocal = static_cast<int64_t>(ND) * NF;
+        (void)nLocal; // buffer extent for checked builds
+        for (int it = threadIdx.x; it < CPB * NF; it += R::threads)
+        {
+            const int cl = it % CPB, fl = it / CPB;
+            const int64_t e = cell0 + cl;
+            if (e >= n)
+                continue;
+            double out[ND];
+            const bool eq = GD && fl == DIM;
+            SfTranspose<double, DIM, GD>([&](int j, int q) { return sT[fl][q][j][cl]; },
+                                         [&](int q) { return eq ? sTV[GD ? q : 0][cl] : 0.; }, out);
+            // entry of node 0: the displacement entries are node-major, the eeq entries follow them
+            const int64_t first = eq ? static_cast<int64_t>(ND) * DIM : fl, step = eq ? 1 : DIM;
+#pragma unroll
+            for (int nd = 0; nd < ND; ++nd)
+                fcell[NG_IDX((first + nd * step) * n + e, nLocal * n, 8)] = out[nd];
+        }
+        __syncwarp(); // the next pass overwrites the shared arrays
+    }
+}
+
+// Both gathers of a residual in one launch: k_gather_cell_vectors' sums (ascending cell order) for the displacement
+// nodes and, in gradient damage, the eeq nodes.
+struct GatherArgs
+{
+    int64_t items[kMaxSlots]; // nodes x components of the slot (0: unused)
+    int ncomp[kMaxSlots], off[kMaxSlots];
+    const int64_t* cellPtr[kMaxSlots];
+    const int32_t* cellIdx[kMaxSlots];
+    const uint8_t* cellLoc[kMaxSlots];
+    const int64_t* gdof[kMaxSlots];
+    int64_t nCells, nLocal, nDofs;
+};
+
+__global__ void __launch_bounds__(256) k_gather_residual(GatherArgs g, const double* __restrict__ fcell,
+                                                         double* __restrict__ f)
+{
+    PdlWait();
+    int64_t it = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+    const bool second = it >= g.items[0];
+    it -= second ? g.items[0] : 0;
+    if (it >= (second ? g.items[1] : g.items[0]))
+        return;
+    const int nc = second ? g.ncomp[1] : g.ncomp[0];
+    const int off = second ? g.off[1] : g.off[0];
+    const int64_t* cellPtr = second ? g.cellPtr[1] : g.cellPtr[0];
+    const int32_t* cellIdx = second ? g.cellIdx[1] : g.cellIdx[0];
+    const uint8_t* cellLoc = second ? g.cellLoc[1] : g.cellLoc[0];
+    const int64_t i = it / nc;
+    const int comp = static_cast<int>(it % nc);
+    const int64_t k1 = cellPtr[i + 1];
+    double sum = 0.;
+    for (int64_t k = cellPtr[i]; k < k1; ++k)
+    {
+        const int64_t e = cellIdx[k];
+        const int64_t entry = off + static_cast<int64_t>(cellLoc[k]) * nc + comp;
+        sum += fcell[NG_IDX(entry * g.nCells + e, g.nLocal * g.nCells, 9)];
+    }
+    f[NG_IDX((second ? g.gdof[1] : g.gdof[0])[i] + comp, g.nDofs, 9)] = sum;
+}
+
 void LaunchResidual(Ctx& c, const double* u, double* f, int blocksPerSm)
 {
     const Slot& D = c.slots[c.prm.disp_slot];
@@ -410,20 +691,75 @@ void LaunchResidual(Ctx& c, const double* u, double* f, int blocksPerSm)
     if (c.slots.size() > static_cast<size_t>(gd ? 2 : 1))
         NG_CUDA(cudaMemsetAsync(f, 0, c.nDofs * sizeof(double), c.stream));
     CellArgs a = MakeCellArgs(c);
-    DispatchCfg(c, [&](auto cfg) {
-        using C = decltype(cfg);
-        constexpr int CPB = MaxI<1, 128 / MaxI<C::nip, C::nd>::v>::v;
-        int64_t blocks = (c.nCells + CPB - 1) / CPB;
-        if (blocksPerSm > 0)
-            blocks = std::min<int64_t>(blocks, static_cast<int64_t>(blocksPerSm) * std::max(c.smCount, 1));
-        k_residual<C::dim, C::nd, C::nip, C::kind><<<static_cast<unsigned>(blocks), 128, 0, c.stream>>>(
-                a, c.law, u, c.dCellVec.p);
-    });
-    AfterLaunch(c, "k_residual");
-    GatherCellVectors(c, D, c.dim, 0, nLocal, f, false);
-    if (gd)
-        GatherCellVectors(c, c.slots[c.prm.eeq_slot], 1, D.nen * c.dim, nLocal, f, false);
-    c.stats.kernel_launches += gd ? 3 : 2;
+    auto grid = [&](int cpb, int perSm) {
+        const int64_t blocks = (c.nCells + cpb - 1) / cpb;
+        return static_cast<unsigned>(
+                perSm > 0 ? std::min<int64_t>(blocks, static_cast<int64_t>(perSm) * std::max(c.smCount, 1)) : blocks);
+    };
+    if (a.jac)
+    {
+        auto run = [&](auto dim, auto kind) {
+            constexpr int DIM = decltype(dim)::value, KIND = decltype(kind)::value;
+            using R = ResShape<DIM, KIND>;
+            // cells per warp: 8 (2D: 16) fill the lanes of every phase; 4 (2D: 8) make a warp's chain of instructions
+            // 1.6 times shorter and are taken while each of the 4 schedulers of an SM then has at most one warp
+            constexpr int BIG = DIM == 3 ? 8 : 16, SMALL = BIG / 2;
+            const bool small = c.nCells <= static_cast<int64_t>(SMALL) * 4 * std::max(c.smCount, 1);
+            // a block of k_residual_sf is a quarter of a block of k_residual
+            if (small)
+                k_residual_sf<DIM, KIND, SMALL><<<grid(SMALL, 4 * blocksPerSm), R::threads, 0, c.stream>>>(
+                        a, c.law, u, c.dCellVec.p);
+            else
+                k_residual_sf<DIM, KIND, BIG><<<grid(BIG, 4 * blocksPerSm), R::threads, 0, c.stream>>>(
+                        a, c.law, u, c.dCellVec.p);
+        };
+        auto kinds = [&](auto dim) {
+            if (gd)
+                run(dim, std::integral_constant<int, NUTO_GPU_GRADIENT_DAMAGE>{});
+            else if (c.prm.kind == NUTO_GPU_MB_LOCAL_DAMAGE)
+                run(dim, std::integral_constant<int, NUTO_GPU_MB_LOCAL_DAMAGE>{});
+            else
+                run(dim, std::integral_constant<int, NUTO_GPU_MB_LINEAR_ELASTIC>{});
+        };
+        if (c.dim == 2)
+            kinds(std::integral_constant<int, 2>{});
+        else
+            kinds(std::integral_constant<int, 3>{});
+        AfterLaunch(c, "k_residual_sf");
+    }
+    else
+    {
+        DispatchCfg(c, [&](auto cfg) {
+            using C = decltype(cfg);
+            if constexpr (C::nd != C::nip) // Quad4 / Hex8 with the two-point rule: above
+            {
+                constexpr int CPB = MaxI<1, 128 / MaxI<C::nip, C::nd>::v>::v;
+                k_residual<C::dim, C::nd, C::nip, C::kind>
+                        <<<grid(CPB, blocksPerSm), 128, 0, c.stream>>>(a, c.law, u, c.dCellVec.p);
+            }
+        });
+        AfterLaunch(c, "k_residual");
+    }
+    GatherArgs g{};
+    g.nCells = c.nCells;
+    g.nLocal = nLocal;
+    g.nDofs = c.nDofs;
+    for (int s = 0; s < (gd ? 2 : 1); ++s)
+    {
+        const Slot& S = s ? c.slots[c.prm.eeq_slot] : D;
+        g.ncomp[s] = s ? 1 : c.dim;
+        g.off[s] = s ? D.nen * c.dim : 0;
+        g.items[s] = S.nNodes * g.ncomp[s];
+        g.cellPtr[s] = S.dCellPtr.p;
+        g.cellIdx[s] = S.dCellIdx.p;
+        g.cellLoc[s] = S.dCellLoc.p;
+        g.gdof[s] = S.dGdof.p;
+    }
+    const int64_t items = g.items[0] + g.items[1];
+    NG_CUDA(LaunchPdl(k_gather_residual, dim3(static_cast<unsigned>((items + 255) / 256)), dim3(256), 0, c.stream, g,
+                      static_cast<const double*>(c.dCellVec.p), f));
+    AfterLaunch(c, "k_gather_residual");
+    c.stats.kernel_launches += 2;
 }
 
 // ---- tangent: FP32 or FP64 values scattered into CSR ---------------------------------------------------------
@@ -1344,6 +1680,8 @@ static void LaunchTangentT(Ctx& c, const double* u, T* vals)
         return;
     }
     NG_CUDA(cudaMemsetAsync(vals, 0, c.nnz * sizeof(T), c.stream));
+    if (sizeof(T) == 4)
+        EnsureGeo32(c);
     CellArgs a = MakeCellArgs(c);
     ScatterArgs s = MakeScatterArgs(c);
     const int ns = static_cast<int>(c.slots.size());

@@ -236,9 +236,11 @@ struct LawParams
     double C11, C12, C33;
     // LinearElasticDamage
     double m3K, m2G, d2; // d2: mD2 factor of the normal components (1 or 1 + nu/(nu-1))
+    double lamD, muD;    // undamaged Lame parameters of LinearElasticDamage: (m3K - m2G) d2 / 3, m2G / 2
     // damage law, strain norm, nonlocal interaction
     double kappa0, beta, alpha;
     double K1, K2, k;
+    double K2o6, K2o4; // K2 / 6, K2 / 4
     double c, R, eta;
 };
 
@@ -372,7 +374,10 @@ struct Ctx
     // geometry caches per integration point: planar [(q * S + k)][cell], S = 1 + nen_d * dim
     bool haveGeo = false;
     DBuf<double> dGeo64;
-    DBuf<float> dGeo32;
+    DBuf<float> dGeo32; // on first use of the FP32 element kernel
+    // w det J and the inverse Jacobian (times SumFac::gradScale) per point, planar [(q * (1 + dim^2) + k)][cell]
+    // (Quad4 / Hex8 cells with the two-point rule)
+    DBuf<double> dJac;
     int geoStride = 0;
 
     // row-gather tangent: integration-point records and the displacement-node -> eeq-node map
@@ -405,11 +410,12 @@ struct Ctx
     // residual: the cell vectors of the last residual (planar [local entry][cell]) gathered per DOF
     DBuf<double> dCellVec;
     // nuto_gpu_build_system: the residual on a second stream beside the tangent, as a persistent grid of
-    // sysResBlocks blocks per SM (the FP64 pipe needs few warps), the rest of every SM left to the tangent's
-    // blocks; the first call of a context runs both in sequence (lazy set-up, autotuning)
+    // 4 sysResBlocks warps per SM (the FP64 pipe needs few warps), the rest of every SM left to the tangent's
+    // blocks; the first call of a context runs both in sequence (lazy set-up, autotuning). 64^3 system pass with
+    // 1 / 2 / 3 / 4: 1835 / 1668 / 1681 / 1689 us
     cudaStream_t sideStream = nullptr;
     cudaEvent_t evFork = nullptr, evJoin = nullptr;
-    int sysResBlocks = 6;
+    int sysResBlocks = 2;
     // nuto_gpu_build_system_host: device copies of the caller's host state, values and vector
     DBuf<double> dHostIoU, dHostIoF;
     DBuf<unsigned char> dHostIoVals;
@@ -458,6 +464,7 @@ struct Ctx
 // ---- host helpers implemented in the .cu files ----
 void BuildTables(Ctx& c);
 void BuildGeometryCache(Ctx& c);
+bool LinearTwoPoint(const Ctx& c);
 void LaunchResidual(Ctx& c, const double* u, double* f, int blocksPerSm = 0); // 0: one block per CPB cells
 void LaunchTangent(Ctx& c, const double* u, int precision, void* values);
 void LaunchTangentExact(Ctx& c, const double* u, double* vals);
@@ -508,6 +515,8 @@ struct CellArgs
     const double* tabN_E;
     const double* geo64;
     const float* geo32;
+    const double* jac; // planar [(q * (1 + dim^2) + k)][cell] or nullptr
+    int64_t jacSize;
     int geoStride;
     double* kappa;
     const double* escale; // per-cell Young's modulus factor (nullptr: 1)
@@ -600,6 +609,32 @@ __host__ __device__ inline void LedStress(const LawParams& p, const T* e, T omeg
         const T dev = normal ? e[i] - eV : e[i];
         s[i] = (normal ? sV : T(0)) + g * (normal ? dev : T(0.5) * dev);
     }
+}
+
+// The same times a weight, s = w * sigma, in the form (1 - omega) w (2 mu eps + lambda tr eps) where the volumetric part is
+// damaged at every point (FULL); phi = 1 - omega. About half the FP64 operations of LedStress and the scaling apart.
+template <typename T, int DIM>
+__device__ __forceinline__ void LedStressWeighted(const LawParams& p, const T* e, T phi, T w, T* s)
+{
+    constexpr int VD = DIM == 2 ? 3 : 6;
+    if (p.damageApp == NUTO_GPU_DAMAGE_UNILATERAL)
+    {
+        LedStress<T, DIM>(p, e, T(1) - phi, s);
+#pragma unroll
+        for (int i = 0; i < VD; ++i)
+            s[i] *= w;
+        return;
+    }
+    T tr = e[0] + e[1];
+    if (DIM == 3)
+        tr += e[2];
+    const T f = phi * w, fm = f * T(p.muD), t = T(p.lamD) * tr;
+#pragma unroll
+    for (int i = 0; i < DIM; ++i)
+        s[i] = f * (T(p.m2G) * e[i] + t);
+#pragma unroll
+    for (int i = DIM; i < VD; ++i)
+        s[i] = fm * e[i];
 }
 
 // LinearElasticDamage::DstressDomega (LinearElasticDamage.h:79-87)
@@ -730,6 +765,32 @@ __host__ __device__ inline void MisesDerivative(const LawParams& p, const T* s, 
     d[0] = dI1 * K1 + inv2A * (T(2) * dI1 * K1 * K1 * I1 + K2 * dxx);
     d[1] = dI1 * K1 + inv2A * (T(2) * dI1 * K1 * K1 * I1 + K2 * dyy);
     d[2] = inv2A * (K2 * T(0.5) * s[2]);
+}
+
+// ModifiedMisesStrainNorm::Value with the constants of J2 multiplied out (3D; MisesValue otherwise)
+template <typename T, int DIM>
+__device__ __forceinline__ T MisesNorm(const LawParams& p, const T* e)
+{
+    if constexpr (DIM == 2)
+        return MisesValue<T, DIM>(p, e);
+    else
+    {
+        const T a = e[0] - e[1], b = e[1] - e[2], c = e[2] - e[0];
+        const T k = T(p.K1) * (e[0] + e[1] + e[2]);
+        const T s = a * a + b * b + c * c;
+        const T g = e[3] * e[3] + e[4] * e[4] + e[5] * e[5];
+        return k + sqrt(k * k + (T(p.K2o6) * s + T(p.K2o4) * g));
+    }
+}
+
+// 1 - omega of DamageLawExponential
+template <typename T>
+__device__ __forceinline__ T DamageIntegrity(const LawParams& p, T kappa)
+{
+    const T k0 = T(p.kappa0);
+    if (kappa < k0)
+        return T(1);
+    return k0 / kappa * (T(1) - T(p.alpha) + T(p.alpha) * exp(T(p.beta) * (k0 - kappa)));
 }
 
 // DamageLawExponential (DamageLawExponential.h:40-52)
