@@ -451,6 +451,7 @@ static void BuildPattern(Ctx& c)
         M.hNbrIdx = std::move(nbr[p].idx);
     }
     FreeAmg(c);
+    c.rowPlanKey = 0;
     c.havePattern = true;
 }
 
@@ -1133,10 +1134,7 @@ int nuto_gpu_build_matrix(nuto_gpu_ctx* ctx, const double* u, int precision, voi
         RequireReady(*ctx);
         NG_CHECK(precision == NUTO_GPU_FP32 || precision == NUTO_GPU_FP64 || precision == NUTO_GPU_FP64X,
                  NUTO_GPU_EINVAL, "precision 32, 64 or 65");
-        if (precision == NUTO_GPU_FP64X)
-            LaunchTangentExact(*ctx, u, static_cast<double*>(values));
-        else
-            LaunchTangent(*ctx, u, precision, values);
+        LaunchTangent(*ctx, u, precision, values);
         return NUTO_GPU_OK;
     });
 }

@@ -28,7 +28,7 @@
 // strain at a point is formed in FP32 with an error bound, and where the bound does not separate it from the
 // history kappa or from kappa0 it is recomputed in FP64 exactly as the FP64 kernels form it. The loading/unloading
 // and damage-threshold branches therefore agree with the FP64 residual at every point; everything else is FP32.
-#include "internal.cuh"
+#include "rows.cuh"
 
 #include <algorithm>
 #include <type_traits>
@@ -44,7 +44,6 @@ constexpr int kFusedRowCap = 128; // values per row buffer: 32 neighbour nodes o
 struct FusedArgs
 {
     int64_t nNodes, nCells, nnz, nRows, nDofs, nNodesD, nNodesE;
-    int64_t nodeBase; // the element-matrix row gathers take nodes nodeBase .. nNodes - 1
     const int32_t* connD; // planar [n][cell]
     const int32_t* connE;
     const int64_t* gdofD; // per node: combined index of component 0
@@ -1123,119 +1122,6 @@ __global__ void __launch_bounds__(W * 32) k_cell_matrices(int64_t nCells, const 
     }
 }
 
-template <int DIM, int ND, int NIP, int KIND, int W>
-__global__ void __launch_bounds__(W * 32) k_rows_from_cells(FusedArgs A, const float* __restrict__ em,
-                                                            float* __restrict__ vals)
-{
-    using CS = CellSlab<DIM, ND, KIND>;
-    constexpr bool GD = CS::GD;
-    constexpr int NR = CS::nr, NC = CS::nc, SL = CS::size;
-    constexpr int PER = (SL + 31) / 32; // slab values per lane
-    __shared__ float sRowAll[W][NR * kFusedRowCap];
-    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t a = A.nodeBase + static_cast<int64_t>(blockIdx.x) * W + wid;
-    if (a >= A.nNodes)
-        return; // the whole warp leaves; only warp-level synchronisation follows
-    float* sRow = sRowAll[wid];
-    int64_t rs[NR];
-    int len[NR];
-    const int64_t g0 = A.gdofD[a];
-#pragma unroll
-    for (int k = 0; k < DIM; ++k)
-    {
-        rs[k] = A.rowPtr[NG_IDX(g0 + k, A.nRows, 72)];
-        len[k] = static_cast<int>(A.rowPtr[g0 + k + 1] - rs[k]);
-    }
-    int32_t ae = 0;
-    if (GD)
-    {
-        ae = A.eOf[a];
-        const int64_t ge = A.gdofE[ae];
-        rs[DIM] = A.rowPtr[NG_IDX(ge, A.nRows, 72)];
-        len[DIM] = static_cast<int>(A.rowPtr[ge + 1] - rs[DIM]);
-    }
-    const int32_t bUU = A.blk[0][a];
-    const int32_t bUE = GD ? A.blk[1][a] : 0;
-    const int32_t bEU = GD ? A.blk[2][ae] : 0;
-    const int32_t bEE = GD ? A.blk[3][ae] : 0;
-#pragma unroll
-    for (int k = 0; k < NR; ++k)
-        for (int i = lane; i < kFusedRowCap; i += 32)
-            sRow[k * kFusedRowCap + i] = 0.f;
-    const int64_t n = A.nCells;
-    const int64_t k0 = A.cellPtr[a], k1 = A.cellPtr[a + 1];
-    // the slab values of the next cell are loaded while the current one is added
-    float nxt[PER];
-    auto load = [&](int64_t kc, float (&v)[PER]) {
-        const int64_t e = A.cellIdx[kc];
-        const int ia = A.cellLoc[kc];
-        const float* slab = em + (NG_IDX(e, n, 73) * ND + ia) * SL;
-#pragma unroll
-        for (int m = 0; m < PER; ++m)
-        {
-            const int i = lane + 32 * m;
-            v[m] = i < SL ? slab[i] : 0.f;
-        }
-    };
-    if (k0 < k1)
-        load(k0, nxt);
-    for (int64_t kc = k0; kc < k1; ++kc)
-    {
-        float cur[PER];
-#pragma unroll
-        for (int m = 0; m < PER; ++m)
-            cur[m] = nxt[m];
-        const int64_t e = A.cellIdx[kc];
-        const int ia = A.cellLoc[kc];
-        // ranks of b in a's neighbour lists: lane b loads them, the others read them by shuffles
-        int r0 = 0, r1 = 0, r2 = 0, r3 = 0;
-        if (lane < ND)
-        {
-            const int64_t ridx = static_cast<int64_t>(ia * ND + lane) * n + e;
-            r0 = A.rank[0][ridx];
-            if (GD)
-            {
-                r1 = A.rank[1][ridx];
-                r2 = A.rank[2][ridx];
-                r3 = A.rank[3][ridx];
-            }
-        }
-        if (kc + 1 < k1)
-            load(kc + 1, nxt);
-#pragma unroll
-        for (int m = 0; m < PER; ++m)
-        {
-            const int i = lane + 32 * m;
-            const int ic = i < SL ? i : 0;
-            const int row = ic / NC, col = ic % NC;
-            const bool ucol = col < ND * DIM;
-            const int b = ucol ? col / DIM : col - ND * DIM;
-            const int l = ucol ? col % DIM : 0;
-            const int rk0 = __shfl_sync(0xffffffffu, r0, b);
-            int pos;
-            if (GD)
-            {
-                const int rk1 = __shfl_sync(0xffffffffu, r1, b);
-                const int rk2 = __shfl_sync(0xffffffffu, r2, b);
-                const int rk3 = __shfl_sync(0xffffffffu, r3, b);
-                if (row < DIM)
-                    pos = ucol ? bUU + DIM * rk0 + l : bUE + rk1;
-                else
-                    pos = ucol ? bEU + DIM * rk2 + l : bEE + rk3;
-            }
-            else
-                pos = bUU + DIM * rk0 + l;
-            if (i < SL)
-                sRow[row * kFusedRowCap + NG_IDX(pos, kFusedRowCap, 74)] += cur[m];
-        }
-        __syncwarp();
-    }
-#pragma unroll
-    for (int k = 0; k < NR; ++k)
-        for (int i = lane; i < len[k]; i += 32)
-            vals[NG_IDX(rs[k] + i, A.nnz, 75)] = sRow[k * kFusedRowCap + i];
-}
-
 // The element matrices with the law evaluated in the same kernel (no records in global memory): a warp takes
 // CPW = 32 / NIP cells; (0) lane (cell, node) stages the node data, (A) lane (cell, point) evaluates PointData into
 // the record layout in shared memory (the values k_point_records writes), (B) the cells one after the other as in
@@ -1387,124 +1273,6 @@ __global__ void __launch_bounds__(W * 32) k_cell_matrices_law(FusedArgs A, LawPa
     }
 }
 
-// The ranks of one (cell entry of a node, neighbour b) packed into one word (UU | UE << 8 | EU << 16 | EE << 24), in
-// the order of the nodes' cell lists: the row gather of a node then reads the ranks of its cells with contiguous
-// loads instead of byte loads from the planar rank tables. Built once per mesh.
-template <int ND>
-__global__ void k_pack_ranks(FusedArgs A, int64_t nEntries, uint32_t* __restrict__ packed)
-{
-    const int64_t it = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (it >= nEntries * ND)
-        return;
-    const int64_t kc = it / ND;
-    const int b = static_cast<int>(it % ND);
-    const int64_t e = A.cellIdx[kc];
-    const int ia = A.cellLoc[kc];
-    const int64_t ridx = static_cast<int64_t>(ia * ND + b) * A.nCells + e;
-    packed[it] = static_cast<uint32_t>(A.rank[0][ridx]) | static_cast<uint32_t>(A.rank[1][ridx]) << 8 |
-                 static_cast<uint32_t>(A.rank[2][ridx]) << 16 | static_cast<uint32_t>(A.rank[3][ridx]) << 24;
-}
-
-// Row gather of the element-matrix form for slabs of exactly 32 columns (Hex8 gradient damage: 24 displacement
-// columns, 8 eeq columns): lane l owns column l of every slab row, so its neighbour b = l / 3 (or l - 24), and the
-// positions in the displacement rows and in the eeq row are fixed per cell. The slab values and packed ranks of a
-// batch of CB cells are loaded before any is added (all loads in flight at once); cells are added in ascending
-// order.
-template <int DIM, int ND, int NIP, int KIND, int W, int CB>
-__global__ void __launch_bounds__(W * 32) k_rows_from_cells32(FusedArgs A, const uint32_t* __restrict__ packed,
-                                                              const float* __restrict__ em, float* __restrict__ vals)
-{
-    using CS = CellSlab<DIM, ND, KIND>;
-    constexpr bool GD = CS::GD;
-    constexpr int NR = CS::nr, SL = CS::size;
-    static_assert(CS::nc == 32 && ND == 8, "one slab column per lane, 8 nodes per cell");
-    static_assert(CB == 2 || CB == 4 || CB == 8, "cells per batch");
-    __shared__ float sRowAll[W][NR * kFusedRowCap];
-    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t a = A.nodeBase + static_cast<int64_t>(blockIdx.x) * W + wid;
-    if (a >= A.nNodes)
-        return; // the whole warp leaves; only warp-level synchronisation follows
-    float* sRow = sRowAll[wid];
-    int64_t rs[NR];
-    int len[NR];
-    const int64_t g0 = A.gdofD[a];
-#pragma unroll
-    for (int k = 0; k < DIM; ++k)
-    {
-        rs[k] = A.rowPtr[NG_IDX(g0 + k, A.nRows, 76)];
-        len[k] = static_cast<int>(A.rowPtr[g0 + k + 1] - rs[k]);
-    }
-    int32_t ae = 0;
-    if (GD)
-    {
-        ae = A.eOf[a];
-        const int64_t ge = A.gdofE[ae];
-        rs[DIM] = A.rowPtr[NG_IDX(ge, A.nRows, 76)];
-        len[DIM] = static_cast<int>(A.rowPtr[ge + 1] - rs[DIM]);
-    }
-    const int32_t bUU = A.blk[0][a];
-    const int32_t bUE = GD ? A.blk[1][a] : 0;
-    const int32_t bEU = GD ? A.blk[2][ae] : 0;
-    const int32_t bEE = GD ? A.blk[3][ae] : 0;
-#pragma unroll
-    for (int k = 0; k < NR; ++k)
-        for (int i = lane; i < kFusedRowCap; i += 32)
-            sRow[k * kFusedRowCap + i] = 0.f;
-    const bool ucol = lane < ND * DIM;
-    const int myB = ucol ? lane / DIM : lane - ND * DIM;
-    const int myL = ucol ? lane % DIM : 0;
-    const int64_t n = A.nCells; // extent of the checked indices
-    (void)n;
-    const int64_t k0 = A.cellPtr[a], k1 = A.cellPtr[a + 1];
-    for (int64_t kb = k0; kb < k1; kb += CB)
-    {
-        const int nc = static_cast<int>(k1 - kb < CB ? k1 - kb : CB);
-        // packed ranks of the batch: lane l holds (cell slot l / 8, b = l % 8) and (cell slot 4 + l / 8, b)
-        uint32_t pk0 = 0, pk1 = 0;
-        if (lane / ND < nc)
-            pk0 = packed[NG_IDX((kb + lane / ND) * ND + lane % ND, n * ND * ND, 77)];
-        if (CB == 8 && 4 + lane / ND < nc)
-            pk1 = packed[NG_IDX((kb + 4 + lane / ND) * ND + lane % ND, n * ND * ND, 77)];
-        float v[CB][NR];
-#pragma unroll
-        for (int c = 0; c < CB; ++c)
-        {
-            if (c < nc)
-            {
-                const int64_t kc = kb + c;
-                const float* slab = em + (NG_IDX(A.cellIdx[kc], n, 78) * ND + A.cellLoc[kc]) * SL;
-#pragma unroll
-                for (int r = 0; r < NR; ++r)
-                    v[c][r] = slab[r * 32 + lane];
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < CB; ++c)
-        {
-            // all lanes take part in the shuffle; cells beyond the batch add nothing
-            const uint32_t w = __shfl_sync(0xffffffffu, c < 4 ? pk0 : pk1, (c & 3) * ND + myB);
-            if (c < nc)
-            {
-                const int r0 = w & 0xff, r1 = (w >> 8) & 0xff, r2 = (w >> 16) & 0xff, r3 = w >> 24;
-                const int posU = ucol ? bUU + DIM * r0 + myL : bUE + r1;
-#pragma unroll
-                for (int k = 0; k < DIM; ++k)
-                    sRow[k * kFusedRowCap + NG_IDX(posU, kFusedRowCap, 79)] += v[c][k];
-                if (GD)
-                {
-                    const int posE = ucol ? bEU + DIM * r2 + myL : bEE + r3;
-                    sRow[DIM * kFusedRowCap + NG_IDX(posE, kFusedRowCap, 79)] += v[c][DIM];
-                }
-            }
-            __syncwarp();
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < NR; ++k)
-        for (int i = lane; i < len[k]; i += 32)
-            vals[NG_IDX(rs[k] + i, A.nnz, 75)] = sRow[k * kFusedRowCap + i];
-}
-
 } // namespace
 
 // FP32 coordinates of every cell's nodes relative to its first node (planar [(n * dim + d)][cell]), formed in FP64
@@ -1624,8 +1392,10 @@ void LaunchTangentFused(Ctx& c, const double* u, float* vals)
                 {
                     using CS = CellSlab<DIM, ND, KIND>;
                     const size_t emFloats = static_cast<size_t>(c.nCells) * ND * CS::size;
-                    if (c.dElemMats.n < emFloats)
-                        c.dElemMats.alloc(emFloats);
+                    if (c.dElemMats.n < emFloats * sizeof(float))
+                        c.dElemMats.alloc(emFloats * sizeof(float));
+                    float* em = reinterpret_cast<float*>(c.dElemMats.p);
+                    const RowPlanArgs plan = EnsureRowPlan(c);
                     if (c.cellsLawFused)
                     {
                         using LS = CellLawShape<DIM, ND, NIP, KIND>;
@@ -1636,7 +1406,7 @@ void LaunchTangentFused(Ctx& c, const double* u, float* vals)
                                                          static_cast<int>(smem)));
                         const int64_t cellsPerBlock = static_cast<int64_t>(WW) * LS::cpw;
                         kern<<<static_cast<unsigned>((c.nCells + cellsPerBlock - 1) / cellsPerBlock), WW * 32, smem,
-                               c.stream>>>(A, c.law, u, c.dElemMats.p);
+                               c.stream>>>(A, c.law, u, em);
                         AfterLaunch(c, "k_cell_matrices_law");
                     }
                     else
@@ -1649,52 +1419,19 @@ void LaunchTangentFused(Ctx& c, const double* u, float* vals)
                             NG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                          static_cast<int>(smem)));
                         kern<<<static_cast<unsigned>((c.nCells + WW - 1) / WW), WW * 32, smem, c.stream>>>(
-                                c.nCells, recs, c.dElemMats.p);
+                                c.nCells, recs, em);
                         AfterLaunch(c, "k_cell_matrices");
-                    }
-                    if constexpr (CS::nc == 32 && ND == 8)
-                    {
-                        // packed ranks in cell-list order, once per mesh
-                        const int64_t entries = static_cast<int64_t>(c.nCells) * ND;
-                        if (c.dPackedRanks.n != static_cast<size_t>(entries * ND))
-                        {
-                            c.dPackedRanks.alloc(static_cast<size_t>(entries * ND));
-                            k_pack_ranks<ND><<<static_cast<unsigned>((entries * ND + 255) / 256), 256, 0, c.stream>>>(
-                                    A, entries, c.dPackedRanks.p);
-                            AfterLaunch(c, "k_pack_ranks");
-                        }
                     }
                     // the row gather, in node chunks when a caller hooks into them (each chunk's rows are complete
                     // when its launch is)
                     const int chunks = c.rowChunks > 1 && c.onRowChunk ? c.rowChunks : 1;
                     for (int ch = 0; ch < chunks; ++ch)
                     {
-                        FusedArgs Ac = A;
-                        Ac.nodeBase = A.nNodes * ch / chunks;
-                        Ac.nNodes = A.nNodes * (ch + 1) / chunks;
-                        const int64_t nodes = Ac.nNodes - Ac.nodeBase;
-                        const unsigned rowBlocks = static_cast<unsigned>((nodes + WW - 1) / WW);
-                        if (rowBlocks > 0)
-                        {
-                            if constexpr (CS::nc == 32 && ND == 8)
-                            {
-                                // 4 cells per batch: 64 registers, 32 resident warps per SM (8 cells: 86 registers,
-                                // 1.14x slower; 2 cells: 1.02x slower, measured at 64^3)
-                                k_rows_from_cells32<DIM, ND, NIP, KIND, WW, 4><<<rowBlocks, WW * 32, 0, c.stream>>>(
-                                        Ac, c.dPackedRanks.p, c.dElemMats.p, vals);
-                                AfterLaunch(c, "k_rows_from_cells32");
-                            }
-                            else
-                            {
-                                k_rows_from_cells<DIM, ND, NIP, KIND, WW><<<rowBlocks, WW * 32, 0, c.stream>>>(
-                                        Ac, c.dElemMats.p, vals);
-                                AfterLaunch(c, "k_rows_from_cells");
-                            }
-                            c.stats.kernel_launches += 1;
-                        }
+                        const int64_t a0 = A.nNodes * ch / chunks, a1 = A.nNodes * (ch + 1) / chunks;
+                        LaunchRows<float, DIM, ND, CS::GD, WW>(c, plan, a0, a1, em, vals);
                         if (chunks > 1)
                         {
-                            c.onRowChunk(Ac.nodeBase, Ac.nNodes);
+                            c.onRowChunk(a0, a1);
                             c.rowChunksDone++;
                         }
                     }

@@ -256,6 +256,25 @@ struct IpTables
 struct SolverWork;
 struct Amg;
 
+// Row gather of the element-matrix tangents (rows.cuh), built once per mesh: per displacement node its rows, the offsets
+// of the blocks in them and its cell list; per entry of the cell lists the slab (cell * nodes per cell + local index) and
+// per (entry, b) the ranks of b in the node's four neighbour lists (UU | UE << 8 | EU << 16 | EE << 24).
+struct RowPlan
+{
+    int64_t rowU, rowE, first;                   // first values of the rows, first entry of the cell list
+    int32_t lenU, lenE, bUU, bUE, bEU, bEE, cells, pad0;
+    int64_t pad1; // 64 bytes: one record per two sectors
+};
+static_assert(sizeof(RowPlan) == 64, "one 64-byte record per node");
+struct RowPlanArgs
+{
+    const RowPlan* plan;
+    const uint32_t* slab;
+    const uint32_t* packed;
+    int64_t nodeFirst, nodeLast; // displacement nodes of the launch
+    int64_t nEntries, nnz;
+};
+
 // Boundary cells of one DOF slot (NeumannBc loads): Line2 faces of a 2D mesh or Quad4 faces of a 3D mesh, on the
 // context's coordinate nodes and the slot's DOF nodes.
 struct BoundaryGroup
@@ -400,9 +419,13 @@ struct Ctx
     int tc20Split = 3;
     bool forceTc20Off = false; // NUTO_GPU_TC20=off
     int tc20LawFp64 = 0;       // NUTO_GPU_TC20=fp64law: the law of every point in FP64
-    DBuf<float> dElemMats;
+    // element matrices of the last tangent in its arithmetic (one buffer for FP32 and FP64: every tangent of a context runs
+    // on its stream) and the plan of the row gather
+    DBuf<unsigned char> dElemMats;
     bool cellsLawFused = true; // element-matrix form: the law in the cell kernel (NUTO_GPU_CELLS_RECORDS=1: records)
-    DBuf<uint32_t> dPackedRanks; // element-matrix form: ranks of (cell entry of a node, b), packed, cell-list order
+    DBuf<RowPlan> dRowPlan;
+    DBuf<uint32_t> dRowSlab, dPackedRanks;
+    int rowPlanKey = 0; // slots the plan was built for (0: not built)
     // device status word of kernels with bounded waits (0 = fine, else NUTO_GPU_ETIMEOUT), read after a stream
     // synchronisation; spinLimit bounds every wait loop (iterations)
     DBuf<int> dStatus;
@@ -467,10 +490,15 @@ void BuildGeometryCache(Ctx& c);
 bool LinearTwoPoint(const Ctx& c);
 void LaunchResidual(Ctx& c, const double* u, double* f, int blocksPerSm = 0); // 0: one block per CPB cells
 void LaunchTangent(Ctx& c, const double* u, int precision, void* values);
-void LaunchTangentExact(Ctx& c, const double* u, double* vals);
 void LaunchTangentNoAlloc(Ctx& c, const double* u, float* values);
 bool FusedTangentSupported(Ctx& c);
 void LaunchTangentFused(Ctx& c, const double* u, float* vals);
+// element matrices in FP64 + row gather for the cells of FusedTangentSupported; false: not done (no memory for them)
+bool LaunchTangent64(Ctx& c, const double* u, double* vals);
+RowPlanArgs EnsureRowPlan(Ctx& c);
+// the context's element-matrix buffer with room for `bytes`; nullptr while it would have to grow during a stream capture or
+// beyond the free device memory
+unsigned char* ElemMatsOrNull(Ctx& c, size_t bytes);
 bool Tc20TangentSupported(Ctx& c);
 void LaunchTangentTc20(Ctx& c, const double* u, float* vals);
 int ReadDeviceStatus(Ctx& c); // after a stream synchronisation: the status word (and reset to 0)

@@ -1,0 +1,128 @@
+// CSR rows from element matrices, the second half of every element-matrix tangent (FP32: fused.cu, FP64: tangent64.cu).
+//
+// An element matrix is ND slabs, one per local node a: NR rows (a's displacement components, then its eeq row) x NC columns
+// (the displacement components of b = 0..ND-1, b-major, then the eeq of b = 0..ND-1). A group of lanes owns one displacement
+// node: lane = slab column; the slabs of the node's cells are added in ascending cell order into a shared copy of the node's
+// rows at the ranks of b (a cell's b are distinct nodes: no conflicts) and the rows are stored once. No atomics: the values
+// are bitwise reproducible.
+//
+// Bound by the latency of the chain node -> cells -> slab. It is kept to three dependent loads: the node's plan (rows,
+// block offsets, cell list: one 64-byte record), the slab numbers and packed ranks of a batch of 4 cells, their slabs.
+// FP32 Hex8 gradient damage at 64^3: 380 us with row pointers, cell indices and block offsets read one after the other,
+// about 315 us now; Quad4 gradient damage (16 lanes per node) 70 -> 30 us for 71 k nodes.
+#pragma once
+
+#include "internal.cuh"
+
+namespace nuto_gpu
+{
+
+constexpr int kRowsCap = 128; // values per row: 32 neighbour nodes of [u | eeq] in 3D
+
+template <int DIM, int ND, bool GD>
+struct Slab
+{
+    static constexpr int nr = DIM + (GD ? 1 : 0);      // rows per local node
+    static constexpr int nc = ND * DIM + (GD ? ND : 0); // columns per row
+    static constexpr int size = nr * nc;
+    // lanes per node: the columns rounded up to a power of two
+    static constexpr int lanes = nc > 16 ? 32 : (nc > 8 ? 16 : 8);
+};
+
+template <typename T, int DIM, int ND, bool GD, int W>
+__global__ void __launch_bounds__(W * 32) k_rows_from_slabs(RowPlanArgs P, const T* __restrict__ em, T* __restrict__ vals)
+{
+    using S = Slab<DIM, ND, GD>;
+    constexpr int NR = S::nr, NC = S::nc, LPN = S::lanes, NPW = 32 / LPN, CB = 4;
+    __shared__ T sRowAll[W * NPW][NR * kRowsCap];
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int grp = lane / LPN, col = lane % LPN;
+    PdlWait();
+    const int64_t a = P.nodeFirst + (static_cast<int64_t>(blockIdx.x) * W + wid) * NPW + grp;
+    T* sRow = sRowAll[wid * NPW + grp];
+    RowPlan p{};
+    if (a < P.nodeLast)
+        p = P.plan[a]; // p.cells = 0 beyond the last node: nothing to add or store
+    for (int k = 0; k < DIM; ++k)
+        for (int i = col; i < p.lenU; i += LPN)
+            sRow[k * kRowsCap + i] = T(0);
+    if (GD)
+        for (int i = col; i < p.lenE; i += LPN)
+            sRow[DIM * kRowsCap + i] = T(0);
+    const bool ucol = col < ND * DIM;
+    const int myB = col < NC ? (ucol ? col / DIM : col - ND * DIM) : 0;
+    const int myL = ucol ? col % DIM : 0;
+    int most = p.cells;
+    if (NPW > 1)
+    {
+#pragma unroll
+        for (int o = LPN; o < 32; o <<= 1)
+            most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+    }
+    __syncwarp();
+    for (int kb = 0; kb < most; kb += CB)
+    {
+        uint32_t slab[CB], word[CB];
+#pragma unroll
+        for (int c = 0; c < CB; ++c)
+        {
+            const bool on = kb + c < p.cells;
+            slab[c] = on ? P.slab[NG_IDX(p.first + kb + c, P.nEntries, 77)] : 0u;
+            word[c] = on ? P.packed[NG_IDX((p.first + kb + c) * ND + myB, P.nEntries * ND, 77)] : 0u;
+        }
+        T v[CB][NR];
+#pragma unroll
+        for (int c = 0; c < CB; ++c)
+        {
+            const bool on = kb + c < p.cells && col < NC;
+            const T* src = em + NG_IDX(slab[c], P.nEntries, 78) * static_cast<int64_t>(S::size) + col;
+#pragma unroll
+            for (int r = 0; r < NR; ++r)
+                v[c][r] = on ? src[r * NC] : T(0);
+        }
+#pragma unroll
+        for (int c = 0; c < CB; ++c)
+        {
+            if (kb + c < p.cells && col < NC)
+            {
+                const int r0 = word[c] & 0xff, r1 = (word[c] >> 8) & 0xff, r2 = (word[c] >> 16) & 0xff, r3 = word[c] >> 24;
+                const int posU = ucol ? p.bUU + DIM * r0 + myL : p.bUE + r1;
+#pragma unroll
+                for (int k = 0; k < DIM; ++k)
+                    sRow[k * kRowsCap + NG_IDX(posU, kRowsCap, 79)] += v[c][k];
+                if (GD)
+                {
+                    const int posE = ucol ? p.bEU + DIM * r2 + myL : p.bEE + r3;
+                    sRow[DIM * kRowsCap + NG_IDX(posE, kRowsCap, 79)] += v[c][DIM];
+                }
+            }
+            __syncwarp();
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < DIM; ++k)
+        for (int i = col; i < p.lenU; i += LPN)
+            vals[NG_IDX(p.rowU + static_cast<int64_t>(k) * p.lenU + i, P.nnz, 75)] = sRow[k * kRowsCap + i];
+    if (GD)
+        for (int i = col; i < p.lenE; i += LPN)
+            vals[NG_IDX(p.rowE + i, P.nnz, 75)] = sRow[DIM * kRowsCap + i];
+}
+
+// Launches the gather for the displacement nodes first .. last - 1.
+template <typename T, int DIM, int ND, bool GD, int W>
+inline void LaunchRows(Ctx& c, const RowPlanArgs& all, int64_t first, int64_t last, const T* em, T* vals)
+{
+    RowPlanArgs P = all;
+    P.nodeFirst = first;
+    P.nodeLast = last;
+    constexpr int perBlock = W * (32 / Slab<DIM, ND, GD>::lanes);
+    if (last <= first)
+        return;
+    NG_CUDA(LaunchPdl(k_rows_from_slabs<T, DIM, ND, GD, W>,
+                      dim3(static_cast<unsigned>((last - first + perBlock - 1) / perBlock)), dim3(W * 32), 0, c.stream, P, em,
+                      vals));
+    AfterLaunch(c, "k_rows_from_slabs");
+    c.stats.kernel_launches += 1;
+}
+
+} // namespace nuto_gpu

@@ -235,4 +235,27 @@ __device__ __forceinline__ void SfValuesToNodes(const T* f, T* out)
     }
 }
 
+// engineering strain from the natural gradients G[c][j] = du_c/dxi_j and the inverse Jacobian J[j][d] = dxi_j/dx_d
+template <typename T, int DIM>
+__device__ __forceinline__ void StrainFromNatural(const T (&G)[DIM][DIM], const T (&J)[DIM][DIM], T* e)
+{
+    auto dot = [&](int c, int d, T s) {
+#pragma unroll
+        for (int j = 0; j < DIM; ++j)
+            s += G[c][j] * J[j][d];
+        return s;
+    };
+#pragma unroll
+    for (int c = 0; c < DIM; ++c)
+        e[c] = dot(c, c, T(0));
+    if (DIM == 2)
+        e[2] = dot(0, 1, dot(1, 0, T(0)));
+    else
+    {
+        e[3] = dot(1, 2, dot(2, 1, T(0)));
+        e[4] = dot(0, 2, dot(2, 0, T(0)));
+        e[5] = dot(0, 1, dot(1, 0, T(0)));
+    }
+}
+
 } // namespace nuto_gpu

@@ -1,0 +1,503 @@
+// FP64 tangent of linear cells through element matrices: SimpleAssembler::BuildMatrix
+// (nuto/mechanics/cell/SimpleAssembler.cpp:100-156) of MomentumBalance::Hessian0 with LinearElastic
+// (nuto/mechanics/integrands/MomentumBalance.h:36-46) and GradientDamage::Hessian0
+// (nuto/mechanics/integrands/GradientDamage.h:92-120) for Quad4 and Hex8 cells with the two-point rule. k_cell_matrices64
+// integrates every cell's element matrix once, k_rows_from_slabs (rows.cuh) adds them into the CSR rows: no atomics, the
+// values are bitwise reproducible.
+//
+// Bound by the FP64 pipe (2 lanes per clock and SM); what is saved against an element kernel that integrates each ordered
+// node pair on its own:
+// - the material tangent is lambda m m^T + mu diag(2..2, 1..1) with one ratio rho = lambda / mu for all points (LinearElastic;
+//   LinearElasticDamage with FULL damage application), so a displacement block is rho S + S^T + tr(S) I with the one sum
+//   S = sum over the points of mu w g_a g_b^T, and the block of (b, a) is the transpose: 9 multiply-adds per point and
+//   unordered pair instead of 33 per ordered pair;
+// - the coupling blocks sum_q P_a(q) N_b(q) are transposed interpolations, sum-factorised over the points (24 multiply-adds
+//   per row of 8 blocks instead of 64, sumfac.cuh).
+// 8,800 FP64 instructions per Hex8 gradient-damage cell against about 33,000; 64^3 14.46 -> 4.66 ms, 40^3 3.57 -> 1.18 ms,
+// 17^3 317 -> 118 us, 200^2 Quad4 elastic 109 -> 39 us (k_cell_matrices64 at 90 % of the FP64 pipe; the gather of 8 KB
+// per cell 12 % of the time). The same values serve NUTO_GPU_FP64X, whose double-float products took 2.03 ms at 40^3.
+#include "rows.cuh"
+#include "sumfac.cuh"
+
+#include <algorithm>
+
+namespace nuto_gpu
+{
+
+namespace
+{
+
+template <int DIM, bool GD>
+struct Cell64
+{
+    static constexpr int nd = SumFac<DIM>::nd, nip = nd;
+    static constexpr int vd = DIM == 2 ? 3 : 6;
+    static constexpr int nf = DIM + (GD ? 1 : 0);
+    static constexpr int threads = 64;
+    static constexpr int cpb = threads / nip; // one thread per (cell, point) and per (cell, node)
+    static constexpr int pairs = nd * (nd + 1) / 2;
+    // per point: the node gradients, the same times mu w; gradient damage: the Voigt vectors of the coupling blocks, the
+    // eeq-gradient coupling vector, w and c g w (all but the gradients scaled as their use below wants them)
+    static constexpr int oG = 0, oM = nd * DIM, oS = 2 * nd * DIM, oT = oS + vd, oC = oT + vd, oW = oC + DIM;
+    static constexpr int rec = GD ? oW + 2 : oS;
+    static constexpr int ng = SumFac<DIM>::ng;
+};
+
+// node pair p of the upper triangle (a <= b), row by row
+template <int ND>
+__device__ __forceinline__ void UnorderedPair(int p, int& a, int& b)
+{
+    a = 0;
+    int row = ND;
+    while (p >= row)
+    {
+        p -= row;
+        --row;
+        ++a;
+    }
+    b = a + p;
+}
+
+template <int DIM, bool GD>
+__global__ void __launch_bounds__(Cell64<DIM, GD>::threads) k_cell_matrices64(CellArgs a, LawParams L,
+                                                                              const double* __restrict__ u,
+                                                                              double* __restrict__ em)
+{
+    using C = Cell64<DIM, GD>;
+    using S = SumFac<DIM>;
+    using SL = Slab<DIM, C::nd, GD>;
+    constexpr int ND = C::nd, NIP = C::nip, VD = C::vd, CPB = C::cpb, REC = C::rec;
+    extern __shared__ double sm64[];
+    double* sRec = sm64;                        // [NIP][REC][CPB]
+    double* sGrad = sRec + NIP * REC * CPB;     // [NF][ng][CPB], later the (eeq, eeq) sums [ND][ND][CPB]
+    double* sEn = sGrad + (C::nf * C::ng > ND * ND ? C::nf * C::ng : ND * ND) * CPB; // nodal eeq [ND][CPB]
+    const int64_t n = a.nCells;
+    const int64_t cell0 = static_cast<int64_t>(blockIdx.x) * CPB;
+    auto at = [&](int q, int k, int cl) -> double& { return sRec[(q * REC + k) * CPB + cl]; };
+
+    // natural gradients of the displacement components and of eeq
+    for (int it = threadIdx.x; it < CPB * C::nf; it += C::threads)
+    {
+        const int cl = it % CPB, fl = it / CPB;
+        const int64_t e = cell0 + cl;
+        if (e >= n)
+            continue;
+        const bool eq = GD && fl == DIM;
+        const int32_t* conn = eq ? a.connE : a.connD;
+        const int64_t* gdof = eq ? a.gdofE : a.gdofD;
+        const int comp = eq ? 0 : fl;
+        double v[ND], g[S::ng];
+#pragma unroll
+        for (int nd = 0; nd < ND; ++nd)
+        {
+            const int64_t gd = gdof[NG_IDX(conn[static_cast<int64_t>(nd) * n + e], eq ? a.nNodesE : a.nNodesD, 2)];
+            v[nd] = u[NG_IDX(gd + comp, a.nDofs, 3)];
+            if (eq)
+                sEn[nd * CPB + cl] = v[nd];
+        }
+        SfForward<double, DIM, false>(v, g, nullptr);
+#pragma unroll
+        for (int k = 0; k < S::ng; ++k)
+            sGrad[(fl * S::ng + k) * CPB + cl] = g[k];
+    }
+    __syncthreads();
+
+    // the law and the node gradients of every point
+    {
+        const int cl = threadIdx.x % CPB, q = threadIdx.x / CPB;
+        const int64_t e = cell0 + cl;
+        if (e < n)
+        {
+            const double* Jq = a.jac + NG_IDX(static_cast<int64_t>(q) * (1 + DIM * DIM) * n + e, a.jacSize, 6);
+            const double wdj = Jq[0];
+            // per-cell Young's modulus factor: scales the material tangent and dsigma/domega (displacement rows)
+            const double wdjE = a.escale ? wdj * a.escale[e] : wdj;
+            double muw;
+            if (!GD)
+                muw = L.C33 * wdjE;
+            else
+            {
+                double J[DIM][DIM], G[DIM][DIM], eps[VD];
+#pragma unroll
+                for (int j = 0; j < DIM; ++j)
+#pragma unroll
+                    for (int d = 0; d < DIM; ++d)
+                        J[j][d] = Jq[(1 + j * DIM + d) * n];
+#pragma unroll
+                for (int c = 0; c < DIM; ++c)
+#pragma unroll
+                    for (int j = 0; j < DIM; ++j)
+                        G[c][j] = sGrad[(c * S::ng + SfGradIndex<DIM>(j, q)) * CPB + cl];
+                StrainFromNatural<double, DIM>(G, J, eps);
+                // eeq in the order of the history update and of the other tangents: a converged loading point has
+                // eeq = kappa there, and the loading test must find it loading
+                double eeq = 0.;
+#pragma unroll
+                for (int nd = 0; nd < ND; ++nd)
+                    eeq = fma(a.tabN_D[q * ND + nd], sEn[nd * CPB + cl], eeq);
+                const double kh = a.kappa[NG_IDX(e * NIP + q, n * NIP, 7)];
+                const double kap = kh > eeq ? kh : eeq;
+                const bool loading = eeq >= kh;
+                double phi = 1., dom = 0.;
+                if (!(kap < L.kappa0))
+                {
+                    const double ki = 1. / kap, ex = L.alpha * exp(L.beta * (L.kappa0 - kap));
+                    const double k0i = L.kappa0 * ki;
+                    phi = k0i * ((1. - L.alpha) + ex);
+                    dom = k0i * ((ki + L.beta) * ex + (1. - L.alpha) * ki);
+                }
+                if (!loading)
+                    dom = 0.;
+                double g = 1., dgdw = 0.;
+                if (L.interaction != NUTO_GPU_INTERACTION_CONSTANT)
+                {
+                    g = InteractionFactor<double>(L, 1. - phi);
+                    dgdw = InteractionDerivative<double>(L, 1. - phi);
+                }
+                muw = phi * L.muD * wdjE;
+                // (disp, eeq): B^T (dsigma/domega omega' kappa') N with dsigma/domega = -(lambda tr + 2 mu eps); the
+                // factor of the sum-factorised transpose goes in here
+                double tr = eps[0] + eps[1];
+                if (DIM == 3)
+                    tr += eps[2];
+                const double f = -S::valScale * dom * wdjE, t = L.lamD * tr, fm = f * L.muD;
+#pragma unroll
+                for (int v = 0; v < VD; ++v)
+                    at(q, C::oS + v, cl) = v < DIM ? f * (L.m2G * eps[v] + t) : fm * eps[v];
+                // (eeq, disp): -N^T (deps_eq/deps)^T B
+                double dn[VD];
+                MisesDerivative<double, DIM>(L, eps, dn);
+                const double fn = -S::valScale * wdj;
+#pragma unroll
+                for (int v = 0; v < VD; ++v)
+                    at(q, C::oT + v, cl) = fn * dn[v];
+                // (eeq, eeq): (w N_a + gs_a) N_b + c g w (g_a . g_b), gs_a = c g' omega' kappa' w (grad eeq . g_a)
+                const double sc = S::valScale * L.c * dgdw * dom * wdj;
+                double ge[DIM];
+#pragma unroll
+                for (int d = 0; d < DIM; ++d)
+                    ge[d] = 0.;
+                if (sc != 0.)
+                {
+#pragma unroll
+                    for (int j = 0; j < DIM; ++j)
+#pragma unroll
+                        for (int d = 0; d < DIM; ++d)
+                            ge[d] += sGrad[(DIM * S::ng + SfGradIndex<DIM>(j, q)) * CPB + cl] * J[j][d];
+                }
+#pragma unroll
+                for (int d = 0; d < DIM; ++d)
+                    at(q, C::oC + d, cl) = sc * ge[d];
+                at(q, C::oW, cl) = S::valScale * wdj;
+                at(q, C::oW + 1, cl) = L.c * g * wdj;
+            }
+            const double* Gq = a.geo64 + NG_IDX(static_cast<int64_t>(q) * a.geoStride * n + e, a.geoSize, 6);
+#pragma unroll
+            for (int k = 0; k < ND * DIM; ++k)
+            {
+                const double g = Gq[(1 + k) * n];
+                at(q, C::oG + k, cl) = g;
+                at(q, C::oM + k, cl) = muw * g;
+            }
+        }
+    }
+    __syncthreads();
+
+    // displacement blocks of the unordered pairs and the gradient part of the (eeq, eeq) entries
+    const double mu0 = GD ? L.muD : L.C33;
+    const double rho = mu0 != 0. ? (GD ? L.lamD : L.C12) / mu0 : 0.;
+    for (int it = threadIdx.x; it < CPB * C::pairs; it += C::threads)
+    {
+        const int cl = it % CPB;
+        int ia, ib;
+        UnorderedPair<ND>(it / CPB, ia, ib);
+        const int64_t e = cell0 + cl;
+        if (e >= n)
+            continue;
+        double s[DIM][DIM], dd = 0.;
+#pragma unroll
+        for (int k = 0; k < DIM; ++k)
+#pragma unroll
+            for (int l = 0; l < DIM; ++l)
+                s[k][l] = 0.;
+#pragma unroll 2
+        for (int q = 0; q < NIP; ++q)
+        {
+            double m[DIM], gb[DIM];
+#pragma unroll
+            for (int d = 0; d < DIM; ++d)
+            {
+                m[d] = at(q, C::oM + ia * DIM + d, cl);
+                gb[d] = at(q, C::oG + ib * DIM + d, cl);
+            }
+#pragma unroll
+            for (int k = 0; k < DIM; ++k)
+#pragma unroll
+                for (int l = 0; l < DIM; ++l)
+                    s[k][l] += m[k] * gb[l];
+            if (GD)
+            {
+                double gab = at(q, C::oG + ia * DIM, cl) * gb[0];
+#pragma unroll
+                for (int d = 1; d < DIM; ++d)
+                    gab += at(q, C::oG + ia * DIM + d, cl) * gb[d];
+                dd += at(q, C::oW + 1, cl) * gab;
+            }
+        }
+        double tr = s[0][0];
+#pragma unroll
+        for (int k = 1; k < DIM; ++k)
+            tr += s[k][k];
+        double* rowA = em + (NG_IDX(e, n, 84) * ND + ia) * SL::size + ib * DIM;
+        double* rowB = em + (e * ND + ib) * SL::size + ia * DIM;
+#pragma unroll
+        for (int k = 0; k < DIM; ++k)
+#pragma unroll
+            for (int l = 0; l < DIM; ++l)
+            {
+                const double v = rho * s[k][l] + (k == l ? s[l][k] + tr : s[l][k]);
+                rowA[k * SL::nc + l] = v;
+                if (ia != ib)
+                    rowB[l * SL::nc + k] = v;
+            }
+        if (GD)
+        {
+            sGrad[(ia * ND + ib) * CPB + cl] = dd;
+            sGrad[(ib * ND + ia) * CPB + cl] = dd;
+        }
+    }
+    if constexpr (GD)
+    {
+        __syncthreads();
+        // coupling blocks: thread (cell, a) the (disp a, eeq) and (eeq a, eeq) rows over all b, then (eeq, disp a)
+        const int cl = threadIdx.x % CPB, ia = threadIdx.x / CPB;
+        const int64_t e = cell0 + cl;
+        if (e >= n)
+            return;
+        double f[DIM + 1][NIP], o[ND];
+#pragma unroll
+        for (int q = 0; q < NIP; ++q)
+        {
+            double g[DIM], sv[VD], P[DIM];
+#pragma unroll
+            for (int d = 0; d < DIM; ++d)
+                g[d] = at(q, C::oG + ia * DIM + d, cl);
+#pragma unroll
+            for (int v = 0; v < VD; ++v)
+                sv[v] = at(q, C::oS + v, cl);
+            BtS<double, DIM>(g, sv, P);
+            double z = at(q, C::oW, cl) * a.tabN_D[q * ND + ia];
+#pragma unroll
+            for (int d = 0; d < DIM; ++d)
+            {
+                f[d][q] = P[d];
+                z += at(q, C::oC + d, cl) * g[d];
+            }
+            f[DIM][q] = z;
+        }
+        double* slab = em + (e * ND + ia) * SL::size;
+#pragma unroll
+        for (int k = 0; k <= DIM; ++k)
+        {
+            SfValuesToNodes<double, DIM>(f[k], o);
+            double* row = slab + k * SL::nc + ND * DIM;
+#pragma unroll
+            for (int b = 0; b < ND; ++b)
+                row[b] = k < DIM ? o[b] : o[b] + sGrad[(ia * ND + b) * CPB + cl];
+        }
+#pragma unroll
+        for (int q = 0; q < NIP; ++q)
+        {
+            double g[DIM], tv[VD], Q[DIM];
+#pragma unroll
+            for (int d = 0; d < DIM; ++d)
+                g[d] = at(q, C::oG + ia * DIM + d, cl);
+#pragma unroll
+            for (int v = 0; v < VD; ++v)
+                tv[v] = at(q, C::oT + v, cl);
+            BtS<double, DIM>(g, tv, Q);
+#pragma unroll
+            for (int d = 0; d < DIM; ++d)
+                f[d][q] = Q[d];
+        }
+#pragma unroll
+        for (int d = 0; d < DIM; ++d)
+        {
+            SfValuesToNodes<double, DIM>(f[d], o);
+#pragma unroll
+            for (int r = 0; r < ND; ++r) // (eeq r, disp (ia, d))
+                em[(e * ND + r) * SL::size + DIM * SL::nc + ia * DIM + d] = o[r];
+        }
+    }
+}
+
+} // namespace
+
+bool LaunchTangent64(Ctx& c, const double* u, double* vals)
+{
+    const bool gd = c.prm.kind == NUTO_GPU_GRADIENT_DAMAGE;
+    const CellArgs a = CellArgsOf(c);
+    const Slot& D = c.slots[c.prm.disp_slot];
+    auto run = [&](auto dim, auto dmg) -> bool {
+        constexpr int DIM = decltype(dim)::value;
+        constexpr bool GD = decltype(dmg)::value;
+        using C = Cell64<DIM, GD>;
+        using SL = Slab<DIM, C::nd, GD>;
+        double* em = reinterpret_cast<double*>(
+                ElemMatsOrNull(c, static_cast<size_t>(c.nCells) * C::nd * SL::size * sizeof(double)));
+        if (!em)
+            return false;
+        const RowPlanArgs P = EnsureRowPlan(c);
+        if (c.slots.size() > static_cast<size_t>(GD ? 2 : 1)) // rows of slots that the integrand does not touch
+            NG_CUDA(cudaMemsetAsync(vals, 0, c.nnz * sizeof(double), c.stream));
+        constexpr int grad = std::max(C::nf * C::ng, C::nd * C::nd);
+        constexpr size_t smem = static_cast<size_t>(C::nip * C::rec + grad + C::nd) * C::cpb * sizeof(double);
+        auto kern = k_cell_matrices64<DIM, GD>;
+        if (smem > 48 * 1024)
+            NG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        kern<<<static_cast<unsigned>((c.nCells + C::cpb - 1) / C::cpb), C::threads, smem, c.stream>>>(a, c.law, u, em);
+        AfterLaunch(c, "k_cell_matrices64");
+        c.stats.kernel_launches += 1;
+        LaunchRows<double, DIM, C::nd, GD, 4>(c, P, 0, D.nNodes, em, vals);
+        return true;
+    };
+    using std::integral_constant;
+    if (c.dim == 2)
+        return gd ? run(integral_constant<int, 2>{}, integral_constant<bool, true>{})
+                  : run(integral_constant<int, 2>{}, integral_constant<bool, false>{});
+    return gd ? run(integral_constant<int, 3>{}, integral_constant<bool, true>{})
+              : run(integral_constant<int, 3>{}, integral_constant<bool, false>{});
+}
+
+// ---- plan of the row gather, once per mesh -----------------------------------------------------------------------
+namespace
+{
+
+struct PlanArgs
+{
+    int64_t nNodes, nCells;
+    int dim;
+    const int64_t* gdofD;
+    const int64_t* gdofE; // nullptr: no eeq rows
+    const int32_t* eOf;
+    const int64_t* cellPtr;
+    const int32_t* cellIdx;
+    const uint8_t* cellLoc;
+    const int64_t* rowPtr;
+    const uint8_t* rank[4]; // UU, UE, EU, EE
+    const int32_t* blk[4];
+};
+
+__global__ void __launch_bounds__(256) k_row_plan(PlanArgs A, RowPlan* __restrict__ plan)
+{
+    const int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+    if (a >= A.nNodes)
+        return;
+    RowPlan p{};
+    const int64_t g = A.gdofD[a];
+    p.rowU = A.rowPtr[g];
+    p.lenU = static_cast<int32_t>(A.rowPtr[g + 1] - p.rowU); // the rows of a node's components have one length
+    p.first = A.cellPtr[a];
+    p.cells = static_cast<int32_t>(A.cellPtr[a + 1] - p.first);
+    p.bUU = A.blk[0][a];
+    if (A.gdofE)
+    {
+        const int32_t ae = A.eOf[a];
+        const int64_t ge = A.gdofE[ae];
+        p.rowE = A.rowPtr[ge];
+        p.lenE = static_cast<int32_t>(A.rowPtr[ge + 1] - p.rowE);
+        p.bUE = A.blk[1][a];
+        p.bEU = A.blk[2][ae];
+        p.bEE = A.blk[3][ae];
+    }
+    plan[a] = p;
+}
+
+template <int ND>
+__global__ void __launch_bounds__(256) k_row_entries(PlanArgs A, int64_t nEntries, uint32_t* __restrict__ slab,
+                                                     uint32_t* __restrict__ packed)
+{
+    const int64_t it = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+    if (it >= nEntries * ND)
+        return;
+    const int64_t kc = it / ND;
+    const int b = static_cast<int>(it % ND);
+    const int64_t e = A.cellIdx[kc];
+    const int ia = A.cellLoc[kc];
+    if (b == 0)
+        slab[kc] = static_cast<uint32_t>(e * ND + ia);
+    const int64_t ridx = static_cast<int64_t>(ia * ND + b) * A.nCells + e;
+    packed[it] = static_cast<uint32_t>(A.rank[0][ridx]) | static_cast<uint32_t>(A.rank[1][ridx]) << 8 |
+                 static_cast<uint32_t>(A.rank[2][ridx]) << 16 | static_cast<uint32_t>(A.rank[3][ridx]) << 24;
+}
+
+} // namespace
+
+RowPlanArgs EnsureRowPlan(Ctx& c)
+{
+    const int ns = static_cast<int>(c.slots.size());
+    const int dS = c.prm.disp_slot;
+    const bool gd = c.prm.kind == NUTO_GPU_GRADIENT_DAMAGE;
+    const int eS = gd ? c.prm.eeq_slot : dS;
+    const Slot& D = c.slots[dS];
+    const int64_t entries = c.nCells * D.nen;
+    // the plan depends on the integrand's slots as well: whether there are eeq rows, and which slot they are in
+    const int key = 1 + dS + kMaxSlots * (gd ? 1 + eS : 0);
+    if (c.rowPlanKey != key)
+    {
+        c.dRowPlan.alloc(static_cast<size_t>(D.nNodes));
+        c.dRowSlab.alloc(static_cast<size_t>(entries));
+        c.dPackedRanks.alloc(static_cast<size_t>(entries * D.nen));
+        PlanArgs A{};
+        A.nNodes = D.nNodes;
+        A.nCells = c.nCells;
+        A.dim = c.dim;
+        A.gdofD = D.dGdof.p;
+        A.gdofE = gd ? c.slots[eS].dGdof.p : nullptr;
+        A.eOf = gd ? c.dEOf.p : nullptr;
+        A.cellPtr = D.dCellPtr.p;
+        A.cellIdx = D.dCellIdx.p;
+        A.cellLoc = D.dCellLoc.p;
+        A.rowPtr = c.dRowPtr.p;
+        const int pr[4] = {dS * ns + dS, dS * ns + eS, eS * ns + dS, eS * ns + eS};
+        for (int k = 0; k < 4; ++k)
+        {
+            A.rank[k] = c.pairs[pr[k]].rank;
+            A.blk[k] = c.pairs[pr[k]].dBlk.p;
+        }
+        k_row_plan<<<static_cast<unsigned>((D.nNodes + 255) / 256), 256, 0, c.stream>>>(A, c.dRowPlan.p);
+        AfterLaunch(c, "k_row_plan");
+        const unsigned blocks = static_cast<unsigned>((entries * D.nen + 255) / 256);
+        if (D.nen == 4)
+            k_row_entries<4><<<blocks, 256, 0, c.stream>>>(A, entries, c.dRowSlab.p, c.dPackedRanks.p);
+        else
+            k_row_entries<8><<<blocks, 256, 0, c.stream>>>(A, entries, c.dRowSlab.p, c.dPackedRanks.p);
+        AfterLaunch(c, "k_row_entries");
+        c.rowPlanKey = key;
+    }
+    RowPlanArgs P{};
+    P.plan = c.dRowPlan.p;
+    P.slab = c.dRowSlab.p;
+    P.packed = c.dPackedRanks.p;
+    P.nEntries = entries;
+    P.nnz = c.nnz;
+    return P;
+}
+
+unsigned char* ElemMatsOrNull(Ctx& c, size_t bytes)
+{
+    if (c.dElemMats.n >= bytes)
+        return c.dElemMats.p;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    NG_CUDA(cudaStreamIsCapturing(c.stream, &cs));
+    if (cs != cudaStreamCaptureStatusNone)
+        return nullptr;
+    size_t free = 0, total = 0;
+    NG_CUDA(cudaMemGetInfo(&free, &total));
+    if (bytes > free + c.dElemMats.n)
+        return nullptr;
+    c.dElemMats.alloc(bytes);
+    return c.dElemMats.p;
+}
+
+} // namespace nuto_gpu

@@ -741,8 +741,10 @@ void LaunchTangentTc20(Ctx& c, const double* u, float* vals)
     const size_t recBytes = static_cast<size_t>(n) * kNip * kRecF4 * 16;
     if (c.dRecords.n < recBytes)
         c.dRecords.alloc(recBytes);
-    if (c.dElemMats.n < static_cast<size_t>(n) * kNd * 180)
-        c.dElemMats.alloc(static_cast<size_t>(n) * kNd * 180);
+    const size_t emBytes = static_cast<size_t>(n) * kNd * 180 * sizeof(float);
+    if (c.dElemMats.n < emBytes)
+        c.dElemMats.alloc(emBytes);
+    float* em = reinterpret_cast<float*>(c.dElemMats.p);
     float4* recs = reinterpret_cast<float4*>(c.dRecords.p);
 
     Tc20Args A{};
@@ -770,7 +772,7 @@ void LaunchTangentTc20(Ctx& c, const double* u, float* vals)
     const unsigned grid = static_cast<unsigned>(std::min<int64_t>(n, c.smCount > 0 ? c.smCount : 1));
     auto tc = [&](auto kern) {
         NG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemTc));
-        kern<<<grid, kTcThreads, kSmemTc, c.stream>>>(n, A.tabDNd, recs, c.dElemMats.p, c.dStatus.p, c.spinLimit);
+        kern<<<grid, kTcThreads, kSmemTc, c.stream>>>(n, A.tabDNd, recs, em, c.dStatus.p, c.spinLimit);
     };
     if (ld)
     {
@@ -801,7 +803,7 @@ void LaunchTangentTc20(Ctx& c, const double* u, float* vals)
     const int p = c.prm.disp_slot * static_cast<int>(c.slots.size()) + c.prm.disp_slot;
     r.rank = c.pairs[p].rank;
     r.blk = c.pairs[p].dBlk.p;
-    k_tc20_rows<<<static_cast<unsigned>((D.nNodes + 3) / 4), 128, 0, c.stream>>>(r, c.dElemMats.p, vals);
+    k_tc20_rows<<<static_cast<unsigned>((D.nNodes + 3) / 4), 128, 0, c.stream>>>(r, em, vals);
     AfterLaunch(c, "k_tc20_rows");
     c.stats.kernel_launches += 3;
 }

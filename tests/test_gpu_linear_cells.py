@@ -1,6 +1,7 @@
-"""Residual of Quad4 / Hex8 cells with the two-point rule (k_residual_sf: sum-factorised gradients, a warp per 8 or 4 Hex8
-cells and per 16 or 8 Quad4 cells) against the oracle on distorted, non-cubic meshes: every integrand kind and law option,
-cell counts below one warp's, with remainders, and on both sides of the switch of the cells per warp."""
+"""Quad4 / Hex8 cells with the two-point rule against the oracle on distorted, non-cubic meshes: every integrand kind and
+law option, cell counts below one warp's or block's, with remainders, and on both sides of the switch of the residual's cells
+per warp. Residual: k_residual_sf (sum-factorised gradients, a warp per 8 or 4 Hex8 cells and per 16 or 8 Quad4 cells); FP64
+tangent: k_cell_matrices64 + k_rows_from_slabs (elastic and gradient damage with FULL damage), else the element kernel."""
 
 import numpy as np
 import pytest
@@ -66,3 +67,17 @@ def test_residual_on_distorted_cells(dim, cells, law):
     f_ref = P.build_vector(u)
     f = g.build_vector(u).cpu().numpy()
     assert np.abs(f - f_ref).max() <= FP64_REL * np.abs(f_ref).max()
+
+
+@pytest.mark.parametrize("dim,cells,law", CASES)
+def test_fp64_tangent_on_distorted_cells(dim, cells, law):
+    import nuto_gb300
+
+    g, P, u = _case(dim, cells, LAWS[law], 8)
+    K = P.build_matrix_scipy(u).tocsr()
+    K.sort_indices()
+    for precision in (nuto_gb300.FP64, nuto_gb300.FP64X):
+        v = g.build_matrix(u, precision).cpu().numpy()
+        assert np.abs(v - K.data).max() <= FP64_REL * np.abs(K.data).max()
+    if law in ("elastic", "elastic_plane_stress", "gradient", "gradient_plane_stress"):  # no atomics
+        assert np.array_equal(v, g.build_matrix(u, nuto_gb300.FP64).cpu().numpy())
