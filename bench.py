@@ -51,11 +51,9 @@ EXACT_BELOW = 1.0e4
 FORCING_FLOOR = 0.05
 # the FP32 tangent's kernels per form the autotuner can choose (nuto_gpu_autotune_info)
 TANGENT_KERNELS = {
-    "cell_matrices": "k_cell_matrices_law<3,8,8,GD,W> + k_rows_from_cells32 (law and element matrix per cell, "
-                     "then one warp per node adds its cells' slabs into its rows)",
-    "node_rows": "k_point_records + k_tangent_fused<3,8,8,GD,STAGED,W> (per-point records, one warp per node "
-                 "integrates its node-pair blocks)",
-    "pipelined": "k_point_records + k_tangent_rows_pipe<3,8,8,GD,W> (node rows on resident blocks)",
+    "cell_matrices": "k_cell_matrices<3,GD,W> + k_rows_from_slabs (law and element matrix per cell, then one warp per "
+                     "node adds its cells' slabs into its rows)",
+    "pipelined": "k_cell_matrices<3,GD,W> on resident blocks + k_rows_from_slabs",
 }
 
 
@@ -632,12 +630,12 @@ def run_ours(args):
            "precision": "FP32 tangent (law branch decisions in FP64), FP64 residual",
            "ms_matrix_per_step": float(np.mean(ms_matrix)), "ms_vector_per_step": float(np.mean(ms_vector)),
            "ms_per_step_sequential": ms_sequential,
-           "step_form": "nuto_gpu_build_system: the FP64 residual on a second stream (%s resident blocks per SM) "
+           "step_form": "nuto_gpu_build_system: the FP64 residual on a second stream (4 x %s resident warps per SM) "
                         "beside the FP32 tangent; ms_matrix/ms_vector_per_step and the rooflines from the same K "
                         "steps run as two calls in sequence" % os.environ.get("NUTO_GPU_SYSTEM_RES_BLOCKS", "6"),
            "max_abs_tangent_value": fp32_check,
            "roofline": roof,
-           "roofline_residual": {"kernel": "k_residual (FP64 internal-force vector)", "bound": "fp64",
+           "roofline_residual": {"kernel": "k_residual_sf + k_gather_residual (FP64 internal-force vector)", "bound": "fp64",
                                  "algorithmic_bytes_per_launch": rb, "mean_launch_ms": res_s * 1e3,
                                  "achieved_gbs": rb / res_s / 1e9},
            "e2e": e2e, "gpu_launches": int(launches), "clocks": clk}

@@ -114,9 +114,9 @@ class GpuCellGroup:
 
     def autotune_info(self):
         """Launch shapes the autotuner chose and the times it measured: {"tangent_warps": W, "tangent_form":
-        "node_rows" | "pipelined" | "cell_matrices", "tangent_pipelined": bool, "tangent_ms": [2, 4, 8 warps],
-        "tangent_pipelined_ms": [2, 4 warps], "tangent_cells_ms": [2, 4 warps], "spmv_lanes": {"f32/f32": G, ...},
-        "spmv_ms": {"f32/f32": [4, 8, 16 lanes], ...}} (0: not tuned)."""
+        "pipelined" (the cell kernel on resident blocks) | "cell_matrices", "tangent_pipelined": bool, "tangent_ms":
+        [2, 4, 8 warps], "tangent_pipelined_ms": [2, 4 warps], "tangent_cells_ms": [2, 4 warps], "spmv_lanes":
+        {"f32/f32": G, ...}, "spmv_ms": {"f32/f32": [4, 8, 16 lanes], ...}} (0: not tuned)."""
         ch = np.zeros(6, dtype=np.int32)
         ms = np.zeros(19, dtype=np.float32)
         self._call("nuto_gpu_autotune_info", _ptr(ch), _ptr(ms))

@@ -577,6 +577,13 @@ static void EnsureSideStream(Ctx& c)
     NG_CUDA(cudaEventCreateWithFlags(&c.evJoin, cudaEventDisableTiming));
 }
 
+// Quad4 gradient damage: the residual and the tangent slow each other down more than the overlap gives (sysResBlocks). With host buffers the copy
+// of the values is longer than either and overlaps them.
+static bool SystemInSequence(const Ctx& c)
+{
+    return c.sysResBlocks <= 0 || (c.dim == 2 && c.prm.kind == NUTO_GPU_GRADIENT_DAMAGE);
+}
+
 // The copy stream of nuto_gpu_build_system_host's chunked values and its events, created on first use.
 static void EnsureCopyStream(Ctx& c, int chunks)
 {
@@ -652,18 +659,10 @@ int nuto_gpu_create(nuto_gpu_ctx** out, int device, void* stream)
     const char* tk = std::getenv("NUTO_GPU_TANGENT");
     c->forceAtomicTangent = tk && std::string(tk) == "atomic";
     c->forceRecordTangent = tk && std::string(tk) == "records";
-    c->tangentStaged = !(tk && std::string(tk) == "fused");
-    if (tk && std::string(tk) == "pipelined")
+    if (tk && (std::string(tk) == "pipelined" || std::string(tk) == "cells"))
     {
-        c->tuning.tangentWarps = 4; // the double-buffered node-row kernel, not tuned
-        c->tuning.tangentForm = 1;
-    }
-    const char* cr = std::getenv("NUTO_GPU_CELLS_RECORDS");
-    c->cellsLawFused = !(cr && cr[0] == '1');
-    if (tk && std::string(tk) == "cells")
-    {
-        c->tuning.tangentWarps = 4; // element matrices + row gather, not tuned
-        c->tuning.tangentForm = 2;
+        c->tuning.tangentWarps = 4; // not tuned: the cell kernel on resident blocks, or one pass per warp
+        c->tuning.tangentForm = std::string(tk) == "pipelined" ? 1 : 2;
     }
     // Hex20 FP32 tangent: tensor cores with split TF32 (default), one TF32 product (tf32) or records + row
     // gather (off)
@@ -1148,7 +1147,7 @@ int nuto_gpu_build_system(nuto_gpu_ctx* ctx, const double* u, int precision, voi
         Ctx& c = *ctx;
         // the first call (lazy set-up of geometry, records and tuning), and contexts that ask for it, run the two
         // launches in sequence on the context's stream
-        if (c.systemCalls++ == 0 || c.sysResBlocks <= 0)
+        if (c.systemCalls++ == 0 || SystemInSequence(c))
         {
             LaunchTangent(c, u, precision, values);
             LaunchResidual(c, u, f);
@@ -1225,8 +1224,10 @@ int nuto_gpu_build_system_host(nuto_gpu_ctx* ctx, const double* hU, int precisio
         // chunk's values go to the host on a copy stream while the next chunks are gathered. (The row kernels writing
         // straight into mapped page-locked host memory were measured slower: 5.4 ms per 64^3 pass against 4.4 ms
         // with one copy after the tangent.)
-        constexpr int kChunks = 4;
-        const bool chunked = precision == NUTO_GPU_FP32 && c.tuning.tangentWarps != 0 && RowsContiguous(c);
+        // A chunk of 8 MB takes 40 us to copy, about what its launch, event and two copies cost the host: smaller values go
+        // in one piece (9^3, 1.5 MB: 89 us in 4 chunks, 50 us in one).
+        const int kChunks = static_cast<int>(std::min<size_t>(4, valBytes >> 23));
+        const bool chunked = kChunks > 1 && precision == NUTO_GPU_FP32 && c.tuning.tangentWarps != 0 && RowsContiguous(c);
         int chunkIdx = 0;
         if (chunked)
         {

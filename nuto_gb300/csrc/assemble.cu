@@ -442,27 +442,27 @@ void GatherCellVectors(Ctx& c, const Slot& S, int ncomp, int off, int64_t nLocal
 }
 
 // The same residual for Quad4 / Hex8 cells with the two-point rule, with the fields' gradients and the transposed sums
-// sum-factorised (sumfac.cuh). A warp takes CPB cells (one warp per block, so that nothing but the warp itself waits
-// and a mesh of a few thousand cells still spreads over the SMs):
+// sum-factorised (sumfac.cuh). A warp takes CPB cells and waits for no other warp:
 //   (1) lane (cell, field): the gradient of one displacement component (or of eeq, with its values) at all points;
 //   (2) lane (cell, point): H = G J^-1, the law, and the stress carried back to natural coordinates, T = w sigma J^-T;
 //   (3) lane (cell, field): the field's entries of the cell vector from T.
 // Bound by the FP64 pipe (2 lanes per clock and SM, 87 % busy): 220 FP64 instructions per Hex8 gradient-damage point, half
 // of them the law, against 352 with the gradients of all nodes read from the cache (k_residual), and 80 bytes of geometry
 // per point instead of 200. 64^3: 1345 -> 881 us with the gathers; 17^3: 56 -> 31 us; 200^2 Quad4 elastic: 26 -> 19 us.
-// (Two warps per 8 cells left one of them idle in phases 1 and 3: 922 us at 64^3.)
+// (Two warps per 8 cells left one of them idle in phases 1 and 3: 922 us at 64^3.) 80 registers: the few spills cost nothing
+// (886 us at 64^3), and beside the FP32 tangent the smaller blocks leave it room (64^3 system pass 1420 -> 1340 us).
 template <int DIM, int KIND>
 struct ResShape
 {
     static constexpr bool GD = KIND == NUTO_GPU_GRADIENT_DAMAGE;
     static constexpr int nip = SumFac<DIM>::nd;
     static constexpr int nf = DIM + (GD ? 1 : 0);
-    static constexpr int threads = 32;
+    static constexpr int warps = 1; // per block: 4 made a 17^3 mesh (154 blocks) 10 us slower and nothing faster
 };
 
 
 template <int DIM, int KIND, int CPB>
-__global__ void __launch_bounds__(32, 16) k_residual_sf(CellArgs a, LawParams L, const double* __restrict__ u,
+__global__ void __launch_bounds__(32, 24) k_residual_sf(CellArgs a, LawParams L, const double* __restrict__ u,
                                                     double* __restrict__ fcell)
 {
     using R = ResShape<DIM, KIND>;
@@ -470,15 +470,19 @@ __global__ void __launch_bounds__(32, 16) k_residual_sf(CellArgs a, LawParams L,
     constexpr bool GD = R::GD;
     constexpr int VD = DIM == 2 ? 3 : 6;
     constexpr int ND = S::nd, NIP = S::nd, NF = R::nf;
-    __shared__ double sG[NF][S::ng][CPB];
-    __shared__ double sV[GD ? NIP : 1][CPB];
-    __shared__ double sT[NF][NIP][DIM][CPB];
-    __shared__ double sTV[GD ? NIP : 1][CPB];
-    const int64_t n = a.nCells;
-    for (int64_t cell0 = static_cast<int64_t>(blockIdx.x) * CPB; cell0 < n;
-         cell0 += static_cast<int64_t>(gridDim.x) * CPB)
+    struct Shared
     {
-        for (int it = threadIdx.x; it < CPB * NF; it += R::threads)
+        double G[NF][S::ng][CPB], V[GD ? NIP : 1][CPB], T[NF][NIP][DIM][CPB], TV[GD ? NIP : 1][CPB];
+    };
+    __shared__ Shared shared[R::warps];
+    Shared& sh = shared[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const int64_t n = a.nCells;
+    // a warp's cells; warps do not wait for each other
+    for (int64_t cell0 = (static_cast<int64_t>(blockIdx.x) * R::warps + (threadIdx.x >> 5)) * CPB; cell0 < n;
+         cell0 += static_cast<int64_t>(gridDim.x) * R::warps * CPB)
+    {
+        for (int it = lane; it < CPB * NF; it += 32)
         {
             const int cl = it % CPB, fl = it / CPB;
             const int64_t e = cell0 + cl;
@@ -501,15 +505,15 @@ __global__ void __launch_bounds__(32, 16) k_residual_sf(CellArgs a, LawParams L,
             {
 #pragma unroll
                 for (int q = 0; q < NIP; ++q)
-                    sV[q][cl] = val[q];
+                    sh.V[q][cl] = val[q];
             }
 #pragma unroll
             for (int k = 0; k < S::ng; ++k)
-                sG[fl][k][cl] = g[k];
+                sh.G[fl][k][cl] = g[k];
         }
         __syncwarp();
 #pragma unroll 1
-        for (int it = threadIdx.x; it < CPB * NIP; it += R::threads)
+        for (int it = lane; it < CPB * NIP; it += 32)
         {
             const int cl = it % CPB, q = it / CPB;
             const int64_t e = cell0 + cl;
@@ -536,7 +540,7 @@ __global__ void __launch_bounds__(32, 16) k_residual_sf(CellArgs a, LawParams L,
                 for (int c = 0; c < DIM; ++c)
 #pragma unroll
                     for (int j = 0; j < DIM; ++j)
-                        G[c][j] = sG[c][gi[j]][cl];
+                        G[c][j] = sh.G[c][gi[j]][cl];
                 StrainFromNatural<double, DIM>(G, J, eps);
                 if (KIND == NUTO_GPU_MB_LINEAR_ELASTIC)
                 {
@@ -552,18 +556,18 @@ __global__ void __launch_bounds__(32, 16) k_residual_sf(CellArgs a, LawParams L,
                 }
                 else
                 {
-                    const double eeq = S::valScale * sV[q][cl];
+                    const double eeq = S::valScale * sh.V[q][cl];
                     const double kap = fmax(kh, eeq); // GradientDamage::Kappa (GradientDamage.h:127-130)
                     const double phi = DamageIntegrity<double>(L, kap);
                     LedStressWeighted<double, DIM>(L, eps, phi, wdjE, sig);
                     double cg = L.c * wdj;
                     if (L.interaction != NUTO_GPU_INTERACTION_CONSTANT)
                         cg *= InteractionFactor<double>(L, 1. - phi);
-                    sTV[q][cl] = (eeq - MisesNorm<double, DIM>(L, eps)) * (S::valScale * wdj);
+                    sh.TV[q][cl] = (eeq - MisesNorm<double, DIM>(L, eps)) * (S::valScale * wdj);
                     double g[DIM], ge[DIM];
 #pragma unroll
                     for (int j = 0; j < DIM; ++j)
-                        g[j] = cg * sG[DIM][gi[j]][cl];
+                        g[j] = cg * sh.G[DIM][gi[j]][cl];
 #pragma unroll
                     for (int d = 0; d < DIM; ++d)
                     {
@@ -580,7 +584,7 @@ __global__ void __launch_bounds__(32, 16) k_residual_sf(CellArgs a, LawParams L,
 #pragma unroll
                         for (int d = 1; d < DIM; ++d)
                             s += ge[d] * J[j][d];
-                        sT[DIM][q][j][cl] = s;
+                        sh.T[DIM][q][j][cl] = s;
                     }
                 }
 #pragma unroll
@@ -590,14 +594,14 @@ __global__ void __launch_bounds__(32, 16) k_residual_sf(CellArgs a, LawParams L,
                     BtS<double, DIM>(J[j], sig, b); // row j of J^-1 in the place of a node gradient
 #pragma unroll
                     for (int c = 0; c < DIM; ++c)
-                        sT[c][q][j][cl] = b[c];
+                        sh.T[c][q][j][cl] = b[c];
                 }
             }
         }
         __syncwarp();
         const int64_t nLocal = static_cast<int64_t>(ND) * NF;
         (void)nLocal; // buffer extent for checked builds
-        for (int it = threadIdx.x; it < CPB * NF; it += R::threads)
+        for (int it = lane; it < CPB * NF; it += 32)
         {
             const int cl = it % CPB, fl = it / CPB;
             const int64_t e = cell0 + cl;
@@ -605,8 +609,8 @@ __global__ void __launch_bounds__(32, 16) k_residual_sf(CellArgs a, LawParams L,
                 continue;
             double out[ND];
             const bool eq = GD && fl == DIM;
-            SfTranspose<double, DIM, GD>([&](int j, int q) { return sT[fl][q][j][cl]; },
-                                         [&](int q) { return eq ? sTV[GD ? q : 0][cl] : 0.; }, out);
+            SfTranspose<double, DIM, GD>([&](int j, int q) { return sh.T[fl][q][j][cl]; },
+                                         [&](int q) { return eq ? sh.TV[GD ? q : 0][cl] : 0.; }, out);
             // entry of node 0: the displacement entries are node-major, the eeq entries follow them
             const int64_t first = eq ? static_cast<int64_t>(ND) * DIM : fl, step = eq ? 1 : DIM;
 #pragma unroll
@@ -682,13 +686,13 @@ void LaunchResidual(Ctx& c, const double* u, double* f, int blocksPerSm)
             // 1.6 times shorter and are taken while each of the 4 schedulers of an SM then has at most one warp
             constexpr int BIG = DIM == 3 ? 8 : 16, SMALL = BIG / 2;
             const bool small = c.nCells <= static_cast<int64_t>(SMALL) * 4 * std::max(c.smCount, 1);
-            // a block of k_residual_sf is a quarter of a block of k_residual
+            constexpr int W = R::warps;
             if (small)
-                k_residual_sf<DIM, KIND, SMALL><<<grid(SMALL, 4 * blocksPerSm), R::threads, 0, c.stream>>>(
-                        a, c.law, u, c.dCellVec.p);
+                k_residual_sf<DIM, KIND, SMALL>
+                        <<<grid(SMALL * W, 4 * blocksPerSm), 32 * W, 0, c.stream>>>(a, c.law, u, c.dCellVec.p);
             else
-                k_residual_sf<DIM, KIND, BIG><<<grid(BIG, 4 * blocksPerSm), R::threads, 0, c.stream>>>(
-                        a, c.law, u, c.dCellVec.p);
+                k_residual_sf<DIM, KIND, BIG>
+                        <<<grid(BIG * W, 4 * blocksPerSm), 32 * W, 0, c.stream>>>(a, c.law, u, c.dCellVec.p);
         };
         auto kinds = [&](auto dim) {
             if (gd)

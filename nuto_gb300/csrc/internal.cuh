@@ -273,6 +273,7 @@ struct RowPlanArgs
     const uint32_t* packed;
     int64_t nodeFirst, nodeLast; // displacement nodes of the launch
     int64_t nEntries, nnz;
+    bool sameGraph; // the eeq row of every node has the positions of its displacement rows
 };
 
 // Boundary cells of one DOF slot (NeumannBc loads): Line2 faces of a 2D mesh or Quad4 faces of a 3D mesh, on the
@@ -339,11 +340,10 @@ struct HostClock
 struct Tuning
 {
     bool enabled = true;             // NUTO_GPU_AUTOTUNE=0 keeps the defaults
-    int tangentWarps = 0;            // warps per block of the FP32 tangent's node-row kernel (2, 4, 8)
-    int tangentForm = 0;             // 0 node rows, 1 double-buffered node rows on resident blocks, 2 element
-                                     // matrices + row gather
-    float tangentMs[7] = {0, 0, 0, 0, 0, 0, 0}; // one assembly with 2, 4, 8 warps per block; double-buffered with 2,
-                                                // 4; element matrices with 2, 4
+    int tangentWarps = 0;            // warps per block of the FP32 tangent's kernels (2, 4, 8)
+    int tangentForm = 2;             // 2 one pass of the cell kernel per warp, 1 on a grid of resident blocks
+    float tangentMs[7] = {0, 0, 0, 0, 0, 0, 0}; // one assembly with 2, 4, 8 warps per block; resident blocks with 2, 4;
+                                                // the first two again
     int spmvGroup[4] = {0, 0, 0, 0}; // lanes per node of the fine-level product, per (value, vector) type pair
     float spmvMs[4][3] = {};         // one product with 4, 8, 16 lanes per node
 };
@@ -406,11 +406,10 @@ struct Ctx
     int gmresRestart = 0;            // NUTO_GPU_GMRES_RESTART; 0 = the default length
     DBuf<int32_t> dEOf;
     DBuf<unsigned char> dRecords;
-    // fused FP32 tangent: -1 not decided, 0 not applicable, 1 used; FP32 node coordinates relative to each cell's
-    // first node (planar [(n * dim + d)][cell])
+    // element-matrix tangents of linear cells: -1 not decided, 0 not applicable, 1 used; FP32 node coordinates relative to
+    // each cell's first node (planar [(n * dim + d)][cell])
     Tuning tuning;
     int fusedMode = -1;
-    bool tangentStaged = true; // per-point records computed once (NUTO_GPU_TANGENT=fused: recomputed per node warp)
     DBuf<float> dRelX;
     // Hex20 FP32 tangent on the tensor cores: -1 not decided, 0 not applicable, 1 used; split 3 = three TF32
     // products per contraction (hi.hi + hi.lo + lo.hi, FP32-level accuracy), 1 = one (NUTO_GPU_TC20=tf32);
@@ -422,10 +421,10 @@ struct Ctx
     // element matrices of the last tangent in its arithmetic (one buffer for FP32 and FP64: every tangent of a context runs
     // on its stream) and the plan of the row gather
     DBuf<unsigned char> dElemMats;
-    bool cellsLawFused = true; // element-matrix form: the law in the cell kernel (NUTO_GPU_CELLS_RECORDS=1: records)
     DBuf<RowPlan> dRowPlan;
     DBuf<uint32_t> dRowSlab, dPackedRanks;
     int rowPlanKey = 0; // slots the plan was built for (0: not built)
+    bool rowPlanSame = false;
     // device status word of kernels with bounded waits (0 = fine, else NUTO_GPU_ETIMEOUT), read after a stream
     // synchronisation; spinLimit bounds every wait loop (iterations)
     DBuf<int> dStatus;
@@ -434,11 +433,12 @@ struct Ctx
     DBuf<double> dCellVec;
     // nuto_gpu_build_system: the residual on a second stream beside the tangent, as a persistent grid of
     // 4 sysResBlocks warps per SM (the FP64 pipe needs few warps), the rest of every SM left to the tangent's
-    // blocks; the first call of a context runs both in sequence (lazy set-up, autotuning). 64^3 system pass with
-    // 1 / 2 / 3 / 4: 1835 / 1668 / 1681 / 1689 us
+    // blocks; the first call of a context runs both in sequence (lazy set-up, autotuning). FP32 64^3 Hex8 system pass:
+    // 1502 us in sequence, 1528 / 1344 / 1280 with 2 / 4 / 6; 17^3: 54 us, 38 with all three; 200^2 Quad4 elastic: 35 us,
+    // 32 / 30 / 30. Quad4 gradient damage runs in sequence: 3 / 10 plates 35 / 141 us, beside each other 62 / 144.
     cudaStream_t sideStream = nullptr;
     cudaEvent_t evFork = nullptr, evJoin = nullptr;
-    int sysResBlocks = 2;
+    int sysResBlocks = 6;
     // nuto_gpu_build_system_host: device copies of the caller's host state, values and vector
     DBuf<double> dHostIoU, dHostIoF;
     DBuf<unsigned char> dHostIoVals;
@@ -722,8 +722,8 @@ __host__ __device__ inline T MisesValue(const LawParams& p, const T* e)
     return K1 * I1 + A;
 }
 
-template <typename T, int DIM>
-__host__ __device__ inline void MisesDerivative(const LawParams& p, const T* s, T* d)
+template <typename T, int DIM, typename P>
+__host__ __device__ inline void MisesDerivative(const P& p, const T* s, T* d)
 {
     const T K1 = T(p.K1), K2 = T(p.K2);
     if (DIM == 3)

@@ -8,8 +8,10 @@
 //
 // Bound by the latency of the chain node -> cells -> slab. It is kept to three dependent loads: the node's plan (rows,
 // block offsets, cell list: one 64-byte record), the slab numbers and packed ranks of a batch of 4 cells, their slabs.
-// FP32 Hex8 gradient damage at 64^3: 380 us with row pointers, cell indices and block offsets read one after the other,
-// about 315 us now; Quad4 gradient damage (16 lanes per node) 70 -> 30 us for 71 k nodes.
+// The rows are kept interleaved where the eeq row has the positions of the displacement rows (every mesh whose DOF types share
+// one node graph): one vector access per column instead of one per row. FP32 Hex8 gradient damage at 48^3: 160 us with row
+// pointers, cell indices and block offsets read one after the other, 139 us with the plan, 118 us interleaved (DRAM floor
+// 95 us; 81 % of the shared-memory wavefronts). Quad4 gradient damage (16 lanes per node) 70 -> 30 us for 71 k nodes.
 #pragma once
 
 #include "internal.cuh"
@@ -29,26 +31,40 @@ struct Slab
     static constexpr int lanes = nc > 16 ? 32 : (nc > 8 ? 16 : 8);
 };
 
-template <typename T, int DIM, int ND, bool GD, int W>
+// One value of every row of a node at one position, read and written as one vector
+template <typename T, int NR>
+struct alignas(NR == 2 ? 2 * sizeof(T) : 16) RowVec
+{
+    static constexpr int n = NR == 3 ? 4 : NR;
+    T v[n];
+};
+
+// SAME: the eeq row has the same positions as the displacement rows (one node graph for both DOF types, and elastic cells
+// with their one): the rows are kept interleaved and updated with one vector access per column
+template <typename T, int DIM, int ND, bool GD, int W, bool SAME>
 __global__ void __launch_bounds__(W * 32) k_rows_from_slabs(RowPlanArgs P, const T* __restrict__ em, T* __restrict__ vals)
 {
     using S = Slab<DIM, ND, GD>;
     constexpr int NR = S::nr, NC = S::nc, LPN = S::lanes, NPW = 32 / LPN, CB = 4;
-    __shared__ T sRowAll[W * NPW][NR * kRowsCap];
+    using V = RowVec<T, NR>;
+    __shared__ V sRowAll[W * NPW][kRowsCap];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int grp = lane / LPN, col = lane % LPN;
     PdlWait();
     const int64_t a = P.nodeFirst + (static_cast<int64_t>(blockIdx.x) * W + wid) * NPW + grp;
-    T* sRow = sRowAll[wid * NPW + grp];
+    V* sVec = sRowAll[wid * NPW + grp];
+    T* sRow = reinterpret_cast<T*>(sVec); // SAME = false: [row][kRowsCap]
     RowPlan p{};
     if (a < P.nodeLast)
         p = P.plan[a]; // p.cells = 0 beyond the last node: nothing to add or store
-    for (int k = 0; k < DIM; ++k)
+    if constexpr (SAME)
+    {
         for (int i = col; i < p.lenU; i += LPN)
-            sRow[k * kRowsCap + i] = T(0);
-    if (GD)
-        for (int i = col; i < p.lenE; i += LPN)
-            sRow[DIM * kRowsCap + i] = T(0);
+            sVec[i] = V{};
+    }
+    else
+        for (int i = col; i < NR * kRowsCap; i += LPN)
+            sRow[i] = T(0);
     const bool ucol = col < ND * DIM;
     const int myB = col < NC ? (ucol ? col / DIM : col - ND * DIM) : 0;
     const int myL = ucol ? col % DIM : 0;
@@ -87,25 +103,52 @@ __global__ void __launch_bounds__(W * 32) k_rows_from_slabs(RowPlanArgs P, const
             {
                 const int r0 = word[c] & 0xff, r1 = (word[c] >> 8) & 0xff, r2 = (word[c] >> 16) & 0xff, r3 = word[c] >> 24;
                 const int posU = ucol ? p.bUU + DIM * r0 + myL : p.bUE + r1;
-#pragma unroll
-                for (int k = 0; k < DIM; ++k)
-                    sRow[k * kRowsCap + NG_IDX(posU, kRowsCap, 79)] += v[c][k];
-                if (GD)
+                if constexpr (SAME)
                 {
-                    const int posE = ucol ? p.bEU + DIM * r2 + myL : p.bEE + r3;
-                    sRow[DIM * kRowsCap + NG_IDX(posE, kRowsCap, 79)] += v[c][DIM];
+                    V& row = sVec[NG_IDX(posU, kRowsCap, 79)];
+                    V x = row;
+#pragma unroll
+                    for (int k = 0; k < NR; ++k)
+                        x.v[k] += v[c][k];
+                    row = x;
+                }
+                else
+                {
+#pragma unroll
+                    for (int k = 0; k < DIM; ++k)
+                        sRow[k * kRowsCap + NG_IDX(posU, kRowsCap, 79)] += v[c][k];
+                    if (GD)
+                    {
+                        const int posE = ucol ? p.bEU + DIM * r2 + myL : p.bEE + r3;
+                        sRow[DIM * kRowsCap + NG_IDX(posE, kRowsCap, 79)] += v[c][DIM];
+                    }
                 }
             }
             __syncwarp();
         }
     }
-#pragma unroll
-    for (int k = 0; k < DIM; ++k)
+    if constexpr (SAME)
+    {
         for (int i = col; i < p.lenU; i += LPN)
-            vals[NG_IDX(p.rowU + static_cast<int64_t>(k) * p.lenU + i, P.nnz, 75)] = sRow[k * kRowsCap + i];
-    if (GD)
-        for (int i = col; i < p.lenE; i += LPN)
-            vals[NG_IDX(p.rowE + i, P.nnz, 75)] = sRow[DIM * kRowsCap + i];
+        {
+            const V x = sVec[i];
+#pragma unroll
+            for (int k = 0; k < DIM; ++k)
+                vals[NG_IDX(p.rowU + static_cast<int64_t>(k) * p.lenU + i, P.nnz, 75)] = x.v[k];
+            if (GD)
+                vals[NG_IDX(p.rowE + i, P.nnz, 75)] = x.v[DIM];
+        }
+    }
+    else
+    {
+#pragma unroll
+        for (int k = 0; k < DIM; ++k)
+            for (int i = col; i < p.lenU; i += LPN)
+                vals[NG_IDX(p.rowU + static_cast<int64_t>(k) * p.lenU + i, P.nnz, 75)] = sRow[k * kRowsCap + i];
+        if (GD)
+            for (int i = col; i < p.lenE; i += LPN)
+                vals[NG_IDX(p.rowE + i, P.nnz, 75)] = sRow[DIM * kRowsCap + i];
+    }
 }
 
 // Launches the gather for the displacement nodes first .. last - 1.
@@ -118,9 +161,11 @@ inline void LaunchRows(Ctx& c, const RowPlanArgs& all, int64_t first, int64_t la
     constexpr int perBlock = W * (32 / Slab<DIM, ND, GD>::lanes);
     if (last <= first)
         return;
-    NG_CUDA(LaunchPdl(k_rows_from_slabs<T, DIM, ND, GD, W>,
-                      dim3(static_cast<unsigned>((last - first + perBlock - 1) / perBlock)), dim3(W * 32), 0, c.stream, P, em,
-                      vals));
+    const dim3 grid(static_cast<unsigned>((last - first + perBlock - 1) / perBlock));
+    if (!GD || P.sameGraph)
+        NG_CUDA(LaunchPdl(k_rows_from_slabs<T, DIM, ND, GD, W, true>, grid, dim3(W * 32), 0, c.stream, P, em, vals));
+    else if constexpr (GD)
+        NG_CUDA(LaunchPdl(k_rows_from_slabs<T, DIM, ND, GD, W, false>, grid, dim3(W * 32), 0, c.stream, P, em, vals));
     AfterLaunch(c, "k_rows_from_slabs");
     c.stats.kernel_launches += 1;
 }

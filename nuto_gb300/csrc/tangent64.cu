@@ -388,7 +388,8 @@ struct PlanArgs
     const int32_t* blk[4];
 };
 
-__global__ void __launch_bounds__(256) k_row_plan(PlanArgs A, RowPlan* __restrict__ plan)
+// *differ becomes 1 where the eeq row of a node has other positions than its displacement rows
+__global__ void __launch_bounds__(256) k_row_plan(PlanArgs A, RowPlan* __restrict__ plan, int* __restrict__ differ)
 {
     const int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
     if (a >= A.nNodes)
@@ -409,13 +410,15 @@ __global__ void __launch_bounds__(256) k_row_plan(PlanArgs A, RowPlan* __restric
         p.bUE = A.blk[1][a];
         p.bEU = A.blk[2][ae];
         p.bEE = A.blk[3][ae];
+        if (p.lenE != p.lenU || p.bEU != p.bUU || p.bEE != p.bUE)
+            *differ = 1;
     }
     plan[a] = p;
 }
 
 template <int ND>
 __global__ void __launch_bounds__(256) k_row_entries(PlanArgs A, int64_t nEntries, uint32_t* __restrict__ slab,
-                                                     uint32_t* __restrict__ packed)
+                                                     uint32_t* __restrict__ packed, int* __restrict__ differ)
 {
     const int64_t it = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
     if (it >= nEntries * ND)
@@ -427,8 +430,10 @@ __global__ void __launch_bounds__(256) k_row_entries(PlanArgs A, int64_t nEntrie
     if (b == 0)
         slab[kc] = static_cast<uint32_t>(e * ND + ia);
     const int64_t ridx = static_cast<int64_t>(ia * ND + b) * A.nCells + e;
-    packed[it] = static_cast<uint32_t>(A.rank[0][ridx]) | static_cast<uint32_t>(A.rank[1][ridx]) << 8 |
-                 static_cast<uint32_t>(A.rank[2][ridx]) << 16 | static_cast<uint32_t>(A.rank[3][ridx]) << 24;
+    const uint32_t r0 = A.rank[0][ridx], r1 = A.rank[1][ridx], r2 = A.rank[2][ridx], r3 = A.rank[3][ridx];
+    if (r0 != r2 || r1 != r3)
+        *differ = 1;
+    packed[it] = r0 | r1 << 8 | r2 << 16 | r3 << 24;
 }
 
 } // namespace
@@ -465,14 +470,21 @@ RowPlanArgs EnsureRowPlan(Ctx& c)
             A.rank[k] = c.pairs[pr[k]].rank;
             A.blk[k] = c.pairs[pr[k]].dBlk.p;
         }
-        k_row_plan<<<static_cast<unsigned>((D.nNodes + 255) / 256), 256, 0, c.stream>>>(A, c.dRowPlan.p);
+        DBuf<int> differ;
+        differ.alloc(1);
+        NG_CUDA(cudaMemsetAsync(differ.p, 0, sizeof(int), c.stream));
+        k_row_plan<<<static_cast<unsigned>((D.nNodes + 255) / 256), 256, 0, c.stream>>>(A, c.dRowPlan.p, differ.p);
         AfterLaunch(c, "k_row_plan");
         const unsigned blocks = static_cast<unsigned>((entries * D.nen + 255) / 256);
         if (D.nen == 4)
-            k_row_entries<4><<<blocks, 256, 0, c.stream>>>(A, entries, c.dRowSlab.p, c.dPackedRanks.p);
+            k_row_entries<4><<<blocks, 256, 0, c.stream>>>(A, entries, c.dRowSlab.p, c.dPackedRanks.p, differ.p);
         else
-            k_row_entries<8><<<blocks, 256, 0, c.stream>>>(A, entries, c.dRowSlab.p, c.dPackedRanks.p);
+            k_row_entries<8><<<blocks, 256, 0, c.stream>>>(A, entries, c.dRowSlab.p, c.dPackedRanks.p, differ.p);
         AfterLaunch(c, "k_row_entries");
+        int h = 0;
+        NG_CUDA(cudaMemcpyAsync(&h, differ.p, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+        NG_CUDA(cudaStreamSynchronize(c.stream));
+        c.rowPlanSame = h == 0;
         c.rowPlanKey = key;
     }
     RowPlanArgs P{};
@@ -481,6 +493,7 @@ RowPlanArgs EnsureRowPlan(Ctx& c)
     P.packed = c.dPackedRanks.p;
     P.nEntries = entries;
     P.nnz = c.nnz;
+    P.sameGraph = c.rowPlanSame;
     return P;
 }
 

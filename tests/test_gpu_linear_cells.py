@@ -81,3 +81,18 @@ def test_fp64_tangent_on_distorted_cells(dim, cells, law):
         assert np.abs(v - K.data).max() <= FP64_REL * np.abs(K.data).max()
     if law in ("elastic", "elastic_plane_stress", "gradient", "gradient_plane_stress"):  # no atomics
         assert np.array_equal(v, g.build_matrix(u, nuto_gb300.FP64).cpu().numpy())
+
+
+@pytest.mark.parametrize("form", ["cells", "pipelined"])
+@pytest.mark.parametrize("dim,cells,law", [c for c in CASES if "unilateral" not in c[2] and c[2] != "local"])
+def test_fp32_tangent_on_distorted_cells(dim, cells, law, form, monkeypatch):
+    """The FP32 element-matrix form, one pass per warp and on resident blocks: the FP32 tangent's tolerance against the
+    oracle, 2e-6 of the largest entry."""
+    import nuto_gb300
+
+    monkeypatch.setenv("NUTO_GPU_TANGENT", form)
+    g, P, u = _case(dim, cells, LAWS[law], 9)
+    K = P.build_matrix_scipy(u).tocsr()
+    K.sort_indices()
+    v = g.build_matrix(u, nuto_gb300.FP32).double().cpu().numpy()
+    assert np.abs(v - K.data).max() <= 2e-6 * np.abs(K.data).max()
