@@ -452,6 +452,8 @@ static void BuildPattern(Ctx& c)
     }
     FreeAmg(c);
     c.rowPlanKey = 0;
+    c.h20Mode = -1;
+    c.tc20Mode = -1;
     c.havePattern = true;
 }
 
@@ -577,8 +579,8 @@ static void EnsureSideStream(Ctx& c)
     NG_CUDA(cudaEventCreateWithFlags(&c.evJoin, cudaEventDisableTiming));
 }
 
-// Quad4 gradient damage: the residual and the tangent slow each other down more than the overlap gives (sysResBlocks). With host buffers the copy
-// of the values is longer than either and overlaps them.
+// Quad4 gradient damage: the residual and the tangent slow each other down more than the overlap gives (sysResBlocks).
+// With host buffers the copy of the values is longer than either and overlaps them.
 static bool SystemInSequence(const Ctx& c)
 {
     return c.sysResBlocks <= 0 || (c.dim == 2 && c.prm.kind == NUTO_GPU_GRADIENT_DAMAGE);
@@ -939,6 +941,8 @@ int nuto_gpu_set_integrand(nuto_gpu_ctx* ctx, const nuto_gpu_integrand* p)
         ctx->haveIntegrand = true;
         ctx->rowsMode = -1;
         ctx->fusedMode = -1;
+        ctx->h20Mode = -1;
+        ctx->tc20Mode = -1;
         ctx->haveGeo = false;
         return NUTO_GPU_OK;
     });

@@ -1472,7 +1472,7 @@ static void LaunchTangentRows(Ctx& c, const double* u, T* vals)
 // done: the element kernel, which needs none, is then taken
 static bool SetUpInCapture(Ctx& c)
 {
-    if (c.rowsMode >= 0 && c.fusedMode >= 0 && c.rowPlanKey != 0)
+    if (c.rowsMode >= 0 && c.fusedMode >= 0 && c.h20Mode >= 0 && c.rowPlanKey != 0)
         return false;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     NG_CUDA(cudaStreamIsCapturing(c.stream, &cs));
@@ -1503,8 +1503,9 @@ static void LaunchTangentT(Ctx& c, const double* u, T* vals)
     // FP64, linear cells with a constant ratio of the Lame parameters: element matrices + row gather (64^3 gradient
     // damage: 4.66 ms against 14.46 ms of the element kernel)
     if constexpr (sizeof(T) == 8)
-        if (!c.forceAtomicTangent && !SetUpInCapture(c) && RowsSupported(c) && FusedTangentSupported(c) &&
-            LaunchTangent64(c, u, vals))
+        if (!c.forceAtomicTangent && !SetUpInCapture(c) && RowsSupported(c) &&
+            ((FusedTangentSupported(c) && LaunchTangent64(c, u, vals)) ||
+             (Hex20RowsSupported(c) && LaunchTangent64H20(c, u, vals))))
             return;
     NG_CUDA(cudaMemsetAsync(vals, 0, c.nnz * sizeof(T), c.stream));
     if (sizeof(T) == 4)

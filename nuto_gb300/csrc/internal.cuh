@@ -415,6 +415,7 @@ struct Ctx
     // products per contraction (hi.hi + hi.lo + lo.hi, FP32-level accuracy), 1 = one (NUTO_GPU_TC20=tf32);
     // per-point records and per-cell element matrices ([cell][a][i][b][j], FP32)
     int tc20Mode = -1;
+    int h20Mode = -1; // Hex20 element matrices + row gather: -1 not decided, 0 not applicable, 1 applicable
     int tc20Split = 3;
     bool forceTc20Off = false; // NUTO_GPU_TC20=off
     int tc20LawFp64 = 0;       // NUTO_GPU_TC20=fp64law: the law of every point in FP64
@@ -495,6 +496,8 @@ bool FusedTangentSupported(Ctx& c);
 void LaunchTangentFused(Ctx& c, const double* u, float* vals);
 // element matrices in FP64 + row gather for the cells of FusedTangentSupported; false: not done (no memory for them)
 bool LaunchTangent64(Ctx& c, const double* u, double* vals);
+bool LaunchTangent64H20(Ctx& c, const double* u, double* vals); // for the cells of Hex20RowsSupported
+bool Hex20RowsSupported(Ctx& c);
 RowPlanArgs EnsureRowPlan(Ctx& c);
 // the context's element-matrix buffer with room for `bytes`; nullptr while it would have to grow during a stream capture or
 // beyond the free device memory
@@ -811,14 +814,15 @@ __device__ __forceinline__ T MisesNorm(const LawParams& p, const T* e)
     }
 }
 
-// 1 - omega of DamageLawExponential
+// 1 - omega of DamageLawExponential, through omega as the law defines it (the difference rounds at 1, which for a nearly
+// destroyed material is not the rounding of k0 / kappa (...) itself)
 template <typename T>
 __device__ __forceinline__ T DamageIntegrity(const LawParams& p, T kappa)
 {
     const T k0 = T(p.kappa0);
     if (kappa < k0)
         return T(1);
-    return k0 / kappa * (T(1) - T(p.alpha) + T(p.alpha) * exp(T(p.beta) * (k0 - kappa)));
+    return T(1) - (T(1) - k0 / kappa * (T(1) - T(p.alpha) + T(p.alpha) * exp(T(p.beta) * (k0 - kappa))));
 }
 
 // DamageLawExponential (DamageLawExponential.h:40-52)

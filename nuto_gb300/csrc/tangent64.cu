@@ -20,6 +20,7 @@
 #include "sumfac.cuh"
 
 #include <algorithm>
+#include <cfloat>
 
 namespace nuto_gpu
 {
@@ -143,7 +144,7 @@ __global__ void __launch_bounds__(Cell64<DIM, GD>::threads) k_cell_matrices64(Ce
                 {
                     const double ki = 1. / kap, ex = L.alpha * exp(L.beta * (L.kappa0 - kap));
                     const double k0i = L.kappa0 * ki;
-                    phi = k0i * ((1. - L.alpha) + ex);
+                    phi = 1. - (1. - k0i * ((1. - L.alpha) + ex)); // as DamageIntegrity
                     dom = k0i * ((ki + L.beta) * ex + (1. - L.alpha) * ki);
                 }
                 if (!loading)
@@ -331,7 +332,230 @@ __global__ void __launch_bounds__(Cell64<DIM, GD>::threads) k_cell_matrices64(Ce
     }
 }
 
+// ---- Hex20 displacement cells, 3 x 3 x 3 points, LinearElastic or LocalIsotropicDamage with FULL damage -------------------
+// One block per cell: (A) threads (point, component) the displacement gradient, then thread (point) the law; (B) the node
+// gradients times mu w and, for the points whose rank-1 part does not vanish, P = B^T (dsigma/domega omega') w and
+// Q = B^T deps_eq/deps (LocalIsotropicDamage::Tangent, nuto/mechanics/constitutive/LocalIsotropicDamage.h:59-68, 115-122);
+// (C) thread = unordered node pair: rho S + S^T + tr(S) I over all points as above, and the rank-1 sums P_a Q_b^T and
+// P_b Q_a^T over the loading points only. Undamaged, unloading points have P or Q = 0 exactly: their terms are left out (a
+// NaN is no zero). Bound by the FP64 pipe (95 % busy): 4,525 FP64 warp instructions per cell with half of the points
+// loading. 13^3: 2261 -> 607 us (the element kernel formed each ordered pair with its own lambda and mu sums and added with
+// atomics), of which the gather 38 us.
+constexpr int kH20Nd = 20, kH20Nip = 27, kH20Pairs = kH20Nd * (kH20Nd + 1) / 2, kH20Threads = 224;
+
+template <bool LD>
+struct H20Shared
+{
+    double u[kH20Nd * 3];
+    double H[kH20Nip][9];
+    double g[kH20Nip][kH20Nd * 3];  // node gradients
+    double m[kH20Nip][kH20Nd * 3];  // the same times mu w
+    double muw[kH20Nip];
+    double st[LD ? kH20Nip : 1][12]; // Voigt vectors of P and Q
+    double P[LD ? kH20Nip : 1][kH20Nd * 3], Q[LD ? kH20Nip : 1][kH20Nd * 3]; // compacted: loading points first
+    int list[kH20Nip];
+    int loading;
+};
+
+template <int KIND>
+__global__ void __launch_bounds__(kH20Threads) k_cell_matrices64_h20(CellArgs a, LawParams L, const double* __restrict__ u,
+                                                                     double* __restrict__ em)
+{
+    constexpr bool LD = KIND == NUTO_GPU_MB_LOCAL_DAMAGE;
+    constexpr int ND = kH20Nd, NIP = kH20Nip;
+    extern __shared__ __align__(16) unsigned char smRaw[];
+    H20Shared<LD>& sh = *reinterpret_cast<H20Shared<LD>*>(smRaw);
+    const int64_t n = a.nCells, e = blockIdx.x;
+    const int tid = threadIdx.x;
+    if (tid < ND)
+    {
+        const int64_t gd = a.gdofD[NG_IDX(a.connD[static_cast<int64_t>(tid) * n + e], a.nNodesD, 2)];
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+            sh.u[tid * 3 + c] = u[NG_IDX(gd + c, a.nDofs, 3)];
+    }
+    for (int it = tid; it < NIP * ND * 3; it += kH20Threads)
+    {
+        const int q = it / (ND * 3), k = it % (ND * 3);
+        sh.g[q][k] = a.geo64[NG_IDX((static_cast<int64_t>(q) * a.geoStride + 1 + k) * n + e, a.geoSize, 6)];
+    }
+    __syncthreads();
+    if (LD)
+    {
+        // in the node order of the history update (EvolutionImplicit): the loading test compares with what it stored
+        for (int it = tid; it < NIP * 3; it += kH20Threads)
+        {
+            const int q = it % NIP, c = it / NIP;
+            double h[3] = {0., 0., 0.};
+#pragma unroll 5
+            for (int nd = 0; nd < ND; ++nd)
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                    h[d] = fma(sh.u[nd * 3 + c], sh.g[q][nd * 3 + d], h[d]);
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                sh.H[q][c * 3 + d] = h[d];
+        }
+        __syncthreads();
+    }
+    if (tid < 32)
+    {
+        const int q = tid;
+        bool on = false;
+        if (q < NIP)
+        {
+            const double wdj = a.geo64[NG_IDX(static_cast<int64_t>(q) * a.geoStride * n + e, a.geoSize, 6)];
+            const double wdjE = a.escale ? wdj * a.escale[e] : wdj;
+            if (!LD)
+                sh.muw[q] = L.C33 * wdjE;
+            else
+            {
+                double H[3][3], eps[6];
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+#pragma unroll
+                    for (int d = 0; d < 3; ++d)
+                        H[c][d] = sh.H[q][c * 3 + d];
+                StrainFromH<double, 3>(H, eps);
+                const double kh = a.kappa[NG_IDX(e * NIP + q, n * NIP, 7)];
+                const double eqs = MisesValue<double, 3>(L, eps);
+                const double kap = eqs > kh ? eqs : kh;
+                double phi = 1., dom = 0.;
+                if (!(kap < L.kappa0))
+                {
+                    const double ki = 1. / kap, ex = L.alpha * exp(L.beta * (L.kappa0 - kap));
+                    const double k0i = L.kappa0 * ki;
+                    phi = 1. - (1. - k0i * ((1. - L.alpha) + ex)); // as DamageIntegrity
+                    dom = k0i * ((ki + L.beta) * ex + (1. - L.alpha) * ki);
+                }
+                sh.muw[q] = phi * L.muD * wdjE;
+                // at a converged state kappa_h is eqs itself, from the history update's own evaluation of the Mises norm, whose
+                // last bits may differ: within 4 ulps below it a point is loading
+                if (!(eqs >= kh - 4.0 * DBL_EPSILON * kh))
+                    dom = eqs == eqs && kh == kh ? 0. : dom;
+                const double tr = eps[0] + eps[1] + eps[2];
+                const double f = -dom * wdjE, t = L.lamD * tr, fm = f * L.muD;
+                double dk[6];
+                on = !(dom == 0.) || !(eqs == eqs);
+                if (on)
+                {
+                    MisesDerivative<double, 3>(L, eps, dk);
+#pragma unroll
+                    for (int v = 0; v < 6; ++v)
+                    {
+                        sh.st[q][v] = v < 3 ? f * (L.m2G * eps[v] + t) : fm * eps[v];
+                        sh.st[q][6 + v] = dk[v];
+                    }
+                }
+            }
+        }
+        const unsigned mask = __ballot_sync(0xffffffffu, on);
+        if (on)
+            sh.list[__popc(mask & ((1u << tid) - 1u))] = q;
+        if (tid == 0)
+            sh.loading = __popc(mask);
+    }
+    __syncthreads();
+    const int loading = LD ? sh.loading : 0;
+    for (int it = tid; it < NIP * ND * 3; it += kH20Threads)
+    {
+        const int q = it / (ND * 3), k = it % (ND * 3);
+        sh.m[q][k] = sh.muw[q] * sh.g[q][k];
+    }
+    if (LD)
+    {
+        for (int it = tid; it < loading * ND; it += kH20Threads)
+        {
+            const int j = it / ND, nd = it % ND, q = sh.list[j];
+            const double g[3] = {sh.g[q][nd * 3], sh.g[q][nd * 3 + 1], sh.g[q][nd * 3 + 2]};
+            BtS<double, 3>(g, sh.st[q], &sh.P[j][nd * 3]);
+            BtS<double, 3>(g, sh.st[q] + 6, &sh.Q[j][nd * 3]);
+        }
+    }
+    __syncthreads();
+    if (tid >= kH20Pairs)
+        return;
+    int ia, ib;
+    UnorderedPair<ND>(tid, ia, ib);
+    double s[3][3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int l = 0; l < 3; ++l)
+            s[k][l] = 0.;
+#pragma unroll 3
+    for (int q = 0; q < NIP; ++q)
+    {
+        const double* m = &sh.m[q][ia * 3];
+        const double* g = &sh.g[q][ib * 3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int l = 0; l < 3; ++l)
+                s[k][l] += m[k] * g[l];
+    }
+    const double mu0 = LD ? L.muD : L.C33;
+    const double rho = mu0 != 0. ? (LD ? L.lamD : L.C12) / mu0 : 0.;
+    const double tr = s[0][0] + s[1][1] + s[2][2];
+    double ab[3][3], ba[3][3]; // the blocks (a, b) and (b, a)
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int l = 0; l < 3; ++l)
+            ab[k][l] = ba[l][k] = rho * s[k][l] + (k == l ? s[l][k] + tr : s[l][k]);
+    if (LD)
+    {
+#pragma unroll 2
+        for (int j = 0; j < loading; ++j)
+        {
+            const double *pa = &sh.P[j][ia * 3], *pb = &sh.P[j][ib * 3], *qa = &sh.Q[j][ia * 3], *qb = &sh.Q[j][ib * 3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+#pragma unroll
+                for (int l = 0; l < 3; ++l)
+                {
+                    ab[k][l] += pa[k] * qb[l];
+                    ba[k][l] += pb[k] * qa[l];
+                }
+        }
+    }
+    double* rowA = em + (NG_IDX(e, n, 84) * ND + ia) * (9 * ND) + ib * 3;
+    double* rowB = em + (e * ND + ib) * (9 * ND) + ia * 3;
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int l = 0; l < 3; ++l)
+        {
+            rowA[k * 3 * ND + l] = ab[k][l];
+            if (ia != ib)
+                rowB[k * 3 * ND + l] = ba[k][l];
+        }
+}
+
 } // namespace
+
+bool LaunchTangent64H20(Ctx& c, const double* u, double* vals)
+{
+    const bool ld = c.prm.kind == NUTO_GPU_MB_LOCAL_DAMAGE;
+    const CellArgs a = CellArgsOf(c);
+    double* em = reinterpret_cast<double*>(
+            ElemMatsOrNull(c, static_cast<size_t>(c.nCells) * kH20Nd * 9 * kH20Nd * sizeof(double)));
+    if (!em)
+        return false;
+    const RowPlanArgs P = EnsureRowPlan(c);
+    auto run = [&](auto kern, size_t smem) {
+        NG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        kern<<<static_cast<unsigned>(c.nCells), kH20Threads, smem, c.stream>>>(a, c.law, u, em);
+    };
+    if (ld)
+        run(k_cell_matrices64_h20<NUTO_GPU_MB_LOCAL_DAMAGE>, sizeof(H20Shared<true>));
+    else
+        run(k_cell_matrices64_h20<NUTO_GPU_MB_LINEAR_ELASTIC>, sizeof(H20Shared<false>));
+    AfterLaunch(c, "k_cell_matrices64_h20");
+    c.stats.kernel_launches += 1;
+    LaunchWideRows<double, kH20Nd>(c, P, c.slots[c.prm.disp_slot].nNodes, em, vals);
+    return true;
+}
 
 bool LaunchTangent64(Ctx& c, const double* u, double* vals)
 {
@@ -478,6 +702,8 @@ RowPlanArgs EnsureRowPlan(Ctx& c)
         const unsigned blocks = static_cast<unsigned>((entries * D.nen + 255) / 256);
         if (D.nen == 4)
             k_row_entries<4><<<blocks, 256, 0, c.stream>>>(A, entries, c.dRowSlab.p, c.dPackedRanks.p, differ.p);
+        else if (D.nen == 20)
+            k_row_entries<20><<<blocks, 256, 0, c.stream>>>(A, entries, c.dRowSlab.p, c.dPackedRanks.p, differ.p);
         else
             k_row_entries<8><<<blocks, 256, 0, c.stream>>>(A, entries, c.dRowSlab.p, c.dPackedRanks.p, differ.p);
         AfterLaunch(c, "k_row_entries");

@@ -22,14 +22,13 @@
 //                   element matrix [a][i][b][j]. With split 3 every operand is the sum of two TF32 numbers
 //                   (hi = round(x), lo = round(x - hi)) and D accumulates lo.hi + hi.lo + hi.hi: about FP32
 //                   accuracy (the dropped lo.lo term is 2^-22 relative); split 1 keeps hi.hi only.
-//   k_tc20_rows     one warp per displacement node adds its rows of the element matrices over the node's cells in
-//                   ascending order into shared rows at the ranks of b and stores the CSR rows once (no atomics:
-//                   bitwise reproducible).
+//   k_rows_from_wide_slabs (rows.cuh)  one warp per displacement node adds its rows of the element matrices over the
+//                   node's cells in ascending order (no atomics: bitwise reproducible).
 // The tensor-memory accumulator is double-buffered (2 x 64 columns): the MMAs of one cell run while the epilogue of
 // the previous cell reads its accumulator. The only wait is on the MMA completion barrier; it is bounded by the
 // context's spin limit and, when it gives up, sets NUTO_GPU_ETIMEOUT in the status word, waits once more (bounded)
 // for the MMAs in flight, frees the tensor memory and returns.
-#include "internal.cuh"
+#include "rows.cuh"
 
 #include <algorithm>
 #include <cfloat>
@@ -45,7 +44,6 @@ namespace
 constexpr int kNd = 20, kNg = 8, kNip = 27;
 constexpr int kRecF4 = 6;          // float4 per point record
 constexpr int kTcThreads = 512;    // 16 warps: 4 per tensor-memory lane quarter
-constexpr int kRowCapTc = 256;     // values per CSR row buffer (81 neighbour nodes x 3 in the interior)
 // shared memory of k_tangent_tc20 (bytes)
 constexpr int kOpAHi = 0, kOpALo = 32768, kOpBHi = 65536, kOpBLo = 81920, kOpEnd = 98304;
 constexpr int kRecOff = kOpEnd;                                // 2 x 27 x 6 float4: this cell's records, the next's
@@ -75,18 +73,6 @@ struct Tc20Args
     const double* tabDNg;  // [q][8][3]
     const double* tabDNd;  // [q][20][3]
     const double* tabW;    // [q]
-};
-
-struct Tc20RowArgs
-{
-    int64_t nNodes, nCells, nnz, nRows;
-    const int64_t* gdofD;
-    const int64_t* cellPtr;
-    const int32_t* cellIdx;
-    const uint8_t* cellLoc;
-    const int64_t* rowPtr;
-    const uint8_t* rank; // UU ranks, [(loc * 20 + b)][cell]
-    const int32_t* blk;
 };
 
 // ---- tcgen05 / mbarrier wrappers (inline PTX, sm_100-class tensor cores) --------------------------------------
@@ -211,204 +197,209 @@ __global__ void __launch_bounds__(128) k_tc20_points(Tc20Args A, LawParams L, co
     __shared__ float sW[kNip];
     __shared__ float sX[CPB][kNg][3];
     __shared__ double sU[CPB][kNd][3];
+    __shared__ float sUr[CPB][kNd][3]; // displacements relative to the cell's first node (LD), formed in FP64
     const int64_t n = A.nCells;
-    const int64_t cell0 = static_cast<int64_t>(blockIdx.x) * CPB;
     for (int i = threadIdx.x; i < kNip * kNg * 3; i += blockDim.x)
         sDNg[i] = static_cast<float>(A.tabDNg[i]);
     for (int i = threadIdx.x; i < kNip * kNd * 3; i += blockDim.x)
         sDNd[i] = static_cast<float>(A.tabDNd[i]);
     for (int i = threadIdx.x; i < kNip; i += blockDim.x)
         sW[i] = static_cast<float>(A.tabW[i]);
-    for (int it = threadIdx.x; it < CPB * kNg * 3; it += blockDim.x)
+    for (int64_t cell0 = static_cast<int64_t>(blockIdx.x) * CPB; cell0 < n; cell0 += static_cast<int64_t>(gridDim.x) * CPB)
     {
-        const int cl = it % CPB, r = it / CPB; // r = node * 3 + d
-        const int64_t e = cell0 + cl;
-        if (e < n)
-            sX[cl][r / 3][r % 3] = A.relX[static_cast<int64_t>(r) * n + e];
-    }
-    for (int it = threadIdx.x; it < CPB * kNd; it += blockDim.x)
-    {
-        const int cl = it % CPB, nd = it / CPB;
-        const int64_t e = cell0 + cl;
-        if (e >= n)
-            continue;
-        const int64_t g = A.gdofD[NG_IDX(A.connD[static_cast<int64_t>(nd) * n + e], A.nNodesD, 60)];
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-            sU[cl][nd][c] = u[NG_IDX(g + c, A.nDofs, 61)];
-    }
-    __syncthreads();
-    const int t = threadIdx.x;
-    if (t >= CPB * kNip)
-        return;
-    const int cl = t / kNip, q = t % kNip;
-    const int64_t e = cell0 + cl;
-    if (e >= n)
-        return;
-    // Jacobian J[i][j] = dx_i / dxi_j from the relative coordinates (k_geometry's formulas in FP32)
-    float J[3][3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
+        for (int it = threadIdx.x; it < CPB * kNg * 3; it += blockDim.x)
         {
-            float s = 0.f;
-#pragma unroll
-            for (int nd = 1; nd < kNg; ++nd) // node 0 sits at the origin of the relative coordinates
-                s += sX[cl][nd][i] * sDNg[(q * kNg + nd) * 3 + j];
-            J[i][j] = s;
+            const int cl = it % CPB, r = it / CPB; // r = node * 3 + d
+            const int64_t e = cell0 + cl;
+            if (e < n)
+                sX[cl][r / 3][r % 3] = A.relX[static_cast<int64_t>(r) * n + e];
         }
-    const float c00 = J[1][1] * J[2][2] - J[1][2] * J[2][1];
-    const float c10 = J[1][2] * J[2][0] - J[1][0] * J[2][2];
-    const float c20 = J[1][0] * J[2][1] - J[1][1] * J[2][0];
-    const float det = J[0][0] * c00 + J[0][1] * c10 + J[0][2] * c20;
-    const float id = 1.f / det;
-    float inv[3][3];
-    inv[0][0] = c00 * id;
-    inv[1][0] = c10 * id;
-    inv[2][0] = c20 * id;
-    inv[0][1] = (J[0][2] * J[2][1] - J[0][1] * J[2][2]) * id;
-    inv[1][1] = (J[0][0] * J[2][2] - J[0][2] * J[2][0]) * id;
-    inv[2][1] = (J[0][1] * J[2][0] - J[0][0] * J[2][1]) * id;
-    inv[0][2] = (J[0][1] * J[1][2] - J[0][2] * J[1][1]) * id;
-    inv[1][2] = (J[0][2] * J[1][0] - J[0][0] * J[1][2]) * id;
-    inv[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) * id;
-    const float wdj = sW[q] * det;
-    const float wdjE = A.escale ? wdj * static_cast<float>(A.escale[e]) : wdj;
-    float lamw, muw, sv[6], tv[6];
-#pragma unroll
-    for (int v = 0; v < 6; ++v)
-        sv[v] = tv[v] = 0.f;
-    if (!LD)
-    {
-        lamw = static_cast<float>(L.C12) * wdjE;
-        muw = static_cast<float>(L.C33) * wdjE;
-    }
-    else
-    {
-        // displacement gradient H = (sum_a u_a (x) dN_a/dxi) J^-1, and the same sums of magnitudes for the bound
-        float Hx[3][3], Ha[3][3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-            for (int j = 0; j < 3; ++j)
-                Hx[c][j] = Ha[c][j] = 0.f;
-        for (int nd = 0; nd < kNd; ++nd)
+        for (int it = threadIdx.x; it < CPB * kNd; it += blockDim.x)
         {
-            const float* dn = sDNd + (q * kNd + nd) * 3;
+            const int cl = it % CPB, nd = it / CPB;
+            const int64_t e = cell0 + cl;
+            if (e >= n)
+                continue;
+            const int64_t g = A.gdofD[NG_IDX(A.connD[static_cast<int64_t>(nd) * n + e], A.nNodesD, 60)];
 #pragma unroll
             for (int c = 0; c < 3; ++c)
-            {
-                const float uc = static_cast<float>(sU[cl][nd][c]);
-#pragma unroll
-                for (int j = 0; j < 3; ++j)
-                {
-                    Hx[c][j] += uc * dn[j];
-                    Ha[c][j] += fabsf(uc) * fabsf(dn[j]);
-                }
-            }
+                sU[cl][nd][c] = u[NG_IDX(g + c, A.nDofs, 61)];
         }
-        float H[3][3], S = 0.f;
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-            for (int k = 0; k < 3; ++k)
+        __syncthreads();
+        if (LD)
+        {
+            for (int it = threadIdx.x; it < CPB * kNd * 3; it += blockDim.x)
             {
-                float h = 0.f, ha = 0.f;
-#pragma unroll
-                for (int j = 0; j < 3; ++j)
-                {
-                    h += Hx[c][j] * inv[j][k];
-                    ha += Ha[c][j] * fabsf(inv[j][k]);
-                }
-                H[c][k] = h;
-                S += ha;
+                const int cl = it / (kNd * 3), k = it % (kNd * 3);
+                (&sUr[cl][0][0])[k] = static_cast<float>((&sU[cl][0][0])[k] - sU[cl][0][k % 3]);
             }
-        float eps[6];
-        StrainFromH<float, 3>(H, eps);
-        const double kh = A.kappa[NG_IDX(e * kNip + q, n * kNip, 62)];
-        const float khf = static_cast<float>(kh), k0f = static_cast<float>(L.kappa0);
-        const float eqs = MisesValue<float, 3>(L, eps);
-        // the FP32 strain differs from k_residual's FP64 strain by well below 1e-5 S (S bounds the magnitudes that
-        // enter H); eq. strain's slope in the strain is below 10, so a margin of 1e-4 S separates both decisions
-        const float bound = 1.0e-4f * S + 1.0e-30f;
-        const float kapf = eqs > khf ? eqs : khf;
-        const bool near = lawFp64 || fabsf(eqs - khf) <= bound + 1.0e-6f * khf ||
-                          fabsf(kapf - k0f) <= bound + 1.0e-6f * k0f;
-        if (!near)
-        {
-            const float omega = DamageOmega<float>(L, kapf);
-            float lam, mu;
-            LedTangentLameParams<float, 3>(L, eps, omega, lam, mu);
-            lamw = lam * wdjE;
-            muw = mu * wdjE;
-            float dsdw[6];
-            LedDstressDomega<float, 3>(L, eps, dsdw);
-            const float dOdK = DamageDerivative<float>(L, kapf);
-            if (eqs >= khf)
-                MisesDerivative<float, 3>(L, eps, tv);
-#pragma unroll
-            for (int v = 0; v < 6; ++v)
-                sv[v] = dsdw[v] * dOdK * wdjE;
+            __syncthreads();
         }
-        else
+        const int cl = threadIdx.x / kNip, q = threadIdx.x % kNip;
+        const int64_t e = cell0 + cl;
+        if (threadIdx.x < CPB * kNip && e < n)
         {
-            // the FP64 strain of k_residual (geometry cache, same order of the sums) and the law in FP64
-            const double* G = A.geo64 + NG_IDX(static_cast<int64_t>(q) * A.geoStride * n + e, A.geoSize, 63);
-            double H64[3][3];
+            // Jacobian J[i][j] = dx_i / dxi_j from the relative coordinates (k_geometry's formulas in FP32)
+            float J[3][3];
 #pragma unroll
             for (int i = 0; i < 3; ++i)
 #pragma unroll
                 for (int j = 0; j < 3; ++j)
-                    H64[i][j] = 0.;
-            for (int nd = 0; nd < kNd; ++nd)
-            {
-                double g[3];
+                {
+                    float s = 0.f;
 #pragma unroll
-                for (int d = 0; d < 3; ++d)
-                    g[d] = G[(1 + nd * 3 + d) * n];
+                    for (int nd = 1; nd < kNg; ++nd) // node 0 sits at the origin of the relative coordinates
+                        s += sX[cl][nd][i] * sDNg[(q * kNg + nd) * 3 + j];
+                    J[i][j] = s;
+                }
+            const float c00 = J[1][1] * J[2][2] - J[1][2] * J[2][1];
+            const float c10 = J[1][2] * J[2][0] - J[1][0] * J[2][2];
+            const float c20 = J[1][0] * J[2][1] - J[1][1] * J[2][0];
+            const float det = J[0][0] * c00 + J[0][1] * c10 + J[0][2] * c20;
+            const float id = 1.f / det;
+            float inv[3][3];
+            inv[0][0] = c00 * id;
+            inv[1][0] = c10 * id;
+            inv[2][0] = c20 * id;
+            inv[0][1] = (J[0][2] * J[2][1] - J[0][1] * J[2][2]) * id;
+            inv[1][1] = (J[0][0] * J[2][2] - J[0][2] * J[2][0]) * id;
+            inv[2][1] = (J[0][1] * J[2][0] - J[0][0] * J[2][1]) * id;
+            inv[0][2] = (J[0][1] * J[1][2] - J[0][2] * J[1][1]) * id;
+            inv[1][2] = (J[0][2] * J[1][0] - J[0][0] * J[1][2]) * id;
+            inv[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) * id;
+            const float wdj = sW[q] * det;
+            const float wdjE = A.escale ? wdj * static_cast<float>(A.escale[e]) : wdj;
+            float lamw, muw, sv[6], tv[6];
+#pragma unroll
+            for (int v = 0; v < 6; ++v)
+                sv[v] = tv[v] = 0.f;
+            if (!LD)
+            {
+                lamw = static_cast<float>(L.C12) * wdjE;
+                muw = static_cast<float>(L.C33) * wdjE;
+            }
+            else
+            {
+                // displacement gradient H = (sum_a u_a (x) dN_a/dxi) J^-1, and the same sums of magnitudes for the bound
+                float Hx[3][3], Ha[3][3];
 #pragma unroll
                 for (int c = 0; c < 3; ++c)
 #pragma unroll
-                    for (int d = 0; d < 3; ++d)
-                        H64[c][d] += sU[cl][nd][c] * g[d];
-            }
-            double e64[6];
-            StrainFromH<double, 3>(H64, e64);
-            const double eq64 = MisesValue<double, 3>(L, e64);
-            const double kap = eq64 > kh ? eq64 : kh;
-            const double omega = DamageOmega<double>(L, kap);
-            double lam, mu, dsdw[6], dk[6];
-            LedTangentLameParams<double, 3>(L, e64, omega, lam, mu);
-            lamw = static_cast<float>(lam) * wdjE;
-            muw = static_cast<float>(mu) * wdjE;
-            LedDstressDomega<double, 3>(L, e64, dsdw);
-            const double dOdK = DamageDerivative<double>(L, kap);
-            // loading (EvolutionImplicit: eq >= kappa_h). At a converged state kappa_h is eq itself, written by
-            // k_history; this kernel's FP64 eq equals it mathematically but may differ in the last bits (the compiler
-            // contracts the sums of squares of the Mises norm into FMAs differently per kernel), so a point within 4
-            // ulps below kappa_h is loading, as it is in the kernels whose arithmetic matches k_history's bit for bit
-            if (eq64 >= kh - 4.0 * DBL_EPSILON * kh)
-                MisesDerivative<double, 3>(L, e64, dk);
-            else
+                    for (int j = 0; j < 3; ++j)
+                        Hx[c][j] = Ha[c][j] = 0.f;
+                for (int nd = 0; nd < kNd; ++nd)
+                {
+                    const float* dn = sDNd + (q * kNd + nd) * 3;
+#pragma unroll
+                    for (int c = 0; c < 3; ++c)
+                    {
+                        const float uc = sUr[cl][nd][c];
+#pragma unroll
+                        for (int j = 0; j < 3; ++j)
+                        {
+                            Hx[c][j] += uc * dn[j];
+                            Ha[c][j] += fabsf(uc) * fabsf(dn[j]);
+                        }
+                    }
+                }
+                float H[3][3], S = 0.f;
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+#pragma unroll
+                    for (int k = 0; k < 3; ++k)
+                    {
+                        float h = 0.f, ha = 0.f;
+#pragma unroll
+                        for (int j = 0; j < 3; ++j)
+                        {
+                            h += Hx[c][j] * inv[j][k];
+                            ha += Ha[c][j] * fabsf(inv[j][k]);
+                        }
+                        H[c][k] = h;
+                        S += ha;
+                    }
+                float eps[6];
+                StrainFromH<float, 3>(H, eps);
+                const double kh = A.kappa[NG_IDX(e * kNip + q, n * kNip, 62)];
+                const float khf = static_cast<float>(kh), k0f = static_cast<float>(L.kappa0);
+                const float eqs = MisesValue<float, 3>(L, eps);
+                // the FP32 strain differs from k_residual's FP64 strain by well below 1e-5 S (S bounds the magnitudes that
+                // enter H); eq. strain's slope in the strain is below 10, so a margin of 1e-4 S separates both decisions.
+                // S is formed with displacements relative to the cell: with absolute ones nearly every warp had a point
+                // inside the margin and took the FP64 strain (265 us at 24^3 against 177 us).
+                const float bound = 1.0e-4f * S + 1.0e-30f;
+                const float kapf = eqs > khf ? eqs : khf;
+                const bool near = lawFp64 || !(fabsf(eqs - khf) > bound + 1.0e-6f * khf) ||
+                                  !(fabsf(kapf - k0f) > bound + 1.0e-6f * k0f);
+                double e64[6];
 #pragma unroll
                 for (int v = 0; v < 6; ++v)
-                    dk[v] = 0.;
+                    e64[v] = static_cast<double>(eps[v]);
+                if (near)
+                {
+                    // the FP64 strain of k_residual (geometry cache, same order of the sums)
+                    const double* G = A.geo64 + NG_IDX(static_cast<int64_t>(q) * A.geoStride * n + e, A.geoSize, 63);
+                    double H64[3][3];
 #pragma unroll
-            for (int v = 0; v < 6; ++v)
-            {
-                sv[v] = static_cast<float>(dsdw[v] * dOdK) * wdjE;
-                tv[v] = static_cast<float>(dk[v]);
+                    for (int i = 0; i < 3; ++i)
+#pragma unroll
+                        for (int j = 0; j < 3; ++j)
+                            H64[i][j] = 0.;
+                    for (int nd = 0; nd < kNd; ++nd)
+                    {
+                        double g[3];
+#pragma unroll
+                        for (int d = 0; d < 3; ++d)
+                            g[d] = G[(1 + nd * 3 + d) * n];
+#pragma unroll
+                        for (int c = 0; c < 3; ++c)
+#pragma unroll
+                            for (int d = 0; d < 3; ++d)
+                                H64[c][d] += sU[cl][nd][c] * g[d];
+                    }
+                    StrainFromH<double, 3>(H64, e64);
+                }
+                // the law in FP64 (FP32 loses up to 4e-6 of the rank-1 part where K1 I1 + sqrt(...) cancels)
+                const double eq64 = MisesValue<double, 3>(L, e64);
+                const double kap = eq64 > kh ? eq64 : kh;
+                double phi = 1., dom = 0.;
+                if (!(kap < L.kappa0))
+                {
+                    const double ki = 1. / kap, ex = L.alpha * exp(L.beta * (L.kappa0 - kap));
+                    const double k0i = L.kappa0 * ki;
+                    phi = 1. - (1. - k0i * ((1. - L.alpha) + ex));
+                    dom = k0i * ((ki + L.beta) * ex + (1. - L.alpha) * ki);
+                }
+                lamw = static_cast<float>(phi * L.lamD) * wdjE;
+                muw = static_cast<float>(phi * L.muD) * wdjE;
+                const double tr = e64[0] + e64[1] + e64[2];
+                const double f = -dom, t = L.lamD * tr, fm = f * L.muD;
+#pragma unroll
+                for (int v = 0; v < 6; ++v)
+                    sv[v] = static_cast<float>(v < 3 ? f * (L.m2G * e64[v] + t) : fm * e64[v]) * wdjE;
+                // loading (EvolutionImplicit: eq >= kappa_h). At a converged state kappa_h is eq itself, written by
+                // k_history; this kernel's FP64 eq equals it mathematically but may differ in the last bits (the compiler
+                // contracts the sums of squares of the Mises norm into FMAs differently per kernel), so a point within 4
+                // ulps below kappa_h is loading, as it is in the kernels whose arithmetic matches k_history's bit for bit
+                if (eq64 >= kh - 4.0 * DBL_EPSILON * kh)
+                {
+                    double dk[6];
+                    MisesDerivative<double, 3>(L, e64, dk);
+#pragma unroll
+                    for (int v = 0; v < 6; ++v)
+                        tv[v] = static_cast<float>(dk[v]);
+                }
             }
+            float4* R = recs + (e * kNip + q) * kRecF4;
+            R[0] = make_float4(inv[0][0], inv[0][1], inv[0][2], inv[1][0]);
+            R[1] = make_float4(inv[1][1], inv[1][2], inv[2][0], inv[2][1]);
+            R[2] = make_float4(inv[2][2], lamw, muw, 0.f);
+            R[3] = make_float4(sv[0], sv[1], sv[2], sv[3]);
+            R[4] = make_float4(sv[4], sv[5], tv[0], tv[1]);
+            R[5] = make_float4(tv[2], tv[3], tv[4], tv[5]);
         }
+        __syncthreads(); // the next pass overwrites the node data
     }
-    float4* R = recs + (e * kNip + q) * kRecF4;
-    R[0] = make_float4(inv[0][0], inv[0][1], inv[0][2], inv[1][0]);
-    R[1] = make_float4(inv[1][1], inv[1][2], inv[2][0], inv[2][1]);
-    R[2] = make_float4(inv[2][2], lamw, muw, 0.f);
-    R[3] = make_float4(sv[0], sv[1], sv[2], sv[3]);
-    R[4] = make_float4(sv[4], sv[5], tv[0], tv[1]);
-    R[5] = make_float4(tv[2], tv[3], tv[4], tv[5]);
 }
 
 // ---- element matrices on the tensor cores ----------------------------------------------------------------------
@@ -646,66 +637,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tangent_tc20(int64_t nCells, 
     }
 }
 
-// ---- CSR rows from the element matrices ------------------------------------------------------------------------
-
-__global__ void __launch_bounds__(128) k_tc20_rows(Tc20RowArgs r, const float* __restrict__ em,
-                                                   float* __restrict__ vals)
-{
-    __shared__ float sRow[4][3][kRowCapTc];
-    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t a = static_cast<int64_t>(blockIdx.x) * 4 + wid;
-    if (a >= r.nNodes)
-        return; // the whole warp leaves; only warp-level synchronisation follows
-    float(*row)[kRowCapTc] = sRow[wid];
-    int64_t rs[3];
-    int len[3];
-    const int64_t g = r.gdofD[a];
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-    {
-        rs[k] = r.rowPtr[NG_IDX(g + k, r.nRows, 64)];
-        len[k] = static_cast<int>(r.rowPtr[g + k + 1] - rs[k]);
-        for (int i = lane; i < len[k]; i += 32)
-            row[k][i] = 0.f;
-    }
-    const int32_t bUU = r.blk[a];
-    __syncwarp();
-    const int64_t k0 = r.cellPtr[a], k1 = r.cellPtr[a + 1];
-    for (int64_t kc = k0; kc < k1; ++kc)
-    {
-        const int64_t e = r.cellIdx[kc];
-        const int ia = r.cellLoc[kc];
-        const int rk = lane < kNd ? r.rank[(static_cast<int64_t>(ia) * kNd + lane) * r.nCells + e] : 0;
-        const float* src = em + NG_IDX((e * kNd + ia) * 180, r.nCells * kNd * 180, 65);
-#pragma unroll
-        for (int m = 0; m < 6; ++m)
-        {
-            const int t = lane + 32 * m; // item (row i, neighbour b, column j) of a's 180 values in this cell
-            const int tc = t < 180 ? t : 179;
-            const int i = tc / 60, b = (tc % 60) / 3, j = tc % 3;
-            const int rb = __shfl_sync(0xffffffffu, rk, b);
-            if (t < 180)
-                row[i][NG_IDX(bUU + 3 * rb + j, kRowCapTc, 66)] += src[t];
-        }
-        __syncwarp();
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-        for (int i = lane; i < len[k]; i += 32)
-            vals[NG_IDX(rs[k] + i, r.nnz, 67)] = row[k][i];
-}
-
 } // namespace
 
 // Hex20 displacement cells on a Hex8 coordinate mesh with 3x3x3 Gauss points, LinearElastic or LocalIsotropicDamage
-// with FULL damage application (UNILATERAL switches on the sign of the volumetric strain, a branch FP32 cannot
-// decide like FP64 near zero), every CSR row within the row buffer.
-bool Tc20TangentSupported(Ctx& c)
+// with FULL damage application (UNILATERAL switches on the sign of the volumetric strain: no constant ratio of the Lame
+// parameters, and a branch FP32 cannot decide like FP64 near zero), every CSR row within the row buffer.
+bool Hex20RowsSupported(Ctx& c)
 {
-    if (c.tc20Mode >= 0)
-        return c.tc20Mode == 1;
-    c.tc20Mode = 0;
-    if (c.forceTc20Off || c.slots.size() != 1)
+    if (c.h20Mode >= 0)
+        return c.h20Mode == 1;
+    c.h20Mode = 0;
+    if (c.slots.size() != 1)
         return false;
     const Slot& D = c.slots[c.prm.disp_slot];
     const bool cells = c.dim == 3 && c.nge == 8 && D.nen == kNd && D.ncomp == 3 && c.ip.nIp == kNip;
@@ -717,11 +659,18 @@ bool Tc20TangentSupported(Ctx& c)
         for (int k = 0; k < 3; ++k)
         {
             const int64_t rr = D.offset + D.dof0[i] + k;
-            if (c.hRowPtr[rr + 1] - c.hRowPtr[rr] > kRowCapTc)
+            if (c.hRowPtr[rr + 1] - c.hRowPtr[rr] > kRowsCapWide)
                 return false;
         }
-    c.tc20Mode = 1;
+    c.h20Mode = 1;
     return true;
+}
+
+bool Tc20TangentSupported(Ctx& c)
+{
+    if (c.tc20Mode < 0)
+        c.tc20Mode = !c.forceTc20Off && Hex20RowsSupported(c) ? 1 : 0;
+    return c.tc20Mode == 1;
 }
 
 void LaunchTangentTc20(Ctx& c, const double* u, float* vals)
@@ -762,7 +711,8 @@ void LaunchTangentTc20(Ctx& c, const double* u, float* vals)
     A.tabDNg = c.dTables.p + c.tabDN[c.geoInterp];
     A.tabDNd = c.dTables.p + c.tabDN[D.interp];
     A.tabW = c.dTables.p + c.tabW;
-    const unsigned pb = static_cast<unsigned>((n + 3) / 4);
+    // resident blocks that walk the cells: the shape tables are converted once per block
+    const unsigned pb = static_cast<unsigned>(std::min<int64_t>((n + 3) / 4, 8LL * std::max(c.smCount, 1)));
     if (ld)
         k_tc20_points<NUTO_GPU_MB_LOCAL_DAMAGE><<<pb, 128, 0, c.stream>>>(A, c.law, u, recs, c.tc20LawFp64);
     else
@@ -790,22 +740,8 @@ void LaunchTangentTc20(Ctx& c, const double* u, float* vals)
     }
     AfterLaunch(c, "k_tangent_tc20");
 
-    Tc20RowArgs r{};
-    r.nNodes = D.nNodes;
-    r.nCells = n;
-    r.nnz = c.nnz;
-    r.nRows = c.nDofs;
-    r.gdofD = D.dGdof.p;
-    r.cellPtr = D.dCellPtr.p;
-    r.cellIdx = D.dCellIdx.p;
-    r.cellLoc = D.dCellLoc.p;
-    r.rowPtr = c.dRowPtr.p;
-    const int p = c.prm.disp_slot * static_cast<int>(c.slots.size()) + c.prm.disp_slot;
-    r.rank = c.pairs[p].rank;
-    r.blk = c.pairs[p].dBlk.p;
-    k_tc20_rows<<<static_cast<unsigned>((D.nNodes + 3) / 4), 128, 0, c.stream>>>(r, em, vals);
-    AfterLaunch(c, "k_tc20_rows");
-    c.stats.kernel_launches += 3;
+    LaunchWideRows<float, kNd>(c, EnsureRowPlan(c), D.nNodes, em, vals);
+    c.stats.kernel_launches += 2;
 }
 
 int ReadDeviceStatus(Ctx& c)
