@@ -50,6 +50,24 @@ static void DispatchCfg(const Ctx& c, F&& f)
     throw Error{NUTO_GPU_EINVAL, "unsupported cell configuration (interpolation / integration points / integrand)"};
 }
 
+// Calls f(dimension, kind) (integral constants) for a configuration of sumfac.cuh.
+template <typename F>
+static void DispatchTwoPoint(const Ctx& c, F&& f)
+{
+    auto kinds = [&](auto dim) {
+        if (c.prm.kind == NUTO_GPU_GRADIENT_DAMAGE)
+            f(dim, std::integral_constant<int, NUTO_GPU_GRADIENT_DAMAGE>{});
+        else if (c.prm.kind == NUTO_GPU_MB_LOCAL_DAMAGE)
+            f(dim, std::integral_constant<int, NUTO_GPU_MB_LOCAL_DAMAGE>{});
+        else
+            f(dim, std::integral_constant<int, NUTO_GPU_MB_LINEAR_ELASTIC>{});
+    };
+    if (c.dim == 2)
+        kinds(std::integral_constant<int, 2>{});
+    else
+        kinds(std::integral_constant<int, 3>{});
+}
+
 // ---- small device helpers -------------------------------------------------------------------------------
 
 // LinearElastic stress sigma = C eps (LinearElastic.h:21-24, CalculateC :47-121)
@@ -694,18 +712,7 @@ void LaunchResidual(Ctx& c, const double* u, double* f, int blocksPerSm)
                 k_residual_sf<DIM, KIND, BIG>
                         <<<grid(BIG * W, 4 * blocksPerSm), 32 * W, 0, c.stream>>>(a, c.law, u, c.dCellVec.p);
         };
-        auto kinds = [&](auto dim) {
-            if (gd)
-                run(dim, std::integral_constant<int, NUTO_GPU_GRADIENT_DAMAGE>{});
-            else if (c.prm.kind == NUTO_GPU_MB_LOCAL_DAMAGE)
-                run(dim, std::integral_constant<int, NUTO_GPU_MB_LOCAL_DAMAGE>{});
-            else
-                run(dim, std::integral_constant<int, NUTO_GPU_MB_LINEAR_ELASTIC>{});
-        };
-        if (c.dim == 2)
-            kinds(std::integral_constant<int, 2>{});
-        else
-            kinds(std::integral_constant<int, 3>{});
+        DispatchTwoPoint(c, run);
         AfterLaunch(c, "k_residual_sf");
     }
     else
@@ -1792,7 +1799,8 @@ void LaunchExternalLoad(Ctx& c, const BoundaryGroup& B, const double* p, double*
 // One thread per (cell, point): strain from the cached FP64 geometry, kappa = max(kappa_h, eeq or eps_eq)
 // (GradientDamage::Kappa, GradientDamage.h:127-130; EvolutionImplicit), omega(kappa), the law's stress.
 // out[(cell * NIP + q) * width + r].
-template <int DIM, int ND, int NIP, int KIND>
+// STRAIN = false: the quantities of gradient damage that need the nonlocal eeq only
+template <int DIM, int ND, int NIP, int KIND, bool STRAIN>
 __global__ void __launch_bounds__(128) k_eval_ip(CellArgs a, LawParams L, const double* __restrict__ u, int quantity,
                                                  double* __restrict__ out)
 {
@@ -1803,27 +1811,30 @@ __global__ void __launch_bounds__(128) k_eval_ip(CellArgs a, LawParams L, const 
         return;
     const int64_t e = it / NIP;
     const int q = static_cast<int>(it % NIP);
-    const double* G = a.geo64 + NG_IDX(static_cast<int64_t>(q) * a.geoStride * n + e, a.geoSize, 6);
-    double H[DIM][DIM];
-#pragma unroll
-    for (int i = 0; i < DIM; ++i)
-#pragma unroll
-        for (int j = 0; j < DIM; ++j)
-            H[i][j] = 0;
-    for (int nd = 0; nd < ND; ++nd)
-    {
-        const int64_t g = a.gdofD[NG_IDX(a.connD[static_cast<int64_t>(nd) * n + e], a.nNodesD, 2)];
-#pragma unroll
-        for (int c = 0; c < DIM; ++c)
-        {
-            const double uc = u[NG_IDX(g + c, a.nDofs, 3)];
-#pragma unroll
-            for (int d = 0; d < DIM; ++d)
-                H[c][d] += uc * G[(1 + nd * DIM + d) * n];
-        }
-    }
     double eps[VD];
-    StrainFromH<double, DIM>(H, eps);
+    if constexpr (STRAIN)
+    {
+        const double* G = a.geo64 + NG_IDX(static_cast<int64_t>(q) * a.geoStride * n + e, a.geoSize, 6);
+        double H[DIM][DIM];
+#pragma unroll
+        for (int i = 0; i < DIM; ++i)
+#pragma unroll
+            for (int j = 0; j < DIM; ++j)
+                H[i][j] = 0;
+        for (int nd = 0; nd < ND; ++nd)
+        {
+            const int64_t g = a.gdofD[NG_IDX(a.connD[static_cast<int64_t>(nd) * n + e], a.nNodesD, 2)];
+#pragma unroll
+            for (int c = 0; c < DIM; ++c)
+            {
+                const double uc = u[NG_IDX(g + c, a.nDofs, 3)];
+#pragma unroll
+                for (int d = 0; d < DIM; ++d)
+                    H[c][d] += uc * G[(1 + nd * DIM + d) * n];
+            }
+        }
+        StrainFromH<double, DIM>(H, eps);
+    }
     double eqs = 0;
     if (KIND == NUTO_GPU_GRADIENT_DAMAGE)
     {
@@ -1831,7 +1842,7 @@ __global__ void __launch_bounds__(128) k_eval_ip(CellArgs a, LawParams L, const 
             eqs += a.tabN_D[q * ND + nd] *
                    u[NG_IDX(a.gdofE[NG_IDX(a.connE[static_cast<int64_t>(nd) * n + e], a.nNodesE, 4)], a.nDofs, 5)];
     }
-    else if (KIND == NUTO_GPU_MB_LOCAL_DAMAGE)
+    else if (STRAIN && KIND == NUTO_GPU_MB_LOCAL_DAMAGE)
         eqs = MisesValue<double, DIM>(L, eps);
     const double kh = a.kappa[NG_IDX(e * NIP + q, n * NIP, 7)];
     const double kap = KIND == NUTO_GPU_MB_LINEAR_ELASTIC ? 0. : fmax(kh, eqs);
@@ -1843,7 +1854,9 @@ __global__ void __launch_bounds__(128) k_eval_ip(CellArgs a, LawParams L, const 
     else if (quantity == NUTO_GPU_IP_DAMAGE)
         o[0] = omega;
     else if (quantity == NUTO_GPU_IP_EEQ)
-        o[0] = KIND == NUTO_GPU_MB_LINEAR_ELASTIC ? MisesValue<double, DIM>(L, eps) : eqs;
+        o[0] = STRAIN && KIND == NUTO_GPU_MB_LINEAR_ELASTIC ? MisesValue<double, DIM>(L, eps) : eqs;
+    else if (!STRAIN)
+        return;
     else if (quantity == NUTO_GPU_IP_STRAIN)
     {
 #pragma unroll
@@ -1864,6 +1877,102 @@ __global__ void __launch_bounds__(128) k_eval_ip(CellArgs a, LawParams L, const 
     }
 }
 
+// Strain or stress of Quad4 / Hex8 cells with the two-point rule: phases 1 and 2 of k_residual_sf (a warp per CPB cells), the
+// values of a warp's cells, consecutive in the output, leave through shared memory. Bound by the FP64 pipe.
+template <int DIM, int KIND, bool STRESS>
+__global__ void __launch_bounds__(32, 20) k_eval_sf(CellArgs a, LawParams L, const double* __restrict__ u,
+                                                    double* __restrict__ out)
+{
+    using S = SumFac<DIM>;
+    constexpr bool GD = KIND == NUTO_GPU_GRADIENT_DAMAGE && STRESS; // the strain does not need eeq
+    constexpr int VD = DIM == 2 ? 3 : 6, ND = S::nd, NIP = S::nd, NF = DIM + (GD ? 1 : 0), CPB = DIM == 3 ? 8 : 16;
+    __shared__ double sG[NF][S::ng][CPB];
+    __shared__ double sV[GD ? NIP : 1][CPB];
+    constexpr int CELL = NIP * VD; // a cell's values, padded by one: its lanes' banks differ from the next cell's
+    __shared__ double sOut[CPB * (CELL + 1)];
+    const int64_t n = a.nCells;
+    const int64_t cell0 = static_cast<int64_t>(blockIdx.x) * CPB;
+    const int lane = threadIdx.x;
+    for (int it = lane; it < CPB * NF; it += 32)
+    {
+        const int cl = it % CPB, fl = it / CPB;
+        const int64_t e = cell0 + cl;
+        if (e >= n)
+            continue;
+        const bool eq = GD && fl == DIM;
+        const int32_t* conn = eq ? a.connE : a.connD;
+        const int64_t* gdof = eq ? a.gdofE : a.gdofD;
+        const int comp = eq ? 0 : fl;
+        double v[ND], g[S::ng], val[NIP];
+#pragma unroll
+        for (int nd = 0; nd < ND; ++nd)
+        {
+            const int64_t gd = gdof[NG_IDX(conn[static_cast<int64_t>(nd) * n + e], eq ? a.nNodesE : a.nNodesD, 2)];
+            v[nd] = u[NG_IDX(gd + comp, a.nDofs, 3)];
+        }
+        SfForward<double, DIM, GD>(v, g, val);
+        if (eq)
+        {
+#pragma unroll
+            for (int q = 0; q < NIP; ++q)
+                sV[q][cl] = val[q];
+        }
+#pragma unroll
+        for (int k = 0; k < S::ng; ++k)
+            sG[fl][k][cl] = g[k];
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int it = lane; it < CPB * NIP; it += 32)
+    {
+        const int cl = it % CPB, q = it / CPB;
+        const int64_t e = cell0 + cl;
+        if (e >= n)
+            continue;
+        const double* Jq = a.jac + NG_IDX(static_cast<int64_t>(q) * (1 + DIM * DIM) * n + e, a.jacSize, 6);
+        double J[DIM][DIM], G[DIM][DIM], v[VD];
+#pragma unroll
+        for (int j = 0; j < DIM; ++j)
+#pragma unroll
+            for (int d = 0; d < DIM; ++d)
+                J[j][d] = Jq[(1 + j * DIM + d) * n];
+#pragma unroll
+        for (int c = 0; c < DIM; ++c)
+#pragma unroll
+            for (int j = 0; j < DIM; ++j)
+                G[c][j] = sG[c][SfGradIndex<DIM>(j, q)][cl];
+        StrainFromNatural<double, DIM>(G, J, v);
+        if (STRESS)
+        {
+            double eps[VD];
+#pragma unroll
+            for (int r = 0; r < VD; ++r)
+                eps[r] = v[r];
+            const double se = a.escale ? a.escale[e] : 1.;
+            if (KIND == NUTO_GPU_MB_LINEAR_ELASTIC)
+            {
+                ElasticStress<double, DIM>(L, eps, v);
+#pragma unroll
+                for (int r = 0; r < VD; ++r)
+                    v[r] *= se;
+            }
+            else
+            {
+                const double kh = a.kappa[NG_IDX(e * NIP + q, n * NIP, 7)];
+                const double eqs = GD ? S::valScale * sV[GD ? q : 0][cl] : MisesNorm<double, DIM>(L, eps);
+                LedStressWeighted<double, DIM>(L, eps, DamageIntegrity<double>(L, fmax(kh, eqs)), se, v);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < VD; ++r)
+            sOut[cl * (CELL + 1) + q * VD + r] = v[r];
+    }
+    __syncwarp();
+    const int64_t cells = n - cell0 < CPB ? n - cell0 : CPB;
+    for (int i = lane; i < cells * CELL; i += 32)
+        out[NG_IDX(cell0 * CELL + i, n * CELL, 11)] = sOut[i + i / CELL];
+}
+
 int IpWidth(const Ctx& c, int quantity)
 {
     return (quantity == NUTO_GPU_IP_STRAIN || quantity == NUTO_GPU_IP_STRESS) ? (c.dim == 2 ? 3 : 6) : 1;
@@ -1874,9 +1983,28 @@ void LaunchEvalIp(Ctx& c, const double* u, int quantity, double* out)
     CellArgs a = MakeCellArgs(c);
     const int64_t items = c.nCells * c.ip.nIp;
     const int blocks = static_cast<int>((items + 127) / 128);
+    const bool strain = quantity == NUTO_GPU_IP_STRAIN || quantity == NUTO_GPU_IP_STRESS;
+    if (strain && a.jac)
+    {
+        auto run = [&](auto dim, auto kind) {
+            constexpr int DIM = decltype(dim)::value, KIND = decltype(kind)::value, CPB = DIM == 3 ? 8 : 16;
+            const unsigned grid = static_cast<unsigned>((c.nCells + CPB - 1) / CPB);
+            if (quantity == NUTO_GPU_IP_STRESS)
+                k_eval_sf<DIM, KIND, true><<<grid, 32, 0, c.stream>>>(a, c.law, u, out);
+            else
+                k_eval_sf<DIM, KIND, false><<<grid, 32, 0, c.stream>>>(a, c.law, u, out);
+        };
+        DispatchTwoPoint(c, run);
+        AfterLaunch(c, "k_eval_sf");
+        c.stats.kernel_launches += 1;
+        return;
+    }
     DispatchCfg(c, [&](auto cfg) {
         using C = decltype(cfg);
-        k_eval_ip<C::dim, C::nd, C::nip, C::kind><<<blocks, 128, 0, c.stream>>>(a, c.law, u, quantity, out);
+        if (C::kind == NUTO_GPU_GRADIENT_DAMAGE && !strain)
+            k_eval_ip<C::dim, C::nd, C::nip, C::kind, false><<<blocks, 128, 0, c.stream>>>(a, c.law, u, quantity, out);
+        else
+            k_eval_ip<C::dim, C::nd, C::nip, C::kind, true><<<blocks, 128, 0, c.stream>>>(a, c.law, u, quantity, out);
     });
     AfterLaunch(c, "k_eval_ip");
     c.stats.kernel_launches += 1;

@@ -96,3 +96,13 @@ def test_fp32_tangent_on_distorted_cells(dim, cells, law, form, monkeypatch):
     K.sort_indices()
     v = g.build_matrix(u, nuto_gb300.FP32).double().cpu().numpy()
     assert np.abs(v - K.data).max() <= 2e-6 * np.abs(K.data).max()
+
+
+@pytest.mark.parametrize("dim,cells,law", CASES)
+def test_point_values_on_distorted_cells(dim, cells, law):
+    """Strain and stress (k_eval_sf) and the scalar quantities at every integration point."""
+    g, P, u = _case(dim, cells, LAWS[law], 10)
+    for quantity in range(5):
+        ref = P.eval_ip(u, quantity)
+        v = g.eval_ip(u, quantity).cpu().numpy().reshape(ref.shape)
+        assert np.abs(v - ref).max() <= FP64_REL * np.abs(ref).max() + 1e-300, quantity
