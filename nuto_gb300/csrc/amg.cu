@@ -49,8 +49,19 @@ constexpr float kCoarseRatio = 30.f;
 template <typename TA>
 struct Num
 {
-    DBuf<TA> vals, dinv, e, b, t, d;
+    DBuf<TA> vals, dinv, e, t, d;
+    TA* b = nullptr; // coarse levels: right-hand side, a part of Amg::rhs (zeroed once per sweep)
     DBuf<TA> nb; // coarse levels: the values in the padded layout of the level's SpMV
+};
+
+// The one-block tail (k_amg_tail) as a dense matrix: its V-cycle is a fixed linear map of at most kTailNodes x 3 values,
+// applied once per sweep; column k = the cycle of unit vector k
+template <typename TA>
+struct TailDense
+{
+    DBuf<TA> m;    // [k][i]
+    DBuf<TA> work; // vectors of the tail levels, one set per column
+    int64_t n = 0;
 };
 
 struct AmgLevel
@@ -113,6 +124,11 @@ struct Amg
     std::vector<float> lmaxHost;
     DBuf<float> in32, out32, res32; // combined-length work vectors of the sweep (FP32 cycle)
     DBuf<double> in64, out64, res64; // the same for the FP64 cycle
+    DBuf<float> rhs32; // right-hand sides of all coarse levels (Num::b)
+    DBuf<double> rhs64;
+    TailDense<float> tail32[kMaxSlots];
+    TailDense<double> tail64[kMaxSlots];
+    bool tailSym = false; // the cycle the tails were formed for
     int prec = 32;                   // arithmetic of the last set-up: that of the tangent values
     const void* fine = nullptr;      // the tangent of the last set-up (level-0 operator)
     const void* setupVals = nullptr;
@@ -134,6 +150,23 @@ struct Amg
     std::string graphError; // why graphs were switched off (diagnostics)
     cudaStream_t capStream = nullptr; // private stream for graph capture (the context's may be the legacy stream)
 };
+
+template <typename TA>
+static DBuf<TA>& Rhs(Amg& M)
+{
+    if constexpr (sizeof(TA) == 4)
+        return M.rhs32;
+    else
+        return M.rhs64;
+}
+template <typename TA>
+static TailDense<TA>& Tail(Amg& M, int slot)
+{
+    if constexpr (sizeof(TA) == 4)
+        return M.tail32[slot];
+    else
+        return M.tail64[slot];
+}
 
 void FreeAmg(Ctx& c)
 {
@@ -255,20 +288,6 @@ static NodeSpmv SlotView(const Ctx& c, int I)
         A.nbSrc32 = c.nb.src32;
         A.nbSrc64 = c.nb.src64;
     }
-    return A;
-}
-
-// whole-row operator restricted to the rows of slot I (K_I0 z_0 + K_II z_I, used with z_I = 0)
-static NodeSpmv RowsView(const Ctx& c, int I)
-{
-    NodeSpmv A = MakeNodeSpmv(c);
-    if (I == 1)
-    {
-        A.firstWarp[1] = 0;
-        A.totalWarps = A.nNodes[1];
-    }
-    else
-        A.totalWarps = A.nNodes[0];
     return A;
 }
 
@@ -586,67 +605,171 @@ __device__ __forceinline__ bool Idle(const int* st)
     return st && st[ST_STATE] != RUN;
 }
 
-// first Chebyshev step from zero: d = dinv b / theta; e = d
+// first Chebyshev step from zero: e = dinv b / theta
 template <typename TA>
-__global__ void k_cheb0(int64_t n, const TA* __restrict__ dinv, const TA* __restrict__ b, TA* d, TA* e, TA invTheta,
-                        const int* st)
+__global__ void k_cheb0(int64_t n, const TA* __restrict__ dinv, const TA* __restrict__ b, TA* e, TA invTheta, const int* st)
 {
     PdlWait();
     PdlTrigger();
     const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
     if (i >= n || Idle(st))
         return;
-    const TA v = dinv[i] * b[i] * invTheta;
-    d[i] = v;
-    e[i] = v;
+    e[i] = dinv[i] * b[i] * invTheta;
 }
 
-// first Chebyshev step from a nonzero e (t = A e): d = dinv (b - t) / theta; e += d
+// One product of the cycle with what precedes and follows it, on the padded layout of one slot pair (rows of ncRow
+// components, columns of ncCol; the structure of k_spmv_nb: G lanes per node, x of the neighbours gathered into shared
+// memory, values streamed with 16-byte loads). With t = A x:
+//   GATHER  how x is formed: CG_VECTOR x = xin; CG_ZERO x = dinv b w0 (the first Chebyshev step from zero); CG_PROLONG
+//           x = xin + P ce (the coarse correction of unconstrained DOFs)
+//   EPI     CE_RESTRICT  cb += P^T (b - t) over unconstrained rows (cb is zero before; with CG_ZERO also xout = x)
+//           CE_FIRST     d = dinv (b - t) w1; xout = x + d       (first Chebyshev step from a nonzero x)
+//           CE_STEP      d = w2 d + w1 dinv (b - t); xout = x + d (later steps; with CG_ZERO the step before is x itself)
+//           CE_RESIDUAL  xout = b - t (constrained rows: b)
+// xin and xout differ (other rows still gather xin). At the sizes of the coarse levels a launch is what costs: a level takes
+// 3 launches instead of 9, and the sweep of a 20^3 beam 25 instead of 92. On large levels CG_ZERO and CG_PROLONG would put
+// more loads behind every neighbour of a product that waits for exactly those, and run as their own kernels (kFuseNodes).
+enum CycleGather
+{
+    CG_VECTOR,
+    CG_ZERO,
+    CG_PROLONG
+};
+enum CycleEpilogue
+{
+    CE_RESTRICT,
+    CE_FIRST,
+    CE_STEP,
+    CE_RESIDUAL
+};
+constexpr int64_t kFuseNodes = 40000;
+
 template <typename TA>
-__global__ void k_cheb1(int64_t n, const TA* __restrict__ dinv, const TA* __restrict__ b, const TA* __restrict__ t,
-                        TA* d, TA* e, TA invTheta, const int* st)
+struct CycleArgs
+{
+    int64_t nNodes, nRows, nbrTotal, nCoarse; // nRows, nbrTotal, nCoarse: extents for checked builds
+    int ncRow, ncCol, seg4;
+    const int64_t *gdof, *nbrPtr, *nbBase;
+    const int32_t *nbrIdx, *nbrCol, *agg;
+    const TA* vals;      // the pair's first padded value
+    const uint8_t* mask; // nullptr: no constrained rows
+    const TA *b, *dinv, *xin, *ce;
+    TA *xout, *d, *cb;
+    TA w0, w1, w2;
+};
+
+template <typename TA, int G, int GATHER, int EPI>
+__global__ void __launch_bounds__(kBS, NbMinBlocks<TA>()) k_cycle(CycleArgs<TA> A, const int* st)
 {
     PdlWait();
     PdlTrigger();
-    const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (i >= n || Idle(st))
+    extern __shared__ __align__(16) unsigned char cySmem[];
+    if (Idle(st))
         return;
-    const TA v = dinv[i] * (b[i] - t[i]) * invTheta;
-    d[i] = v;
-    e[i] += v;
+    const int gl = threadIdx.x & (G - 1);
+    TA* xs = reinterpret_cast<TA*>(cySmem) + (threadIdx.x / G) * A.seg4;
+    const int64_t a = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) / G;
+    const bool valid = a < A.nNodes;
+    const int ncR = valid ? A.ncRow : 0, ncC = A.ncCol;
+    int64_t q0 = 0;
+    int nn = 0;
+    const TA* vp = A.vals;
+    if (valid)
+    {
+        q0 = A.nbrPtr[a];
+        nn = static_cast<int>(A.nbrPtr[a + 1] - q0);
+        vp += A.nbBase[a];
+    }
+    // x of one DOF: global row g, component c of node `node`
+    auto value = [&](int64_t g, int32_t coarse, int c) -> TA {
+        if (GATHER == CG_ZERO)
+            return A.dinv[g] * A.b[g] * A.w0;
+        TA v = A.xin[g];
+        if (GATHER == CG_PROLONG && !(A.mask && A.mask[g]))
+            v += A.ce[NG_IDX(static_cast<int64_t>(coarse) * ncC + c, A.nCoarse, 34)];
+        return v;
+    };
+#pragma unroll 4
+    for (int t = gl; t < nn; t += G)
+    {
+        const int64_t col = A.nbrCol[NG_IDX(q0 + t, A.nbrTotal, 60)];
+        const int32_t coarse = GATHER == CG_PROLONG ? A.agg[A.nbrIdx[q0 + t]] : 0;
+        for (int d = 0; d < ncC; ++d)
+            xs[t * ncC + d] = value(NG_IDX(col + d, A.nRows, 62), coarse, d);
+    }
+    const int sg = (ncC * nn + 3) & ~3;
+    for (int t = ncC * nn + gl; t < sg; t += G)
+        xs[t] = TA(0);
+    __syncwarp();
+    TA s[kMaxComp];
+#pragma unroll
+    for (int c = 0; c < kMaxComp; ++c)
+        s[c] = TA(0);
+#pragma unroll 2
+    for (int f = 4 * gl; f < sg; f += 4 * G)
+    {
+        TA xv[4];
+        Load4(xs + f, xv);
+#pragma unroll
+        for (int c = 0; c < kMaxComp; ++c)
+            if (c < ncR)
+            {
+                TA v[4];
+                Load4(vp + c * sg + f, v);
+                s[c] += v[0] * xv[0] + v[1] * xv[1] + v[2] * xv[2] + v[3] * xv[3];
+            }
+    }
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int c = 0; c < kMaxComp; ++c)
+            s[c] += __shfl_xor_sync(0xffffffffu, s[c], o);
+    if (gl >= ncR)
+        return;
+    // lane c of the group finishes component c
+    TA t = s[0];
+#pragma unroll
+    for (int c = 1; c < kMaxComp; ++c)
+        t = gl == c ? s[c] : t;
+    const int64_t r = NG_IDX(A.gdof[a] + gl, A.nRows, 64);
+    const bool fixed = A.mask && A.mask[r];
+    if (EPI == CE_RESIDUAL)
+    {
+        A.xout[r] = fixed ? A.b[r] : A.b[r] - t;
+        return;
+    }
+    const TA x = value(r, GATHER == CG_PROLONG ? A.agg[a] : 0, gl);
+    const TA res = A.b[r] - (fixed ? x : t);
+    if (EPI == CE_RESTRICT)
+    {
+        if (GATHER == CG_ZERO)
+            A.xout[r] = x;
+        if (!fixed)
+            atomicAdd(A.cb + NG_IDX(static_cast<int64_t>(A.agg[a]) * A.ncRow + gl, A.nCoarse, 33), res);
+        return;
+    }
+    const TA d = EPI == CE_FIRST ? A.dinv[r] * res * A.w1
+                                 : A.w2 * (GATHER == CG_ZERO ? x : A.d[r]) + A.w1 * A.dinv[r] * res;
+    A.d[r] = d;
+    A.xout[r] = x + d;
 }
 
-// later Chebyshev steps (t = A e): d = c1 d + c2 dinv (b - t); e += d
-template <typename TA>
-__global__ void k_chebk(int64_t n, const TA* __restrict__ dinv, const TA* __restrict__ b, const TA* __restrict__ t,
-                        TA* d, TA* e, TA c1, TA c2, const int* st)
+template <typename TA, int GATHER, int EPI>
+static void LaunchCycle(Ctx& c, const CycleArgs<TA>& A, const int* st)
 {
-    PdlWait();
-    PdlTrigger();
-    const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (i >= n || Idle(st))
-        return;
-    const TA v = c1 * d[i] + c2 * dinv[i] * (b[i] - t[i]);
-    d[i] = v;
-    e[i] += v;
-}
-
-// coarse b = P^T (b - t) with t = A e (cb zeroed before); constrained finer DOFs are skipped
-template <typename TA>
-__global__ void k_restrict(NodeSpmv F, const uint8_t* __restrict__ fmask, const TA* __restrict__ b,
-                           const TA* __restrict__ t, const int32_t* __restrict__ agg, NodeSpmv C, TA* cb,
-                           const int* st)
-{
-    PdlWait();
-    PdlTrigger();
-    const int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (a >= F.totalWarps || Idle(st))
-        return;
-    const int64_t g0 = F.gdof[0][a];
-    const int64_t G0 = C.gdof[0][agg[a]];
-    for (int c = 0; c < F.ncomp[0]; ++c)
-        if (!fmask[g0 + c])
-            atomicAdd(cb + NG_IDX(G0 + c, C.nRows, 33), b[g0 + c] - t[g0 + c]);
+    const bool narrow = A.ncRow == 1 && A.ncCol == 1; // one short segment per node
+    const int G = narrow ? 4 : kNbG;
+    const size_t perGroup = static_cast<size_t>(A.seg4) * sizeof(TA);
+    int threads = kBS;
+    while (threads > 32 && (threads / G) * perGroup > 48 * 1024)
+        threads -= 32;
+    const unsigned blocks = static_cast<unsigned>((A.nNodes * G + threads - 1) / threads);
+    const size_t smem = (threads / G) * perGroup;
+    if (narrow)
+        NG_CUDA(LaunchPdl(k_cycle<TA, 4, GATHER, EPI>, blocks, threads, smem, c.stream, A, st));
+    else
+        NG_CUDA(LaunchPdl(k_cycle<TA, kNbG, GATHER, EPI>, blocks, threads, smem, c.stream, A, st));
+    c.stats.kernel_launches += 1;
 }
 
 // e += P ce
@@ -666,18 +789,6 @@ __global__ void k_prolong(NodeSpmv F, const uint8_t* __restrict__ fmask, const i
             e[g0 + c] += ce[NG_IDX(G0 + c, C.nRows, 34)];
 }
 
-// y = a - b (elementwise); a == nullptr gives y = 0
-template <typename TA>
-__global__ void k_sub(int64_t n, const TA* a, const TA* b, TA* y, const int* st)
-{
-    PdlWait();
-    PdlTrigger();
-    const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (i >= n || Idle(st))
-        return;
-    y[i] = a ? a[i] - b[i] : TA(0);
-}
-
 template <typename TA, typename TB>
 __global__ void k_convert(int64_t n, const TA* __restrict__ a, TB* __restrict__ b, const int* st)
 {
@@ -689,11 +800,14 @@ __global__ void k_convert(int64_t n, const TA* __restrict__ a, TB* __restrict__ 
 }
 
 // ---- device: the coarsest levels in one block ----------------------------------------------------------------
-// Levels with at most kTailNodes nodes (and every coarser one) do microseconds of work per launch; run as separate
-// launches they cost about 29 launches per slot and cycle. One block of kTailThreads threads runs their whole
-// V-cycle instead: the same Chebyshev recurrences (coefficients from the same double-precision formulas), the same
-// restriction and prolongation, and a warp-per-node product on the coarse node-block CSR, with block barriers
-// between the steps. The level vectors stay in global memory (L2-resident at these sizes).
+// Levels with at most kTailNodes nodes (and every coarser one) do microseconds of work per launch. Their whole V-cycle is a
+// fixed linear map of at most 384 values, so it is formed once per tangent as a dense matrix: block k of k_amg_tail runs the
+// cycle on unit vector k (the same Chebyshev recurrences, coefficients from the same double-precision formulas, the same
+// restriction and prolongation, a warp-per-node product on the coarse node-block CSR, block barriers between the steps),
+// and every sweep applies it with one small product. Run once per sweep in one block instead, the cycle took 55-73 us per
+// slot in FP32 and more in FP64, whose pipe is 2 lanes per clock and SM; the product takes 3-6 us, forming the matrix (90 nodes
+// x 3) 150 us in FP32 and 227 us in FP64 per tangent. Solves to 1e-13 with the fused cycle (k_cycle) and this: FP32 24^3
+// 130 -> 69 ms, FP64 20^3 203 -> 123 ms (launches per iteration 92 -> 33).
 constexpr int kTailNodes = 128;
 constexpr int kTailMax = 8;
 constexpr int kTailThreads = 1024;
@@ -720,6 +834,8 @@ struct TailArgs
     int pre, post, coarse;
     double smoothRatio, coarseRatio;
     TailLevel<TA> L[kTailMax];
+    int64_t stride; // block k works on vectors k * stride behind the levels'
+    TA* columns;    // [k][i]: block k's result
 };
 
 template <typename TA>
@@ -802,19 +918,30 @@ __device__ void TailCheb(const TailLevel<TA>& L, int degree, bool fromZero, doub
     }
 }
 
-// e = V-cycle(b) on the tail levels: the first level's b is the restriction from the finer level, its e is read by
-// the finer level's prolongation
+// Block k runs the V-cycle of the tail levels on unit vector k of the first level and stores the result as column k of the
+// tail's matrix (TailDense).
 template <typename TA>
-__global__ void __launch_bounds__(kTailThreads) k_amg_tail(TailArgs<TA> T, const int* st)
+__global__ void __launch_bounds__(kTailThreads) k_amg_tail(TailArgs<TA> T)
 {
-    PdlWait();
-    PdlTrigger();
-    if (Idle(st))
-        return;
+    __shared__ TailLevel<TA> L[kTailMax];
+    for (int l = threadIdx.x; l < T.nl; l += blockDim.x)
+    {
+        TailLevel<TA> F = T.L[l];
+        const int64_t o = blockIdx.x * T.stride;
+        F.b += o;
+        F.e += o;
+        F.t += o;
+        F.d += o;
+        L[l] = F;
+    }
+    __syncthreads();
+    for (int64_t i = threadIdx.x; i < L[0].nDofs; i += blockDim.x)
+        L[0].b[i] = i == blockIdx.x ? TA(1) : TA(0);
+    __syncthreads();
     for (int l = 0; l + 1 < T.nl; ++l)
     {
-        const TailLevel<TA>& F = T.L[l];
-        const TailLevel<TA>& C = T.L[l + 1];
+        const TailLevel<TA>& F = L[l];
+        const TailLevel<TA>& C = L[l + 1];
         TailCheb(F, T.pre, true, T.smoothRatio);
         TailSpmv(F, F.e, F.t);
         for (int64_t i = threadIdx.x; i < C.nDofs; i += blockDim.x)
@@ -828,11 +955,11 @@ __global__ void __launch_bounds__(kTailThreads) k_amg_tail(TailArgs<TA> T, const
         }
         __syncthreads();
     }
-    TailCheb(T.L[T.nl - 1], T.coarse, true, T.coarseRatio);
+    TailCheb(L[T.nl - 1], T.coarse, true, T.coarseRatio);
     for (int l = T.nl - 2; l >= 0; --l)
     {
-        const TailLevel<TA>& F = T.L[l];
-        const TailLevel<TA>& C = T.L[l + 1];
+        const TailLevel<TA>& F = L[l];
+        const TailLevel<TA>& C = L[l + 1];
         for (int64_t a = threadIdx.x; a < F.nNodes; a += blockDim.x)
         {
             const int64_t A = F.agg[a];
@@ -841,6 +968,42 @@ __global__ void __launch_bounds__(kTailThreads) k_amg_tail(TailArgs<TA> T, const
         }
         __syncthreads();
         TailCheb(F, T.post, false, T.smoothRatio);
+    }
+    const int64_t n = L[0].nDofs;
+    for (int64_t i = threadIdx.x; i < n; i += blockDim.x)
+        T.columns[blockIdx.x * n + i] = L[0].e[i];
+}
+
+// e = M b with the tail's matrix (columns m[k]): a block owns 32 rows, its warps a share of the columns each
+constexpr int kDenseWarps = 16;
+template <typename TA>
+__global__ void __launch_bounds__(kDenseWarps * 32) k_amg_tail_dense(int n, const TA* __restrict__ m,
+                                                                     const TA* __restrict__ b, TA* __restrict__ e,
+                                                                     const int* st)
+{
+    PdlWait();
+    PdlTrigger();
+    __shared__ TA part[kDenseWarps][32];
+    if (Idle(st))
+        return;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
+    TA s = TA(0);
+    if (i < n)
+    {
+#pragma unroll 8
+        for (int k = wid; k < n; k += kDenseWarps)
+            s += m[static_cast<int64_t>(k) * n + i] * b[k];
+    }
+    part[wid][lane] = s;
+    __syncthreads();
+    if (wid == 0 && i < n)
+    {
+        TA t = TA(0);
+#pragma unroll
+        for (int w = 0; w < kDenseWarps; ++w)
+            t += part[w][lane];
+        e[i] = t;
     }
 }
 
@@ -854,12 +1017,14 @@ static unsigned Blocks(int64_t n, int bs = 256)
 template <typename TA>
 static void EnsureNum(Ctx& c, Amg& M)
 {
+    int64_t rhs = 0;
     for (int I = 0; I < M.ns; ++I)
         for (size_t l = 0; l < M.h[I].size(); ++l)
         {
             AmgLevel& L = M.h[I][l];
             Num<TA>& U = N<TA>(L);
             const int64_t n = l == 0 ? c.nDofs : L.nDofs;
+            rhs += l > 0 ? L.nDofs : 0;
             if (U.dinv.n == static_cast<size_t>(n))
                 continue;
             if (l > 0)
@@ -867,16 +1032,96 @@ static void EnsureNum(Ctx& c, Amg& M)
                 U.vals.alloc(L.nnz);
                 U.nb.alloc(std::max<int64_t>(L.nbTotal, 4));
             }
-            for (DBuf<TA>* b : {&U.dinv, &U.e, &U.b, &U.t, &U.d})
+            for (DBuf<TA>* b : {&U.dinv, &U.e, &U.t, &U.d})
                 b->alloc(n);
         }
+    DBuf<TA>& R = Rhs<TA>(M);
+    if (R.n != static_cast<size_t>(rhs))
+    {
+        R.alloc(rhs);
+        int64_t at = 0;
+        for (int I = 0; I < M.ns; ++I)
+            for (size_t l = 1; l < M.h[I].size(); ++l)
+            {
+                N<TA>(M.h[I][l]).b = R.p + at;
+                at += M.h[I][l].nDofs;
+            }
+    }
+}
+
+// first level (>= 1) from which every level has at most kTailNodes nodes, if they fit one tail launch; 0: none
+static size_t TailStart(const std::vector<AmgLevel>& H)
+{
+    for (size_t l = 1; l < H.size(); ++l)
+        if (H[l].nNodes <= kTailNodes)
+            return H.size() - l <= static_cast<size_t>(kTailMax) ? l : 0;
+    return 0;
+}
+
+// the dense matrix of slot I's tail for the current coarse operators
+template <typename TA>
+static void BuildTail(Ctx& c, int I, bool sym)
+{
+    Amg& M = *c.amg;
+    std::vector<AmgLevel>& H = M.h[I];
+    const size_t l0 = TailStart(H);
+    TailDense<TA>& D = Tail<TA>(M, I);
+    if (l0 == 0)
+    {
+        D.n = 0;
+        return;
+    }
+    int64_t sum = 0; // values of one level-vector set
+    for (size_t l = l0; l < H.size(); ++l)
+        sum += H[l].nDofs;
+    D.n = H[l0].nDofs;
+    if (D.m.n != static_cast<size_t>(D.n * D.n))
+        D.m.alloc(D.n * D.n);
+    if (D.work.n != static_cast<size_t>(4 * sum * D.n))
+        D.work.alloc(4 * sum * D.n);
+    TailArgs<TA> T{};
+    T.nl = static_cast<int>(H.size() - l0);
+    T.pre = sym ? kPostDegree : kPreDegree;
+    T.post = kPostDegree;
+    T.coarse = CoarseDegree<TA>();
+    T.smoothRatio = kSmoothRatio;
+    T.coarseRatio = kCoarseRatio;
+    T.stride = 4 * sum;
+    T.columns = D.m.p;
+    int64_t at = 0;
+    for (int k = 0; k < T.nl; ++k)
+    {
+        AmgLevel& Lk = H[l0 + k];
+        Num<TA>& Uk = N<TA>(Lk);
+        TailLevel<TA>& F = T.L[k];
+        F.rowPtr = Lk.rowPtr.p;
+        F.nbrPtr = Lk.nbrPtr.p;
+        F.nbrCol = Lk.nbrCol.p;
+        F.agg = l0 + k + 1 < H.size() ? H[l0 + k + 1].aggOf.p : nullptr;
+        F.vals = Uk.vals.p;
+        F.dinv = Uk.dinv.p;
+        for (TA** v : {&F.b, &F.e, &F.t, &F.d})
+        {
+            *v = D.work.p + at;
+            at += Lk.nDofs;
+        }
+        F.nNodes = Lk.nNodes;
+        F.nnz = Lk.nnz;
+        F.nDofs = Lk.nDofs;
+        F.nbrTotal = static_cast<int64_t>(Lk.nbrIdx.n);
+        F.ncomp = Lk.ncomp;
+        F.lmax = Lk.lmax;
+    }
+    k_amg_tail<TA><<<static_cast<unsigned>(D.n), kTailThreads, 0, c.stream>>>(T);
+    AfterLaunch(c, "k_amg_tail");
+    c.stats.kernel_launches += 1;
 }
 
 // Builds the hierarchy on first use and the coarse operators for the tangent `vals` unless they were built for
 // the same values already (same pointer and tangent version). The preconditioner works in the arithmetic of the
 // tangent values: FP32 for FP32 tangents, FP64 for FP64 tangents.
 template <typename TV>
-void AmgSetup(Ctx& c, const TV* vals)
+void AmgSetup(Ctx& c, const TV* vals, bool sym)
 {
     HostClock hc(&c.hostMs[HP_AMG_SETUP]);
     if (!c.amg)
@@ -889,7 +1134,15 @@ void AmgSetup(Ctx& c, const TV* vals)
     if (!M.built)
         BuildHierarchy(c);
     if (M.setupVals == static_cast<const void*>(vals) && M.setupVersion == c.valsVersion)
+    {
+        if (M.tailSym != sym) // the same values for the other Krylov method: its cycle differs in the pre-smoothing
+        {
+            for (int I = 0; I < M.ns; ++I)
+                BuildTail<TV>(c, I, sym);
+            M.tailSym = sym;
+        }
         return;
+    }
     EnsureNum<TV>(c, M);
     M.prec = sizeof(TV) == 4 ? 32 : 64;
     M.fine = vals;
@@ -949,122 +1202,177 @@ void AmgSetup(Ctx& c, const TV* vals)
             const float v = M.lmaxHost[slot++];
             L.lmax = v > 0.f ? v : 1.f;
         }
+    for (int I = 0; I < M.ns; ++I)
+        BuildTail<TV>(c, I, sym);
+    M.tailSym = sym;
     M.setupVals = vals;
     M.setupVersion = c.valsVersion;
     M.setups++;
 }
-template void AmgSetup<float>(Ctx&, const float*);
-template void AmgSetup<double>(Ctx&, const double*);
+template void AmgSetup<float>(Ctx&, const float*, bool);
+template void AmgSetup<double>(Ctx&, const double*, bool);
 
-// Chebyshev smoothing of A e = b on [lmax / ratio, lmax]. Vectors are base pointers of the level (combined
-// length on level 0); elementwise work runs over rows [off, off + n). fromZero starts at e = 0 (no product).
-template <typename TA>
-static void Chebyshev(Ctx& c, AmgLevel& L, const TA* vals, const uint8_t* mask, const TA* b, TA* e, int degree,
-                      bool fromZero, float ratio, const int* st)
+// Chebyshev coefficients on [lmax / ratio, lmax]: step k multiplies the last step by w2 and dinv (b - A e) by w1
+struct Cheb
 {
-    Num<TA>& U = N<TA>(L);
-    const int64_t n = L.nDofs, o = L.off;
-    const double lmax = L.lmax, lmin = L.lmax / ratio;
-    const double theta = 0.5 * (lmax + lmin), delta = 0.5 * (lmax - lmin);
-    const double sigma = theta / delta;
-    int* stw = const_cast<int*>(st); // the SpMV only reads the state when it computes no dot products
-    double rho = 1. / sigma;
-    if (fromZero)
-        NG_CUDA(LaunchPdl(k_cheb0<TA>, Blocks(n), 256, 0, c.stream, n, U.dinv.p + o, b + o, U.d.p + o, e + o,
-                          TA(1. / theta), st));
-    else
+    double theta, delta, sigma, rho;
+    Cheb(const AmgLevel& L, float ratio)
     {
-        SpmvNode<TA, TA, 0>(c.stream, L.spmv, vals, e, U.t.p, nullptr, nullptr, stw, 0, mask);
-        NG_CUDA(LaunchPdl(k_cheb1<TA>, Blocks(n), 256, 0, c.stream, n, U.dinv.p + o, b + o, U.t.p + o, U.d.p + o,
-                          e + o, TA(1. / theta), st));
-        c.stats.kernel_launches += 1;
+        const double lmax = L.lmax, lmin = L.lmax / ratio;
+        theta = 0.5 * (lmax + lmin);
+        delta = 0.5 * (lmax - lmin);
+        sigma = theta / delta;
+        rho = 1. / sigma;
     }
-    c.stats.kernel_launches += 1;
-    for (int k = 1; k < degree; ++k)
+    void step(double& w2, double& w1)
     {
         const double rhoNew = 1. / (2. * sigma - rho);
-        SpmvNode<TA, TA, 0>(c.stream, L.spmv, vals, e, U.t.p, nullptr, nullptr, stw, 0, mask);
-        NG_CUDA(LaunchPdl(k_chebk<TA>, Blocks(n), 256, 0, c.stream, n, U.dinv.p + o, b + o, U.t.p + o, U.d.p + o,
-                          e + o, TA(rhoNew * rho), TA(2. * rhoNew / delta), st));
-        c.stats.kernel_launches += 2;
+        w2 = rhoNew * rho;
+        w1 = 2. * rhoNew / delta;
         rho = rhoNew;
     }
-}
+};
 
-// first level (>= 1) from which every level has at most kTailNodes nodes, if they fit one tail launch; 0: none
-static size_t TailStart(const std::vector<AmgLevel>& H)
-{
-    for (size_t l = 1; l < H.size(); ++l)
-        if (H[l].nNodes <= kTailNodes)
-            return H.size() - l <= static_cast<size_t>(kTailMax) ? l : 0;
-    return 0;
-}
-
-// e = V-cycle(b) on level l of hierarchy H
+// the diagonal block of a level for k_cycle (vectors are base pointers of the level: combined length on level 0)
 template <typename TA>
-static void VCycle(Ctx& c, std::vector<AmgLevel>& H, size_t l, const TA* b, TA* e, const int* st, bool sym)
+static CycleArgs<TA> LevelArgs(Ctx& c, AmgLevel& L, bool fine)
+{
+    const NodeSpmv& V = L.spmv;
+    CycleArgs<TA> A{};
+    NG_CHECK(SpmvPadded(V, fine ? static_cast<const TA*>(c.amg->fine) : N<TA>(L).vals.p), NUTO_GPU_ESTATE,
+             "the padded layout does not hold the level's values");
+    A.nNodes = L.nNodes;
+    A.nRows = V.nRows;
+    A.nbrTotal = V.nbrTotal[0];
+    A.ncRow = A.ncCol = L.ncomp;
+    A.seg4 = V.nbSeg4;
+    A.gdof = V.gdof[0];
+    A.nbrPtr = V.nbrPtr[0];
+    A.nbrIdx = V.nbrIdx[0];
+    A.nbrCol = V.nbrCol[0];
+    A.nbBase = V.nbBase[0];
+    A.vals = NbValues<TA>(V) + V.nbOff[0];
+    A.mask = fine ? c.dMask.p : nullptr;
+    A.dinv = N<TA>(L).dinv.p;
+    A.d = N<TA>(L).d.p;
+    return A;
+}
+
+// e = V-cycle(b) on level l of slot I's hierarchy
+template <typename TA>
+static void VCycle(Ctx& c, int I, size_t l, const TA* b, TA* e, const int* st, bool sym)
 {
     Amg& M = *c.amg;
+    std::vector<AmgLevel>& H = M.h[I];
     AmgLevel& L = H[l];
     Num<TA>& U = N<TA>(L);
-    const TA* vals = l == 0 ? static_cast<const TA*>(M.fine) : U.vals.p;
-    const uint8_t* mask = l == 0 ? c.dMask.p : L.zeroMask.p;
     if (l > 0 && l == TailStart(H))
     {
-        // this level and every coarser one in one block (b = U.b, e = U.e of this level)
-        TailArgs<TA> T{};
-        T.nl = static_cast<int>(H.size() - l);
-        T.pre = sym ? kPostDegree : kPreDegree;
-        T.post = kPostDegree;
-        T.coarse = CoarseDegree<TA>();
-        T.smoothRatio = kSmoothRatio;
-        T.coarseRatio = kCoarseRatio;
-        for (int k = 0; k < T.nl; ++k)
-        {
-            AmgLevel& Lk = H[l + k];
-            Num<TA>& Uk = N<TA>(Lk);
-            TailLevel<TA>& D = T.L[k];
-            D.rowPtr = Lk.rowPtr.p;
-            D.nbrPtr = Lk.nbrPtr.p;
-            D.nbrCol = Lk.nbrCol.p;
-            D.agg = l + k + 1 < H.size() ? H[l + k + 1].aggOf.p : nullptr;
-            D.vals = Uk.vals.p;
-            D.dinv = Uk.dinv.p;
-            D.b = Uk.b.p;
-            D.e = Uk.e.p;
-            D.t = Uk.t.p;
-            D.d = Uk.d.p;
-            D.nNodes = Lk.nNodes;
-            D.nnz = Lk.nnz;
-            D.nDofs = Lk.nDofs;
-            D.nbrTotal = static_cast<int64_t>(Lk.nbrIdx.n);
-            D.ncomp = Lk.ncomp;
-            D.lmax = Lk.lmax;
-        }
-        // the level's b and e are the ones the caller passed (its own U.b, U.e)
-        NG_CUDA(LaunchPdl(k_amg_tail<TA>, 1, kTailThreads, 0, c.stream, T, st));
+        const TailDense<TA>& D = Tail<TA>(M, I);
+        NG_CUDA(LaunchPdl(k_amg_tail_dense<TA>, Blocks(D.n, 32), kDenseWarps * 32, 0, c.stream, static_cast<int>(D.n), D.m.p,
+                          b, e, st));
         c.stats.kernel_launches += 1;
         return;
     }
+    CycleArgs<TA> A = LevelArgs<TA>(c, L, l == 0);
+    A.b = b;
+    const int64_t n = L.nDofs, o = L.off;
+    const bool fuse = L.nNodes <= kFuseNodes;
+    // from zero: x = dinv b / theta, in the product's gather or in a kernel of its own (into `to`)
+    auto fromZero = [&](const Cheb& C, TA* to) {
+        A.w0 = TA(1. / C.theta);
+        if (fuse)
+            return;
+        NG_CUDA(LaunchPdl(k_cheb0<TA>, Blocks(n), 256, 0, c.stream, n, U.dinv.p + o, b + o, to + o, A.w0, st));
+        c.stats.kernel_launches += 1;
+        A.xin = to;
+    };
+    auto stepFromZero = [&](TA* out) {
+        A.xout = out;
+        if (fuse)
+            LaunchCycle<TA, CG_ZERO, CE_STEP>(c, A, st);
+        else
+        {
+            // the step before is x itself: d = x
+            NG_CUDA(cudaMemcpyAsync(U.d.p + o, A.xin + o, n * sizeof(TA), cudaMemcpyDeviceToDevice, c.stream));
+            LaunchCycle<TA, CG_VECTOR, CE_STEP>(c, A, st);
+        }
+    };
+    auto coefficients = [&](Cheb& C) {
+        double w2, w1;
+        C.step(w2, w1);
+        A.w1 = TA(w1);
+        A.w2 = TA(w2);
+    };
     if (l + 1 == H.size())
     {
-        Chebyshev<TA>(c, L, vals, mask, b, e, CoarseDegree<TA>(), true, kCoarseRatio, st);
+        // Chebyshev solve; the steps alternate between t and e and end in e
+        Cheb C(L, kCoarseRatio);
+        const int steps = CoarseDegree<TA>() - 1;
+        TA* buf[2] = {U.t.p, e}; // step s writes buf[(steps - s) & 1 ? 0 : 1]
+        fromZero(C, steps & 1 ? U.t.p : e);
+        for (int s = 1; s <= steps; ++s)
+        {
+            coefficients(C);
+            TA* out = buf[(steps - s) & 1 ? 0 : 1];
+            if (s == 1)
+                stepFromZero(out);
+            else
+            {
+                A.xout = out;
+                LaunchCycle<TA, CG_VECTOR, CE_STEP>(c, A, st);
+            }
+            A.xin = out;
+        }
         return;
     }
-    AmgLevel& C = H[l + 1];
-    Num<TA>& CU = N<TA>(C);
-    int* stw = const_cast<int*>(st);
-    Chebyshev<TA>(c, L, vals, mask, b, e, sym ? kPostDegree : kPreDegree, true, kSmoothRatio, st);
-    SpmvNode<TA, TA, 0>(c.stream, L.spmv, vals, e, U.t.p, nullptr, nullptr, stw, 0, mask);
-    NG_CUDA(LaunchPdl(k_sub<TA>, Blocks(C.nDofs), 256, 0, c.stream, C.nDofs, nullptr, nullptr, CU.b.p, st));
-    NG_CUDA(LaunchPdl(k_restrict<TA>, Blocks(L.nNodes), 256, 0, c.stream, L.spmv, mask, b, U.t.p, C.aggOf.p, C.spmv,
-                      CU.b.p, st));
-    c.stats.kernel_launches += 3;
-    VCycle<TA>(c, H, l + 1, CU.b.p, CU.e.p, st, sym);
-    NG_CUDA(LaunchPdl(k_prolong<TA>, Blocks(L.nNodes), 256, 0, c.stream, L.spmv, mask, C.aggOf.p, C.spmv, CU.e.p, e,
-                      st));
-    c.stats.kernel_launches += 1;
-    Chebyshev<TA>(c, L, vals, mask, b, e, kPostDegree, false, kSmoothRatio, st);
+    AmgLevel& Co = H[l + 1];
+    Num<TA>& CU = N<TA>(Co);
+    // pre-smoothing from zero (one step, two in the symmetric cycle), then the residual restricted
+    A.agg = Co.aggOf.p;
+    A.cb = CU.b;
+    A.nCoarse = Co.nDofs;
+    {
+        Cheb C(L, kSmoothRatio);
+        if (sym)
+        {
+            fromZero(C, U.t.p);
+            coefficients(C);
+            stepFromZero(e);
+            A.xin = e;
+            LaunchCycle<TA, CG_VECTOR, CE_RESTRICT>(c, A, st);
+        }
+        else
+        {
+            fromZero(C, e);
+            A.xout = e;
+            if (fuse)
+                LaunchCycle<TA, CG_ZERO, CE_RESTRICT>(c, A, st);
+            else
+                LaunchCycle<TA, CG_VECTOR, CE_RESTRICT>(c, A, st);
+        }
+    }
+    VCycle<TA>(c, I, l + 1, CU.b, CU.e.p, st, sym);
+    // coarse correction and two post-smoothing steps: e -> t -> e
+    A.ce = CU.e.p;
+    A.xin = e;
+    A.xout = U.t.p;
+    Cheb C(L, kSmoothRatio);
+    A.w1 = TA(1. / C.theta);
+    if (fuse)
+        LaunchCycle<TA, CG_PROLONG, CE_FIRST>(c, A, st);
+    else
+    {
+        NG_CUDA(LaunchPdl(k_prolong<TA>, Blocks(L.nNodes), 256, 0, c.stream, L.spmv, l == 0 ? c.dMask.p : L.zeroMask.p,
+                          Co.aggOf.p, Co.spmv, static_cast<const TA*>(CU.e.p), e, st));
+        c.stats.kernel_launches += 1;
+        LaunchCycle<TA, CG_VECTOR, CE_FIRST>(c, A, st);
+    }
+    static_assert(kPostDegree == 2, "two post-smoothing steps");
+    coefficients(C);
+    A.xin = U.t.p;
+    A.xout = e;
+    LaunchCycle<TA, CG_VECTOR, CE_STEP>(c, A, st);
 }
 
 // block Gauss-Seidel sweep in slot order on combined vectors: z_0 = V_0(v_0), z_1 = V_1(v_1 - K_10 z_0)
@@ -1072,18 +1380,33 @@ template <typename TA>
 static void Sweep(Ctx& c, const TA* v, TA* z, TA* res, const int* st, bool sym)
 {
     Amg& M = *c.amg;
-    VCycle<TA>(c, M.h[0], 0, v, z, st, sym);
+    if (Rhs<TA>(M).n > 0)
+        NG_CUDA(cudaMemsetAsync(Rhs<TA>(M).p, 0, Rhs<TA>(M).n * sizeof(TA), c.stream));
+    VCycle<TA>(c, 0, 0, v, z, st, sym);
     for (int I = 1; I < M.ns; ++I)
     {
-        AmgLevel& L = M.h[I][0];
-        const int64_t o = L.off, n = L.nDofs;
-        // z_I = 0, res = K z on the rows of slot I, res = v_I - res
-        NG_CUDA(LaunchPdl(k_sub<TA>, Blocks(n), 256, 0, c.stream, n, nullptr, nullptr, z + o, st));
-        SpmvNode<TA, TA, 0>(c.stream, RowsView(c, I), static_cast<const TA*>(M.fine), z, res, nullptr, nullptr,
-                            const_cast<int*>(st), 0, c.dMask.p);
-        NG_CUDA(LaunchPdl(k_sub<TA>, Blocks(n), 256, 0, c.stream, n, v + o, res + o, res + o, st));
-        c.stats.kernel_launches += 3;
-        VCycle<TA>(c, M.h[I], 0, res, z, st, sym);
+        // res = v_I - K_I0 z_0 on the rows of slot I
+        const PairMap& P = c.pairs[I * M.ns];
+        const NbLayout::Pair& nb = c.nb.pair[I * M.ns];
+        CycleArgs<TA> A{};
+        A.nNodes = c.slots[I].nNodes;
+        A.nRows = c.nDofs;
+        A.nbrTotal = static_cast<int64_t>(P.dNbrIdx.n);
+        A.ncRow = c.slots[I].ncomp;
+        A.ncCol = c.slots[0].ncomp;
+        A.seg4 = nb.maxSeg4;
+        A.gdof = c.slots[I].dGdof.p;
+        A.nbrPtr = P.dNbrPtr.p;
+        A.nbrIdx = P.dNbrIdx.p;
+        A.nbrCol = P.dNbrCol.p;
+        A.nbBase = nb.base.p;
+        A.vals = NbValues<TA>(M.h[I][0].spmv) + nb.off;
+        A.mask = c.dMask.p;
+        A.b = v;
+        A.xin = z;
+        A.xout = res;
+        LaunchCycle<TA, CG_VECTOR, CE_RESIDUAL>(c, A, st);
+        VCycle<TA>(c, I, 0, res, z, st, sym);
     }
 }
 

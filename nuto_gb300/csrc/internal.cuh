@@ -518,7 +518,7 @@ int DoStep(Ctx& c, double tNew, const nuto_gpu_step_options& o, int* iters);
 void FreeSolverWork(Ctx& c);
 void FreeAmg(Ctx& c);
 template <typename TV>
-void AmgSetup(Ctx& c, const TV* vals);
+void AmgSetup(Ctx& c, const TV* vals, bool sym); // sym: as in AmgApply
 template <typename T>
 void AmgApply(Ctx& c, const T* v, T* z, const int* st, bool sym);
 int AmgLevels(const Ctx& c);

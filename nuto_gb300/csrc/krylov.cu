@@ -1137,7 +1137,7 @@ static int GmresSolve(Ctx& c, const TV* vals, const double* b, double* x64, bool
     EnsureNb(c, vals);
     if (amg)
     {
-        AmgSetup<TV>(c, vals);
+        AmgSetup<TV>(c, vals, false);
         G.ensureZ();
     }
     else
@@ -1297,7 +1297,7 @@ static int KrylovSolve(Ctx& c, int method, const TV* vals, const double* b, doub
     const bool amg = pcg && c.precond == NUTO_GPU_PRECOND_AMG;
     EnsureNb(c, vals);
     if (amg)
-        AmgSetup<TV>(c, vals);
+        AmgSetup<TV>(c, vals, true);
     else
         k_diag_inv<TV, T><<<static_cast<unsigned>((n + 255) / 256), 256, 0, c.stream>>>(
                 n, c.dRowPtr.p, c.dColIdx.p, vals, c.dMask.p, V.dinv.p);

@@ -300,7 +300,7 @@ __device__ __forceinline__ void Load4(const T* p, T (&o)[4])
 }
 
 template <typename TV>
-__device__ __forceinline__ const TV* NbValues(const NodeSpmv& A)
+__host__ __device__ __forceinline__ const TV* NbValues(const NodeSpmv& A)
 {
     if constexpr (sizeof(TV) == 4)
         return A.nb32;
