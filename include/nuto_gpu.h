@@ -160,7 +160,8 @@ typedef struct nuto_gpu_stats
     double ms_assemble_vector;
     double ms_krylov;
     double ms_total;
-    double ms_spmv;          /* device time of the Krylov sparse matrix-vector products (CUDA events) */
+    double ms_spmv;          /* device time of the Krylov sparse matrix-vector products (CUDA events around every
+                                eighth one, times the number of products) */
     int64_t spmv_launches;
     int64_t kernel_launches; /* kernels launched by the step */
 } nuto_gpu_stats;

@@ -754,21 +754,32 @@ __global__ void __launch_bounds__(kBS, NbMinBlocks<TA>()) k_cycle(CycleArgs<TA> 
     A.xout[r] = x + d;
 }
 
+// Lanes per node and threads per block: 8 lanes (4 for one-component rows and columns, one short segment per node) and 256
+// threads stream a large level; on small ones the chain of one node is what takes the time, so more lanes share it and the
+// blocks shrink until every SM has one.
 template <typename TA, int GATHER, int EPI>
 static void LaunchCycle(Ctx& c, const CycleArgs<TA>& A, const int* st)
 {
-    const bool narrow = A.ncRow == 1 && A.ncCol == 1; // one short segment per node
-    const int G = narrow ? 4 : kNbG;
+    const bool narrow = A.ncRow == 1 && A.ncCol == 1;
+    const int64_t sms = std::max(c.smCount, 1);
+    int G = narrow ? 4 : 8;
+    const int most = narrow ? 8 : 32;
+    while (G < most && A.nNodes * G * 2 <= sms * 512)
+        G *= 2;
     const size_t perGroup = static_cast<size_t>(A.seg4) * sizeof(TA);
-    int threads = kBS;
+    int threads = static_cast<int>(std::min<int64_t>(kBS, std::max<int64_t>(32, A.nNodes * G / sms / 32 * 32)));
     while (threads > 32 && (threads / G) * perGroup > 48 * 1024)
         threads -= 32;
     const unsigned blocks = static_cast<unsigned>((A.nNodes * G + threads - 1) / threads);
     const size_t smem = (threads / G) * perGroup;
-    if (narrow)
+    if (G == 4)
         NG_CUDA(LaunchPdl(k_cycle<TA, 4, GATHER, EPI>, blocks, threads, smem, c.stream, A, st));
+    else if (G == 8)
+        NG_CUDA(LaunchPdl(k_cycle<TA, 8, GATHER, EPI>, blocks, threads, smem, c.stream, A, st));
+    else if (G == 16)
+        NG_CUDA(LaunchPdl(k_cycle<TA, 16, GATHER, EPI>, blocks, threads, smem, c.stream, A, st));
     else
-        NG_CUDA(LaunchPdl(k_cycle<TA, kNbG, GATHER, EPI>, blocks, threads, smem, c.stream, A, st));
+        NG_CUDA(LaunchPdl(k_cycle<TA, 32, GATHER, EPI>, blocks, threads, smem, c.stream, A, st));
     c.stats.kernel_launches += 1;
 }
 
@@ -1498,6 +1509,50 @@ static bool SweepGraphRun(Ctx& c, TA* in, TA* out, TA* res, const int* st, bool 
     return true;
 }
 
+template <typename T>
+void AmgVectors(Ctx& c, T** in, T** out)
+{
+    Amg& M = *c.amg;
+    *in = *out = nullptr;
+    if (M.prec != static_cast<int>(8 * sizeof(T)))
+        return;
+    DBuf<T>*vi, *vo, *vr;
+    if constexpr (sizeof(T) == 4)
+    {
+        vi = &M.in32;
+        vo = &M.out32;
+        vr = &M.res32;
+    }
+    else
+    {
+        vi = &M.in64;
+        vo = &M.out64;
+        vr = &M.res64;
+    }
+    for (DBuf<T>* b : {vi, vo, vr})
+        if (b->n != static_cast<size_t>(c.nDofs))
+            b->alloc(c.nDofs);
+    *in = vi->p;
+    *out = vo->p;
+}
+template void AmgVectors<float>(Ctx&, float**, float**);
+template void AmgVectors<double>(Ctx&, double**, double**);
+
+template <typename T>
+void AmgSweep(Ctx& c, const int* st, bool sym)
+{
+    T *in, *out, *res;
+    AmgVectors<T>(c, &in, &out);
+    if constexpr (sizeof(T) == 4)
+        res = c.amg->res32.p;
+    else
+        res = c.amg->res64.p;
+    if (!SweepGraphRun<T>(c, in, out, res, st, sym))
+        Sweep<T>(c, in, out, res, st, sym);
+}
+template void AmgSweep<float>(Ctx&, const int*, bool);
+template void AmgSweep<double>(Ctx&, const int*, bool);
+
 // z = M^-1 v for the tangent of the last AmgSetup, in that tangent's arithmetic (FP64 Krylov vectors with an
 // FP32 tangent are converted). With st given, every kernel returns at once when the Krylov state is not RUN.
 // sym = true runs equal pre- and post-smoothing (a symmetric cycle for PCG on a single slot); otherwise the
@@ -1505,61 +1560,27 @@ static bool SweepGraphRun(Ctx& c, TA* in, TA* out, TA* res, const int* st, bool 
 template <typename T>
 void AmgApply(Ctx& c, const T* v, T* z, const int* st, bool sym)
 {
-    Amg& M = *c.amg;
     const int64_t n = c.nDofs;
-    const size_t bytesN = static_cast<size_t>(n);
-    if (M.prec == 64)
+    T *in, *out;
+    AmgVectors<T>(c, &in, &out);
+    if (in)
     {
-        if constexpr (sizeof(T) == 8)
-        {
-            if (M.res64.n != bytesN)
-            {
-                M.res64.alloc(n);
-                M.in64.alloc(n);
-                M.out64.alloc(n);
-            }
-            if (M.graphs)
-            {
-                NG_CUDA(cudaMemcpyAsync(M.in64.p, v, n * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
-                if (SweepGraphRun<double>(c, M.in64.p, M.out64.p, M.res64.p, st, sym))
-                {
-                    NG_CUDA(cudaMemcpyAsync(z, M.out64.p, n * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
-                    return;
-                }
-            }
-            Sweep<double>(c, v, z, M.res64.p, st, sym);
-        }
-        else
-            throw Error{NUTO_GPU_EINVAL, "FP32 Krylov vectors with an FP64 multigrid set-up"};
+        NG_CUDA(cudaMemcpyAsync(in, v, n * sizeof(T), cudaMemcpyDeviceToDevice, c.stream));
+        AmgSweep<T>(c, st, sym);
+        NG_CUDA(cudaMemcpyAsync(z, out, n * sizeof(T), cudaMemcpyDeviceToDevice, c.stream));
         return;
     }
-    if (M.res32.n != bytesN)
+    if constexpr (sizeof(T) == 8)
     {
-        M.res32.alloc(n);
-        M.in32.alloc(n);
-        M.out32.alloc(n);
-    }
-    if constexpr (sizeof(T) == 4)
-    {
-        if (M.graphs)
-        {
-            NG_CUDA(cudaMemcpyAsync(M.in32.p, v, n * sizeof(float), cudaMemcpyDeviceToDevice, c.stream));
-            if (SweepGraphRun<float>(c, M.in32.p, M.out32.p, M.res32.p, st, sym))
-            {
-                NG_CUDA(cudaMemcpyAsync(z, M.out32.p, n * sizeof(float), cudaMemcpyDeviceToDevice, c.stream));
-                return;
-            }
-        }
-        Sweep<float>(c, v, z, M.res32.p, st, sym);
-    }
-    else
-    {
-        NG_CUDA(LaunchPdl(k_convert<double, float>, Blocks(n), 256, 0, c.stream, n, v, M.in32.p, st));
-        if (!SweepGraphRun<float>(c, M.in32.p, M.out32.p, M.res32.p, st, sym))
-            Sweep<float>(c, M.in32.p, M.out32.p, M.res32.p, st, sym);
-        NG_CUDA(LaunchPdl(k_convert<float, double>, Blocks(n), 256, 0, c.stream, n, M.out32.p, z, st));
+        float *in32, *out32;
+        AmgVectors<float>(c, &in32, &out32);
+        NG_CUDA(LaunchPdl(k_convert<double, float>, Blocks(n), 256, 0, c.stream, n, v, in32, st));
+        AmgSweep<float>(c, st, sym);
+        NG_CUDA(LaunchPdl(k_convert<float, double>, Blocks(n), 256, 0, c.stream, n, static_cast<const float*>(out32), z, st));
         c.stats.kernel_launches += 2;
     }
+    else
+        throw Error{NUTO_GPU_EINVAL, "FP32 Krylov vectors with an FP64 multigrid set-up"};
 }
 template void AmgApply<float>(Ctx&, const float*, float*, const int*, bool);
 template void AmgApply<double>(Ctx&, const double*, double*, const int*, bool);

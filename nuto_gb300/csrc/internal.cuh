@@ -521,6 +521,12 @@ template <typename TV>
 void AmgSetup(Ctx& c, const TV* vals, bool sym); // sym: as in AmgApply
 template <typename T>
 void AmgApply(Ctx& c, const T* v, T* z, const int* st, bool sym);
+// the fixed input and output vectors of the sweep where its arithmetic (that of the last set-up) is T, else nullptrs, and
+// the sweep on them
+template <typename T>
+void AmgVectors(Ctx& c, T** in, T** out);
+template <typename T>
+void AmgSweep(Ctx& c, const int* st, bool sym);
 int AmgLevels(const Ctx& c);
 // y = K x for FP32 or FP64 CSR values and FP64 vectors (FP64 accumulation), and the compensated FP32 form
 void SpmvFull64(Ctx& c, int precision, const void* vals, const double* x, double* y);

@@ -475,8 +475,8 @@ template void EnsureNb<float>(Ctx&, const float*);
 template void EnsureNb<double>(Ctx&, const double*);
 
 // Autotuner of the fine-level product: the first product of a context with a given value and vector type (outside
-// any stream capture) times the padded-layout kernel with 4, 8 and 16 lanes per node (one warm-up and one timed
-// launch each, y = K x without dot products, so the tuning launches only write the y the real call writes again)
+// any stream capture) times the padded-layout kernel with 4, 8 and 16 lanes per node (one warm-up and eight timed
+// launches each, y = K x without dot products, so the tuning launches only write the y the real call writes again)
 // and keeps the fastest; NUTO_GPU_AUTOTUNE=0 keeps the default.
 template <typename TV, typename TX>
 static int SpmvGroup(Ctx& c, const NodeSpmv& A, const TV* vals, const TX* x, TX* y, const uint8_t* mask)
@@ -499,13 +499,16 @@ static int SpmvGroup(Ctx& c, const NodeSpmv& A, const TV* vals, const TX* x, TX*
     int pick = kNbG;
     for (int k = 0; k < 3; ++k)
     {
+        constexpr int runs = 8; // one launch between two events is mostly the events at small sizes
         SpmvNode<TV, TX, 0>(c.stream, A, vals, x, y, nullptr, nullptr, nullptr, FIN_NONE, mask, cand[k]);
         NG_CUDA(cudaEventRecord(e0, c.stream));
-        SpmvNode<TV, TX, 0>(c.stream, A, vals, x, y, nullptr, nullptr, nullptr, FIN_NONE, mask, cand[k]);
+        for (int i = 0; i < runs; ++i)
+            SpmvNode<TV, TX, 0>(c.stream, A, vals, x, y, nullptr, nullptr, nullptr, FIN_NONE, mask, cand[k]);
         NG_CUDA(cudaEventRecord(e1, c.stream));
         NG_CUDA(cudaEventSynchronize(e1));
         float ms = 0.f;
         NG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+        ms /= runs;
         T.spmvMs[key][k] = ms;
         if (k == 0 || ms < best)
         {
@@ -515,7 +518,7 @@ static int SpmvGroup(Ctx& c, const NodeSpmv& A, const TV* vals, const TX* x, TX*
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    c.stats.kernel_launches += 6;
+    c.stats.kernel_launches += 27;
     T.spmvGroup[key] = pick;
     return pick;
 }
@@ -529,12 +532,20 @@ static void SpmvLaunch(Ctx& c, const TV* vals, const TX* x, TX* y, const TX* w0,
     SpmvNode<TV, TX, NDOT>(c.stream, A, vals, x, y, w0, sc, st, fin, mask, g);
 }
 
-// Krylov SpMV with a CUDA-event pair around it (device time of the dominant kernel, collected by SpmvCollect)
+// Krylov SpMV, every eighth one with a CUDA-event pair around it (device time of the dominant kernel, collected by
+// SpmvCollect). An event between two kernels keeps the second from being scheduled while the first drains.
+constexpr int kSpmvSample = 8;
 template <typename TV, typename TX, int NDOT>
 static void SpmvTimed(Ctx& c, const TV* vals, const TX* x, TX* y, const TX* w0, double* sc, int* st, int fin,
                       const uint8_t* mask)
 {
     SolverWork& w = Work(c);
+    c.stats.kernel_launches += 1;
+    if (w.spmvCount++ % kSpmvSample != 0)
+    {
+        SpmvLaunch<TV, TX, NDOT>(c, vals, x, y, w0, sc, st, fin, mask);
+        return;
+    }
     if (w.spmvNext == w.spmvEv.size())
     {
         std::pair<cudaEvent_t, cudaEvent_t> p;
@@ -546,21 +557,24 @@ static void SpmvTimed(Ctx& c, const TV* vals, const TX* x, TX* y, const TX* w0, 
     NG_CUDA(cudaEventRecord(ev.first, c.stream));
     SpmvLaunch<TV, TX, NDOT>(c, vals, x, y, w0, sc, st, fin, mask);
     NG_CUDA(cudaEventRecord(ev.second, c.stream));
-    c.stats.kernel_launches += 1;
 }
 
 // after a stream synchronisation: add the recorded SpMV times to the statistics
 static void SpmvCollect(Ctx& c)
 {
     SolverWork& w = Work(c);
+    double sum = 0.;
     for (size_t i = 0; i < w.spmvNext; ++i)
     {
         float ms = 0;
         NG_CUDA(cudaEventElapsedTime(&ms, w.spmvEv[i].first, w.spmvEv[i].second));
-        c.stats.ms_spmv += ms;
+        sum += ms;
     }
-    c.stats.spmv_launches += static_cast<int64_t>(w.spmvNext);
+    if (w.spmvNext > 0)
+        c.stats.ms_spmv += sum * static_cast<double>(w.spmvCount) / static_cast<double>(w.spmvNext);
+    c.stats.spmv_launches += w.spmvCount;
     w.spmvNext = 0;
+    w.spmvCount = 0;
 }
 
 double MaskedNorm(Ctx& c, const double* v)
@@ -774,15 +788,23 @@ void SpmvFull64(Ctx& c, int precision, const void* vals, const double* x, double
 // is enqueued without a host round trip. The basis is stored in T (FP32 or FP64).
 using GL = GmresLayout;
 
-// Projections on the basis in warp units: a unit is 32 x kUnitRows consecutive rows, lane l reading rows
-// base + l + 32 k, so every basis vector is streamed once per pass with coalesced loads. Per basis vector and unit
-// the lanes' products are summed by a warp butterfly in T; lane i % 32 keeps the running sum of vector i in a
-// register, and at the end of the block the warps' sums are added in T and each block adds one FP64 value per
-// vector to the accumulator. No FP64 arithmetic per row or per unit (the FP64 pipe is narrow on this part).
-constexpr int kUnitRows = 4;
+// Projections on the basis in warp units: a unit is 32 x K consecutive rows, lane l reading rows base + l + 32 k, so every
+// basis vector is streamed once per pass with coalesced loads. The lanes' products with 8 vectors at a time are summed by one
+// butterfly that halves the number of values in its first three steps (9 additions instead of 40); the lane of vector i keeps
+// its running sum in a register, and at the end of the block the warps' sums are added in T and each block adds one FP64 value
+// per vector to the accumulator. K = 1, 2 or 4 (UnitRows): few rows per unit spread a small system over all SMs, which for
+// FP64 (2 lanes per clock and SM) is what bounds these kernels: 37,044 rows and 40 vectors took 46 us with 37 blocks of
+// 4-row units and a butterfly per vector, 12.5 us now.
 constexpr int kGmresFirstChunk = 4; // iterations enqueued before the first look at the residual estimate
 constexpr int kGmresMaxChunk = 16;
 constexpr int kProjChunks = (GL::m + 1 + 31) / 32;
+
+// rows per lane and unit: the largest that still gives every SM 16 warps
+static int UnitRows(const Ctx& c, int64_t n)
+{
+    const int64_t warps = static_cast<int64_t>(std::max(c.smCount, 1)) * 16;
+    return n >= warps * 128 ? 4 : (n >= warps * 64 ? 2 : 1);
+}
 
 template <typename T>
 __device__ __forceinline__ T WarpAllSum(T v)
@@ -791,6 +813,28 @@ __device__ __forceinline__ T WarpAllSum(T v)
     for (int o = 16; o > 0; o >>= 1)
         v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
+}
+
+// sums of p[0..7] over the warp: lane l returns the sum of p[l & 7]
+template <typename T>
+__device__ __forceinline__ T WarpSum8(T (&p)[8])
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int h = 4, o = 16; h > 0; h >>= 1, o >>= 1)
+    {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < h; ++i)
+        {
+            const T send = up ? p[i] : p[i + h], keep = up ? p[i + h] : p[i];
+            p[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    T v = p[0]; // of vector (lane >> 4 & 1) * 4 + (lane >> 3 & 1) * 2 + (lane >> 2 & 1)
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    return __shfl_sync(0xffffffffu, v, (lane & 7) * 4);
 }
 
 // adds the block's per-vector sums (lane registers acc[c] hold vector lane + 32 c of each warp) to out[0, nv)
@@ -813,45 +857,47 @@ __device__ __forceinline__ void ProjFlush(const T (&acc)[kProjChunks], int nv, d
     }
 }
 
-// products of the unit's rows (held in r[]) with basis vectors 0 .. nv-1, summed into acc
-template <typename T>
-__device__ __forceinline__ void ProjUnit(const T* __restrict__ V, int64_t n, int nv, int64_t base, bool full,
-                                         const T (&r)[kUnitRows], T (&acc)[kProjChunks])
+// products of the unit's rows (held in r[], zero beyond n) with basis vectors 0 .. nv-1, summed into acc
+template <typename T, int K>
+__device__ __forceinline__ void ProjUnit(const T* __restrict__ V, int64_t n, int nv, int64_t base, const T (&r)[K],
+                                         T (&acc)[kProjChunks])
 {
     const int lane = threadIdx.x & 31;
+    bool in[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        in[k] = base + 32 * k < n;
 #pragma unroll
     for (int c = 0; c < kProjChunks; ++c)
     {
         if (c * 32 >= nv)
             break;
-        const int iend = min(32, nv - c * 32);
-#pragma unroll 4
-        for (int ii = 0; ii < iend; ++ii)
+#pragma unroll 1
+        for (int g = 0; g < 4; ++g)
         {
-            const T* Vi = V + static_cast<int64_t>(c * 32 + ii) * n;
-            T p = T(0);
-            if (full)
-            {
+            const int i0 = c * 32 + g * 8;
+            if (i0 >= nv)
+                break;
+            T p[8];
 #pragma unroll
-                for (int k = 0; k < kUnitRows; ++k)
-                    p += Vi[base + 32 * k] * r[k];
-            }
-            else
+            for (int i = 0; i < 8; ++i)
             {
+                const T* Vi = V + static_cast<int64_t>(i0 + i) * n + base;
+                p[i] = T(0);
 #pragma unroll
-                for (int k = 0; k < kUnitRows; ++k)
-                    if (base + 32 * k < n)
-                        p += Vi[base + 32 * k] * r[k];
+                for (int k = 0; k < K; ++k)
+                    if (i0 + i < nv && in[k])
+                        p[i] += Vi[32 * k] * r[k];
             }
-            p = WarpAllSum(p);
-            if (lane == ii)
-                acc[c] += p;
+            const T v = WarpSum8(p);
+            if ((lane >> 3) == g)
+                acc[c] += v;
         }
     }
 }
 
 // acc[i] += V_i . w for i < nv
-template <typename T>
+template <typename T, int K>
 __global__ void __launch_bounds__(kBS) k_gm_proj(int64_t n, const T* __restrict__ V, int nv, const T* __restrict__ w,
                                                   double* acc, const int* st)
 {
@@ -864,24 +910,23 @@ __global__ void __launch_bounds__(kBS) k_gm_proj(int64_t n, const T* __restrict_
 #pragma unroll
     for (int c = 0; c < kProjChunks; ++c)
         sums[c] = T(0);
-    const int64_t units = (n + 32 * kUnitRows - 1) / (32 * kUnitRows);
+    const int64_t units = (n + 32 * K - 1) / (32 * K);
     const int64_t warps = static_cast<int64_t>(gridDim.x) * (kBS / 32);
     for (int64_t u = blockIdx.x * static_cast<int64_t>(kBS / 32) + (threadIdx.x >> 5); u < units; u += warps)
     {
-        const int64_t base = u * 32 * kUnitRows + lane;
-        const bool full = (u + 1) * 32 * kUnitRows <= n;
-        T r[kUnitRows];
+        const int64_t base = u * 32 * K + lane;
+        T r[K];
 #pragma unroll
-        for (int k = 0; k < kUnitRows; ++k)
+        for (int k = 0; k < K; ++k)
             r[k] = base + 32 * k < n ? w[base + 32 * k] : T(0);
-        ProjUnit(V, n, nv, base, full, r, sums);
+        ProjUnit<T, K>(V, n, nv, base, r, sums);
     }
     ProjFlush(sums, nv, acc);
 }
 
 // w -= sum_i h_i V_i with h the first projection (gs + H1), then acc2[i] += V_i . w: the update of classical
 // Gram-Schmidt and the re-orthogonalisation's projection in one pass (the unit's V values are re-read from cache)
-template <typename T>
+template <typename T, int K>
 __global__ void __launch_bounds__(kBS) k_gm_update_proj(int64_t n, const T* __restrict__ V, int nv, const double* h,
                                                          T* __restrict__ w, double* acc2, const int* st)
 {
@@ -898,41 +943,41 @@ __global__ void __launch_bounds__(kBS) k_gm_update_proj(int64_t n, const T* __re
 #pragma unroll
     for (int c = 0; c < kProjChunks; ++c)
         sums[c] = T(0);
-    const int64_t units = (n + 32 * kUnitRows - 1) / (32 * kUnitRows);
+    const int64_t units = (n + 32 * K - 1) / (32 * K);
     const int64_t warps = static_cast<int64_t>(gridDim.x) * (kBS / 32);
     for (int64_t u = blockIdx.x * static_cast<int64_t>(kBS / 32) + (threadIdx.x >> 5); u < units; u += warps)
     {
-        const int64_t base = u * 32 * kUnitRows + lane;
-        const bool full = (u + 1) * 32 * kUnitRows <= n;
-        T r[kUnitRows];
+        const int64_t base = u * 32 * K + lane;
+        T r[K];
 #pragma unroll
-        for (int k = 0; k < kUnitRows; ++k)
+        for (int k = 0; k < K; ++k)
             r[k] = base + 32 * k < n ? w[base + 32 * k] : T(0);
-#pragma unroll 4
+#pragma unroll 8
         for (int i = 0; i < nv; ++i)
         {
             const T hi = hs[i];
-            const T* Vi = V + static_cast<int64_t>(i) * n;
+            const T* Vi = V + static_cast<int64_t>(i) * n + base;
 #pragma unroll
-            for (int k = 0; k < kUnitRows; ++k)
+            for (int k = 0; k < K; ++k)
                 if (base + 32 * k < n)
-                    r[k] -= hi * Vi[base + 32 * k];
+                    r[k] -= hi * Vi[32 * k];
         }
 #pragma unroll
-        for (int k = 0; k < kUnitRows; ++k)
+        for (int k = 0; k < K; ++k)
             if (base + 32 * k < n)
                 w[base + 32 * k] = r[k];
-        ProjUnit(V, n, nv, base, full, r, sums);
+        ProjUnit<T, K>(V, n, nv, base, r, sums);
     }
     ProjFlush(sums, nv, acc2);
 }
 
 // w -= sum_i h_i V_i with h the second projection (gs + H2), |w|^2; the last block completes Arnoldi column j:
 // H(:, j) = h1 + h2, H(j+1, j) = |w|, earlier rotations applied, new rotation formed, residual estimate |g(j+1)|
-// tested. Row sums of |w|^2 are formed in T per thread and block, one FP64 atomic per block.
+// tested. Row sums of |w|^2 are formed in T per thread and block, one FP64 atomic per block. zsrc (the sweep's output) is
+// kept as the preconditioned basis vector zdst.
 template <typename T>
 __global__ void __launch_bounds__(kBS) k_gm_update(int64_t n, const T* __restrict__ V, int nv, double* gs, T* w,
-                                                    int* st, int j)
+                                                    const T* __restrict__ zsrc, T* __restrict__ zdst, int* st, int j)
 {
     PdlWait();
     PdlTrigger();
@@ -949,9 +994,12 @@ __global__ void __launch_bounds__(kBS) k_gm_update(int64_t n, const T* __restric
          r += static_cast<int64_t>(gridDim.x) * blockDim.x)
     {
         T a = w[r];
+#pragma unroll 8
         for (int i = 0; i < nv; ++i)
             a -= hs[i] * V[static_cast<int64_t>(i) * n + r];
         w[r] = a;
+        if (zsrc)
+            zdst[r] = zsrc[r];
         nrm += a * a;
     }
     nrm = WarpAllSum(nrm);
@@ -965,48 +1013,63 @@ __global__ void __launch_bounds__(kBS) k_gm_update(int64_t n, const T* __restric
             t += sh[q];
         atomicAdd(gs + GL::ACC, static_cast<double>(t));
     }
-    if (LastBlock(st + ST_COUNTER) && threadIdx.x == 0)
+    if (!LastBlock(st + ST_COUNTER))
+        return;
+    // the column and the rotations through shared memory: read one after the other from global memory they took most of
+    // this kernel's time (34 us at j = 44)
+    __shared__ double sH[GL::m + 2], sC[GL::m], sS[GL::m];
+    double* H = gs + GL::H + static_cast<int64_t>(j) * (GL::m + 1);
+    for (int i = threadIdx.x; i <= j; i += blockDim.x)
+    {
+        sH[i] = VRead(gs + GL::H1 + i) + VRead(gs + GL::H2 + i);
+        gs[GL::H1 + i] = 0.;
+        gs[GL::H2 + i] = 0.;
+        if (i < j)
+        {
+            sC[i] = gs[GL::CS + i];
+            sS[i] = gs[GL::SN + i];
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
     {
         st[ST_COUNTER] = 0;
-        double* H = gs + GL::H + static_cast<int64_t>(j) * (GL::m + 1);
-        for (int i = 0; i <= j; ++i)
-        {
-            H[i] = VRead(gs + GL::H1 + i) + VRead(gs + GL::H2 + i);
-            gs[GL::H1 + i] = 0.;
-            gs[GL::H2 + i] = 0.;
-        }
         const double hn = sqrt(VRead(gs + GL::ACC));
         gs[GL::ACC] = 0.;
         // earlier rotations
+        double a = sH[0];
+#pragma unroll 4
         for (int i = 0; i < j; ++i)
         {
-            const double c = gs[GL::CS + i], s = gs[GL::SN + i];
-            const double a = H[i], b = H[i + 1];
-            H[i] = c * a + s * b;
-            H[i + 1] = -s * a + c * b;
+            const double c = sC[i], s = sS[i], b = sH[i + 1];
+            sH[i] = c * a + s * b;
+            a = -s * a + c * b;
         }
-        const double a = H[j], b = hn;
-        const double r = hypot(a, b);
-        const double c = r > 0. ? a / r : 1., s = r > 0. ? b / r : 0.;
+        const double r = hypot(a, hn);
+        const double c = r > 0. ? a / r : 1., s = r > 0. ? hn / r : 0.;
         gs[GL::CS + j] = c;
         gs[GL::SN + j] = s;
-        H[j] = r;
-        H[j + 1] = 0.;
+        sH[j] = r;
+        sH[j + 1] = 0.;
         const double gj = gs[GL::G + j];
         gs[GL::G + j] = c * gj;
-        gs[GL::G + j + 1] = -s * gj;
+        const double gn = -s * gj;
+        gs[GL::G + j + 1] = gn;
         gs[GL::NRM] = hn;
         st[ST_ITERS] += 1;
         st[ST_JDONE] = j + 1;
-        const double res = fabs(gs[GL::G + j + 1]);
+        const double res = fabs(gn);
         if (!isfinite(res) || !isfinite(hn))
             st[ST_STATE] = NONFINITE;
         else if (res * res <= gs[GL::TOL2] || hn == 0.)
             st[ST_STATE] = CONVERGED;
     }
+    __syncthreads();
+    for (int i = threadIdx.x; i <= j + 1; i += blockDim.x)
+        H[i] = sH[i];
 }
 
-// v_j = w / nrm; z = dinv v_j (Jacobi; z == nullptr when the multigrid cycle computes z)
+// v_j = w / nrm; z = dinv v_j (Jacobi) or, with dinv == nullptr, z = v_j (the sweep's input vector)
 template <typename T>
 __global__ void __launch_bounds__(kBS) k_gm_normalize(int64_t n, const T* __restrict__ w, T* vj, T* z,
                                                        const T* __restrict__ dinv, const double* gs, const int* st)
@@ -1022,7 +1085,7 @@ __global__ void __launch_bounds__(kBS) k_gm_normalize(int64_t n, const T* __rest
         const T v = w[r] * inv;
         vj[r] = v;
         if (z)
-            z[r] = dinv[r] * v;
+            z[r] = dinv ? dinv[r] * v : v;
     }
 }
 
@@ -1128,17 +1191,22 @@ static int GmresSolve(Ctx& c, const TV* vals, const double* b, double* x64, bool
     NG_CUDA(cudaMemsetAsync(st, 0, ST_COUNT * sizeof(int), c.stream));
     NG_CUDA(cudaMemsetAsync(gs, 0, GL::SIZE * sizeof(double), c.stream));
     const int grid = GridFor(c, n);
-    // projection kernels: warp units of 32 kUnitRows rows, four blocks per SM
-    const int64_t units = (n + 32 * kUnitRows - 1) / (32 * kUnitRows);
+    // projection kernels: warp units of 32 K rows, four blocks per SM
+    const int unitRows = UnitRows(c, n);
+    const int64_t units = (n + 32 * unitRows - 1) / (32 * unitRows);
     const int gridP = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>((units + kBS / 32 - 1) / (kBS / 32),
                                                                              static_cast<int64_t>(c.smCount) * 4)));
     const unsigned g256 = static_cast<unsigned>((n + 255) / 256);
     const bool amg = c.precond == NUTO_GPU_PRECOND_AMG;
     EnsureNb(c, vals);
+    // the sweep's own input and output vectors where it works in T: the basis vector is written to the one when it is
+    // normalised, the product and the stored basis read the other (FP64 Krylov vectors on an FP32 cycle are converted)
+    T *sweepIn = nullptr, *sweepOut = nullptr;
     if (amg)
     {
         AmgSetup<TV>(c, vals, false);
         G.ensureZ();
+        AmgVectors<T>(c, &sweepIn, &sweepOut);
     }
     else
         k_diag_inv<TV, T><<<g256, 256, 0, c.stream>>>(n, c.dRowPtr.p, c.dColIdx.p, vals, c.dMask.p, K.dinv.p);
@@ -1162,8 +1230,9 @@ static int GmresSolve(Ctx& c, const TV* vals, const double* b, double* x64, bool
         c.stats.kernel_launches += 2;
         k_gm_start<T><<<grid, kBS, 0, c.stream>>>(n, K.r.p, G.w.p, first ? 0 : 1, gs, st);
         first = false;
-        NG_CUDA(LaunchPdl(k_gm_normalize<T>, grid, kBS, 0, c.stream, n, G.w.p, G.V.p, amg ? nullptr : G.z.p, K.dinv.p,
-                          gs, st));
+        T* const znext = amg ? sweepIn : G.z.p;
+        const T* const zdinv = amg ? nullptr : K.dinv.p;
+        NG_CUDA(LaunchPdl(k_gm_normalize<T>, grid, kBS, 0, c.stream, n, G.w.p, G.V.p, znext, zdinv, gs, st));
         const int cols = std::min(m, maxit - total);
         // The cycle is enqueued in chunks: after each chunk the host reads the state and the residual estimate and
         // sizes the next chunk from the observed convergence rate (the iterations still needed, 1 .. 16). Kernels
@@ -1178,17 +1247,30 @@ static int GmresSolve(Ctx& c, const TV* vals, const double* b, double* x64, bool
             {
                 T* vj1 = G.V.p + static_cast<int64_t>(j + 1) * n;
                 T* zj = amg ? G.Z.p + static_cast<int64_t>(j) * n : G.z.p;
-                if (amg)
+                const T* zx = zj; // what the product reads
+                if (sweepIn)
+                {
+                    AmgSweep<T>(c, st, false);
+                    zx = sweepOut;
+                }
+                else if (amg)
                     AmgApply<T>(c, G.V.p + static_cast<int64_t>(j) * n, zj, st, false);
-                SpmvTimed<TV, T, 0>(c, vals, zj, G.w.p, nullptr, nullptr, st, FIN_NONE, c.dMask.p);
+                SpmvTimed<TV, T, 0>(c, vals, zx, G.w.p, nullptr, nullptr, st, FIN_NONE, c.dMask.p);
                 c.stats.kernel_launches += 3 + (j + 1 < cols ? 1 : 0);
-                NG_CUDA(LaunchPdl(k_gm_proj<T>, gridP, kBS, 0, c.stream, n, G.V.p, j + 1, G.w.p, gs + GL::H1, st));
-                NG_CUDA(LaunchPdl(k_gm_update_proj<T>, gridP, kBS, 0, c.stream, n, G.V.p, j + 1, gs + GL::H1, G.w.p,
-                                  gs + GL::H2, st));
-                NG_CUDA(LaunchPdl(k_gm_update<T>, grid, kBS, 0, c.stream, n, G.V.p, j + 1, gs, G.w.p, st, j));
+                auto project = [&](auto k1, auto k2) {
+                    NG_CUDA(LaunchPdl(k1, gridP, kBS, 0, c.stream, n, G.V.p, j + 1, G.w.p, gs + GL::H1, st));
+                    NG_CUDA(LaunchPdl(k2, gridP, kBS, 0, c.stream, n, G.V.p, j + 1, gs + GL::H1, G.w.p, gs + GL::H2, st));
+                };
+                if (unitRows == 4)
+                    project(k_gm_proj<T, 4>, k_gm_update_proj<T, 4>);
+                else if (unitRows == 2)
+                    project(k_gm_proj<T, 2>, k_gm_update_proj<T, 2>);
+                else
+                    project(k_gm_proj<T, 1>, k_gm_update_proj<T, 1>);
+                NG_CUDA(LaunchPdl(k_gm_update<T>, grid, kBS, 0, c.stream, n, G.V.p, j + 1, gs, G.w.p,
+                                  sweepIn ? zx : nullptr, zj, st, j));
                 if (j + 1 < cols)
-                    NG_CUDA(LaunchPdl(k_gm_normalize<T>, grid, kBS, 0, c.stream, n, G.w.p, vj1, amg ? nullptr : G.z.p,
-                                      K.dinv.p, gs, st));
+                    NG_CUDA(LaunchPdl(k_gm_normalize<T>, grid, kBS, 0, c.stream, n, G.w.p, vj1, znext, zdinv, gs, st));
             }
             if (j >= cols)
                 break;

@@ -126,9 +126,10 @@ struct SolverWork
     DBuf<float> xsplit;       // 2n: x as (hi, lo) floats for the compensated FP32 product
     DBuf<uint8_t> zeroMask;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
-    // CUDA-event pairs around the Krylov SpMV launches, folded into stats at synchronisation points
+    // CUDA-event pairs around a sample of the Krylov SpMV launches, folded into stats at synchronisation points
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> spmvEv;
     size_t spmvNext = 0;
+    int64_t spmvCount = 0; // products since the times were last collected
     ~SolverWork();
 };
 
