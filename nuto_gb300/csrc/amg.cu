@@ -922,19 +922,20 @@ __global__ void k_cheb0(int64_t n, const TA* __restrict__ dinv, const TA* __rest
 // One product of the cycle with what precedes and follows it, on the padded layout of one slot pair (rows of ncRow
 // components, columns of ncCol; the structure of k_spmv_nb: G lanes per node, x of the neighbours gathered into shared
 // memory, values streamed with 16-byte loads). With t = A x:
-//   GATHER  how x is formed: CG_VECTOR x = xin; CG_ZERO x = dinv b w0 (the first Chebyshev step from zero)
+//   GATHER  how x is formed: CG_VECTOR x = xin; CG_ZERO x = dinv b w0 (the first Chebyshev step from zero); CG_PROLONG
+//           x = xin + P ce (the coarse correction of unconstrained DOFs)
 //   EPI     CE_RESTRICT  cb += P^T (b - t) over unconstrained rows (cb is zero before; with CG_ZERO also xout = x)
 //           CE_FIRST     d = dinv (b - t) w1; xout = x + d       (first Chebyshev step from a nonzero x)
 //           CE_STEP      d = w2 d + w1 dinv (b - t); xout = x + d (later steps; with CG_ZERO the step before is x itself)
 //           CE_RESIDUAL  xout = b - t (constrained rows: b)
 // xin and xout differ (other rows still gather xin). At the sizes of the coarse levels a launch is what costs: a level takes
-// 3 products and the prolongation (whose up to 8 coarse values per node would be gathered again for each neighbour). On large
-// levels CG_ZERO would put two more loads behind every neighbour of a product that waits for exactly those, and runs as its
-// own kernel (kFuseNodes).
+// 3 products. CG_ZERO puts two more loads behind every neighbour of a product that waits for exactly those, CG_PROLONG up to 8
+// coarse values per component; on larger levels both run as kernels of their own (kFuseNodes, kProlongNodes).
 enum CycleGather
 {
     CG_VECTOR,
-    CG_ZERO
+    CG_ZERO,
+    CG_PROLONG
 };
 enum CycleEpilogue
 {
@@ -944,36 +945,36 @@ enum CycleEpilogue
     CE_RESIDUAL
 };
 constexpr int64_t kFuseNodes = 40000;
+constexpr int64_t kProlongNodes = 2500;
 
 template <typename TA>
 struct CycleArgs
 {
     int64_t nNodes, nRows, nbrTotal, nCoarse; // nRows, nbrTotal, nCoarse: extents for checked builds
     int ncRow, ncCol, seg4;
+    bool early; // the values may be read before the kernel in front has finished
     const int64_t *gdof, *nbrPtr, *nbBase;
-    const int32_t *nbrCol, *pNode;
+    const int32_t *nbrIdx, *nbrCol, *pNode;
     const float* pWeight;
     const TA* vals;      // the pair's first padded value
     const uint8_t* mask; // nullptr: no constrained rows
-    const TA *b, *dinv, *xin;
+    const TA *b, *dinv, *xin, *ce;
     TA *xout, *d, *cb;
     TA w0, w1, w2;
 };
 
 template <typename TA, int G, int GATHER, int EPI>
-__global__ void __launch_bounds__(kBS, NbMinBlocks<TA>()) k_cycle(CycleArgs<TA> A, const int* st)
+__global__ void __launch_bounds__(kBS, sizeof(TA) == 4 ? 5 : 4) k_cycle(CycleArgs<TA> A, const int* st)
 {
-    PdlWait();
-    PdlTrigger();
     extern __shared__ __align__(16) unsigned char cySmem[];
-    if (Idle(st))
-        return;
+    // the structure, and on coarse levels the values, were complete before the kernel in front of this one started: they are
+    // fetched while that kernel runs
     const int gl = threadIdx.x & (G - 1);
     TA* xs = reinterpret_cast<TA*>(cySmem) + (threadIdx.x / G) * A.seg4;
     const int64_t a = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) / G;
     const bool valid = a < A.nNodes;
     const int ncR = valid ? A.ncRow : 0, ncC = A.ncCol;
-    int64_t q0 = 0;
+    int64_t q0 = 0, g0 = 0;
     int nn = 0;
     const TA* vp = A.vals;
     if (valid)
@@ -981,26 +982,74 @@ __global__ void __launch_bounds__(kBS, NbMinBlocks<TA>()) k_cycle(CycleArgs<TA> 
         q0 = A.nbrPtr[a];
         nn = static_cast<int>(A.nbrPtr[a + 1] - q0);
         vp += A.nbBase[a];
-    }
-    // x of one DOF: global row g, component c of node `node`
-    auto value = [&](int64_t g) -> TA { return GATHER == CG_ZERO ? A.dinv[g] * A.b[g] * A.w0 : A.xin[g]; };
-#pragma unroll 4
-    for (int t = gl; t < nn; t += G)
-    {
-        const int64_t col = A.nbrCol[NG_IDX(q0 + t, A.nbrTotal, 60)];
-        for (int d = 0; d < ncC; ++d)
-            xs[t * ncC + d] = value(NG_IDX(col + d, A.nRows, 62));
+        g0 = A.gdof[a];
     }
     const int sg = (ncC * nn + 3) & ~3;
+    int32_t cols[kNbCols];
+#pragma unroll
+    for (int k = 0; k < kNbCols; ++k)
+        cols[k] = gl + k * G < nn ? A.nbrCol[NG_IDX(q0 + gl + k * G, A.nbrTotal, 60)] : 0;
+    TA v0[kMaxComp][4];
+    auto first = [&]() {
+#pragma unroll
+        for (int c = 0; c < kMaxComp; ++c)
+        {
+            if (c < ncR && 4 * gl < sg)
+                Load4(vp + c * sg + 4 * gl, v0[c]);
+            else
+                v0[c][0] = v0[c][1] = v0[c][2] = v0[c][3] = TA(0);
+        }
+    };
+    if (A.early)
+        first();
+    PdlWait();
+    PdlTrigger();
+    if (Idle(st))
+        return;
+    if (!A.early)
+        first();
+    // x of component c at row g of level node b
+    auto value = [&](int64_t g, int64_t b, int c) -> TA {
+        if (GATHER == CG_ZERO)
+            return A.dinv[g] * A.b[g] * A.w0;
+        TA v = A.xin[g];
+        if (GATHER == CG_PROLONG && !(A.mask && A.mask[g]))
+        {
+            int32_t node[kInterp];
+            float w[kInterp];
+            LoadInterp(A.pNode, A.pWeight, b, node, w);
+#pragma unroll
+            for (int k = 0; k < kInterp; ++k)
+                if (node[k] >= 0)
+                    v += static_cast<TA>(w[k]) * A.ce[NG_IDX(static_cast<int64_t>(node[k]) * ncC + c, A.nCoarse, 34)];
+        }
+        return v;
+    };
+    auto gather = [&](int t, int64_t col) {
+        const int64_t b = GATHER == CG_PROLONG ? A.nbrIdx[q0 + t] : 0;
+        for (int d = 0; d < ncC; ++d)
+            xs[t * ncC + d] = value(NG_IDX(col + d, A.nRows, 62), b, d);
+    };
+#pragma unroll
+    for (int k = 0; k < kNbCols; ++k)
+        if (gl + k * G < nn)
+            gather(gl + k * G, cols[k]);
+    for (int t = gl + kNbCols * G; t < nn; t += G)
+        gather(t, A.nbrCol[NG_IDX(q0 + t, A.nbrTotal, 60)]);
     for (int t = ncC * nn + gl; t < sg; t += G)
         xs[t] = TA(0);
     __syncwarp();
     TA s[kMaxComp];
+    {
+        TA xv[4] = {TA(0), TA(0), TA(0), TA(0)};
+        if (4 * gl < sg)
+            Load4(xs + 4 * gl, xv);
 #pragma unroll
-    for (int c = 0; c < kMaxComp; ++c)
-        s[c] = TA(0);
+        for (int c = 0; c < kMaxComp; ++c)
+            s[c] = v0[c][0] * xv[0] + v0[c][1] * xv[1] + v0[c][2] * xv[2] + v0[c][3] * xv[3];
+    }
 #pragma unroll 2
-    for (int f = 4 * gl; f < sg; f += 4 * G)
+    for (int f = 4 * gl + 4 * G; f < sg; f += 4 * G)
     {
         TA xv[4];
         Load4(xs + f, xv);
@@ -1013,26 +1062,18 @@ __global__ void __launch_bounds__(kBS, NbMinBlocks<TA>()) k_cycle(CycleArgs<TA> 
                 s[c] += v[0] * xv[0] + v[1] * xv[1] + v[2] * xv[2] + v[3] * xv[3];
             }
     }
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1)
-#pragma unroll
-        for (int c = 0; c < kMaxComp; ++c)
-            s[c] += __shfl_xor_sync(0xffffffffu, s[c], o);
-    if (gl >= ncR)
+    int comp;
+    const TA t = GroupSum3<G>(s, gl, A.ncRow == 1, comp);
+    if (comp < 0 || comp >= ncR)
         return;
-    // lane c of the group finishes component c
-    TA t = s[0];
-#pragma unroll
-    for (int c = 1; c < kMaxComp; ++c)
-        t = gl == c ? s[c] : t;
-    const int64_t r = NG_IDX(A.gdof[a] + gl, A.nRows, 64);
+    const int64_t r = NG_IDX(g0 + comp, A.nRows, 64);
     const bool fixed = A.mask && A.mask[r];
     if (EPI == CE_RESIDUAL)
     {
         A.xout[r] = fixed ? A.b[r] : A.b[r] - t;
         return;
     }
-    const TA x = value(r);
+    const TA x = value(r, a, comp);
     const TA res = A.b[r] - (fixed ? x : t);
     if (EPI == CE_RESTRICT)
     {
@@ -1046,7 +1087,7 @@ __global__ void __launch_bounds__(kBS, NbMinBlocks<TA>()) k_cycle(CycleArgs<TA> 
 #pragma unroll
         for (int k = 0; k < kInterp; ++k)
             if (node[k] >= 0)
-                atomicAdd(A.cb + NG_IDX(static_cast<int64_t>(node[k]) * A.ncRow + gl, A.nCoarse, 33),
+                atomicAdd(A.cb + NG_IDX(static_cast<int64_t>(node[k]) * A.ncRow + comp, A.nCoarse, 33),
                           static_cast<TA>(w[k]) * res);
         return;
     }
@@ -1594,6 +1635,8 @@ static CycleArgs<TA> LevelArgs(Ctx& c, AmgLevel& L, bool fine)
     A.gdof = V.gdof[0];
     A.nbrPtr = V.nbrPtr[0];
     A.nbrCol = V.nbrCol[0];
+    A.nbrIdx = V.nbrIdx[0];
+    A.early = !fine; // filled by the set-up, which ends with a synchronisation
     A.nbBase = V.nbBase[0];
     A.vals = NbValues<TA>(V) + V.nbOff[0];
     A.mask = fine ? c.dMask.p : nullptr;
@@ -1699,15 +1742,21 @@ static void VCycle(Ctx& c, int I, size_t l, const TA* b, TA* e, const int* st, b
     }
     VCycle<TA>(c, I, l + 1, CU.b, CU.e.p, st, sym);
     // coarse correction and two post-smoothing steps: e -> t -> e
-    NG_CUDA(LaunchPdl(k_prolong<TA>, Blocks(n), 256, 0, c.stream, L.spmv, l == 0 ? c.dMask.p : L.zeroMask.p,
-                      static_cast<const int32_t*>(Co.nodes->pNode.p), static_cast<const float*>(Co.nodes->pWeight.p), Co.nDofs,
-                      static_cast<const TA*>(CU.e.p), e, st));
-    c.stats.kernel_launches += 1;
     A.xin = e;
     A.xout = U.t.p;
+    A.ce = CU.e.p;
     Cheb C(L, kSmoothRatio);
     A.w1 = TA(1. / C.theta);
-    LaunchCycle<TA, CG_VECTOR, CE_FIRST>(c, A, st);
+    if (L.nNodes <= kProlongNodes)
+        LaunchCycle<TA, CG_PROLONG, CE_FIRST>(c, A, st);
+    else
+    {
+        NG_CUDA(LaunchPdl(k_prolong<TA>, Blocks(n), 256, 0, c.stream, L.spmv, l == 0 ? c.dMask.p : L.zeroMask.p,
+                          static_cast<const int32_t*>(Co.nodes->pNode.p), static_cast<const float*>(Co.nodes->pWeight.p),
+                          Co.nDofs, static_cast<const TA*>(CU.e.p), e, st));
+        c.stats.kernel_launches += 1;
+        LaunchCycle<TA, CG_VECTOR, CE_FIRST>(c, A, st);
+    }
     static_assert(kPostDegree == 2, "two post-smoothing steps");
     coefficients(C);
     A.xin = U.t.p;

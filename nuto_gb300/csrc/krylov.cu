@@ -1017,7 +1017,7 @@ __global__ void __launch_bounds__(kBS) k_gm_update(int64_t n, const T* __restric
         return;
     // the column and the rotations through shared memory: read one after the other from global memory they took most of
     // this kernel's time (34 us at j = 44)
-    __shared__ double sH[GL::m + 2], sC[GL::m], sS[GL::m];
+    __shared__ double sH[GL::m + 1], sC[GL::m], sS[GL::m], sA[GL::m], sB[GL::m];
     double* H = gs + GL::H + static_cast<int64_t>(j) * (GL::m + 1);
     for (int i = threadIdx.x; i <= j; i += blockDim.x)
     {
@@ -1031,26 +1031,29 @@ __global__ void __launch_bounds__(kBS) k_gm_update(int64_t n, const T* __restric
         }
     }
     __syncthreads();
+    for (int i = threadIdx.x; i < j; i += blockDim.x)
+        sB[i] = sC[i] * sH[i + 1];
+    __syncthreads();
     if (threadIdx.x == 0)
     {
         st[ST_COUNTER] = 0;
         const double hn = sqrt(VRead(gs + GL::ACC));
         gs[GL::ACC] = 0.;
-        // earlier rotations
+        // earlier rotations: the serial part is one fused multiply-add per rotation, the rest is formed by all threads
+        // before (sB) and after (sH)
         double a = sH[0];
 #pragma unroll 4
         for (int i = 0; i < j; ++i)
         {
-            const double c = sC[i], s = sS[i], b = sH[i + 1];
-            sH[i] = c * a + s * b;
-            a = -s * a + c * b;
+            sA[i] = a;
+            a = sB[i] - sS[i] * a;
         }
         const double r = hypot(a, hn);
         const double c = r > 0. ? a / r : 1., s = r > 0. ? hn / r : 0.;
         gs[GL::CS + j] = c;
         gs[GL::SN + j] = s;
-        sH[j] = r;
-        sH[j + 1] = 0.;
+        H[j] = r;
+        H[j + 1] = 0.;
         const double gj = gs[GL::G + j];
         gs[GL::G + j] = c * gj;
         const double gn = -s * gj;
@@ -1065,8 +1068,8 @@ __global__ void __launch_bounds__(kBS) k_gm_update(int64_t n, const T* __restric
             st[ST_STATE] = CONVERGED;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i <= j + 1; i += blockDim.x)
-        H[i] = sH[i];
+    for (int i = threadIdx.x; i < j; i += blockDim.x)
+        H[i] = sC[i] * sA[i] + sS[i] * sH[i + 1];
 }
 
 // v_j = w / nrm; z = dinv v_j (Jacobi) or, with dinv == nullptr, z = v_j (the sweep's input vector)

@@ -317,17 +317,44 @@ constexpr int NbMinBlocks()
     return sizeof(TV) == 4 ? 6 : 4;
 }
 
+// Sums of s[0..2] over groups of G lanes. Three components: the first two steps halve the number of values a lane holds (4
+// additions for 8 lanes instead of 9; FP64 additions are what the small levels of the cycle spend their time on), and the lane
+// that returns with comp >= 0 holds the sum of component comp. One component (scalar): lane 0.
+template <int G, typename T>
+__device__ __forceinline__ T GroupSum3(const T (&s)[kMaxComp], int gl, bool scalar, int& comp)
+{
+    static_assert(kMaxComp == 3 && G >= 4, "pairs of components over the two upper lane bits");
+    if (scalar)
+    {
+        T t = s[0];
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1)
+            t += __shfl_xor_sync(0xffffffffu, t, o);
+        comp = gl == 0 ? 0 : -1;
+        return t;
+    }
+    const bool hi = gl & (G / 2), mid = gl & (G / 4);
+    T a0 = hi ? s[2] : s[0], a1 = hi ? T(0) : s[1];
+    a0 += __shfl_xor_sync(0xffffffffu, hi ? s[0] : s[2], G / 2);
+    a1 += __shfl_xor_sync(0xffffffffu, hi ? s[1] : T(0), G / 2);
+    T t = (mid ? a1 : a0) + __shfl_xor_sync(0xffffffffu, mid ? a0 : a1, G / 4);
+#pragma unroll
+    for (int o = G / 8; o > 0; o >>= 1)
+        t += __shfl_xor_sync(0xffffffffu, t, o);
+    comp = (gl & (G / 4 - 1)) == 0 && !(hi && mid) ? (hi ? 2 : 0) + (mid ? 1 : 0) : -1;
+    return t;
+}
+
+constexpr int kNbCols = 4; // neighbours per lane whose columns are fetched before the wait: 27 over 8 lanes
+
 template <typename TV, typename TX, int NDOT, int G>
 __global__ void __launch_bounds__(kBS, NbMinBlocks<TV>()) k_spmv_nb(NodeSpmv A, const uint8_t* __restrict__ mask,
                                                   const TX* __restrict__ x, TX* __restrict__ y,
                                                   const TX* __restrict__ w0, double* sc, int* st, int fin)
 {
-    PdlWait();
-    PdlTrigger();
     extern __shared__ __align__(16) unsigned char nbSmem[];
     __shared__ double sh[kBS / 32];
-    if (st && st[ST_STATE] != RUN)
-        return;
+    // the structure (host-built) is fetched while the kernel in front still runs
     const TV* __restrict__ vals = NbValues<TV>(A);
     const int gl = threadIdx.x & (G - 1);
     const int L = A.nbSeg4;
@@ -368,18 +395,34 @@ __global__ void __launch_bounds__(kBS, NbMinBlocks<TV>()) k_spmv_nb(NodeSpmv A, 
     // x of all neighbours of all column slots into the group's segment buffers (unrolled: several neighbour ->
     // x chains in flight per lane)
     const int nc0 = A.ncomp[0], nc1 = A.ns > 1 ? A.ncomp[1] : 0;
-#pragma unroll 4
-    for (int t = gl; t < tot; t += G)
-    {
+    auto column = [&](int t) -> int32_t {
         const int J = t >= nn[0] ? 1 : 0;
-        const int kk = t - (J ? nn[0] : 0);
-        const int ncJ = J ? nc1 : nc0;
         const int p = I * A.ns + J;
-        const int64_t col = A.nbrCol[p][NG_IDX((J ? q0[1] : q0[0]) + kk, A.nbrTotal[p], 60)];
-        const int xb = (J ? xoff[1] : 0) + kk * ncJ;
+        return A.nbrCol[p][NG_IDX((J ? q0[1] : q0[0]) + t - (J ? nn[0] : 0), A.nbrTotal[p], 60)];
+    };
+    auto gather = [&](int t, int64_t col) {
+        const int J = t >= nn[0] ? 1 : 0;
+        const int ncJ = J ? nc1 : nc0;
+        const int xb = (J ? xoff[1] : 0) + (t - (J ? nn[0] : 0)) * ncJ;
         for (int d = 0; d < ncJ; ++d)
             xs[NG_IDX(xb + d, L, 61)] = x[NG_IDX(col + d, A.nRows, 62)];
-    }
+    };
+    int32_t cols[kNbCols];
+#pragma unroll
+    for (int k = 0; k < kNbCols; ++k)
+        cols[k] = gl + k * G < tot ? column(gl + k * G) : 0;
+    const int64_t g0 = valid ? A.gdof[I][a] : 0;
+    PdlWait();
+    PdlTrigger();
+    if (st && st[ST_STATE] != RUN)
+        return;
+#pragma unroll
+    for (int k = 0; k < kNbCols; ++k)
+        if (gl + k * G < tot)
+            gather(gl + k * G, cols[k]);
+#pragma unroll 4
+    for (int t = gl + kNbCols * G; t < tot; t += G)
+        gather(t, column(t));
 #pragma unroll
     for (int J = 0; J < kMaxSlots; ++J)
     {
@@ -414,28 +457,18 @@ __global__ void __launch_bounds__(kBS, NbMinBlocks<TV>()) k_spmv_nb(NodeSpmv A, 
                 }
         }
     }
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1)
-#pragma unroll
-        for (int c = 0; c < kMaxComp; ++c)
-            s[c] += __shfl_xor_sync(0xffffffffu, s[c], o);
+    int comp;
+    const TX sum = GroupSum3<G>(s, gl, A.ncMaxRows == 1, comp);
     double d0 = 0., d1 = 0.;
-    if (valid && gl == 0)
+    if (comp >= 0 && comp < ncI)
     {
-        const int64_t g0 = A.gdof[I][a];
-#pragma unroll
-        for (int c = 0; c < kMaxComp; ++c)
-        {
-            if (c >= ncI)
-                break;
-            const int64_t r = NG_IDX(g0 + c, A.nRows, 64);
-            const TX yv = mask[r] ? x[r] : s[c];
-            y[r] = yv;
-            if (NDOT >= 1)
-                d0 += static_cast<double>(w0[r]) * static_cast<double>(yv);
-            if (NDOT >= 2)
-                d1 += static_cast<double>(yv) * static_cast<double>(yv);
-        }
+        const int64_t r = NG_IDX(g0 + comp, A.nRows, 64);
+        const TX yv = mask[r] ? x[r] : sum;
+        y[r] = yv;
+        if (NDOT >= 1)
+            d0 += static_cast<double>(w0[r]) * static_cast<double>(yv);
+        if (NDOT >= 2)
+            d1 += static_cast<double>(yv) * static_cast<double>(yv);
     }
     if (NDOT == 0)
         return;
