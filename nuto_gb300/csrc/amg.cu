@@ -964,7 +964,7 @@ struct CycleArgs
 };
 
 template <typename TA, int G, int GATHER, int EPI>
-__global__ void __launch_bounds__(kBS, sizeof(TA) == 4 ? 5 : 4) k_cycle(CycleArgs<TA> A, const int* st)
+__global__ void __launch_bounds__(kBS, sizeof(TA) == 4 ? 5 : 3) k_cycle(CycleArgs<TA> A, const int* st)
 {
     extern __shared__ __align__(16) unsigned char cySmem[];
     // the structure, and on coarse levels the values, were complete before the kernel in front of this one started: they are

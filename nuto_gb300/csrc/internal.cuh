@@ -74,8 +74,8 @@ __device__ __forceinline__ long long CheckedIndex(long long i, long long n, int 
 // ---- programmatic dependent launch -----------------------------------------------------------------------------
 // The kernels of the Krylov iteration and the multigrid cycle are launched with programmatic stream serialisation:
 // a kernel's blocks may be scheduled while its predecessor in the stream drains, which hides most of the gap
-// between the many short launches of a cycle. Every such kernel calls PdlWait() before its first global memory
-// access (it returns once the predecessor grid has completed and its writes are visible; without the launch
+// between the many short launches of a cycle. Every such kernel calls PdlWait() before its first access to anything that the
+// kernel in front of it writes (it returns once the predecessor grid has completed and its writes are visible; without the launch
 // attribute it returns at once) and PdlTrigger() right after, so that its own successor may be scheduled once all
 // of its blocks are running. NUTO_GPU_PDL=0 launches them normally.
 __device__ __forceinline__ void PdlWait()

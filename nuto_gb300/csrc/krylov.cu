@@ -784,8 +784,8 @@ void SpmvFull64(Ctx& c, int precision, const void* vals, const double* x, double
 // ---- restarted GMRES(m), right Jacobi preconditioning ----------------------------------------------------------
 // Arnoldi with classical Gram-Schmidt and one re-orthogonalisation (CGS2) in three passes over the basis
 // (projection; update fused with the second projection; second update with the norm). The FP64 Hessenberg column,
-// its Givens rotation and the residual estimate are formed by the last block of the second update, so a whole cycle
-// is enqueued without a host round trip. The basis is stored in T (FP32 or FP64).
+// its Givens rotation and the residual estimate are formed by one block of the normalisation, so a whole cycle is enqueued
+// without a host round trip. The basis is stored in T (FP32 or FP64).
 using GL = GmresLayout;
 
 // Projections on the basis in warp units: a unit is 32 x K consecutive rows, lane l reading rows base + l + 32 k, so every
@@ -899,12 +899,14 @@ __device__ __forceinline__ void ProjUnit(const T* __restrict__ V, int64_t n, int
 // acc[i] += V_i . w for i < nv
 template <typename T, int K>
 __global__ void __launch_bounds__(kBS) k_gm_proj(int64_t n, const T* __restrict__ V, int nv, const T* __restrict__ w,
-                                                  double* acc, const int* st)
+                                                  double* acc, double* norm, const int* st)
 {
     PdlWait();
     PdlTrigger();
     if (st[ST_STATE] != RUN)
         return;
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        *norm = 0.; // k_gm_update adds to it, k_gm_normalize of the iteration before has read it
     const int lane = threadIdx.x & 31;
     T sums[kProjChunks];
 #pragma unroll
@@ -977,7 +979,7 @@ __global__ void __launch_bounds__(kBS) k_gm_update_proj(int64_t n, const T* __re
 // kept as the preconditioned basis vector zdst.
 template <typename T>
 __global__ void __launch_bounds__(kBS) k_gm_update(int64_t n, const T* __restrict__ V, int nv, double* gs, T* w,
-                                                    const T* __restrict__ zsrc, T* __restrict__ zdst, int* st, int j)
+                                                    const T* __restrict__ zsrc, T* __restrict__ zdst, const int* st)
 {
     PdlWait();
     PdlTrigger();
@@ -1013,49 +1015,64 @@ __global__ void __launch_bounds__(kBS) k_gm_update(int64_t n, const T* __restric
             t += sh[q];
         atomicAdd(gs + GL::ACC, static_cast<double>(t));
     }
-    if (!LastBlock(st + ST_COUNTER))
+}
+
+// Column j of the Hessenberg matrix (both projections' sums and the norm), its rotations and the residual estimate; the first
+// warp of a block. The earlier rotations leave a_i+1 = c_i h_i+1 - s_i a_i: composed as affine maps by a scan over the lanes,
+// since one dependent FP64 operation takes about 50 ns here and a column has up to kGmresMax of them.
+static __device__ __forceinline__ void GivensColumn(double* gs, int* st, int j)
+{
+    __shared__ double sH[GL::m + 1];
+    const int lane = threadIdx.x;
+    if (lane >= 32)
         return;
-    // the column and the rotations through shared memory: read one after the other from global memory they took most of
-    // this kernel's time (34 us at j = 44)
-    __shared__ double sH[GL::m + 1], sC[GL::m], sS[GL::m], sA[GL::m], sB[GL::m];
     double* H = gs + GL::H + static_cast<int64_t>(j) * (GL::m + 1);
-    for (int i = threadIdx.x; i <= j; i += blockDim.x)
+    for (int i = lane; i <= j; i += 32)
     {
         sH[i] = VRead(gs + GL::H1 + i) + VRead(gs + GL::H2 + i);
         gs[GL::H1 + i] = 0.;
         gs[GL::H2 + i] = 0.;
-        if (i < j)
-        {
-            sC[i] = gs[GL::CS + i];
-            sS[i] = gs[GL::SN + i];
-        }
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < j; i += blockDim.x)
-        sB[i] = sC[i] * sH[i + 1];
-    __syncthreads();
-    if (threadIdx.x == 0)
+    const double hn2 = VRead(gs + GL::ACC);
+    __syncwarp();
+    double a = sH[0]; // in front of rotation i0
+    for (int i0 = 0; i0 < j; i0 += 32)
     {
-        st[ST_COUNTER] = 0;
-        const double hn = sqrt(VRead(gs + GL::ACC));
-        gs[GL::ACC] = 0.;
-        // earlier rotations: the serial part is one fused multiply-add per rotation, the rest is formed by all threads
-        // before (sB) and after (sH)
-        double a = sH[0];
-#pragma unroll 4
-        for (int i = 0; i < j; ++i)
+        const int i = i0 + lane;
+        const double c = i < j ? gs[GL::CS + i] : 0., s = i < j ? gs[GL::SN + i] : 0.;
+        const double h = i < j ? sH[i + 1] : 0.;
+        // behind rotation i: m a + b
+        double m = i < j ? -s : 1., b = c * h;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
         {
-            sA[i] = a;
-            a = sB[i] - sS[i] * a;
+            const double mb = __shfl_up_sync(0xffffffffu, m, o), bb = __shfl_up_sync(0xffffffffu, b, o);
+            if (lane >= o)
+            {
+                b += m * bb;
+                m *= mb;
+            }
         }
-        const double r = hypot(a, hn);
-        const double c = r > 0. ? a / r : 1., s = r > 0. ? hn / r : 0.;
-        gs[GL::CS + j] = c;
-        gs[GL::SN + j] = s;
+        const double after = m * a + b;
+        const double up = __shfl_up_sync(0xffffffffu, after, 1);
+        const double before = lane == 0 ? a : up;
+        if (i < j)
+            H[i] = c * before + s * h;
+        a = __shfl_sync(0xffffffffu, after, 31);
+    }
+    // the new rotation: lane 0 forms c, lane 1 s
+    const double r = sqrt(a * a + hn2);
+    const double top = lane == 1 ? sqrt(hn2) : a;
+    const double cs = r > 0. ? top / r : (lane == 1 ? 0. : 1.);
+    const double hn = __shfl_sync(0xffffffffu, top, 1), s = __shfl_sync(0xffffffffu, cs, 1);
+    if (lane == 0)
+    {
         H[j] = r;
         H[j + 1] = 0.;
+        gs[GL::CS + j] = cs;
+        gs[GL::SN + j] = s;
         const double gj = gs[GL::G + j];
-        gs[GL::G + j] = c * gj;
+        gs[GL::G + j] = cs * gj;
         const double gn = -s * gj;
         gs[GL::G + j + 1] = gn;
         gs[GL::NRM] = hn;
@@ -1067,28 +1084,35 @@ __global__ void __launch_bounds__(kBS) k_gm_update(int64_t n, const T* __restric
         else if (res * res <= gs[GL::TOL2] || hn == 0.)
             st[ST_STATE] = CONVERGED;
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < j; i += blockDim.x)
-        H[i] = sC[i] * sA[i] + sS[i] * sH[i + 1];
 }
 
-// v_j = w / nrm; z = dinv v_j (Jacobi) or, with dinv == nullptr, z = v_j (the sweep's input vector)
+// v = w / |w|; z = dinv v (Jacobi) or, with dinv == nullptr, z = v (the sweep's input vector). j >= 0: |w|^2 is the sum left by
+// k_gm_update, and block 0 finishes column j meanwhile (nothing is in the next kernels' way but the state); a state that ends the
+// solve may keep other blocks from writing v and z, which nothing reads then. j < 0: |w| from k_gm_start. v == nullptr: only
+// the column.
 template <typename T>
-__global__ void __launch_bounds__(kBS) k_gm_normalize(int64_t n, const T* __restrict__ w, T* vj, T* z,
-                                                       const T* __restrict__ dinv, const double* gs, const int* st)
+__global__ void __launch_bounds__(kBS) k_gm_normalize(int64_t n, const T* __restrict__ w, T* v, T* z,
+                                                       const T* __restrict__ dinv, double* gs, int* st, int j)
 {
     PdlWait();
     PdlTrigger();
     if (st[ST_STATE] != RUN)
         return;
-    const T inv = static_cast<T>(1. / gs[GL::NRM]);
-    for (int64_t r = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; r < n;
-         r += static_cast<int64_t>(gridDim.x) * blockDim.x)
+    if (j >= 0 && blockIdx.x == 0)
     {
-        const T v = w[r] * inv;
-        vj[r] = v;
+        GivensColumn(gs, st, j);
+        return;
+    }
+    const double nrm = j >= 0 ? sqrt(gs[GL::ACC]) : gs[GL::NRM];
+    const T inv = static_cast<T>(nrm > 0. ? 1. / nrm : 0.);
+    const int first = j >= 0 ? 1 : 0;
+    for (int64_t r = (blockIdx.x - first) * static_cast<int64_t>(blockDim.x) + threadIdx.x; r < n;
+         r += static_cast<int64_t>(gridDim.x - first) * blockDim.x)
+    {
+        const T a = w[r] * inv;
+        v[r] = a;
         if (z)
-            z[r] = dinv ? dinv[r] * v : v;
+            z[r] = dinv ? dinv[r] * a : a;
     }
 }
 
@@ -1231,11 +1255,12 @@ static int GmresSolve(Ctx& c, const TV* vals, const double* b, double* x64, bool
         if (!first)
             SpmvTimed<TV, T, 0>(c, vals, K.x.p, G.w.p, nullptr, nullptr, nullptr, FIN_NONE, c.dMask.p);
         c.stats.kernel_launches += 2;
+        NG_CUDA(cudaMemsetAsync(gs + GL::ACC, 0, sizeof(double), c.stream)); // holds the last column's norm
         k_gm_start<T><<<grid, kBS, 0, c.stream>>>(n, K.r.p, G.w.p, first ? 0 : 1, gs, st);
         first = false;
         T* const znext = amg ? sweepIn : G.z.p;
         const T* const zdinv = amg ? nullptr : K.dinv.p;
-        NG_CUDA(LaunchPdl(k_gm_normalize<T>, grid, kBS, 0, c.stream, n, G.w.p, G.V.p, znext, zdinv, gs, st));
+        NG_CUDA(LaunchPdl(k_gm_normalize<T>, grid, kBS, 0, c.stream, n, G.w.p, G.V.p, znext, zdinv, gs, st, -1));
         const int cols = std::min(m, maxit - total);
         // The cycle is enqueued in chunks: after each chunk the host reads the state and the residual estimate and
         // sizes the next chunk from the observed convergence rate (the iterations still needed, 1 .. 16). Kernels
@@ -1259,9 +1284,10 @@ static int GmresSolve(Ctx& c, const TV* vals, const double* b, double* x64, bool
                 else if (amg)
                     AmgApply<T>(c, G.V.p + static_cast<int64_t>(j) * n, zj, st, false);
                 SpmvTimed<TV, T, 0>(c, vals, zx, G.w.p, nullptr, nullptr, st, FIN_NONE, c.dMask.p);
-                c.stats.kernel_launches += 3 + (j + 1 < cols ? 1 : 0);
+                c.stats.kernel_launches += 4;
                 auto project = [&](auto k1, auto k2) {
-                    NG_CUDA(LaunchPdl(k1, gridP, kBS, 0, c.stream, n, G.V.p, j + 1, G.w.p, gs + GL::H1, st));
+                    NG_CUDA(LaunchPdl(k1, gridP, kBS, 0, c.stream, n, G.V.p, j + 1, G.w.p, gs + GL::H1,
+                                      gs + GL::ACC, st));
                     NG_CUDA(LaunchPdl(k2, gridP, kBS, 0, c.stream, n, G.V.p, j + 1, gs + GL::H1, G.w.p, gs + GL::H2, st));
                 };
                 if (unitRows == 4)
@@ -1271,9 +1297,11 @@ static int GmresSolve(Ctx& c, const TV* vals, const double* b, double* x64, bool
                 else
                     project(k_gm_proj<T, 1>, k_gm_update_proj<T, 1>);
                 NG_CUDA(LaunchPdl(k_gm_update<T>, grid, kBS, 0, c.stream, n, G.V.p, j + 1, gs, G.w.p,
-                                  sweepIn ? zx : nullptr, zj, st, j));
-                if (j + 1 < cols)
-                    NG_CUDA(LaunchPdl(k_gm_normalize<T>, grid, kBS, 0, c.stream, n, G.w.p, vj1, znext, zdinv, gs, st));
+                                  sweepIn ? zx : nullptr, zj, st));
+                // the last column of a cycle has no next vector
+                const bool last = j + 1 == cols;
+                NG_CUDA(LaunchPdl(k_gm_normalize<T>, last ? 1 : grid + 1, kBS, 0, c.stream, n, G.w.p, last ? nullptr : vj1,
+                                  znext, zdinv, gs, st, j));
             }
             if (j >= cols)
                 break;
@@ -1554,7 +1582,7 @@ int SolveLinear(Ctx& c, int precision, int method, const void* values, const dou
     double rel = bnorm > 0 ? 1. : 0.;
     for (int sweep = 0; sweep < 30 && rel > rtol && total < maxit; ++sweep)
     {
-        const double inner = std::max(rtol / std::max(rel, 1e-300), 1e-5);
+        const double inner = std::max(rtol / std::max(rel, 1e-300), 1e-4);
         int it = 0;
         KrylovSolve<float, float>(c, meth, static_cast<const float*>(values), w.rhs.p, x, true,
                                   std::min(inner, 0.5), maxit - total, &it, nullptr);
