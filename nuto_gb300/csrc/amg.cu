@@ -85,6 +85,7 @@ struct LevelNodes
     DBuf<int32_t> dNbrIdx;
     DBuf<int32_t> pNode; // kInterp per finer node: nodes of this level, -1 behind the last
     DBuf<float> pWeight; // and their weights
+    DBuf<double> pWeight64; // the same values for the FP64 cycle (a conversion is an FP64 instruction), on first use
 };
 
 struct AmgLevel
@@ -169,6 +170,14 @@ struct Amg
     cudaStream_t capStream = nullptr; // private stream for graph capture (the context's may be the legacy stream)
 };
 
+template <typename TA>
+static DBuf<TA>& Weights(LevelNodes& X)
+{
+    if constexpr (sizeof(TA) == 4)
+        return X.pWeight;
+    else
+        return X.pWeight64;
+}
 template <typename TA>
 static DBuf<TA>& Rhs(Amg& M)
 {
@@ -889,21 +898,23 @@ __device__ __forceinline__ bool Idle(const int* st)
 }
 
 // the interpolation entries of node a
-__device__ __forceinline__ void LoadInterp(const int32_t* __restrict__ pNode, const float* __restrict__ pWeight, int64_t a,
-                                           int32_t (&node)[kInterp], float (&w)[kInterp])
+template <typename TA>
+__device__ __forceinline__ void LoadInterp(const int32_t* __restrict__ pNode, const TA* __restrict__ pWeight, int64_t a,
+                                           int32_t (&node)[kInterp], TA (&w)[kInterp])
 {
-    static_assert(kInterp == 8, "two 16-byte loads each");
-    const int4* pn = reinterpret_cast<const int4*>(pNode + a * kInterp);
-    const float4* pw = reinterpret_cast<const float4*>(pWeight + a * kInterp);
-    const int4 n0 = pn[0], n1 = pn[1];
-    const float4 w0 = pw[0], w1 = pw[1];
-    const int32_t n[8] = {n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, n1.z, n1.w};
-    const float v[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
-    for (int k = 0; k < kInterp; ++k)
+    for (int k = 0; k < kInterp; k += 4)
     {
-        node[k] = n[k];
-        w[k] = v[k];
+        const int4 n = *reinterpret_cast<const int4*>(pNode + a * kInterp + k);
+        node[k] = n.x;
+        node[k + 1] = n.y;
+        node[k + 2] = n.z;
+        node[k + 3] = n.w;
+        TA v[4];
+        Load4(pWeight + a * kInterp + k, v);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            w[k + q] = v[q];
     }
 }
 
@@ -947,6 +958,20 @@ enum CycleEpilogue
 constexpr int64_t kFuseNodes = 40000;
 constexpr int64_t kProlongNodes = 2500;
 
+// Quadruples of values per row that a lane holds before it has x. FP64: a whole row of 27 neighbours x 3 components, with the
+// registers of 2 blocks per SM (20^3: 16.4 us with one quadruple and 3 blocks, 10.9 us); FP32: one, with those of 5 (two to
+// three and 4 blocks were 5 % slower at 64^3).
+template <typename TA, int G>
+constexpr int CycleAhead()
+{
+    return sizeof(TA) == 4 || G >= 32 ? 1 : (G >= 16 ? 2 : 3);
+}
+template <typename TA>
+constexpr int CycleMinBlocks()
+{
+    return sizeof(TA) == 4 ? 5 : 2;
+}
+
 template <typename TA>
 struct CycleArgs
 {
@@ -955,7 +980,7 @@ struct CycleArgs
     bool early; // the values may be read before the kernel in front has finished
     const int64_t *gdof, *nbrPtr, *nbBase;
     const int32_t *nbrIdx, *nbrCol, *pNode;
-    const float* pWeight;
+    const TA* pWeight;
     const TA* vals;      // the pair's first padded value
     const uint8_t* mask; // nullptr: no constrained rows
     const TA *b, *dinv, *xin, *ce;
@@ -964,7 +989,7 @@ struct CycleArgs
 };
 
 template <typename TA, int G, int GATHER, int EPI>
-__global__ void __launch_bounds__(kBS, sizeof(TA) == 4 ? 5 : 3) k_cycle(CycleArgs<TA> A, const int* st)
+__global__ void __launch_bounds__(kBS, CycleMinBlocks<TA>()) k_cycle(CycleArgs<TA> A, const int* st)
 {
     extern __shared__ __align__(16) unsigned char cySmem[];
     // the structure, and on coarse levels the values, were complete before the kernel in front of this one started: they are
@@ -989,21 +1014,24 @@ __global__ void __launch_bounds__(kBS, sizeof(TA) == 4 ? 5 : 3) k_cycle(CycleArg
 #pragma unroll
     for (int k = 0; k < kNbCols; ++k)
         cols[k] = gl + k * G < nn ? A.nbrCol[NG_IDX(q0 + gl + k * G, A.nbrTotal, 60)] : 0;
-    TA v0[kMaxComp][4];
+    constexpr int kAhead = CycleAhead<TA, G>();
+    TA v0[kAhead][kMaxComp][4];
     auto first = [&]() {
 #pragma unroll
-        for (int c = 0; c < kMaxComp; ++c)
-        {
-            if (c < ncR && 4 * gl < sg)
-                Load4(vp + c * sg + 4 * gl, v0[c]);
-            else
-                v0[c][0] = v0[c][1] = v0[c][2] = v0[c][3] = TA(0);
-        }
+        for (int h = 0; h < kAhead; ++h)
+#pragma unroll
+            for (int c = 0; c < kMaxComp; ++c)
+            {
+                const int f = 4 * (gl + h * G);
+                if (c < ncR && f < sg)
+                    Load4(vp + c * sg + f, v0[h][c]);
+                else
+                    v0[h][c][0] = v0[h][c][1] = v0[h][c][2] = v0[h][c][3] = TA(0);
+            }
     };
     if (A.early)
         first();
     PdlWait();
-    PdlTrigger();
     if (Idle(st))
         return;
     if (!A.early)
@@ -1016,12 +1044,12 @@ __global__ void __launch_bounds__(kBS, sizeof(TA) == 4 ? 5 : 3) k_cycle(CycleArg
         if (GATHER == CG_PROLONG && !(A.mask && A.mask[g]))
         {
             int32_t node[kInterp];
-            float w[kInterp];
+            TA w[kInterp];
             LoadInterp(A.pNode, A.pWeight, b, node, w);
 #pragma unroll
             for (int k = 0; k < kInterp; ++k)
                 if (node[k] >= 0)
-                    v += static_cast<TA>(w[k]) * A.ce[NG_IDX(static_cast<int64_t>(node[k]) * ncC + c, A.nCoarse, 34)];
+                    v += w[k] * A.ce[NG_IDX(static_cast<int64_t>(node[k]) * ncC + c, A.nCoarse, 34)];
         }
         return v;
     };
@@ -1040,16 +1068,21 @@ __global__ void __launch_bounds__(kBS, sizeof(TA) == 4 ? 5 : 3) k_cycle(CycleArg
         xs[t] = TA(0);
     __syncwarp();
     TA s[kMaxComp];
-    {
-        TA xv[4] = {TA(0), TA(0), TA(0), TA(0)};
-        if (4 * gl < sg)
-            Load4(xs + 4 * gl, xv);
 #pragma unroll
-        for (int c = 0; c < kMaxComp; ++c)
-            s[c] = v0[c][0] * xv[0] + v0[c][1] * xv[1] + v0[c][2] * xv[2] + v0[c][3] * xv[3];
-    }
+    for (int c = 0; c < kMaxComp; ++c)
+        s[c] = TA(0);
+#pragma unroll
+    for (int h = 0; h < kAhead; ++h)
+        if (4 * (gl + h * G) < sg)
+        {
+            TA xv[4];
+            Load4(xs + 4 * (gl + h * G), xv);
+#pragma unroll
+            for (int c = 0; c < kMaxComp; ++c)
+                s[c] += v0[h][c][0] * xv[0] + v0[h][c][1] * xv[1] + v0[h][c][2] * xv[2] + v0[h][c][3] * xv[3];
+        }
 #pragma unroll 2
-    for (int f = 4 * gl + 4 * G; f < sg; f += 4 * G)
+    for (int f = 4 * (gl + kAhead * G); f < sg; f += 4 * G)
     {
         TA xv[4];
         Load4(xs + f, xv);
@@ -1062,6 +1095,7 @@ __global__ void __launch_bounds__(kBS, sizeof(TA) == 4 ? 5 : 3) k_cycle(CycleArg
                 s[c] += v[0] * xv[0] + v[1] * xv[1] + v[2] * xv[2] + v[3] * xv[3];
             }
     }
+    PdlTrigger();
     int comp;
     const TA t = GroupSum3<G>(s, gl, A.ncRow == 1, comp);
     if (comp < 0 || comp >= ncR)
@@ -1082,13 +1116,13 @@ __global__ void __launch_bounds__(kBS, sizeof(TA) == 4 ? 5 : 3) k_cycle(CycleArg
         if (fixed)
             return;
         int32_t node[kInterp];
-        float w[kInterp];
+        TA w[kInterp];
         LoadInterp(A.pNode, A.pWeight, a, node, w);
 #pragma unroll
         for (int k = 0; k < kInterp; ++k)
             if (node[k] >= 0)
                 atomicAdd(A.cb + NG_IDX(static_cast<int64_t>(node[k]) * A.ncRow + comp, A.nCoarse, 33),
-                          static_cast<TA>(w[k]) * res);
+                          w[k] * res);
         return;
     }
     const TA d = EPI == CE_FIRST ? A.dinv[r] * res * A.w1
@@ -1129,7 +1163,7 @@ static void LaunchCycle(Ctx& c, const CycleArgs<TA>& A, const int* st)
 // e += P ce on the unconstrained rows, one thread per row
 template <typename TA>
 __global__ void k_prolong(NodeSpmv F, const uint8_t* __restrict__ fmask, const int32_t* __restrict__ pNode,
-                          const float* __restrict__ pWeight, int64_t nCoarse, const TA* __restrict__ ce, TA* e,
+                          const TA* __restrict__ pWeight, int64_t nCoarse, const TA* __restrict__ ce, TA* e,
                           const int* st)
 {
     PdlWait();
@@ -1143,13 +1177,13 @@ __global__ void k_prolong(NodeSpmv F, const uint8_t* __restrict__ fmask, const i
     if (fmask[r])
         return;
     int32_t node[kInterp];
-    float w[kInterp];
+    TA w[kInterp];
     LoadInterp(pNode, pWeight, a, node, w);
     TA s = e[r];
 #pragma unroll
     for (int k = 0; k < kInterp; ++k)
         if (node[k] >= 0)
-            s += static_cast<TA>(w[k]) * ce[NG_IDX(static_cast<int64_t>(node[k]) * nc + c, nCoarse, 34)];
+            s += w[k] * ce[NG_IDX(static_cast<int64_t>(node[k]) * nc + c, nCoarse, 34)];
     e[r] = s;
 }
 
@@ -1183,7 +1217,7 @@ struct TailLevel
     const int64_t* nbrPtr;
     const int32_t* nbrCol;
     const int32_t* pNode; // interpolation from the next coarser level (unused on the coarsest)
-    const float* pWeight;
+    const TA* pWeight;
     const TA* vals;
     const TA* dinv;
     TA *b, *e, *t, *d;
@@ -1315,7 +1349,7 @@ __global__ void __launch_bounds__(kTailThreads) k_amg_tail(TailArgs<TA> T)
         for (int64_t a = threadIdx.x; a < F.nNodes; a += blockDim.x)
         {
             int32_t node[kInterp];
-            float w[kInterp];
+            TA w[kInterp];
             LoadInterp(F.pNode, F.pWeight, a, node, w);
             for (int c = 0; c < F.ncomp; ++c)
             {
@@ -1324,7 +1358,7 @@ __global__ void __launch_bounds__(kTailThreads) k_amg_tail(TailArgs<TA> T)
                 for (int k = 0; k < kInterp; ++k)
                     if (node[k] >= 0)
                         atomicAdd(C.b + NG_IDX(static_cast<int64_t>(node[k]) * C.ncomp + c, C.nDofs, 73),
-                                  static_cast<TA>(w[k]) * res);
+                                  w[k] * res);
             }
         }
         __syncthreads();
@@ -1337,7 +1371,7 @@ __global__ void __launch_bounds__(kTailThreads) k_amg_tail(TailArgs<TA> T)
         for (int64_t a = threadIdx.x; a < F.nNodes; a += blockDim.x)
         {
             int32_t node[kInterp];
-            float w[kInterp];
+            TA w[kInterp];
             LoadInterp(F.pNode, F.pWeight, a, node, w);
             for (int c = 0; c < F.ncomp; ++c)
             {
@@ -1345,7 +1379,7 @@ __global__ void __launch_bounds__(kTailThreads) k_amg_tail(TailArgs<TA> T)
 #pragma unroll
                 for (int k = 0; k < kInterp; ++k)
                     if (node[k] >= 0)
-                        s += static_cast<TA>(w[k]) * C.e[NG_IDX(static_cast<int64_t>(node[k]) * C.ncomp + c, C.nDofs, 74)];
+                        s += w[k] * C.e[NG_IDX(static_cast<int64_t>(node[k]) * C.ncomp + c, C.nDofs, 74)];
                 F.e[a * F.ncomp + c] = s;
             }
         }
@@ -1412,6 +1446,14 @@ static void EnsureNum(Ctx& c, Amg& M)
                 continue;
             if (l > 0)
             {
+                LevelNodes& X = *L.nodes;
+                if (sizeof(TA) == 8 && X.pWeight64.n != X.pWeight.n)
+                {
+                    X.pWeight64.alloc(X.pWeight.n);
+                    const int64_t m = static_cast<int64_t>(X.pWeight.n);
+                    k_convert<float, double><<<Blocks(m), 256, 0, c.stream>>>(m, X.pWeight.p, X.pWeight64.p, nullptr);
+                    c.stats.kernel_launches += 1;
+                }
                 U.vals.alloc(L.nnz);
                 U.nb.alloc(std::max<int64_t>(L.nbTotal, 4));
             }
@@ -1481,7 +1523,7 @@ static void BuildTail(Ctx& c, int I, bool sym)
         F.nbrPtr = Lk.nodes->dNbrPtr.p;
         F.nbrCol = Lk.nbrCol.p;
         F.pNode = l0 + k + 1 < H.size() ? H[l0 + k + 1].nodes->pNode.p : nullptr;
-        F.pWeight = l0 + k + 1 < H.size() ? H[l0 + k + 1].nodes->pWeight.p : nullptr;
+        F.pWeight = l0 + k + 1 < H.size() ? Weights<TA>(*H[l0 + k + 1].nodes).p : nullptr;
         F.vals = Uk.vals.p;
         F.dinv = Uk.dinv.p;
         for (TA** v : {&F.b, &F.e, &F.t, &F.d})
@@ -1717,7 +1759,7 @@ static void VCycle(Ctx& c, int I, size_t l, const TA* b, TA* e, const int* st, b
     Num<TA>& CU = N<TA>(Co);
     // pre-smoothing from zero (one step, two in the symmetric cycle), then the residual restricted
     A.pNode = Co.nodes->pNode.p;
-    A.pWeight = Co.nodes->pWeight.p;
+    A.pWeight = Weights<TA>(*Co.nodes).p;
     A.cb = CU.b;
     A.nCoarse = Co.nDofs;
     {
@@ -1747,12 +1789,12 @@ static void VCycle(Ctx& c, int I, size_t l, const TA* b, TA* e, const int* st, b
     A.ce = CU.e.p;
     Cheb C(L, kSmoothRatio);
     A.w1 = TA(1. / C.theta);
-    if (L.nNodes <= kProlongNodes)
+    if (sizeof(TA) == 4 && L.nNodes <= kProlongNodes)
         LaunchCycle<TA, CG_PROLONG, CE_FIRST>(c, A, st);
     else
     {
         NG_CUDA(LaunchPdl(k_prolong<TA>, Blocks(n), 256, 0, c.stream, L.spmv, l == 0 ? c.dMask.p : L.zeroMask.p,
-                          static_cast<const int32_t*>(Co.nodes->pNode.p), static_cast<const float*>(Co.nodes->pWeight.p),
+                          static_cast<const int32_t*>(Co.nodes->pNode.p), static_cast<const TA*>(Weights<TA>(*Co.nodes).p),
                           Co.nDofs, static_cast<const TA*>(CU.e.p), e, st));
         c.stats.kernel_launches += 1;
         LaunchCycle<TA, CG_VECTOR, CE_FIRST>(c, A, st);

@@ -76,8 +76,9 @@ __device__ __forceinline__ long long CheckedIndex(long long i, long long n, int 
 // a kernel's blocks may be scheduled while its predecessor in the stream drains, which hides most of the gap
 // between the many short launches of a cycle. Every such kernel calls PdlWait() before its first access to anything that the
 // kernel in front of it writes (it returns once the predecessor grid has completed and its writes are visible; without the launch
-// attribute it returns at once) and PdlTrigger() right after, so that its own successor may be scheduled once all
-// of its blocks are running. NUTO_GPU_PDL=0 launches them normally.
+// attribute it returns at once) and PdlTrigger() when its main work is done: the successor's blocks are then scheduled while
+// it drains. Triggered at the start, they are placed wherever the running kernel leaves room, several on one SM and none on
+// others, and the FP64 projections of a 37,044-row basis took 23.6 us instead of 12.6. NUTO_GPU_PDL=0 launches them normally.
 __device__ __forceinline__ void PdlWait()
 {
     asm volatile("griddepcontrol.wait;\n" ::: "memory");

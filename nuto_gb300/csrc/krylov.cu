@@ -902,7 +902,6 @@ __global__ void __launch_bounds__(kBS) k_gm_proj(int64_t n, const T* __restrict_
                                                   double* acc, double* norm, const int* st)
 {
     PdlWait();
-    PdlTrigger();
     if (st[ST_STATE] != RUN)
         return;
     if (blockIdx.x == 0 && threadIdx.x == 0)
@@ -923,6 +922,7 @@ __global__ void __launch_bounds__(kBS) k_gm_proj(int64_t n, const T* __restrict_
             r[k] = base + 32 * k < n ? w[base + 32 * k] : T(0);
         ProjUnit<T, K>(V, n, nv, base, r, sums);
     }
+    PdlTrigger();
     ProjFlush(sums, nv, acc);
 }
 
@@ -933,7 +933,6 @@ __global__ void __launch_bounds__(kBS) k_gm_update_proj(int64_t n, const T* __re
                                                          T* __restrict__ w, double* acc2, const int* st)
 {
     PdlWait();
-    PdlTrigger();
     __shared__ T hs[GL::m + 1];
     if (st[ST_STATE] != RUN)
         return;
@@ -970,6 +969,7 @@ __global__ void __launch_bounds__(kBS) k_gm_update_proj(int64_t n, const T* __re
                 w[base + 32 * k] = r[k];
         ProjUnit<T, K>(V, n, nv, base, r, sums);
     }
+    PdlTrigger();
     ProjFlush(sums, nv, acc2);
 }
 
@@ -982,7 +982,6 @@ __global__ void __launch_bounds__(kBS) k_gm_update(int64_t n, const T* __restric
                                                     const T* __restrict__ zsrc, T* __restrict__ zdst, const int* st)
 {
     PdlWait();
-    PdlTrigger();
     __shared__ T sh[kBS / 32];
     __shared__ T hs[GL::m + 1];
     if (st[ST_STATE] != RUN)
@@ -1004,6 +1003,7 @@ __global__ void __launch_bounds__(kBS) k_gm_update(int64_t n, const T* __restric
             zdst[r] = zsrc[r];
         nrm += a * a;
     }
+    PdlTrigger();
     nrm = WarpAllSum(nrm);
     if ((threadIdx.x & 31) == 0)
         sh[threadIdx.x >> 5] = nrm;

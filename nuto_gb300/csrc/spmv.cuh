@@ -413,7 +413,6 @@ __global__ void __launch_bounds__(kBS, NbMinBlocks<TV>()) k_spmv_nb(NodeSpmv A, 
         cols[k] = gl + k * G < tot ? column(gl + k * G) : 0;
     const int64_t g0 = valid ? A.gdof[I][a] : 0;
     PdlWait();
-    PdlTrigger();
     if (st && st[ST_STATE] != RUN)
         return;
 #pragma unroll
@@ -457,6 +456,7 @@ __global__ void __launch_bounds__(kBS, NbMinBlocks<TV>()) k_spmv_nb(NodeSpmv A, 
                 }
         }
     }
+    PdlTrigger();
     int comp;
     const TX sum = GroupSum3<G>(s, gl, A.ncMaxRows == 1, comp);
     double d0 = 0., d1 = 0.;
