@@ -423,8 +423,8 @@ struct Ctx
     // element matrices of the last tangent in its arithmetic (one buffer for FP32 and FP64: every tangent of a context runs
     // on its stream) and the plan of the row gather
     DBuf<unsigned char> dElemMats;
-    DBuf<RowPlan> dRowPlan;
-    DBuf<uint32_t> dRowSlab, dPackedRanks;
+    DBuf<unsigned char> dRowPlan; // RowPlan per node, then slab numbers and packed ranks:
+    uint32_t *rowSlab = nullptr, *packedRanks = nullptr;
     int rowPlanKey = 0; // slots the plan was built for (0: not built)
     bool rowPlanSame = false;
     // device status word of kernels with bounded waits (0 = fine, else NUTO_GPU_ETIMEOUT), read after a stream

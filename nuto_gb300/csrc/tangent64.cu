@@ -674,9 +674,14 @@ RowPlanArgs EnsureRowPlan(Ctx& c)
     const int key = 1 + dS + kMaxSlots * (gd ? 1 + eS : 0);
     if (c.rowPlanKey != key)
     {
-        c.dRowPlan.alloc(static_cast<size_t>(D.nNodes));
-        c.dRowSlab.alloc(static_cast<size_t>(entries));
-        c.dPackedRanks.alloc(static_cast<size_t>(entries * D.nen));
+        // one allocation: the nodes' records, slab numbers, packed ranks, and the flag that the kernels below may raise
+        const size_t plans = static_cast<size_t>(D.nNodes) * sizeof(RowPlan);
+        const size_t numbers = static_cast<size_t>(entries) * (1 + D.nen) + 1;
+        c.dRowPlan.alloc(plans + numbers * sizeof(uint32_t));
+        c.rowSlab = reinterpret_cast<uint32_t*>(c.dRowPlan.p + plans);
+        c.packedRanks = c.rowSlab + entries;
+        RowPlan* plan = reinterpret_cast<RowPlan*>(c.dRowPlan.p);
+        int* differ = reinterpret_cast<int*>(c.packedRanks + entries * D.nen);
         PlanArgs A{};
         A.nNodes = D.nNodes;
         A.nCells = c.nCells;
@@ -694,29 +699,27 @@ RowPlanArgs EnsureRowPlan(Ctx& c)
             A.rank[k] = c.pairs[pr[k]].rank;
             A.blk[k] = c.pairs[pr[k]].dBlk.p;
         }
-        DBuf<int> differ;
-        differ.alloc(1);
-        NG_CUDA(cudaMemsetAsync(differ.p, 0, sizeof(int), c.stream));
-        k_row_plan<<<static_cast<unsigned>((D.nNodes + 255) / 256), 256, 0, c.stream>>>(A, c.dRowPlan.p, differ.p);
+        NG_CUDA(cudaMemsetAsync(differ, 0, sizeof(int), c.stream));
+        k_row_plan<<<static_cast<unsigned>((D.nNodes + 255) / 256), 256, 0, c.stream>>>(A, plan, differ);
         AfterLaunch(c, "k_row_plan");
         const unsigned blocks = static_cast<unsigned>((entries * D.nen + 255) / 256);
         if (D.nen == 4)
-            k_row_entries<4><<<blocks, 256, 0, c.stream>>>(A, entries, c.dRowSlab.p, c.dPackedRanks.p, differ.p);
+            k_row_entries<4><<<blocks, 256, 0, c.stream>>>(A, entries, c.rowSlab, c.packedRanks, differ);
         else if (D.nen == 20)
-            k_row_entries<20><<<blocks, 256, 0, c.stream>>>(A, entries, c.dRowSlab.p, c.dPackedRanks.p, differ.p);
+            k_row_entries<20><<<blocks, 256, 0, c.stream>>>(A, entries, c.rowSlab, c.packedRanks, differ);
         else
-            k_row_entries<8><<<blocks, 256, 0, c.stream>>>(A, entries, c.dRowSlab.p, c.dPackedRanks.p, differ.p);
+            k_row_entries<8><<<blocks, 256, 0, c.stream>>>(A, entries, c.rowSlab, c.packedRanks, differ);
         AfterLaunch(c, "k_row_entries");
         int h = 0;
-        NG_CUDA(cudaMemcpyAsync(&h, differ.p, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+        NG_CUDA(cudaMemcpyAsync(&h, differ, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
         NG_CUDA(cudaStreamSynchronize(c.stream));
         c.rowPlanSame = h == 0;
         c.rowPlanKey = key;
     }
     RowPlanArgs P{};
-    P.plan = c.dRowPlan.p;
-    P.slab = c.dRowSlab.p;
-    P.packed = c.dPackedRanks.p;
+    P.plan = reinterpret_cast<const RowPlan*>(c.dRowPlan.p);
+    P.slab = c.rowSlab;
+    P.packed = c.packedRanks;
     P.nEntries = entries;
     P.nnz = c.nnz;
     P.sameGraph = c.rowPlanSame;
@@ -731,12 +734,17 @@ unsigned char* ElemMatsOrNull(Ctx& c, size_t bytes)
     NG_CUDA(cudaStreamIsCapturing(c.stream, &cs));
     if (cs != cudaStreamCaptureStatusNone)
         return nullptr;
-    size_t free = 0, total = 0;
-    NG_CUDA(cudaMemGetInfo(&free, &total));
-    if (bytes > free + c.dElemMats.n)
+    // the attempt itself tells whether the memory is there (asking for the free memory first costs as much as a small assembly)
+    c.dElemMats.free();
+    unsigned char* p = nullptr;
+    if (cudaMalloc(&p, bytes) != cudaSuccess)
+    {
+        cudaGetLastError();
         return nullptr;
-    c.dElemMats.alloc(bytes);
-    return c.dElemMats.p;
+    }
+    c.dElemMats.p = p;
+    c.dElemMats.n = bytes;
+    return p;
 }
 
 } // namespace nuto_gpu
