@@ -452,6 +452,7 @@ static void BuildPattern(Ctx& c)
     }
     FreeAmg(c);
     c.rowPlanKey = 0;
+    c.cellChunkEnd.clear();
     c.h20Mode = -1;
     c.tc20Mode = -1;
     c.havePattern = true;
@@ -1206,32 +1207,38 @@ int nuto_gpu_build_system_host(nuto_gpu_ctx* ctx, const double* hU, int precisio
             NG_CUDA(cudaStreamSynchronize(c.stream));
             return NUTO_GPU_OK;
         }
-        EnsureSideStream(c);
-        // the residual and its copy back on the side stream; the tangent and its copy back on the context's stream,
-        // where the copy of the values starts as soon as the tangent is done, while the residual still runs
-        NG_CUDA(cudaEventRecord(c.evFork, c.stream));
-        NG_CUDA(cudaStreamWaitEvent(c.sideStream, c.evFork, 0));
-        const cudaStream_t main = c.stream;
-        c.stream = c.sideStream;
-        try
-        {
-            LaunchResidual(c, c.dHostIoU.p, c.dHostIoF.p, c.sysResBlocks);
-            NG_CUDA(cudaMemcpyAsync(hF, c.dHostIoF.p, vecBytes, cudaMemcpyDeviceToHost, c.stream));
-        }
-        catch (...)
-        {
-            c.stream = main;
-            throw;
-        }
-        c.stream = main;
         // FP32 element-matrix form over rows that follow the node order: the row gather runs in node chunks, and each
         // chunk's values go to the host on a copy stream while the next chunks are gathered. (The row kernels writing
         // straight into mapped page-locked host memory were measured slower: 5.4 ms per 64^3 pass against 4.4 ms
         // with one copy after the tangent.)
-        // A chunk of 8 MB takes 40 us to copy, about what its launch, event and two copies cost the host: smaller values go
+        // A chunk of 8 MB takes 40 us to copy, about what its launches, event and two copies cost the host: smaller values go
         // in one piece (9^3, 1.5 MB: 89 us in 4 chunks, 50 us in one).
-        const int kChunks = static_cast<int>(std::min<size_t>(4, valBytes >> 23));
+        const int kChunks = static_cast<int>(std::min<size_t>(8, valBytes >> 23));
         const bool chunked = kChunks > 1 && precision == NUTO_GPU_FP32 && c.tuning.tangentWarps != 0 && RowsContiguous(c);
+        // The residual and its copy back on the side stream: beside the tangent, whose values are copied as soon as it is done;
+        // in the chunked form behind the tangent's kernels, since the copy of the values takes longer than both and starts the
+        // earlier the sooner the first chunk is there (40^3: 849 us
+        // beside, 697 behind; the copy alone 580).
+        EnsureSideStream(c);
+        auto residual = [&](int blocks) {
+            NG_CUDA(cudaEventRecord(c.evFork, c.stream));
+            NG_CUDA(cudaStreamWaitEvent(c.sideStream, c.evFork, 0));
+            const cudaStream_t main = c.stream;
+            c.stream = c.sideStream;
+            try
+            {
+                LaunchResidual(c, c.dHostIoU.p, c.dHostIoF.p, blocks);
+                NG_CUDA(cudaMemcpyAsync(hF, c.dHostIoF.p, vecBytes, cudaMemcpyDeviceToHost, c.stream));
+            }
+            catch (...)
+            {
+                c.stream = main;
+                throw;
+            }
+            c.stream = main;
+        };
+        if (!chunked)
+            residual(c.sysResBlocks);
         int chunkIdx = 0;
         if (chunked)
         {
@@ -1273,6 +1280,8 @@ int nuto_gpu_build_system_host(nuto_gpu_ctx* ctx, const double* hU, int precisio
         const bool copiedInChunks = chunked && c.rowChunksDone == kChunks;
         c.onRowChunk = nullptr;
         c.rowChunks = 0;
+        if (chunked)
+            residual(0);
         if (copiedInChunks)
         {
             NG_CUDA(cudaEventRecord(c.evCopy, c.copyStream));

@@ -34,7 +34,8 @@ namespace
 struct FusedArgs
 {
     int64_t nCells, nDofs, nNodesD, nNodesE;
-    const int32_t* connD; // planar [n][cell]
+    int64_t cellFirst, cellLast; // cells of this launch
+    const int32_t* connD;        // planar [n][cell]
     const int32_t* connE;
     const int64_t* gdofD; // per node: combined index of component 0
     const int64_t* gdofE;
@@ -345,15 +346,15 @@ __global__ void __launch_bounds__(W * 32, 16 / W) k_cell_matrices(FusedArgs A, L
     for (int i = threadIdx.x; i < NIP; i += blockDim.x)
         sWq[i] = static_cast<float>(A.tabW[i]);
     __syncthreads();
-    const int64_t n = A.nCells;
+    const int64_t n = A.nCells, last = A.cellLast;
     const int64_t stride = RESIDENT ? static_cast<int64_t>(gridDim.x) * W * CPW : n;
     // the warp's own cells: only warp-level synchronisation follows
-    for (int64_t c0 = (static_cast<int64_t>(blockIdx.x) * W + wid) * CPW; c0 < n; c0 += stride)
+    for (int64_t c0 = A.cellFirst + (static_cast<int64_t>(blockIdx.x) * W + wid) * CPW; c0 < last; c0 += stride)
     {
         // (0) lane (cell slot, node): the node data; (A) lane (cell slot, point): geometry and law
         const int cl = lane / ND, ia = lane % ND;
         const int64_t e = c0 + cl;
-        if (e < n)
+        if (e < last)
         {
             const int32_t nD = static_cast<int32_t>(NG_IDX(A.connD[static_cast<int64_t>(ia) * n + e], A.nNodesD, 80));
             const int64_t gd = A.gdofD[nD];
@@ -377,12 +378,12 @@ __global__ void __launch_bounds__(W * 32, 16 / W) k_cell_matrices(FusedArgs A, L
             sU[cl * ND + ia] = make_float4(v[0], v[1], v[2], 0.f);
         }
         __syncwarp();
-        if (e < n)
+        if (e < last)
             PointRecord<DIM, KIND>(A, L, sT + ia * C::tabRow, sWq[ia], sX + cl * ND, sU + cl * ND, GD ? sE + cl * ND : nullptr, ia,
                                    e, sR + cl * C::cell + ia * C::rec);
         __syncwarp();
         // (B) lane (cell slot, a): the slab of a, row by row through the staging rows
-        const bool on = e < n;
+        const bool on = e < last;
         float* R = sR + cl * C::cell;
         float4* st = reinterpret_cast<float4*>(sStage + lane * C::stRow);
         auto flush = [&](int k) {
@@ -392,7 +393,7 @@ __global__ void __launch_bounds__(W * 32, 16 / W) k_cell_matrices(FusedArgs A, L
             {
                 const int row = i / P4, j = i % P4;
                 const int64_t er = c0 + row / ND;
-                if (er < n)
+                if (er < last)
                     *reinterpret_cast<float4*>(em + (NG_IDX(er, n, 84) * ND + row % ND) * SL::size + k * NC + 4 * j) =
                             *reinterpret_cast<const float4*>(sStage + row * C::stRow + 4 * j);
             }
@@ -632,6 +633,29 @@ bool FusedTangentSupported(Ctx& c)
     return true;
 }
 
+// cellChunkEnd[k]: one past the last cell with a node of the first k + 1 node chunks
+static void EnsureCellChunks(Ctx& c, const Slot& D, int chunks)
+{
+    if (static_cast<int>(c.cellChunkEnd.size()) == chunks)
+        return;
+    std::vector<int64_t> end(chunks, 0);
+    for (int64_t e = 0; e < c.nCells; ++e)
+    {
+        int64_t node = D.nNodes;
+        for (int n = 0; n < D.nen; ++n)
+            node = std::min<int64_t>(node, D.conn[e * D.nen + n]);
+        int ch = static_cast<int>(node * chunks / D.nNodes); // or the chunk behind it, where the bounds round down
+        while (ch > 0 && node < D.nNodes * ch / chunks)
+            --ch;
+        while (ch + 1 < chunks && node >= D.nNodes * (ch + 1) / chunks)
+            ++ch;
+        end[ch] = e + 1;
+    }
+    for (int k = 1; k < chunks; ++k)
+        end[k] = std::max(end[k], end[k - 1]);
+    c.cellChunkEnd = std::move(end);
+}
+
 void LaunchTangentFused(Ctx& c, const double* u, float* vals)
 {
     if (c.dRelX.n == 0)
@@ -689,7 +713,7 @@ void LaunchTangentFused(Ctx& c, const double* u, float* vals)
                     NG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  static_cast<int>(smem)));
                 constexpr int64_t perBlock = static_cast<int64_t>(WW) * C::cpw;
-                int64_t blocks = (c.nCells + perBlock - 1) / perBlock;
+                int64_t blocks = (A.cellLast - A.cellFirst + perBlock - 1) / perBlock;
                 if (resident)
                 {
                     int perSm = 0;
@@ -700,16 +724,23 @@ void LaunchTangentFused(Ctx& c, const double* u, float* vals)
                 AfterLaunch(c, "k_cell_matrices");
                 c.stats.kernel_launches += 1;
             };
-            if (form == 1)
-                cells(k_cell_matrices<DIM, KIND, WW, true>, true);
-            else
-                cells(k_cell_matrices<DIM, KIND, WW, false>, false);
-            // the row gather, in node chunks when a caller hooks into them (each chunk's rows are complete when its
-            // launch is)
+            // in node chunks when a caller hooks into them: the cells that a chunk's rows are the first to need, then its
+            // rows, which are complete when their launch is
             const int chunks = c.rowChunks > 1 && c.onRowChunk ? c.rowChunks : 1;
+            if (chunks > 1)
+                EnsureCellChunks(c, D, chunks);
             for (int ch = 0; ch < chunks; ++ch)
             {
                 const int64_t a0 = D.nNodes * ch / chunks, a1 = D.nNodes * (ch + 1) / chunks;
+                A.cellFirst = ch > 0 ? c.cellChunkEnd[ch - 1] : 0;
+                A.cellLast = chunks > 1 ? c.cellChunkEnd[ch] : c.nCells;
+                if (A.cellLast > A.cellFirst)
+                {
+                    if (form == 1)
+                        cells(k_cell_matrices<DIM, KIND, WW, true>, true);
+                    else
+                        cells(k_cell_matrices<DIM, KIND, WW, false>, false);
+                }
                 LaunchRows<float, DIM, C::nd, C::GD, WW>(c, plan, a0, a1, em, vals);
                 if (chunks > 1)
                 {

@@ -674,6 +674,7 @@ RowPlanArgs EnsureRowPlan(Ctx& c)
     const int key = 1 + dS + kMaxSlots * (gd ? 1 + eS : 0);
     if (c.rowPlanKey != key)
     {
+        c.cellChunkEnd.clear();
         // one allocation: the nodes' records, slab numbers, packed ranks, and the flag that the kernels below may raise
         const size_t plans = static_cast<size_t>(D.nNodes) * sizeof(RowPlan);
         const size_t numbers = static_cast<size_t>(entries) * (1 + D.nen) + 1;
