@@ -24,14 +24,15 @@
 //                   accuracy (the dropped lo.lo term is 2^-22 relative); split 1 keeps hi.hi only.
 //   k_rows_from_wide_slabs (rows.cuh)  one warp per displacement node adds its rows of the element matrices over the
 //                   node's cells in ascending order (no atomics: bitwise reproducible).
-// The tensor-memory accumulator is double-buffered (2 x 64 columns): the MMAs of one cell run while the epilogue of
-// the previous cell reads its accumulator. The only wait is on the MMA completion barrier; it is bounded by the
-// context's spin limit and, when it gives up, sets NUTO_GPU_ETIMEOUT in the status word, waits once more (bounded)
+// The tensor-memory accumulator is double-buffered (2 x 64 columns): one group of warps forms the operands of a cell while
+// another reads the accumulator of the cell before it. The waits between them and on the MMAs are on mbarriers, bounded by the
+// context's spin limit; when one gives up, the kernel sets NUTO_GPU_ETIMEOUT in the status word, waits once more (bounded)
 // for the MMAs in flight, frees the tensor memory and returns.
 #include "rows.cuh"
 
 #include <algorithm>
 #include <cfloat>
+#include <type_traits>
 
 namespace nuto_gpu
 {
@@ -43,7 +44,13 @@ namespace
 
 constexpr int kNd = 20, kNg = 8, kNip = 27;
 constexpr int kRecF4 = 6;          // float4 per point record
-constexpr int kTcThreads = 512;    // 16 warps: 4 per tensor-memory lane quarter
+// k_tangent_tc20: kBuildWarps warps form the operands of a cell (4 of the 27 points each) while kEpiWarps consecutive
+// warps read the accumulator of the cell before it (kEpiWarps / 4 per tensor-memory lane quarter, kEpiCols columns each)
+constexpr int kBuildWarps = 7, kEpiWarps = 8;
+constexpr int kEpiCols = 256 / kEpiWarps;
+static_assert(kEpiWarps % 4 == 0 && kEpiCols % 16 == 0, "whole quarters, loads of 16 columns");
+constexpr int kBuildThreads = kBuildWarps * 32, kEpiThreads = kEpiWarps * 32;
+constexpr int kTcThreads = kBuildThreads + kEpiThreads;
 // shared memory of k_tangent_tc20 (bytes)
 constexpr int kOpAHi = 0, kOpALo = 32768, kOpBHi = 65536, kOpBLo = 81920, kOpEnd = 98304;
 constexpr int kRecOff = kOpEnd;                                // 2 x 27 x 6 float4: this cell's records, the next's
@@ -52,8 +59,8 @@ constexpr int kMuStride = 61;
 constexpr int kOutOff = kMuOff + 60 * kMuStride * 4;           // element matrix staging [a][181]
 constexpr int kOutStride = 181;
 constexpr int kTabOff = kOutOff + kNd * kOutStride * 4;        // dN/dxi of the 20 nodes at the 27 points
-constexpr int kBarOff = kTabOff + kNip * kNd * 3 * 4;          // 2 mbarriers, the tensor-memory address
-constexpr int kSmemTc = kBarOff + 32;
+constexpr int kBarOff = kTabOff + kNip * kNd * 3 * 4;          // 4 mbarriers, the tensor-memory address
+constexpr int kSmemTc = kBarOff + 48;
 static_assert(kRecOff % 16 == 0 && kMuOff % 16 == 0 && kOutOff % 16 == 0 && kTabOff % 16 == 0 && kBarOff % 16 == 0,
               "16-byte aligned regions");
 static_assert(kSmemTc <= 227 * 1024, "fits one block per SM");
@@ -421,6 +428,23 @@ __device__ __forceinline__ void PutOp(unsigned char* hi, unsigned char* lo, int 
         *reinterpret_cast<float*>(lo + off) = Tf32Round(x - h);
 }
 
+__device__ __forceinline__ void BarArrive(uint32_t bar)
+{
+    asm volatile("{\n.reg .b64 t;\nmbarrier.arrive.shared::cta.b64 t, [%0];\n}\n" ::"r"(bar) : "memory");
+}
+// barrier `id` of `threads` threads (a group of warps)
+__device__ __forceinline__ void GroupSync(int id, int threads)
+{
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// One block per SM walks the cells. The operand buffer is single, so a cell costs the time from the completion of its MMAs to
+// the completion of the next cell's: the build warps wait for the MMAs of cell k - 1, form the operands of cell k and issue
+// its MMAs; the epilogue warps meanwhile read the accumulator of cell k - 1 (two accumulators; "free" barriers hand them
+// back). 24^3, 13,824 cells: 300 us with all 16 warps first building and then reading, 270 with 8 + 8 warps, 240 with 7 + 8
+// and a warp per 4 points; more warps on either side do not help (11 + 8: 250, 7 + 16: 250): of the 5,000 cycles per cell
+// the MMAs take 1,600 and shared memory about 3,300 wavefronts. A group that gives up a wait leaves its loop; the other one's
+// waits run out too, so both reach the end.
 template <bool RANK1, int SPLIT>
 __global__ void __launch_bounds__(kTcThreads, 1) k_tangent_tc20(int64_t nCells, const double* __restrict__ tabDNd,
                                                                const float4* __restrict__ recs,
@@ -428,14 +452,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tangent_tc20(int64_t nCells, 
                                                                long long spin)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
-    __shared__ int sFail;
+    __shared__ int sFailBuild, sFailEpi;
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
     float4* sRec = reinterpret_cast<float4*>(sm + kRecOff);
     float* sMu = reinterpret_cast<float*>(sm + kMuOff);
     float* sOut = reinterpret_cast<float*>(sm + kOutOff);
     float* sDN = reinterpret_cast<float*>(sm + kTabOff);
     const uint32_t smBase = static_cast<uint32_t>(__cvta_generic_to_shared(sm));
-    const uint32_t bar0 = smBase + kBarOff;
+    const uint32_t bar0 = smBase + kBarOff;  // MMAs of a cell done, per accumulator
+    const uint32_t free0 = bar0 + 16;        // accumulator read, per accumulator
     const int64_t n = nCells;
     if (static_cast<int64_t>(blockIdx.x) >= n)
         return; // the grid has at most one block per cell; a block without a cell allocates nothing
@@ -449,168 +474,206 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tangent_tc20(int64_t nCells, 
     {
         BarInit(bar0, 1);
         BarInit(bar0 + 8, 1);
+        BarInit(free0, kEpiWarps);
+        BarInit(free0 + 8, kEpiWarps);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        sFail = 0;
+        sFailBuild = 0;
+        sFailEpi = 0;
     }
     if (wid == 0)
     {
-        TmemAlloc(smBase + kBarOff + 16, kTmemCols);
+        TmemAlloc(smBase + kBarOff + 32, kTmemCols);
         TmemRelinquish();
     }
     TcFenceBefore();
     __syncthreads();
     TcFenceAfter();
-    const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(sm + kBarOff + 16);
+    const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(sm + kBarOff + 32);
 
     const int64_t stride = gridDim.x;
-    auto issueRecs = [&](int64_t cell, int buf) {
-        const float4* src = recs + cell * (kNip * kRecF4);
-        float4* dst = sRec + buf * (kNip * kRecF4);
-        for (int i = tid; i < kNip * kRecF4; i += kTcThreads)
-            AsyncCopy16(dst + i, src + i);
-    };
-    // epilogue of the cell whose MMAs committed to accumulator acc (their completion has been observed)
-    auto epilogue = [&](int64_t cell, int acc) {
-        TcFenceAfter();
-        const int quarter = wid & 3, chunk = wid >> 2; // lanes 32 quarter.., columns 16 chunk..
-        const int row = quarter * 32 + lane;
-        float v[16];
-        TmemLoad16(tmem + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(acc * 64 + chunk * 16),
-                   v);
-        TcFenceBefore();
-        if (row >= 64 && row < 124)
-#pragma unroll
-            for (int t = 0; t < 16; ++t)
-            {
-                const int col = chunk * 16 + t;
-                if (col < 60)
-                    sMu[(row - 64) * kMuStride + col] = v[t];
-            }
-        __syncthreads();
-        if (row < 60)
-        {
-            const int i = row / 20, a = row % 20;
-#pragma unroll
-            for (int t = 0; t < 16; ++t)
-            {
-                const int col = chunk * 16 + t;
-                if (col >= 60)
-                    continue;
-                const int j = col / 20, b = col % 20;
-                float x = v[t] + sMu[(j * 20 + a) * kMuStride + i * 20 + b];
-                if (i == j)
-                    x += sMu[a * kMuStride + b] + sMu[(20 + a) * kMuStride + 20 + b] +
-                         sMu[(40 + a) * kMuStride + 40 + b];
-                sOut[a * kOutStride + i * 60 + b * 3 + j] = x;
-            }
-        }
-        __syncthreads();
-        float* dst = em + cell * (kNd * 180);
-        for (int t = tid; t < kNd * 180; t += kTcThreads)
-            dst[t] = sOut[(t / 180) * kOutStride + t % 180];
-    };
-
-    int64_t e = blockIdx.x;
-    int k = 0;
-    issueRecs(e, 0);
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-    for (; e < n; e += stride, ++k)
+    int issued = 0; // thread 0: cells whose MMAs were committed
+    if (tid < kBuildThreads)
     {
-        const int b = k & 1;
-        if (e + stride < n)
-            issueRecs(e + stride, b ^ 1);
+        auto issueRecs = [&](int64_t cell, int buf) {
+            const float4* src = recs + cell * (kNip * kRecF4);
+            float4* dst = sRec + buf * (kNip * kRecF4);
+            for (int i = tid; i < kNip * kRecF4; i += kBuildThreads)
+                AsyncCopy16(dst + i, src + i);
+        };
+        int64_t e = blockIdx.x;
+        issueRecs(e, 0);
         asm volatile("cp.async.commit_group;\n" ::: "memory");
-        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-        // the operand buffer is free once the MMAs of the previous cell have completed
-        if (k > 0 && !BarWait(bar0 + 8 * (b ^ 1), ((k - 1) >> 1) & 1, spin))
-            sFail = 1;
-        __syncthreads();
-        if (sFail)
-            break;
-        // operands: item (node a, point q); a warp covers 8 nodes x 4 points, which puts its 32 stores of one
-        // value on 32 distinct banks
-        const float4* R = sRec + b * (kNip * kRecF4);
-        unsigned char* aHi = sm + kOpAHi;
-        unsigned char* aLo = sm + kOpALo;
-        unsigned char* bHi = sm + kOpBHi;
-        unsigned char* bLo = sm + kOpBLo;
-        for (int it = tid; it < 21 * 32; it += kTcThreads)
+        for (int k = 0; e < n; e += stride, ++k)
         {
-            const int grp = it >> 5, l = it & 31;
-            const int a = (grp / 7) * 8 + (l >> 2), q = (grp % 7) * 4 + (l & 3);
-            if (a >= kNd || q >= kNip)
-                continue;
-            const float4* Rq = R + q * kRecF4;
+            const int b = k & 1;
+            // the operand buffer is free, and record buffer b ^ 1 with it, once the MMAs of the previous cell have completed
+            if (k > 0 && !BarWait(bar0 + 8 * (b ^ 1), ((k - 1) >> 1) & 1, spin))
+                *static_cast<volatile int*>(&sFailBuild) = 1;
+            if (e + stride < n)
+                issueRecs(e + stride, b ^ 1);
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+            GroupSync(1, kBuildThreads);
+            if (*static_cast<volatile int*>(&sFailBuild))
+                break;
+            // operands: a warp takes 4 points, whose records it reads once, and 8 nodes at a time, which puts its 32 stores of
+            // one value on 32 distinct banks (an LDS.128 takes 4 wavefronts however few addresses it has)
+            const float4* R = sRec + b * (kNip * kRecF4);
+            unsigned char* aHi = sm + kOpAHi;
+            unsigned char* aLo = sm + kOpALo;
+            unsigned char* bHi = sm + kOpBHi;
+            unsigned char* bLo = sm + kOpBLo;
+            static_assert(kBuildWarps * 4 >= kNip, "a warp per 4 points");
+            const int q = wid * 4 + (lane & 3);
+            const float4* Rq = R + (q < kNip ? q : 0) * kRecF4;
             const float4 r0 = Rq[0], r1 = Rq[1], r2 = Rq[2];
             const float inv[3][3] = {{r0.x, r0.y, r0.z}, {r0.w, r1.x, r1.y}, {r1.z, r1.w, r2.x}};
             const float lamw = r2.y, muw = r2.z;
-            const float* dn = sDN + (q * kNd + a) * 3;
-            float g[3];
-#pragma unroll
-            for (int kk = 0; kk < 3; ++kk)
-                g[kk] = dn[0] * inv[0][kk] + dn[1] * inv[1][kk] + dn[2] * inv[2][kk];
-            float P[3] = {0.f, 0.f, 0.f}, Q[3] = {0.f, 0.f, 0.f};
+            float s[6] = {}, tt[6] = {};
             if (RANK1)
             {
                 const float4 r3 = Rq[3], r4 = Rq[4], r5 = Rq[5];
-                const float s[6] = {r3.x, r3.y, r3.z, r3.w, r4.x, r4.y};
-                const float tt[6] = {r4.z, r4.w, r5.x, r5.y, r5.z, r5.w};
-                BtS<float, 3>(g, s, P);
-                BtS<float, 3>(g, tt, Q);
+                s[0] = r3.x, s[1] = r3.y, s[2] = r3.z, s[3] = r3.w, s[4] = r4.x, s[5] = r4.y;
+                tt[0] = r4.z, tt[1] = r4.w, tt[2] = r5.x, tt[3] = r5.y, tt[4] = r5.z, tt[5] = r5.w;
             }
 #pragma unroll
-            for (int i = 0; i < 3; ++i)
+            for (int grp = 0; grp < 3; ++grp)
             {
-                const int r = i * 20 + a;
-                PutOp<SPLIT>(aHi, aLo, OpOff(r, q), lamw * g[i]);
-                PutOp<SPLIT>(aHi, aLo, OpOff(64 + r, q), muw * g[i]);
-                PutOp<SPLIT>(bHi, bLo, OpOff(r, q), g[i]);
+                const int a = grp * 8 + (lane >> 2);
+                if (a >= kNd || q >= kNip)
+                    continue;
+                const float* dn = sDN + (q * kNd + a) * 3;
+                float g[3];
+#pragma unroll
+                for (int kk = 0; kk < 3; ++kk)
+                    g[kk] = dn[0] * inv[0][kk] + dn[1] * inv[1][kk] + dn[2] * inv[2][kk];
+                float P[3] = {0.f, 0.f, 0.f}, Q[3] = {0.f, 0.f, 0.f};
                 if (RANK1)
                 {
-                    PutOp<SPLIT>(aHi, aLo, OpOff(r, 32 + q), P[i]);
-                    PutOp<SPLIT>(bHi, bLo, OpOff(r, 32 + q), Q[i]);
+                    BtS<float, 3>(g, s, P);
+                    BtS<float, 3>(g, tt, Q);
                 }
-            }
-        }
-        FenceProxyAsync();
-        __syncthreads();
-        if (tid == 0)
-        {
-            TcFenceAfter();
-            const uint32_t d = tmem + static_cast<uint32_t>(b * 64);
-            constexpr int KS = RANK1 ? 8 : 4; // K = 8 per instruction
 #pragma unroll
-            for (int s = 0; s < KS; ++s)
-            {
-                const uint32_t off = static_cast<uint32_t>(s * 256);
-                if (SPLIT == 3)
+                for (int i = 0; i < 3; ++i)
                 {
-                    MmaTf32(d, SmemDesc(smBase + kOpALo + off), SmemDesc(smBase + kOpBHi + off), s > 0 ? 1u : 0u);
-                    MmaTf32(d, SmemDesc(smBase + kOpAHi + off), SmemDesc(smBase + kOpBLo + off), 1u);
-                    MmaTf32(d, SmemDesc(smBase + kOpAHi + off), SmemDesc(smBase + kOpBHi + off), 1u);
+                    const int r = i * 20 + a;
+                    PutOp<SPLIT>(aHi, aLo, OpOff(r, q), lamw * g[i]);
+                    PutOp<SPLIT>(aHi, aLo, OpOff(64 + r, q), muw * g[i]);
+                    PutOp<SPLIT>(bHi, bLo, OpOff(r, q), g[i]);
+                    if (RANK1)
+                    {
+                        PutOp<SPLIT>(aHi, aLo, OpOff(r, 32 + q), P[i]);
+                        PutOp<SPLIT>(bHi, bLo, OpOff(r, 32 + q), Q[i]);
+                    }
                 }
-                else
-                    MmaTf32(d, SmemDesc(smBase + kOpAHi + off), SmemDesc(smBase + kOpBHi + off), s > 0 ? 1u : 0u);
             }
-            MmaCommit(bar0 + 8 * b);
+            FenceProxyAsync();
+            GroupSync(1, kBuildThreads);
+            if (tid == 0)
+            {
+                if (k >= 2 && !BarWait(free0 + 8 * b, ((k - 2) >> 1) & 1, spin))
+                    *static_cast<volatile int*>(&sFailBuild) = 1; // seen by the group at the next cell
+                else
+                {
+                    TcFenceAfter();
+                    const uint32_t d = tmem + static_cast<uint32_t>(b * 64);
+                    constexpr int KS = RANK1 ? 8 : 4; // K = 8 per instruction
+#pragma unroll
+                    for (int s = 0; s < KS; ++s)
+                    {
+                        const uint32_t off = static_cast<uint32_t>(s * 256);
+                        if (SPLIT == 3)
+                        {
+                            MmaTf32(d, SmemDesc(smBase + kOpALo + off), SmemDesc(smBase + kOpBHi + off), s > 0 ? 1u : 0u);
+                            MmaTf32(d, SmemDesc(smBase + kOpAHi + off), SmemDesc(smBase + kOpBLo + off), 1u);
+                            MmaTf32(d, SmemDesc(smBase + kOpAHi + off), SmemDesc(smBase + kOpBHi + off), 1u);
+                        }
+                        else
+                            MmaTf32(d, SmemDesc(smBase + kOpAHi + off), SmemDesc(smBase + kOpBHi + off), s > 0 ? 1u : 0u);
+                    }
+                    MmaCommit(bar0 + 8 * b);
+                    ++issued;
+                }
+            }
         }
-        if (k > 0)
-            epilogue(e - stride, b ^ 1);
-        __syncthreads();
     }
-    if (!sFail && k > 0)
+    else
     {
-        // the last cell
-        const int b = (k - 1) & 1;
-        if (!BarWait(bar0 + 8 * b, ((k - 1) >> 1) & 1, spin))
-            sFail = 1;
-        __syncthreads();
-        if (!sFail)
-            epilogue(e - stride, b);
+        const int et = tid - kBuildThreads;
+        const int quarter = wid & 3, part = (wid - kBuildWarps) >> 2; // lanes 32 quarter.., columns kEpiCols part..
+        const int row = quarter * 32 + lane;
+        int64_t e = blockIdx.x;
+        for (int k = 0; e < n; e += stride, ++k)
+        {
+            const int acc = k & 1;
+            if (!BarWait(bar0 + 8 * acc, (k >> 1) & 1, spin))
+                *static_cast<volatile int*>(&sFailEpi) = 1;
+            GroupSync(2, kEpiThreads); // also: the stores of the cell before have read sOut
+            if (*static_cast<volatile int*>(&sFailEpi))
+                break;
+            TcFenceAfter();
+            float v[kEpiCols / 16][16];
+#pragma unroll
+            for (int h = 0; h < kEpiCols / 16; ++h)
+                TmemLoad16(tmem + (static_cast<uint32_t>(quarter * 32) << 16) +
+                                   static_cast<uint32_t>(acc * 64 + part * kEpiCols + h * 16),
+                           v[h]);
+            TcFenceBefore();
+            __syncwarp();
+            if (lane == 0)
+                BarArrive(free0 + 8 * acc);
+            // a part's columns as compile-time numbers
+            auto muRows = [&](auto h) {
+                if (row >= 64 && row < 124)
+#pragma unroll
+                    for (int t = 0; t < kEpiCols; ++t)
+                    {
+                        const int col = decltype(h)::value * kEpiCols + t;
+                        if (col < 60)
+                            sMu[(row - 64) * kMuStride + col] = v[t >> 4][t & 15];
+                    }
+            };
+            auto blocks = [&](auto h) {
+                if (row >= 60)
+                    return;
+                const int i = row / 20, a = row % 20;
+                const float* mu = sMu + a * kMuStride;
+                float* out = sOut + a * kOutStride + i * 60;
+#pragma unroll
+                for (int t = 0; t < kEpiCols; ++t)
+                {
+                    const int col = decltype(h)::value * kEpiCols + t;
+                    if (col >= 60)
+                        continue;
+                    const int j = col / 20, b = col % 20;
+                    float x = v[t >> 4][t & 15] + mu[j * 20 * kMuStride + i * 20 + b];
+                    if (i == j)
+                        x += mu[b] + mu[20 * kMuStride + 20 + b] + mu[40 * kMuStride + 40 + b];
+                    out[b * 3 + j] = x;
+                }
+            };
+            auto withPart = [&](auto&& f) {
+                if (part == 0)
+                    f(std::integral_constant<int, 0>{});
+                else if (part == 1)
+                    f(std::integral_constant<int, 1>{});
+                else if (part == 2)
+                    f(std::integral_constant<int, 2>{});
+                else
+                    f(std::integral_constant<int, 3>{});
+            };
+            withPart(muRows);
+            GroupSync(2, kEpiThreads);
+            withPart(blocks);
+            GroupSync(2, kEpiThreads);
+            float* dst = em + e * (kNd * 180);
+            for (int t = et; t < kNd * 180; t += kEpiThreads)
+                dst[t] = sOut[(t / 180) * kOutStride + t % 180];
+        }
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
-    if (sFail)
+    if (sFailBuild || sFailEpi)
     {
         // the MMAs of cells 0 .. issued - 1 were committed, alternately to barrier 0 and 1; wait (bounded by a fixed
         // limit, independent of the caller's spin limit) for the last phase of each barrier before the tensor memory
@@ -618,7 +681,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tangent_tc20(int64_t nCells, 
         if (tid == 0)
         {
             atomicExch(status, NUTO_GPU_ETIMEOUT);
-            const int issued = k;
             for (int bb = 0; bb < 2; ++bb)
             {
                 const int commits = (issued + 1 - bb) / 2;
