@@ -414,15 +414,14 @@ def run_newton(args, s, g, barrier):
                        "|C^T r| <= 1e-8 |C^T (r + K db)| per load step, Eisenstat-Walker forcing with floor %g"
                        % (len(t_values), LOAD_STEPS, FORCING_FLOOR),
            "mixed": summary(sec32, agg32)}
-    out["mixed"]["path"] = ("FP32 tangent (k_tangent_fused), FP32 GMRES(80) with the FP32 "
+    out["mixed"]["path"] = ("FP32 tangent (k_cell_matrices), FP32 GMRES(80) with the FP32 "
                             "multigrid, FP64 residual, history, Newton test and refinement residual; iterations "
-                            "with |C^T r| < %g tol use the FP64-accurate tangent (k_tangent, FP64 law, double-float "
-                            "products) for the refinement" % EXACT_BELOW)
+                            "with |C^T r| < %g tol use the FP64 tangent (k_cell_matrices64) for the refinement" % EXACT_BELOW)
     if not args.skip_fp64:
         sec64, agg64, x64 = schedule(opts64)
         out["fp64"] = summary(sec64, agg64)
-        out["fp64"]["path"] = ("FP64 tangent (k_tangent element kernel with FP64 atomics), FP64 GMRES(80) with the "
-                               "FP64 multigrid, FP64 residual and history")
+        out["fp64"]["path"] = ("FP64 tangent (k_cell_matrices64 + k_rows_from_slabs), FP64 GMRES(80) with the FP64 "
+                               "multigrid, FP64 residual and history")
         opts_t = g.default_options(precision=nuto_gb300.FP64, newton_rtol=1e-11, krylov_rtol=1e-6, max_newton=40,
                                    max_krylov=20000)
         try:
@@ -895,9 +894,9 @@ def run_hex20(args):
         res["mixed_vs_fp64_path"] = {"max": float(np.abs(a - b).max() / np.abs(b).max()),
                                      "l2": float(np.linalg.norm(a - b) / np.linalg.norm(b))}
         res["speedup_newton_step_mixed_vs_fp64"] = out["fp64"]["newton_step_ms"] / out["mixed"]["newton_step_ms"]
-    # the FP32 tangent (tensor cores: k_tc20_points + k_tangent_tc20 + k_tc20_rows) at the final state of the last
+    # the FP32 tangent (tensor cores: k_tc20_points + k_tangent_tc20 + k_rows_from_wide_slabs) at the final state of the last
     # run (damaged points at the fixed face's edges), timed with CUDA events, and its error against the FP64
-    # tangent (element kernel, FP64 law and products) at the same state
+    # tangent (k_cell_matrices64_h20) at the same state
     x_end = torch.as_tensor(g.get_state()[0], device="cuda")
     k64 = g.build_matrix(x_end, nuto_gb300.FP64)
     k32 = torch.empty(g.nnz, dtype=torch.float32, device="cuda")
@@ -915,7 +914,7 @@ def run_hex20(args):
     tb = tangent_bytes(s, g.nnz, 4)
     peak, peak_kind = load_peaks()
     res["tangent_fp32"] = {"kernels": "k_tc20_points + k_tangent_tc20 (tcgen05.mma kind::tf32, three-product split, "
-                                      "accumulators in tensor memory) + k_tc20_rows",
+                                      "accumulators in tensor memory) + k_rows_from_wide_slabs",
                            "ms_per_assembly": ms, "assembled_dofs_per_s": g.n_dofs / (ms / 1e3),
                            "algorithmic_bytes": tb, "hbm_frac": tb / (ms / 1e3) / 1e9 / peak, "peak_kind": peak_kind,
                            "max_rel_error_vs_fp64_tangent": err,

@@ -96,7 +96,7 @@ extern "C" {
 
 /* preconditioners of PCG and GMRES (nuto_gpu_set_preconditioner) */
 #define NUTO_GPU_PRECOND_JACOBI 1 /* diagonal */
-#define NUTO_GPU_PRECOND_AMG 2    /* aggregation multigrid V-cycle in FP32 (default) */
+#define NUTO_GPU_PRECOND_AMG 2    /* multigrid V-cycle in the tangent's arithmetic (default) */
 
 typedef struct nuto_gpu_ctx nuto_gpu_ctx;
 
@@ -312,7 +312,7 @@ int nuto_gpu_solve(nuto_gpu_ctx* ctx, int precision, int method, const void* d_v
 int nuto_gpu_spmv(nuto_gpu_ctx* ctx, int precision, const void* d_values, const double* d_x, double* d_y,
                   int compensated);
 /* Preconditioner of the PCG and GMRES solves of nuto_gpu_solve and nuto_gpu_do_step (NUTO_GPU_PRECOND_*). The
-   multigrid hierarchy (spatial aggregates of the DOF nodes, piecewise-constant transfer per component) is built
+   multigrid hierarchy (kept DOF nodes per level, linear interpolation between them) is built
    on the first solve after build_pattern; its coarse operators are rebuilt once per tangent. No counterpart in
    the reference, which factorises the matrix (EigenSparseSolve.cpp:22-73). */
 int nuto_gpu_set_preconditioner(nuto_gpu_ctx* ctx, int preconditioner);

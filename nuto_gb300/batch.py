@@ -6,8 +6,8 @@ touch (NuTo's AddDofInterpolation merges DOF nodes at equal coordinates). Every 
 tangent, history, the Krylov solver and its multigrid -- then runs once over all cells and DOFs of the batch per
 launch. The work unit of every launch is the cell (or the node row), not the specimen, so specimens of uneven size
 need no load balancing: a plate of 120 x 120 cells and one of 20 x 20 are the same stream of cells. The matrix is
-block diagonal with one block per specimen; the multigrid's aggregates never cross a specimen because no matrix
-entry does.
+block diagonal with one block per specimen; the multigrid's interpolation never crosses a specimen because no
+matrix entry does.
 
 Equivalence to solving each specimen alone (what NuTo's QuasistaticSolver does per problem,
 nuto/mechanics/tools/QuasistaticSolver.cpp:51-147):

@@ -13,15 +13,15 @@
 // count (the 1 x 1 x 4 beam first coarsens across its short sides). A kept node hands its value on; any other interpolates
 // between its (at most 8, the nearest) kept neighbours with weights 1 / distance, which on a lattice is the multilinear
 // interpolation. Quadratic cells first drop to their corner nodes with the linear shape functions as weights. Levels stop at
-// kCoarsest nodes. Restriction is the transpose; constrained DOFs take part in neither. Against aggregates of the same size
-// with piecewise constant transfer, GMRES on a damaged, distorted beam to 1e-13 went from 306
-// iterations (52 ms) to 96 (18.5 ms) at 24^3 in FP32 and from 302 (88 ms) to 57 (18 ms) at 20^3 in FP64.
+// kCoarsest nodes. Restriction is the transpose; constrained DOFs take part in neither. Against aggregates of the same size with
+// piecewise constant transfer, GMRES on a damaged, distorted beam to 1e-13 went from 306 iterations (52 ms) to 96 (18.5 ms) at
+// 24^3 in FP32 and from 302 (88 ms) to 57 (18 ms) at 20^3 in FP64; with exact solves of both blocks it takes 25 at 16^3.
 // Coarse operators keep the node-block CSR layout, so the node SpMV serves every level; level 0 is a diagonal-block view of
 // the tangent itself.
 //
 // Per tangent (device, in the arithmetic of the tangent: FP32 or FP64): Galerkin coarse values A_c = P^T A P by
-// one pass over the finer values, A P in shared memory and the rest with atomics; Jacobi diagonals and Gershgorin bounds of D^-1 A per level. Cycle: V(1,2) with Chebyshev-Jacobi
-// smoothing on [lmax / 10, lmax] and a degree-6 Chebyshev solve on the coarsest level. The sweep is a fixed
+// one pass over the finer values, A P in shared memory and the rest with atomics; Jacobi diagonals and Gershgorin
+// bounds of D^-1 A per level. Cycle: V(1,2) with Chebyshev-Jacobi smoothing on [lmax / 10, lmax] and a degree-6 Chebyshev solve on the coarsest level. The sweep is a fixed
 // linear operator; GMRES uses it in flexible form (stored preconditioned basis) so rounding inside the cycle does
 // not limit the attainable residual.
 #include "spmv.cuh"

@@ -1496,8 +1496,8 @@ static void LaunchTangentT(Ctx& c, const double* u, T* vals)
     // atomics.
     if (sizeof(T) == 4 && RowsSupported(c) && !c.forceAtomicTangent)
     {
-        // linear cells: node rows from per-point records; Hex20: element matrices on the tensor cores + row
-        // gather; otherwise FP64-law records + row gather
+        // linear cells: element matrices + row gather; Hex20: the same with the element matrices from the tensor cores;
+        // otherwise FP64-law records + row gather
         if (!c.forceRecordTangent && FusedTangentSupported(c))
             LaunchTangentFused(c, u, reinterpret_cast<float*>(vals));
         else if (!c.forceRecordTangent && Tc20TangentSupported(c))

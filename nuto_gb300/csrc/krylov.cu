@@ -1,5 +1,5 @@
 // Preconditioned Krylov solvers (PCG for SPD tangents; GMRES and BiCGStab for the non-symmetric damage tangents;
-// Jacobi or the aggregation multigrid cycle of amg.cu) on the CSR tangent, replacing the sparse direct solve of the reference (Solve.cpp:8-34 with
+// Jacobi or the multigrid cycle of amg.cu) on the CSR tangent, replacing the sparse direct solve of the reference (Solve.cpp:8-34 with
 // EigenSparseSolve.cpp:22-73). The constrained system C^T K C y = C^T b of unit (Dirichlet) constraints is
 // solved in place: dependent rows act as identity and the iterates stay zero there, so the dependent columns
 // never contribute.
