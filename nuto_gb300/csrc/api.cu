@@ -199,6 +199,9 @@ void BuildTables(Ctx& c)
     }
     c.dTables.alloc(packed.size());
     NG_CUDA(cudaMemcpy(c.dTables.p, packed.data(), packed.size() * sizeof(double), cudaMemcpyHostToDevice));
+    const std::vector<float> packed32(packed.begin(), packed.end());
+    c.dTables32.alloc(packed32.size());
+    NG_CUDA(cudaMemcpy(c.dTables32.p, packed32.data(), packed32.size() * sizeof(float), cudaMemcpyHostToDevice));
 }
 
 template <typename T>

@@ -368,6 +368,7 @@ struct Ctx
     std::vector<double> hCoords;
     std::vector<int32_t> hGeoConn;
     DBuf<double> dTables; // w | N(interp) | dN(interp) packed, see TableOffsets
+    DBuf<float> dTables32; // the same in FP32
     int tabW = 0, tabN[3] = {0, 0, 0}, tabDN[3] = {0, 0, 0};
 
     // DOF types

@@ -77,9 +77,9 @@ struct Tc20Args
     const double* escale;  // per-cell Young's modulus factor (nullptr: 1)
     const double* geo64;   // FP64 geometry cache (the fallback strain)
     int geoStride;
-    const double* tabDNg;  // [q][8][3]
-    const double* tabDNd;  // [q][20][3]
-    const double* tabW;    // [q]
+    const float* tabDNg;   // [q][8][3]
+    const float* tabDNd;   // [q][20][3]
+    const float* tabW;     // [q]
 };
 
 // ---- tcgen05 / mbarrier wrappers (inline PTX, sm_100-class tensor cores) --------------------------------------
@@ -193,12 +193,22 @@ __device__ __forceinline__ float Tf32Round(float x)
 
 // ---- records: geometry and law per (cell, point) ------------------------------------------------------------
 
-template <int KIND>
-__global__ void __launch_bounds__(128) k_tc20_points(Tc20Args A, LawParams L, const double* __restrict__ u,
+// A block takes 7 cells, 189 of its 192 lanes a point each: the FP64 pipe, which bounds the kernel, takes as long for a warp
+// with idle lanes as for a full one (24^3: 180 us with 4 cells in 128 lanes and resident blocks that convert the tables,
+// 145 us). With fewer than 3 blocks of 7 cells per SM, 4 cells in 128 lanes spread
+// the work better (whole tangent, 4 against 7 cells: 13^3 97 and 101 us, 15^3 141 and 140, 16^3 165 and 159). The tables
+// come in FP32: a conversion is an FP64-pipe instruction.
+template <int CPB>
+constexpr int PointThreads()
+{
+    return (CPB * kNip + 31) / 32 * 32;
+}
+
+template <int KIND, int CPB>
+__global__ void __launch_bounds__(PointThreads<CPB>()) k_tc20_points(Tc20Args A, LawParams L, const double* __restrict__ u,
                                                       float4* __restrict__ recs, int lawFp64)
 {
     constexpr bool LD = KIND == NUTO_GPU_MB_LOCAL_DAMAGE;
-    constexpr int CPB = 4; // cells per block: 108 of 128 threads evaluate a point
     __shared__ float sDNg[kNip * kNg * 3];
     __shared__ float sDNd[kNip * kNd * 3];
     __shared__ float sW[kNip];
@@ -207,205 +217,202 @@ __global__ void __launch_bounds__(128) k_tc20_points(Tc20Args A, LawParams L, co
     __shared__ float sUr[CPB][kNd][3]; // displacements relative to the cell's first node (LD), formed in FP64
     const int64_t n = A.nCells;
     for (int i = threadIdx.x; i < kNip * kNg * 3; i += blockDim.x)
-        sDNg[i] = static_cast<float>(A.tabDNg[i]);
+        sDNg[i] = A.tabDNg[i];
     for (int i = threadIdx.x; i < kNip * kNd * 3; i += blockDim.x)
-        sDNd[i] = static_cast<float>(A.tabDNd[i]);
+        sDNd[i] = A.tabDNd[i];
     for (int i = threadIdx.x; i < kNip; i += blockDim.x)
-        sW[i] = static_cast<float>(A.tabW[i]);
-    for (int64_t cell0 = static_cast<int64_t>(blockIdx.x) * CPB; cell0 < n; cell0 += static_cast<int64_t>(gridDim.x) * CPB)
+        sW[i] = A.tabW[i];
+    const int64_t cell0 = static_cast<int64_t>(blockIdx.x) * CPB;
+    for (int it = threadIdx.x; it < CPB * kNg * 3; it += blockDim.x)
     {
-        for (int it = threadIdx.x; it < CPB * kNg * 3; it += blockDim.x)
-        {
-            const int cl = it % CPB, r = it / CPB; // r = node * 3 + d
-            const int64_t e = cell0 + cl;
-            if (e < n)
-                sX[cl][r / 3][r % 3] = A.relX[static_cast<int64_t>(r) * n + e];
-        }
-        for (int it = threadIdx.x; it < CPB * kNd; it += blockDim.x)
-        {
-            const int cl = it % CPB, nd = it / CPB;
-            const int64_t e = cell0 + cl;
-            if (e >= n)
-                continue;
-            const int64_t g = A.gdofD[NG_IDX(A.connD[static_cast<int64_t>(nd) * n + e], A.nNodesD, 60)];
+        const int cl = it % CPB, r = it / CPB; // r = node * 3 + d
+        const int64_t e = cell0 + cl;
+        if (e < n)
+            sX[cl][r / 3][r % 3] = A.relX[static_cast<int64_t>(r) * n + e];
+    }
+    for (int it = threadIdx.x; it < CPB * kNd; it += blockDim.x)
+    {
+        const int cl = it % CPB, nd = it / CPB;
+        const int64_t e = cell0 + cl;
+        if (e >= n)
+            continue;
+        const int64_t g = A.gdofD[NG_IDX(A.connD[static_cast<int64_t>(nd) * n + e], A.nNodesD, 60)];
 #pragma unroll
-            for (int c = 0; c < 3; ++c)
-                sU[cl][nd][c] = u[NG_IDX(g + c, A.nDofs, 61)];
+        for (int c = 0; c < 3; ++c)
+            sU[cl][nd][c] = u[NG_IDX(g + c, A.nDofs, 61)];
+    }
+    __syncthreads();
+    if (LD)
+    {
+        for (int it = threadIdx.x; it < CPB * kNd * 3; it += blockDim.x)
+        {
+            const int cl = it / (kNd * 3), k = it % (kNd * 3);
+            (&sUr[cl][0][0])[k] = static_cast<float>((&sU[cl][0][0])[k] - sU[cl][0][k % 3]);
         }
         __syncthreads();
-        if (LD)
-        {
-            for (int it = threadIdx.x; it < CPB * kNd * 3; it += blockDim.x)
-            {
-                const int cl = it / (kNd * 3), k = it % (kNd * 3);
-                (&sUr[cl][0][0])[k] = static_cast<float>((&sU[cl][0][0])[k] - sU[cl][0][k % 3]);
-            }
-            __syncthreads();
-        }
-        const int cl = threadIdx.x / kNip, q = threadIdx.x % kNip;
-        const int64_t e = cell0 + cl;
-        if (threadIdx.x < CPB * kNip && e < n)
-        {
-            // Jacobian J[i][j] = dx_i / dxi_j from the relative coordinates (k_geometry's formulas in FP32)
-            float J[3][3];
+    }
+    const int cl = threadIdx.x / kNip, q = threadIdx.x % kNip;
+    const int64_t e = cell0 + cl;
+    if (threadIdx.x < CPB * kNip && e < n)
+    {
+        // Jacobian J[i][j] = dx_i / dxi_j from the relative coordinates (k_geometry's formulas in FP32)
+        float J[3][3];
 #pragma unroll
-            for (int i = 0; i < 3; ++i)
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+            {
+                float s = 0.f;
+#pragma unroll
+                for (int nd = 1; nd < kNg; ++nd) // node 0 sits at the origin of the relative coordinates
+                    s += sX[cl][nd][i] * sDNg[(q * kNg + nd) * 3 + j];
+                J[i][j] = s;
+            }
+        const float c00 = J[1][1] * J[2][2] - J[1][2] * J[2][1];
+        const float c10 = J[1][2] * J[2][0] - J[1][0] * J[2][2];
+        const float c20 = J[1][0] * J[2][1] - J[1][1] * J[2][0];
+        const float det = J[0][0] * c00 + J[0][1] * c10 + J[0][2] * c20;
+        const float id = 1.f / det;
+        float inv[3][3];
+        inv[0][0] = c00 * id;
+        inv[1][0] = c10 * id;
+        inv[2][0] = c20 * id;
+        inv[0][1] = (J[0][2] * J[2][1] - J[0][1] * J[2][2]) * id;
+        inv[1][1] = (J[0][0] * J[2][2] - J[0][2] * J[2][0]) * id;
+        inv[2][1] = (J[0][1] * J[2][0] - J[0][0] * J[2][1]) * id;
+        inv[0][2] = (J[0][1] * J[1][2] - J[0][2] * J[1][1]) * id;
+        inv[1][2] = (J[0][2] * J[1][0] - J[0][0] * J[1][2]) * id;
+        inv[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) * id;
+        const float wdj = sW[q] * det;
+        const float wdjE = A.escale ? wdj * static_cast<float>(A.escale[e]) : wdj;
+        float lamw, muw, sv[6], tv[6];
+#pragma unroll
+        for (int v = 0; v < 6; ++v)
+            sv[v] = tv[v] = 0.f;
+        if (!LD)
+        {
+            lamw = static_cast<float>(L.C12) * wdjE;
+            muw = static_cast<float>(L.C33) * wdjE;
+        }
+        else
+        {
+            // displacement gradient H = (sum_a u_a (x) dN_a/dxi) J^-1, and the same sums of magnitudes for the bound
+            float Hx[3][3], Ha[3][3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
 #pragma unroll
                 for (int j = 0; j < 3; ++j)
-                {
-                    float s = 0.f;
-#pragma unroll
-                    for (int nd = 1; nd < kNg; ++nd) // node 0 sits at the origin of the relative coordinates
-                        s += sX[cl][nd][i] * sDNg[(q * kNg + nd) * 3 + j];
-                    J[i][j] = s;
-                }
-            const float c00 = J[1][1] * J[2][2] - J[1][2] * J[2][1];
-            const float c10 = J[1][2] * J[2][0] - J[1][0] * J[2][2];
-            const float c20 = J[1][0] * J[2][1] - J[1][1] * J[2][0];
-            const float det = J[0][0] * c00 + J[0][1] * c10 + J[0][2] * c20;
-            const float id = 1.f / det;
-            float inv[3][3];
-            inv[0][0] = c00 * id;
-            inv[1][0] = c10 * id;
-            inv[2][0] = c20 * id;
-            inv[0][1] = (J[0][2] * J[2][1] - J[0][1] * J[2][2]) * id;
-            inv[1][1] = (J[0][0] * J[2][2] - J[0][2] * J[2][0]) * id;
-            inv[2][1] = (J[0][1] * J[2][0] - J[0][0] * J[2][1]) * id;
-            inv[0][2] = (J[0][1] * J[1][2] - J[0][2] * J[1][1]) * id;
-            inv[1][2] = (J[0][2] * J[1][0] - J[0][0] * J[1][2]) * id;
-            inv[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) * id;
-            const float wdj = sW[q] * det;
-            const float wdjE = A.escale ? wdj * static_cast<float>(A.escale[e]) : wdj;
-            float lamw, muw, sv[6], tv[6];
-#pragma unroll
-            for (int v = 0; v < 6; ++v)
-                sv[v] = tv[v] = 0.f;
-            if (!LD)
+                    Hx[c][j] = Ha[c][j] = 0.f;
+            for (int nd = 0; nd < kNd; ++nd)
             {
-                lamw = static_cast<float>(L.C12) * wdjE;
-                muw = static_cast<float>(L.C33) * wdjE;
-            }
-            else
-            {
-                // displacement gradient H = (sum_a u_a (x) dN_a/dxi) J^-1, and the same sums of magnitudes for the bound
-                float Hx[3][3], Ha[3][3];
+                const float* dn = sDNd + (q * kNd + nd) * 3;
 #pragma unroll
                 for (int c = 0; c < 3; ++c)
+                {
+                    const float uc = sUr[cl][nd][c];
 #pragma unroll
                     for (int j = 0; j < 3; ++j)
-                        Hx[c][j] = Ha[c][j] = 0.f;
-                for (int nd = 0; nd < kNd; ++nd)
-                {
-                    const float* dn = sDNd + (q * kNd + nd) * 3;
-#pragma unroll
-                    for (int c = 0; c < 3; ++c)
                     {
-                        const float uc = sUr[cl][nd][c];
-#pragma unroll
-                        for (int j = 0; j < 3; ++j)
-                        {
-                            Hx[c][j] += uc * dn[j];
-                            Ha[c][j] += fabsf(uc) * fabsf(dn[j]);
-                        }
+                        Hx[c][j] += uc * dn[j];
+                        Ha[c][j] += fabsf(uc) * fabsf(dn[j]);
                     }
-                }
-                float H[3][3], S = 0.f;
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
-#pragma unroll
-                    for (int k = 0; k < 3; ++k)
-                    {
-                        float h = 0.f, ha = 0.f;
-#pragma unroll
-                        for (int j = 0; j < 3; ++j)
-                        {
-                            h += Hx[c][j] * inv[j][k];
-                            ha += Ha[c][j] * fabsf(inv[j][k]);
-                        }
-                        H[c][k] = h;
-                        S += ha;
-                    }
-                float eps[6];
-                StrainFromH<float, 3>(H, eps);
-                const double kh = A.kappa[NG_IDX(e * kNip + q, n * kNip, 62)];
-                const float khf = static_cast<float>(kh), k0f = static_cast<float>(L.kappa0);
-                const float eqs = MisesValue<float, 3>(L, eps);
-                // the FP32 strain differs from k_residual's FP64 strain by well below 1e-5 S (S bounds the magnitudes that
-                // enter H); eq. strain's slope in the strain is below 10, so a margin of 1e-4 S separates both decisions.
-                // S is formed with displacements relative to the cell: with absolute ones nearly every warp had a point
-                // inside the margin and took the FP64 strain (265 us at 24^3 against 177 us).
-                const float bound = 1.0e-4f * S + 1.0e-30f;
-                const float kapf = eqs > khf ? eqs : khf;
-                const bool near = lawFp64 || !(fabsf(eqs - khf) > bound + 1.0e-6f * khf) ||
-                                  !(fabsf(kapf - k0f) > bound + 1.0e-6f * k0f);
-                double e64[6];
-#pragma unroll
-                for (int v = 0; v < 6; ++v)
-                    e64[v] = static_cast<double>(eps[v]);
-                if (near)
-                {
-                    // the FP64 strain of k_residual (geometry cache, same order of the sums)
-                    const double* G = A.geo64 + NG_IDX(static_cast<int64_t>(q) * A.geoStride * n + e, A.geoSize, 63);
-                    double H64[3][3];
-#pragma unroll
-                    for (int i = 0; i < 3; ++i)
-#pragma unroll
-                        for (int j = 0; j < 3; ++j)
-                            H64[i][j] = 0.;
-                    for (int nd = 0; nd < kNd; ++nd)
-                    {
-                        double g[3];
-#pragma unroll
-                        for (int d = 0; d < 3; ++d)
-                            g[d] = G[(1 + nd * 3 + d) * n];
-#pragma unroll
-                        for (int c = 0; c < 3; ++c)
-#pragma unroll
-                            for (int d = 0; d < 3; ++d)
-                                H64[c][d] += sU[cl][nd][c] * g[d];
-                    }
-                    StrainFromH<double, 3>(H64, e64);
-                }
-                // the law in FP64 (FP32 loses up to 4e-6 of the rank-1 part where K1 I1 + sqrt(...) cancels)
-                const double eq64 = MisesValue<double, 3>(L, e64);
-                const double kap = eq64 > kh ? eq64 : kh;
-                double phi = 1., dom = 0.;
-                if (!(kap < L.kappa0))
-                {
-                    const double ki = 1. / kap, ex = L.alpha * exp(L.beta * (L.kappa0 - kap));
-                    const double k0i = L.kappa0 * ki;
-                    phi = 1. - (1. - k0i * ((1. - L.alpha) + ex));
-                    dom = k0i * ((ki + L.beta) * ex + (1. - L.alpha) * ki);
-                }
-                lamw = static_cast<float>(phi * L.lamD) * wdjE;
-                muw = static_cast<float>(phi * L.muD) * wdjE;
-                const double tr = e64[0] + e64[1] + e64[2];
-                const double f = -dom, t = L.lamD * tr, fm = f * L.muD;
-#pragma unroll
-                for (int v = 0; v < 6; ++v)
-                    sv[v] = static_cast<float>(v < 3 ? f * (L.m2G * e64[v] + t) : fm * e64[v]) * wdjE;
-                // loading (EvolutionImplicit: eq >= kappa_h). At a converged state kappa_h is eq itself, written by
-                // k_history; this kernel's FP64 eq equals it mathematically but may differ in the last bits (the compiler
-                // contracts the sums of squares of the Mises norm into FMAs differently per kernel), so a point within 4
-                // ulps below kappa_h is loading, as it is in the kernels whose arithmetic matches k_history's bit for bit
-                if (eq64 >= kh - 4.0 * DBL_EPSILON * kh)
-                {
-                    double dk[6];
-                    MisesDerivative<double, 3>(L, e64, dk);
-#pragma unroll
-                    for (int v = 0; v < 6; ++v)
-                        tv[v] = static_cast<float>(dk[v]);
                 }
             }
-            float4* R = recs + (e * kNip + q) * kRecF4;
-            R[0] = make_float4(inv[0][0], inv[0][1], inv[0][2], inv[1][0]);
-            R[1] = make_float4(inv[1][1], inv[1][2], inv[2][0], inv[2][1]);
-            R[2] = make_float4(inv[2][2], lamw, muw, 0.f);
-            R[3] = make_float4(sv[0], sv[1], sv[2], sv[3]);
-            R[4] = make_float4(sv[4], sv[5], tv[0], tv[1]);
-            R[5] = make_float4(tv[2], tv[3], tv[4], tv[5]);
+            float H[3][3], S = 0.f;
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+#pragma unroll
+                for (int k = 0; k < 3; ++k)
+                {
+                    float h = 0.f, ha = 0.f;
+#pragma unroll
+                    for (int j = 0; j < 3; ++j)
+                    {
+                        h += Hx[c][j] * inv[j][k];
+                        ha += Ha[c][j] * fabsf(inv[j][k]);
+                    }
+                    H[c][k] = h;
+                    S += ha;
+                }
+            float eps[6];
+            StrainFromH<float, 3>(H, eps);
+            const double kh = A.kappa[NG_IDX(e * kNip + q, n * kNip, 62)];
+            const float khf = static_cast<float>(kh), k0f = static_cast<float>(L.kappa0);
+            const float eqs = MisesValue<float, 3>(L, eps);
+            // the FP32 strain differs from k_residual's FP64 strain by well below 1e-5 S (S bounds the magnitudes that
+            // enter H); eq. strain's slope in the strain is below 10, so a margin of 1e-4 S separates both decisions.
+            // S is formed with displacements relative to the cell: with absolute ones nearly every warp had a point
+            // inside the margin and took the FP64 strain (265 us at 24^3 against 177 us).
+            const float bound = 1.0e-4f * S + 1.0e-30f;
+            const float kapf = eqs > khf ? eqs : khf;
+            const bool near = lawFp64 || !(fabsf(eqs - khf) > bound + 1.0e-6f * khf) ||
+                              !(fabsf(kapf - k0f) > bound + 1.0e-6f * k0f);
+            double e64[6];
+#pragma unroll
+            for (int v = 0; v < 6; ++v)
+                e64[v] = static_cast<double>(eps[v]);
+            if (near)
+            {
+                // the FP64 strain of k_residual (geometry cache, same order of the sums)
+                const double* G = A.geo64 + NG_IDX(static_cast<int64_t>(q) * A.geoStride * n + e, A.geoSize, 63);
+                double H64[3][3];
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+#pragma unroll
+                    for (int j = 0; j < 3; ++j)
+                        H64[i][j] = 0.;
+                for (int nd = 0; nd < kNd; ++nd)
+                {
+                    double g[3];
+#pragma unroll
+                    for (int d = 0; d < 3; ++d)
+                        g[d] = G[(1 + nd * 3 + d) * n];
+#pragma unroll
+                    for (int c = 0; c < 3; ++c)
+#pragma unroll
+                        for (int d = 0; d < 3; ++d)
+                            H64[c][d] += sU[cl][nd][c] * g[d];
+                }
+                StrainFromH<double, 3>(H64, e64);
+            }
+            // the law in FP64 (FP32 loses up to 4e-6 of the rank-1 part where K1 I1 + sqrt(...) cancels)
+            const double eq64 = MisesValue<double, 3>(L, e64);
+            const double kap = eq64 > kh ? eq64 : kh;
+            double phi = 1., dom = 0.;
+            if (!(kap < L.kappa0))
+            {
+                const double ki = 1. / kap, ex = L.alpha * exp(L.beta * (L.kappa0 - kap));
+                const double k0i = L.kappa0 * ki;
+                phi = 1. - (1. - k0i * ((1. - L.alpha) + ex));
+                dom = k0i * ((ki + L.beta) * ex + (1. - L.alpha) * ki);
+            }
+            lamw = static_cast<float>(phi * L.lamD) * wdjE;
+            muw = static_cast<float>(phi * L.muD) * wdjE;
+            const double tr = e64[0] + e64[1] + e64[2];
+            const double f = -dom, t = L.lamD * tr, fm = f * L.muD;
+#pragma unroll
+            for (int v = 0; v < 6; ++v)
+                sv[v] = static_cast<float>(v < 3 ? f * (L.m2G * e64[v] + t) : fm * e64[v]) * wdjE;
+            // loading (EvolutionImplicit: eq >= kappa_h). At a converged state kappa_h is eq itself, written by
+            // k_history; this kernel's FP64 eq equals it mathematically but may differ in the last bits (the compiler
+            // contracts the sums of squares of the Mises norm into FMAs differently per kernel), so a point within 4
+            // ulps below kappa_h is loading, as it is in the kernels whose arithmetic matches k_history's bit for bit
+            if (eq64 >= kh - 4.0 * DBL_EPSILON * kh)
+            {
+                double dk[6];
+                MisesDerivative<double, 3>(L, e64, dk);
+#pragma unroll
+                for (int v = 0; v < 6; ++v)
+                    tv[v] = static_cast<float>(dk[v]);
+            }
         }
-        __syncthreads(); // the next pass overwrites the node data
+        float4* R = recs + (e * kNip + q) * kRecF4;
+        R[0] = make_float4(inv[0][0], inv[0][1], inv[0][2], inv[1][0]);
+        R[1] = make_float4(inv[1][1], inv[1][2], inv[2][0], inv[2][1]);
+        R[2] = make_float4(inv[2][2], lamw, muw, 0.f);
+        R[3] = make_float4(sv[0], sv[1], sv[2], sv[3]);
+        R[4] = make_float4(sv[4], sv[5], tv[0], tv[1]);
+        R[5] = make_float4(tv[2], tv[3], tv[4], tv[5]);
     }
 }
 
@@ -446,7 +453,7 @@ __device__ __forceinline__ void GroupSync(int id, int threads)
 // the MMAs take 1,600 and shared memory about 3,300 wavefronts. A group that gives up a wait leaves its loop; the other one's
 // waits run out too, so both reach the end.
 template <bool RANK1, int SPLIT>
-__global__ void __launch_bounds__(kTcThreads, 1) k_tangent_tc20(int64_t nCells, const double* __restrict__ tabDNd,
+__global__ void __launch_bounds__(kTcThreads, 1) k_tangent_tc20(int64_t nCells, const float* __restrict__ tabDNd,
                                                                const float4* __restrict__ recs,
                                                                float* __restrict__ em, int* __restrict__ status,
                                                                long long spin)
@@ -469,7 +476,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tangent_tc20(int64_t nCells, 
     for (int i = tid; i < kOpEnd / 16; i += kTcThreads)
         reinterpret_cast<float4*>(sm)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int i = tid; i < kNip * kNd * 3; i += kTcThreads)
-        sDN[i] = static_cast<float>(tabDNd[i]);
+        sDN[i] = tabDNd[i];
     if (tid == 0)
     {
         BarInit(bar0, 1);
@@ -770,15 +777,23 @@ void LaunchTangentTc20(Ctx& c, const double* u, float* vals)
     A.escale = c.dEScale.n ? c.dEScale.p : nullptr;
     A.geo64 = c.dGeo64.p;
     A.geoStride = c.geoStride;
-    A.tabDNg = c.dTables.p + c.tabDN[c.geoInterp];
-    A.tabDNd = c.dTables.p + c.tabDN[D.interp];
-    A.tabW = c.dTables.p + c.tabW;
-    // resident blocks that walk the cells: the shape tables are converted once per block
-    const unsigned pb = static_cast<unsigned>(std::min<int64_t>((n + 3) / 4, 8LL * std::max(c.smCount, 1)));
-    if (ld)
-        k_tc20_points<NUTO_GPU_MB_LOCAL_DAMAGE><<<pb, 128, 0, c.stream>>>(A, c.law, u, recs, c.tc20LawFp64);
+    A.tabDNg = c.dTables32.p + c.tabDN[c.geoInterp];
+    A.tabDNd = c.dTables32.p + c.tabDN[D.interp];
+    A.tabW = c.dTables32.p + c.tabW;
+    auto points = [&](auto cells) {
+        constexpr int CPB = decltype(cells)::value;
+        const unsigned blocks = static_cast<unsigned>((n + CPB - 1) / CPB);
+        if (ld)
+            k_tc20_points<NUTO_GPU_MB_LOCAL_DAMAGE, CPB>
+                    <<<blocks, PointThreads<CPB>(), 0, c.stream>>>(A, c.law, u, recs, c.tc20LawFp64);
+        else
+            k_tc20_points<NUTO_GPU_MB_LINEAR_ELASTIC, CPB>
+                    <<<blocks, PointThreads<CPB>(), 0, c.stream>>>(A, c.law, u, recs, 0);
+    };
+    if (n >= 7LL * 3 * std::max(c.smCount, 1))
+        points(std::integral_constant<int, 7>{});
     else
-        k_tc20_points<NUTO_GPU_MB_LINEAR_ELASTIC><<<pb, 128, 0, c.stream>>>(A, c.law, u, recs, 0);
+        points(std::integral_constant<int, 4>{});
     AfterLaunch(c, "k_tc20_points");
 
     const unsigned grid = static_cast<unsigned>(std::min<int64_t>(n, c.smCount > 0 ? c.smCount : 1));

@@ -1,4 +1,4 @@
-"""k_tangent_tc20 with one to four cells per block: its two accumulators and their barriers are handed between two groups of
+"""k_tangent_tc20 with one to 22 cells per block: its two accumulators and their barriers are handed between two groups of
 warps, so what can go wrong depends on how many cells a block walks (152 blocks on a GB300)."""
 import numpy as np
 import pytest
@@ -6,7 +6,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("cells", [(1, 1, 1), (8, 19, 1), (9, 17, 1), (16, 19, 1), (5, 61, 1), (457, 1, 1)])
+@pytest.mark.parametrize("cells", [(1, 1, 1), (8, 19, 1), (9, 17, 1), (16, 19, 1), (5, 61, 1), (457, 1, 1), (13, 19, 13)])
 @pytest.mark.parametrize("kind", [0, 1])
 def test_cells_per_block(cells, kind):
     """FP32 against the FP64 tangent at 2e-6 of the largest entry, twice with the same bits."""
