@@ -322,6 +322,7 @@ static void BuildPattern(Ctx& c)
     c.hRowPtr.assign(c.nDofs + 1, 0);
     for (int64_t r = 0; r < c.nDofs; ++r)
         c.hRowPtr[r + 1] = c.hRowPtr[r] + rowLen[r];
+    c.maxRowLen = rowLen.empty() ? 0 : static_cast<int64_t>(*std::max_element(rowLen.begin(), rowLen.end()));
     c.nnz = c.hRowPtr.back();
     NG_CHECK(c.nnz < (int64_t(1) << 40), NUTO_GPU_EINVAL, "pattern too large");
     NG_CHECK(*std::max_element(rowLen.begin(), rowLen.end()) <= 256, NUTO_GPU_EINVAL,

@@ -620,6 +620,8 @@ bool FusedTangentSupported(Ctx& c)
     const int eS = gd ? c.prm.eeq_slot : c.prm.disp_slot;
     for (int s : {c.prm.disp_slot, eS})
     {
+        if (c.maxRowLen <= kRowsCap)
+            break; // as on every lattice: no scan
         const Slot& S = c.slots[s];
         for (int64_t i = 0; i < S.nNodes; ++i)
             for (int k = 0; k < S.ncomp; ++k)

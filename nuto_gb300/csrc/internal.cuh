@@ -450,6 +450,7 @@ struct Ctx
     int rowChunks = 0;
     std::function<void(int64_t, int64_t)> onRowChunk;
     int rowChunksDone = 0;
+    int64_t maxRowLen = 0; // longest CSR row
     std::vector<int64_t> cellChunkEnd; // per chunk: one past the last cell its rows need
     cudaStream_t copyStream = nullptr;
     cudaEvent_t evCopy = nullptr;

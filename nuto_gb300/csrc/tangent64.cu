@@ -711,9 +711,12 @@ RowPlanArgs EnsureRowPlan(Ctx& c)
         else
             k_row_entries<8><<<blocks, 256, 0, c.stream>>>(A, entries, c.rowSlab, c.packedRanks, differ);
         AfterLaunch(c, "k_row_entries");
-        int h = 0;
-        NG_CUDA(cudaMemcpyAsync(&h, differ, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-        NG_CUDA(cudaStreamSynchronize(c.stream));
+        int h = 0; // without eeq rows there is nothing that could differ
+        if (gd)
+        {
+            NG_CUDA(cudaMemcpyAsync(&h, differ, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+            NG_CUDA(cudaStreamSynchronize(c.stream));
+        }
         c.rowPlanSame = h == 0;
         c.rowPlanKey = key;
     }

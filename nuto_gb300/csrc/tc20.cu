@@ -724,7 +724,7 @@ bool Hex20RowsSupported(Ctx& c)
                      (c.prm.kind == NUTO_GPU_MB_LOCAL_DAMAGE && c.prm.damage_application == NUTO_GPU_DAMAGE_FULL);
     if (!cells || !law)
         return false;
-    for (int64_t i = 0; i < D.nNodes; ++i)
+    for (int64_t i = 0; c.maxRowLen > kRowsCapWide && i < D.nNodes; ++i)
         for (int k = 0; k < 3; ++k)
         {
             const int64_t rr = D.offset + D.dof0[i] + k;
