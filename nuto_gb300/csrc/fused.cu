@@ -705,10 +705,10 @@ void LaunchTangentFused(Ctx& c, const double* u, float* vals)
             constexpr int DIM = decltype(dim)::value, KIND = decltype(kind)::value, WW = decltype(warps)::value;
             using C = CellShape<DIM, KIND>;
             using SL = Slab<DIM, C::nd, C::GD>;
-            const size_t bytes = static_cast<size_t>(c.nCells) * C::nd * SL::size * sizeof(float);
-            if (c.dElemMats.n < bytes)
-                c.dElemMats.alloc(bytes);
-            float* em = reinterpret_cast<float*>(c.dElemMats.p);
+            const size_t count = static_cast<size_t>(c.nCells) * C::nd * SL::size;
+            if (c.dElemMats32.n < count)
+                c.dElemMats32.alloc(count);
+            float* em = c.dElemMats32.p;
             constexpr size_t smem = C::smem(WW);
             auto cells = [&](auto kern, bool resident) {
                 if (smem > 48 * 1024)

@@ -421,9 +421,10 @@ struct Ctx
     int tc20Split = 3;
     bool forceTc20Off = false; // NUTO_GPU_TC20=off
     int tc20LawFp64 = 0;       // NUTO_GPU_TC20=fp64law: the law of every point in FP64
-    // element matrices of the last tangent in its arithmetic (one buffer for FP32 and FP64: every tangent of a context runs
-    // on its stream) and the plan of the row gather
-    DBuf<unsigned char> dElemMats;
+    // element matrices of the last tangent in each arithmetic, and the plan of the row gather. One buffer per arithmetic, sized
+    // at its first tangent: a captured tangent holds its address, which a first tangent of the other arithmetic must not move.
+    DBuf<float> dElemMats32;
+    DBuf<double> dElemMats64;
     DBuf<unsigned char> dRowPlan; // RowPlan per node, then slab numbers and packed ranks:
     uint32_t *rowSlab = nullptr, *packedRanks = nullptr;
     int rowPlanKey = 0; // slots the plan was built for (0: not built)
@@ -503,9 +504,9 @@ bool LaunchTangent64(Ctx& c, const double* u, double* vals);
 bool LaunchTangent64H20(Ctx& c, const double* u, double* vals); // for the cells of Hex20RowsSupported
 bool Hex20RowsSupported(Ctx& c);
 RowPlanArgs EnsureRowPlan(Ctx& c);
-// the context's element-matrix buffer with room for `bytes`; nullptr while it would have to grow during a stream capture or
-// beyond the free device memory
-unsigned char* ElemMatsOrNull(Ctx& c, size_t bytes);
+// the context's FP64 element-matrix buffer with room for `count` values; nullptr while it would have to grow during a stream
+// capture or beyond the free device memory
+double* ElemMats64OrNull(Ctx& c, size_t count);
 bool Tc20TangentSupported(Ctx& c);
 void LaunchTangentTc20(Ctx& c, const double* u, float* vals);
 int ReadDeviceStatus(Ctx& c); // after a stream synchronisation: the status word (and reset to 0)

@@ -538,8 +538,7 @@ bool LaunchTangent64H20(Ctx& c, const double* u, double* vals)
 {
     const bool ld = c.prm.kind == NUTO_GPU_MB_LOCAL_DAMAGE;
     const CellArgs a = CellArgsOf(c);
-    double* em = reinterpret_cast<double*>(
-            ElemMatsOrNull(c, static_cast<size_t>(c.nCells) * kH20Nd * 9 * kH20Nd * sizeof(double)));
+    double* em = ElemMats64OrNull(c, static_cast<size_t>(c.nCells) * kH20Nd * 9 * kH20Nd);
     if (!em)
         return false;
     const RowPlanArgs P = EnsureRowPlan(c);
@@ -567,8 +566,7 @@ bool LaunchTangent64(Ctx& c, const double* u, double* vals)
         constexpr bool GD = decltype(dmg)::value;
         using C = Cell64<DIM, GD>;
         using SL = Slab<DIM, C::nd, GD>;
-        double* em = reinterpret_cast<double*>(
-                ElemMatsOrNull(c, static_cast<size_t>(c.nCells) * C::nd * SL::size * sizeof(double)));
+        double* em = ElemMats64OrNull(c, static_cast<size_t>(c.nCells) * C::nd * SL::size);
         if (!em)
             return false;
         const RowPlanArgs P = EnsureRowPlan(c);
@@ -730,24 +728,25 @@ RowPlanArgs EnsureRowPlan(Ctx& c)
     return P;
 }
 
-unsigned char* ElemMatsOrNull(Ctx& c, size_t bytes)
+double* ElemMats64OrNull(Ctx& c, size_t count)
 {
-    if (c.dElemMats.n >= bytes)
-        return c.dElemMats.p;
+    DBuf<double>& B = c.dElemMats64;
+    if (B.n >= count)
+        return B.p;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     NG_CUDA(cudaStreamIsCapturing(c.stream, &cs));
     if (cs != cudaStreamCaptureStatusNone)
         return nullptr;
     // the attempt itself tells whether the memory is there (asking for the free memory first costs as much as a small assembly)
-    c.dElemMats.free();
-    unsigned char* p = nullptr;
-    if (cudaMalloc(&p, bytes) != cudaSuccess)
+    B.free();
+    double* p = nullptr;
+    if (cudaMalloc(&p, count * sizeof(double)) != cudaSuccess)
     {
         cudaGetLastError();
         return nullptr;
     }
-    c.dElemMats.p = p;
-    c.dElemMats.n = bytes;
+    B.p = p;
+    B.n = count;
     return p;
 }
 

@@ -759,10 +759,10 @@ void LaunchTangentTc20(Ctx& c, const double* u, float* vals)
     const size_t recBytes = static_cast<size_t>(n) * kNip * kRecF4 * 16;
     if (c.dRecords.n < recBytes)
         c.dRecords.alloc(recBytes);
-    const size_t emBytes = static_cast<size_t>(n) * kNd * 180 * sizeof(float);
-    if (c.dElemMats.n < emBytes)
-        c.dElemMats.alloc(emBytes);
-    float* em = reinterpret_cast<float*>(c.dElemMats.p);
+    const size_t emCount = static_cast<size_t>(n) * kNd * 180;
+    if (c.dElemMats32.n < emCount)
+        c.dElemMats32.alloc(emCount);
+    float* em = c.dElemMats32.p;
     float4* recs = reinterpret_cast<float4*>(c.dRecords.p);
 
     Tc20Args A{};
