@@ -1430,6 +1430,15 @@ static bool RowsSupported(Ctx& c)
             else if (m != E.conn[i])
                 return false;
         }
+        // nodes of no cell (empty rows in both fields) pair up in order
+        int32_t free = 0;
+        for (int32_t& m : eOf)
+            if (m < 0)
+            {
+                while (seen[free])
+                    ++free;
+                m = free++;
+            }
         c.dEOf.alloc(eOf.size());
         NG_CUDA(cudaMemcpy(c.dEOf.p, eOf.data(), eOf.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
         c.hEOf = eOf;
