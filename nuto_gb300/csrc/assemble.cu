@@ -1510,10 +1510,12 @@ static void LaunchTangentRows(Ctx& c, const double* u, T* vals)
 }
 
 // true while the context's stream is being captured and the FP64 tangent's first-use set-up (maps, buffers) is still to be
-// done: the element kernel, which needs none, is then taken
+// done: the element kernel, which needs none, is then taken. The Hex20 form is looked at only where the linear one does not
+// apply, so its mode stays undecided for linear cells.
 static bool SetUpInCapture(Ctx& c)
 {
-    if (c.rowsMode >= 0 && c.fusedMode >= 0 && c.h20Mode >= 0 && c.rowPlanKey != 0)
+    const bool decided = c.rowsMode >= 0 && c.fusedMode >= 0 && (c.fusedMode == 1 || c.h20Mode >= 0);
+    if (decided && RowPlanReady(c))
         return false;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     NG_CUDA(cudaStreamIsCapturing(c.stream, &cs));

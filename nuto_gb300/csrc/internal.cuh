@@ -504,6 +504,7 @@ bool LaunchTangent64(Ctx& c, const double* u, double* vals);
 bool LaunchTangent64H20(Ctx& c, const double* u, double* vals); // for the cells of Hex20RowsSupported
 bool Hex20RowsSupported(Ctx& c);
 RowPlanArgs EnsureRowPlan(Ctx& c);
+bool RowPlanReady(const Ctx& c); // the plan of the present pattern and integrand is there
 // the context's FP64 element-matrix buffer with room for `count` values; nullptr while it would have to grow during a stream
 // capture or beyond the free device memory
 double* ElemMats64OrNull(Ctx& c, size_t count);

@@ -660,6 +660,17 @@ __global__ void __launch_bounds__(256) k_row_entries(PlanArgs A, int64_t nEntrie
 
 } // namespace
 
+// the plan depends on the integrand's slots: whether there are eeq rows, and which slot they are in
+static int RowPlanKey(const Ctx& c)
+{
+    return 1 + c.prm.disp_slot + kMaxSlots * (c.prm.kind == NUTO_GPU_GRADIENT_DAMAGE ? 1 + c.prm.eeq_slot : 0);
+}
+
+bool RowPlanReady(const Ctx& c)
+{
+    return c.rowPlanKey == RowPlanKey(c);
+}
+
 RowPlanArgs EnsureRowPlan(Ctx& c)
 {
     const int ns = static_cast<int>(c.slots.size());
@@ -668,9 +679,7 @@ RowPlanArgs EnsureRowPlan(Ctx& c)
     const int eS = gd ? c.prm.eeq_slot : dS;
     const Slot& D = c.slots[dS];
     const int64_t entries = c.nCells * D.nen;
-    // the plan depends on the integrand's slots as well: whether there are eeq rows, and which slot they are in
-    const int key = 1 + dS + kMaxSlots * (gd ? 1 + eS : 0);
-    if (c.rowPlanKey != key)
+    if (!RowPlanReady(c))
     {
         c.cellChunkEnd.clear();
         // one allocation: the nodes' records, slab numbers, packed ranks, and the flag that the kernels below may raise
@@ -716,7 +725,7 @@ RowPlanArgs EnsureRowPlan(Ctx& c)
             NG_CUDA(cudaStreamSynchronize(c.stream));
         }
         c.rowPlanSame = h == 0;
-        c.rowPlanKey = key;
+        c.rowPlanKey = RowPlanKey(c);
     }
     RowPlanArgs P{};
     P.plan = reinterpret_cast<const RowPlan*>(c.dRowPlan.p);

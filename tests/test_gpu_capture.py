@@ -78,3 +78,44 @@ def test_replay_after_the_first_tangent_of_the_other_arithmetic(kind, n, precisi
     else:
         assert (out - direct).abs().max() <= 1e-12 * direct.abs().max()
     assert torch.isfinite(other).all()
+
+
+@pytest.mark.parametrize("kind,n", [("quad4", 9), ("plate", 12), ("hex8", 7), ("hex20", 3)])
+def test_captured_fp64_tangent_is_the_direct_call(kind, n):
+    """After one FP64 tangent everything a capture needs is there: the captured call runs the direct call's kernels and its
+    replays give the same bits."""
+    torch = _cuda()
+    s, u0, kappa = _case(kind, n)
+    stream = torch.cuda.Stream()
+    g = _group(s, kappa, stream)
+    u = torch.as_tensor(u0, device="cuda")
+    out = g.build_matrix(u, 64)
+    graph = _capture(g, stream, u, 64, out)
+    u.mul_(-0.75)
+    for _ in range(2):
+        out.zero_()
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        direct = g.build_matrix(u, 64)
+        torch.cuda.synchronize()
+        assert torch.equal(out, direct)
+
+
+@pytest.mark.parametrize("kind,n", [("quad4", 9), ("plate", 12), ("hex8", 7), ("hex20", 3)])
+@pytest.mark.parametrize("before", ["residual", "fp32"])
+def test_first_fp64_tangent_inside_a_capture(kind, n, before):
+    """Without an FP64 tangent before it the captured call allocates nothing and gives the tangent to rounding."""
+    torch = _cuda()
+    s, u0, kappa = _case(kind, n)
+    stream = torch.cuda.Stream()
+    g = _group(s, kappa, stream)
+    u = torch.as_tensor(u0, device="cuda")
+    g.build_vector(u) if before == "residual" else g.build_matrix(u, 32)
+    out = torch.empty(g.nnz, dtype=torch.float64, device="cuda")
+    graph = _capture(g, stream, u, 64, out)
+    graph.replay()
+    torch.cuda.synchronize()
+    direct = g.build_matrix(u, 64)
+    torch.cuda.synchronize()
+    assert (out - direct).abs().max() <= 1e-12 * direct.abs().max()
