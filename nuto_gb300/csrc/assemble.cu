@@ -1533,12 +1533,10 @@ static void LaunchTangentT(Ctx& c, const double* u, T* vals)
     if (sizeof(T) == 4 && RowsSupported(c) && !c.forceAtomicTangent)
     {
         // linear cells: element matrices + row gather; Hex20: the same with the element matrices from the tensor cores;
-        // otherwise FP64-law records + row gather
-        if (!c.forceRecordTangent && FusedTangentSupported(c))
-            LaunchTangentFused(c, u, reinterpret_cast<float*>(vals));
-        else if (!c.forceRecordTangent && Tc20TangentSupported(c))
-            LaunchTangentTc20(c, u, reinterpret_cast<float*>(vals));
-        else
+        // otherwise, and without memory for them, FP64-law records + row gather
+        float* v = reinterpret_cast<float*>(vals);
+        if (c.forceRecordTangent || !((FusedTangentSupported(c) && LaunchTangentFused(c, u, v)) ||
+                                      (Tc20TangentSupported(c) && LaunchTangentTc20(c, u, v))))
             LaunchTangentRows<T>(c, u, vals);
         PrepareNoAlloc(c);
         return;

@@ -658,14 +658,19 @@ static void EnsureCellChunks(Ctx& c, const Slot& D, int chunks)
     c.cellChunkEnd = std::move(end);
 }
 
-void LaunchTangentFused(Ctx& c, const double* u, float* vals)
+bool LaunchTangentFused(Ctx& c, const double* u, float* vals)
 {
-    if (c.dRelX.n == 0)
-        BuildRelativeCoordinates(c);
     const int dS = c.prm.disp_slot;
     const bool gd = c.prm.kind == NUTO_GPU_GRADIENT_DAMAGE;
     const int eS = gd ? c.prm.eeq_slot : dS;
     const Slot& D = c.slots[dS];
+    const size_t slab = c.dim == 3 ? (gd ? Slab<3, 8, true>::size : Slab<3, 8, false>::size)
+                                   : (gd ? Slab<2, 4, true>::size : Slab<2, 4, false>::size);
+    float* em = ElemMatsOrNull<float>(c, static_cast<size_t>(c.nCells) * D.nen * slab);
+    if (!em)
+        return false;
+    if (c.dRelX.n == 0)
+        BuildRelativeCoordinates(c);
     FusedArgs A{};
     A.nCells = c.nCells;
     A.nDofs = c.nDofs;
@@ -704,11 +709,6 @@ void LaunchTangentFused(Ctx& c, const double* u, float* vals)
         auto run = [&](auto dim, auto kind, auto warps) {
             constexpr int DIM = decltype(dim)::value, KIND = decltype(kind)::value, WW = decltype(warps)::value;
             using C = CellShape<DIM, KIND>;
-            using SL = Slab<DIM, C::nd, C::GD>;
-            const size_t count = static_cast<size_t>(c.nCells) * C::nd * SL::size;
-            if (c.dElemMats32.n < count)
-                c.dElemMats32.alloc(count);
-            float* em = c.dElemMats32.p;
             constexpr size_t smem = C::smem(WW);
             auto cells = [&](auto kern, bool resident) {
                 if (smem > 48 * 1024)
@@ -816,6 +816,7 @@ void LaunchTangentFused(Ctx& c, const double* u, float* vals)
         }
     }
     assemble(T.tangentWarps ? T.tangentWarps : 4, T.tangentForm);
+    return true;
 }
 
 } // namespace nuto_gpu

@@ -277,6 +277,16 @@ struct RowPlanArgs
     bool sameGraph; // the eeq row of every node has the positions of its displacement rows
 };
 
+// Element matrices in one arithmetic, scratch of its tangents. One buffer per arithmetic, sized at its first tangent: a captured
+// tangent holds its address, which a first tangent of the other arithmetic must not move. A count that did not fit is remembered
+// until the pattern or the integrand changes: the tangents take the forms without element matrices and ask no more.
+template <typename T>
+struct ElemMats
+{
+    DBuf<T> buf;
+    size_t refused = 0;
+};
+
 // Boundary cells of one DOF slot (NeumannBc loads): Line2 faces of a 2D mesh or Quad4 faces of a 3D mesh, on the
 // context's coordinate nodes and the slot's DOF nodes.
 struct BoundaryGroup
@@ -421,10 +431,9 @@ struct Ctx
     int tc20Split = 3;
     bool forceTc20Off = false; // NUTO_GPU_TC20=off
     int tc20LawFp64 = 0;       // NUTO_GPU_TC20=fp64law: the law of every point in FP64
-    // element matrices of the last tangent in each arithmetic, and the plan of the row gather. One buffer per arithmetic, sized
-    // at its first tangent: a captured tangent holds its address, which a first tangent of the other arithmetic must not move.
-    DBuf<float> dElemMats32;
-    DBuf<double> dElemMats64;
+    // element matrices of the last tangent in each arithmetic, and the plan of the row gather
+    ElemMats<float> elemMats32;
+    ElemMats<double> elemMats64;
     DBuf<unsigned char> dRowPlan; // RowPlan per node, then slab numbers and packed ranks:
     uint32_t *rowSlab = nullptr, *packedRanks = nullptr;
     int rowPlanKey = 0; // slots the plan was built for (0: not built)
@@ -498,18 +507,20 @@ void LaunchResidual(Ctx& c, const double* u, double* f, int blocksPerSm = 0); //
 void LaunchTangent(Ctx& c, const double* u, int precision, void* values);
 void LaunchTangentNoAlloc(Ctx& c, const double* u, float* values);
 bool FusedTangentSupported(Ctx& c);
-void LaunchTangentFused(Ctx& c, const double* u, float* vals);
+bool LaunchTangentFused(Ctx& c, const double* u, float* vals); // false: not done (no memory for the element matrices)
 // element matrices in FP64 + row gather for the cells of FusedTangentSupported; false: not done (no memory for them)
 bool LaunchTangent64(Ctx& c, const double* u, double* vals);
 bool LaunchTangent64H20(Ctx& c, const double* u, double* vals); // for the cells of Hex20RowsSupported
 bool Hex20RowsSupported(Ctx& c);
 RowPlanArgs EnsureRowPlan(Ctx& c);
 bool RowPlanReady(const Ctx& c); // the plan of the present pattern and integrand is there
-// the context's FP64 element-matrix buffer with room for `count` values; nullptr while it would have to grow during a stream
-// capture or beyond the free device memory
-double* ElemMats64OrNull(Ctx& c, size_t count);
+// the context's element matrices in T with room for `count` values; nullptr while the buffer would have to grow during a stream
+// capture or beyond the memory that can be had (FP64: beyond what the solves leave)
+template <typename T>
+T* ElemMatsOrNull(Ctx& c, size_t count);
+size_t SolverBytesToCome(const Ctx& c); // device memory that a first FP64 solve of the context will take (krylov.cu)
 bool Tc20TangentSupported(Ctx& c);
-void LaunchTangentTc20(Ctx& c, const double* u, float* vals);
+bool LaunchTangentTc20(Ctx& c, const double* u, float* vals); // false: not done (no memory for the element matrices)
 int ReadDeviceStatus(Ctx& c); // after a stream synchronisation: the status word (and reset to 0)
 void LaunchHistory(Ctx& c, const double* u);
 void LaunchLumpedMass(Ctx& c, double rho, double* m);

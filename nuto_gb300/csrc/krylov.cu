@@ -1552,6 +1552,22 @@ int ResolveMethod(const Ctx& c, int method)
     return c.prm.kind == NUTO_GPU_MB_LINEAR_ELASTIC ? NUTO_GPU_SOLVER_PCG : NUTO_GPU_SOLVER_GMRES;
 }
 
+// Device memory that a first FP64 solve of the context takes: the padded values, the multigrid's coarse levels (values in two
+// layouts; a fourth of the fine ones is on the safe side on lattices), its and the solver's vectors, and for GMRES both bases.
+size_t SolverBytesToCome(const Ctx& c)
+{
+    const size_t n = static_cast<size_t>(c.nDofs), nnz = static_cast<size_t>(c.nnz);
+    const SolverWork* w = c.work;
+    size_t values = 0;
+    if (c.nb.v64.n == 0)
+        values += static_cast<size_t>(c.nb.total) + nnz / 2 + 20 * n;
+    if (!w || w->v64.n == 0)
+        values += 21 * n;
+    if (c.prm.kind != NUTO_GPU_MB_LINEAR_ELASTIC && (!w || w->g64.n == 0))
+        values += (2 * static_cast<size_t>(c.gmresRestart > 1 ? std::min(c.gmresRestart, static_cast<int>(GL::m)) : kGmresRestart) + 3) * n;
+    return values * sizeof(double);
+}
+
 // nuto_gpu_solve: FP64 solve, or FP32 Krylov inside an FP64 iterative refinement (r = b - K x in FP64 with the
 // FP32 values) until |r| <= rtol |b|.
 int SolveLinear(Ctx& c, int precision, int method, const void* values, const double* b, double* x, double rtol,

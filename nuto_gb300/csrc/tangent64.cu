@@ -538,7 +538,7 @@ bool LaunchTangent64H20(Ctx& c, const double* u, double* vals)
 {
     const bool ld = c.prm.kind == NUTO_GPU_MB_LOCAL_DAMAGE;
     const CellArgs a = CellArgsOf(c);
-    double* em = ElemMats64OrNull(c, static_cast<size_t>(c.nCells) * kH20Nd * 9 * kH20Nd);
+    double* em = ElemMatsOrNull<double>(c, static_cast<size_t>(c.nCells) * kH20Nd * 9 * kH20Nd);
     if (!em)
         return false;
     const RowPlanArgs P = EnsureRowPlan(c);
@@ -566,7 +566,7 @@ bool LaunchTangent64(Ctx& c, const double* u, double* vals)
         constexpr bool GD = decltype(dmg)::value;
         using C = Cell64<DIM, GD>;
         using SL = Slab<DIM, C::nd, GD>;
-        double* em = ElemMats64OrNull(c, static_cast<size_t>(c.nCells) * C::nd * SL::size);
+        double* em = ElemMatsOrNull<double>(c, static_cast<size_t>(c.nCells) * C::nd * SL::size);
         if (!em)
             return false;
         const RowPlanArgs P = EnsureRowPlan(c);
@@ -737,26 +737,46 @@ RowPlanArgs EnsureRowPlan(Ctx& c)
     return P;
 }
 
-double* ElemMats64OrNull(Ctx& c, size_t count)
+template <typename T>
+T* ElemMatsOrNull(Ctx& c, size_t count)
 {
-    DBuf<double>& B = c.dElemMats64;
-    if (B.n >= count)
-        return B.p;
+    ElemMats<T>* E;
+    if constexpr (sizeof(T) == 4)
+        E = &c.elemMats32;
+    else
+        E = &c.elemMats64;
+    if (E->buf.n >= count)
+        return E->buf.p;
+    if (E->refused != 0 && count >= E->refused)
+        return nullptr;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     NG_CUDA(cudaStreamIsCapturing(c.stream, &cs));
     if (cs != cudaStreamCaptureStatusNone)
         return nullptr;
-    // the attempt itself tells whether the memory is there (asking for the free memory first costs as much as a small assembly)
-    B.free();
-    double* p = nullptr;
-    if (cudaMalloc(&p, count * sizeof(double)) != cudaSuccess)
+    const size_t bytes = count * sizeof(T);
+    bool room = true;
+    // The element kernel needs no scratch, so a large FP64 problem may have just the memory for its solver. Asking for the free
+    // memory costs as much as a small assembly: below this size (1 GB of tangent at most) the attempt alone decides.
+    if (sizeof(T) == 8 && bytes >= (size_t(256) << 20))
     {
+        size_t free = 0, total = 0;
+        NG_CUDA(cudaMemGetInfo(&free, &total));
+        room = bytes + SolverBytesToCome(c) <= free;
+    }
+    T* p = nullptr;
+    if (room && cudaMalloc(&p, bytes) != cudaSuccess)
         cudaGetLastError();
+    if (!p)
+    {
+        E->refused = count;
         return nullptr;
     }
-    B.p = p;
-    B.n = count;
+    E->buf.free();
+    E->buf.p = p;
+    E->buf.n = count;
     return p;
 }
+template float* ElemMatsOrNull<float>(Ctx&, size_t);
+template double* ElemMatsOrNull<double>(Ctx&, size_t);
 
 } // namespace nuto_gpu

@@ -742,8 +742,11 @@ bool Tc20TangentSupported(Ctx& c)
     return c.tc20Mode == 1;
 }
 
-void LaunchTangentTc20(Ctx& c, const double* u, float* vals)
+bool LaunchTangentTc20(Ctx& c, const double* u, float* vals)
 {
+    float* em = ElemMatsOrNull<float>(c, static_cast<size_t>(c.nCells) * kNd * 180);
+    if (!em)
+        return false;
     if (c.dRelX.n == 0)
         BuildRelativeCoordinates(c);
     if (!c.haveGeo)
@@ -759,10 +762,6 @@ void LaunchTangentTc20(Ctx& c, const double* u, float* vals)
     const size_t recBytes = static_cast<size_t>(n) * kNip * kRecF4 * 16;
     if (c.dRecords.n < recBytes)
         c.dRecords.alloc(recBytes);
-    const size_t emCount = static_cast<size_t>(n) * kNd * 180;
-    if (c.dElemMats32.n < emCount)
-        c.dElemMats32.alloc(emCount);
-    float* em = c.dElemMats32.p;
     float4* recs = reinterpret_cast<float4*>(c.dRecords.p);
 
     Tc20Args A{};
@@ -819,6 +818,7 @@ void LaunchTangentTc20(Ctx& c, const double* u, float* vals)
 
     LaunchWideRows<float, kNd>(c, EnsureRowPlan(c), D.nNodes, em, vals);
     c.stats.kernel_launches += 2;
+    return true;
 }
 
 int ReadDeviceStatus(Ctx& c)
