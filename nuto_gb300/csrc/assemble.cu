@@ -217,7 +217,8 @@ void BuildGeometryCache(Ctx& c)
     c.haveGeo = true;
 }
 
-// FP32 copy of the geometry cache, made the first time the FP32 element kernel (atomics) runs on this geometry
+// FP32 copy of the geometry cache, made the first time the FP32 element kernel (atomics) runs on this geometry; in a stream
+// capture, which allows no allocation, that kernel converts the FP64 values instead (the same numbers)
 __global__ void __launch_bounds__(256) k_geometry32(int64_t n, const double* __restrict__ geo64,
                                                     float* __restrict__ geo32)
 {
@@ -229,6 +230,10 @@ __global__ void __launch_bounds__(256) k_geometry32(int64_t n, const double* __r
 static void EnsureGeo32(Ctx& c)
 {
     if (c.dGeo32.n == c.dGeo64.n)
+        return;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    NG_CUDA(cudaStreamIsCapturing(c.stream, &cs));
+    if (cs != cudaStreamCaptureStatusNone)
         return;
     c.dGeo32.alloc(c.dGeo64.n);
     k_geometry32<<<static_cast<unsigned>(std::max(c.smCount, 1) * 8), 256, 0, c.stream>>>(
@@ -885,10 +890,7 @@ __global__ void __launch_bounds__(256) k_tangent(CellArgs a, LawParams L, Scatte
         if (e >= n)
             continue;
         const int64_t idx = NG_IDX((static_cast<int64_t>(q) * a.geoStride + 1 + nd * DIM + d) * n + e, a.geoSize, 6);
-        if (sizeof(T) == 4)
-            sG[cl][q][nd][d] = static_cast<T>(a.geo32[idx]);
-        else
-            sG[cl][q][nd][d] = static_cast<T>(a.geo64[idx]);
+        sG[cl][q][nd][d] = sizeof(T) == 4 && a.geo32 ? static_cast<T>(a.geo32[idx]) : static_cast<T>(a.geo64[idx]);
     }
     __syncthreads();
 
@@ -900,7 +902,7 @@ __global__ void __launch_bounds__(256) k_tangent(CellArgs a, LawParams L, Scatte
         if (e >= n)
             continue;
         const int64_t widx = NG_IDX(static_cast<int64_t>(q) * a.geoStride * n + e, a.geoSize, 6);
-        const T wdj = sizeof(T) == 4 ? static_cast<T>(a.geo32[widx]) : static_cast<T>(a.geo64[widx]);
+        const T wdj = sizeof(T) == 4 && a.geo32 ? static_cast<T>(a.geo32[widx]) : static_cast<T>(a.geo64[widx]);
         // per-cell Young's modulus factor: scales the material tangent and dsigma/domega (displacement rows)
         const T wdjE = a.escale ? wdj * static_cast<T>(a.escale[e]) : wdj;
         T H[DIM][DIM];

@@ -568,7 +568,7 @@ struct CellArgs
     const double* tabN_D; // nIp x nenD
     const double* tabN_E;
     const double* geo64;
-    const float* geo32;
+    const float* geo32; // nullptr: not made (the FP32 element kernel then converts geo64)
     const double* jac; // planar [(q * (1 + dim^2) + k)][cell] or nullptr
     int64_t jacSize;
     int geoStride;

@@ -119,3 +119,23 @@ def test_first_fp64_tangent_inside_a_capture(kind, n, before):
     direct = g.build_matrix(u, 64)
     torch.cuda.synchronize()
     assert (out - direct).abs().max() <= 1e-12 * direct.abs().max()
+
+
+@pytest.mark.parametrize("kind,n", [("quad4", 9), ("hex20", 3)])
+def test_first_fp32_element_kernel_inside_a_capture(kind, n, monkeypatch):
+    """The FP32 element kernel needs the geometry of the residual and no memory of its own: what it is first called in may be a
+    capture. Each value sums at most 8 cells' blocks by atomics, in any order: 2e-6 of the largest."""
+    torch = _cuda()
+    monkeypatch.setenv("NUTO_GPU_TANGENT", "atomic")
+    s, u0, kappa = _case(kind, n)
+    stream = torch.cuda.Stream()
+    g = _group(s, kappa, stream)
+    u = torch.as_tensor(u0, device="cuda")
+    g.build_vector(u)
+    out = torch.empty(g.nnz, dtype=torch.float32, device="cuda")
+    graph = _capture(g, stream, u, 32, out)
+    graph.replay()
+    torch.cuda.synchronize()
+    direct = g.build_matrix(u, 32)
+    torch.cuda.synchronize()
+    assert (out - direct).abs().max() <= 2e-6 * direct.abs().max()
