@@ -585,12 +585,31 @@ static void EnsureSideStream(Ctx& c)
     NG_CUDA(cudaEventCreateWithFlags(&c.evJoin, cudaEventDisableTiming));
 }
 
-// Quad4 gradient damage: the residual and the tangent slow each other down more than the overlap gives (sysResBlocks).
-// With host buffers the copy of the values is longer than either and overlaps them.
-static bool SystemInSequence(const Ctx& c)
+// The residual and the tangent side by side: until it ends, the launches of their kernels ask for one split of shared memory
+// and L1. Kernels that want different splits share no SM: one waits until the other's blocks on it are done, and with few
+// cells (a wave or less of each kernel) the pass took longer than the two in sequence. In sequence / with the driver's splits /
+// with one split: FP64 Hex8 9^3 72 / 115 / 56 us, 13^3 81 / 107 / 72 us; FP64 gradient-damage plates 40^2 32 / 55 / 22 us,
+// 100^2 66 / 81 / 56 us; FP32 80^2 29 / 46 / 20 us. It costs the row gather its L1: from 24^3 on 1 to 2 % slower (15^3 to 22^3
+// equal), plates of 400^2 3 % faster in FP32. The limits lie in between.
+class SideBySide
 {
-    return c.sysResBlocks <= 0 || (c.dim == 2 && c.prm.kind == NUTO_GPU_GRADIENT_DAMAGE);
-}
+public:
+    explicit SideBySide(Ctx& ctx, bool on = true)
+        : c(ctx)
+    {
+        if (on && c.nCells <= static_cast<int64_t>(c.dim == 3 ? 50 : 500) * std::max(c.smCount, 1))
+            c.carveout = 100;
+    }
+    ~SideBySide()
+    {
+        c.carveout = -1;
+    }
+    SideBySide(const SideBySide&) = delete;
+    SideBySide& operator=(const SideBySide&) = delete;
+
+private:
+    Ctx& c;
+};
 
 // The copy stream of nuto_gpu_build_system_host's chunked values and its events, created on first use.
 static void EnsureCopyStream(Ctx& c, int chunks)
@@ -1158,13 +1177,14 @@ int nuto_gpu_build_system(nuto_gpu_ctx* ctx, const double* u, int precision, voi
         Ctx& c = *ctx;
         // the first call (lazy set-up of geometry, records and tuning), and contexts that ask for it, run the two
         // launches in sequence on the context's stream
-        if (c.systemCalls++ == 0 || SystemInSequence(c))
+        if (c.systemCalls++ == 0 || c.sysResBlocks <= 0)
         {
             LaunchTangent(c, u, precision, values);
             LaunchResidual(c, u, f);
             return NUTO_GPU_OK;
         }
         EnsureSideStream(c);
+        const SideBySide together(c);
         // fork: the residual (persistent grid, launched first so that its blocks hold their SM slots) on the side
         // stream; the tangent on the context's stream; join before anything else runs on the context's stream
         NG_CUDA(cudaEventRecord(c.evFork, c.stream));
@@ -1243,6 +1263,7 @@ int nuto_gpu_build_system_host(nuto_gpu_ctx* ctx, const double* hU, int precisio
             }
             c.stream = main;
         };
+        const SideBySide together(c, !chunked);
         if (!chunked)
             residual(c.sysResBlocks);
         int chunkIdx = 0;

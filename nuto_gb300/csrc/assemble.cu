@@ -735,12 +735,9 @@ void LaunchResidual(Ctx& c, const double* u, double* f, int blocksPerSm)
             constexpr int BIG = DIM == 3 ? 8 : 16, SMALL = BIG / 2;
             const bool small = c.nCells <= static_cast<int64_t>(SMALL) * 4 * std::max(c.smCount, 1);
             constexpr int W = R::warps;
-            if (small)
-                k_residual_sf<DIM, KIND, SMALL>
-                        <<<grid(SMALL * W, 4 * blocksPerSm), 32 * W, 0, c.stream>>>(a, c.law, u, c.dCellVec.p);
-            else
-                k_residual_sf<DIM, KIND, BIG>
-                        <<<grid(BIG * W, 4 * blocksPerSm), 32 * W, 0, c.stream>>>(a, c.law, u, c.dCellVec.p);
+            NG_CUDA(LaunchEx(false, c.carveout, small ? k_residual_sf<DIM, KIND, SMALL> : k_residual_sf<DIM, KIND, BIG>,
+                             dim3(grid((small ? SMALL : BIG) * W, 4 * blocksPerSm)), dim3(32 * W), 0, c.stream, a, c.law, u,
+                             c.dCellVec.p));
         };
         DispatchTwoPoint(c, run);
         AfterLaunch(c, "k_residual_sf");
@@ -774,8 +771,9 @@ void LaunchResidual(Ctx& c, const double* u, double* f, int blocksPerSm)
         g.gdof[s] = S.dGdof.p;
     }
     const int64_t items = g.items[0] + g.items[1];
-    NG_CUDA(LaunchPdl(c.dim == 2 ? k_gather_residual<4> : k_gather_residual<8>, dim3(static_cast<unsigned>((items + 255) / 256)), dim3(256), 0, c.stream, g,
-                      static_cast<const double*>(c.dCellVec.p), f));
+    NG_CUDA(LaunchEx(true, c.carveout, c.dim == 2 ? k_gather_residual<4> : k_gather_residual<8>,
+                     dim3(static_cast<unsigned>((items + 255) / 256)), dim3(256), 0, c.stream, g,
+                     static_cast<const double*>(c.dCellVec.p), f));
     AfterLaunch(c, "k_gather_residual");
     c.stats.kernel_launches += 2;
 }

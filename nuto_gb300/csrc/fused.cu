@@ -722,7 +722,8 @@ bool LaunchTangentFused(Ctx& c, const double* u, float* vals)
                     NG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kern, WW * 32, smem));
                     blocks = std::max<int64_t>(1, std::min<int64_t>(blocks, static_cast<int64_t>(perSm) * c.smCount));
                 }
-                kern<<<static_cast<unsigned>(blocks), WW * 32, smem, c.stream>>>(A, c.law, u, em);
+                NG_CUDA(LaunchEx(false, c.carveout, kern, dim3(static_cast<unsigned>(blocks)), dim3(WW * 32), smem, c.stream, A,
+                                 c.law, u, em));
                 AfterLaunch(c, "k_cell_matrices");
                 c.stats.kernel_launches += 1;
             };

@@ -88,21 +88,35 @@ __device__ __forceinline__ void PdlTrigger()
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 }
 bool PdlEnabled();
+// pdl: programmatic stream serialisation; carveout: preferred share of shared memory in percent (-1: the driver's choice)
 template <typename... KArgs, typename... Args>
-inline cudaError_t LaunchPdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                             Args... args)
+inline cudaError_t LaunchEx(bool pdl, int carveout, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                            cudaStream_t stream, Args... args)
 {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
     cfg.attrs = attr;
-    cfg.numAttrs = PdlEnabled() ? 1 : 0;
+    if (pdl && PdlEnabled())
+    {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (carveout >= 0)
+    {
+        attr[cfg.numAttrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        attr[cfg.numAttrs++].val.sharedMemCarveout = static_cast<unsigned>(carveout);
+    }
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t LaunchPdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                             Args... args)
+{
+    return LaunchEx(true, -1, kernel, grid, block, smem, stream, args...);
 }
 
 struct Ctx;
@@ -448,10 +462,11 @@ struct Ctx
     // 4 sysResBlocks warps per SM (the FP64 pipe needs few warps), the rest of every SM left to the tangent's
     // blocks; the first call of a context runs both in sequence (lazy set-up, autotuning). FP32 64^3 Hex8 system pass:
     // 1502 us in sequence, 1528 / 1344 / 1280 with 2 / 4 / 6; 17^3: 54 us, 38 with all three; 200^2 Quad4 elastic: 35 us,
-    // 32 / 30 / 30. Quad4 gradient damage runs in sequence: 3 / 10 plates 35 / 141 us, beside each other 62 / 144.
+    // 32 / 30 / 30. Batches of 10 / 128 / 512 plates: 135 / 1289 / 5275 us in sequence, 127 / 1149 / 4666 us.
     cudaStream_t sideStream = nullptr;
     cudaEvent_t evFork = nullptr, evJoin = nullptr;
     int sysResBlocks = 6;
+    int carveout = -1; // LaunchEx of the assembly kernels: set while the two run side by side (SideBySide)
     // nuto_gpu_build_system_host: device copies of the caller's host state, values and vector
     DBuf<double> dHostIoU, dHostIoF;
     DBuf<unsigned char> dHostIoVals;

@@ -259,9 +259,11 @@ inline void LaunchRows(Ctx& c, const RowPlanArgs& all, int64_t first, int64_t la
         return;
     const dim3 grid(static_cast<unsigned>((last - first + perBlock - 1) / perBlock));
     if (!GD || P.sameGraph)
-        NG_CUDA(LaunchPdl(k_rows_from_slabs<T, DIM, ND, GD, W, true>, grid, dim3(W * 32), 0, c.stream, P, em, vals));
+        NG_CUDA(LaunchEx(true, c.carveout, k_rows_from_slabs<T, DIM, ND, GD, W, true>, grid, dim3(W * 32), 0, c.stream, P, em,
+                         vals));
     else if constexpr (GD)
-        NG_CUDA(LaunchPdl(k_rows_from_slabs<T, DIM, ND, GD, W, false>, grid, dim3(W * 32), 0, c.stream, P, em, vals));
+        NG_CUDA(LaunchEx(true, c.carveout, k_rows_from_slabs<T, DIM, ND, GD, W, false>, grid, dim3(W * 32), 0, c.stream, P,
+                         em, vals));
     AfterLaunch(c, "k_rows_from_slabs");
     c.stats.kernel_launches += 1;
 }

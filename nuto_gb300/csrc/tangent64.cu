@@ -577,7 +577,8 @@ bool LaunchTangent64(Ctx& c, const double* u, double* vals)
         auto kern = k_cell_matrices64<DIM, GD>;
         if (smem > 48 * 1024)
             NG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-        kern<<<static_cast<unsigned>((c.nCells + C::cpb - 1) / C::cpb), C::threads, smem, c.stream>>>(a, c.law, u, em);
+        NG_CUDA(LaunchEx(false, c.carveout, kern, dim3(static_cast<unsigned>((c.nCells + C::cpb - 1) / C::cpb)),
+                         dim3(C::threads), smem, c.stream, a, c.law, u, em));
         AfterLaunch(c, "k_cell_matrices64");
         c.stats.kernel_launches += 1;
         LaunchRows<double, DIM, C::nd, GD, 4>(c, P, 0, D.nNodes, em, vals);
