@@ -458,6 +458,7 @@ static void BuildPattern(Ctx& c)
     c.rowPlanKey = 0;
     c.cellChunkEnd.clear();
     c.elemMats32.refused = c.elemMats64.refused = 0;
+    c.rowPlanRoom = nullptr;
     c.h20Mode = -1;
     c.tc20Mode = -1;
     c.havePattern = true;
@@ -967,6 +968,7 @@ int nuto_gpu_set_integrand(nuto_gpu_ctx* ctx, const nuto_gpu_integrand* p)
         ctx->rowsMode = -1;
         ctx->fusedMode = -1;
         ctx->elemMats32.refused = ctx->elemMats64.refused = 0;
+        ctx->rowPlanRoom = nullptr;
         ctx->h20Mode = -1;
         ctx->tc20Mode = -1;
         ctx->haveGeo = false;

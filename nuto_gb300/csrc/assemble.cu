@@ -198,19 +198,18 @@ void BuildGeometryCache(Ctx& c)
     const Slot& D = c.slots[c.prm.disp_slot];
     c.geoStride = 1 + D.nen * c.dim;
     const size_t total = static_cast<size_t>(c.geoStride) * c.ip.nIp * c.nCells;
-    c.dGeo64.alloc(total);
-    const bool linear = LinearTwoPoint(c);
-    if (linear)
-        c.dJac.alloc(static_cast<size_t>(1 + c.dim * c.dim) * c.ip.nIp * c.nCells);
-    else
-        c.dJac.free();
+    const size_t inverse = LinearTwoPoint(c) ? static_cast<size_t>(1 + c.dim * c.dim) * c.ip.nIp * c.nCells : 0;
+    c.dGeo64.alloc(total + inverse);
+    c.geoCount = total;
+    c.jac = inverse ? c.dGeo64.p + total : nullptr;
+    c.jacCount = inverse;
     const int64_t items = c.nCells * c.ip.nIp;
     const int blocks = static_cast<int>((items + 127) / 128);
     DispatchCfg(c, [&](auto cfg) {
         using C = decltype(cfg);
         k_geometry<C::dim, C::ng, C::nd, C::nip><<<blocks, 128, 0, c.stream>>>(
                 c.nCells, static_cast<int64_t>(c.dCoords.n), c.dCoords.p, c.dGeoConnT.p, c.dTables.p, c.tabW, c.tabDN[c.geoInterp], c.tabDN[D.interp],
-                c.geoStride, c.dGeo64.p, linear ? c.dJac.p : nullptr, SumFac<C::dim>::gradScale);
+                c.geoStride, c.dGeo64.p, c.jac, SumFac<C::dim>::gradScale);
     });
     AfterLaunch(c, "k_geometry");
     c.dGeo32.free(); // FP32 copy: made by EnsureGeo32 where a kernel reads it
@@ -229,15 +228,15 @@ __global__ void __launch_bounds__(256) k_geometry32(int64_t n, const double* __r
 
 static void EnsureGeo32(Ctx& c)
 {
-    if (c.dGeo32.n == c.dGeo64.n)
+    if (c.dGeo32.n == c.geoCount)
         return;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     NG_CUDA(cudaStreamIsCapturing(c.stream, &cs));
     if (cs != cudaStreamCaptureStatusNone)
         return;
-    c.dGeo32.alloc(c.dGeo64.n);
+    c.dGeo32.alloc(c.geoCount);
     k_geometry32<<<static_cast<unsigned>(std::max(c.smCount, 1) * 8), 256, 0, c.stream>>>(
-            static_cast<int64_t>(c.dGeo64.n), c.dGeo64.p, c.dGeo32.p);
+            static_cast<int64_t>(c.geoCount), c.dGeo64.p, c.dGeo32.p);
     AfterLaunch(c, "k_geometry32");
 }
 
@@ -257,7 +256,7 @@ static CellArgs MakeCellArgs(Ctx& c)
     a.nCells = c.nCells;
     a.nNodesD = D.nNodes;
     a.nDofs = c.nDofs;
-    a.geoSize = static_cast<int64_t>(c.dGeo64.n);
+    a.geoSize = static_cast<int64_t>(c.geoCount);
     a.connD = D.dConnT.p;
     a.gdofD = D.dGdof.p;
     a.tabN_D = c.dTables.p + c.tabN[D.interp];
@@ -271,8 +270,8 @@ static CellArgs MakeCellArgs(Ctx& c)
     }
     a.geo64 = c.dGeo64.p;
     a.geo32 = c.dGeo32.p;
-    a.jac = c.dJac.n ? c.dJac.p : nullptr;
-    a.jacSize = static_cast<int64_t>(c.dJac.n);
+    a.jac = c.jac;
+    a.jacSize = static_cast<int64_t>(c.jacCount);
     a.geoStride = c.geoStride;
     a.kappa = c.dKappa.p;
     a.escale = c.dEScale.n ? c.dEScale.p : nullptr;

@@ -273,12 +273,14 @@ struct Amg;
 
 // Row gather of the element-matrix tangents (rows.cuh), built once per mesh: per displacement node its rows, the offsets
 // of the blocks in them and its cell list; per entry of the cell lists the slab (cell * nodes per cell + local index) and
-// per (entry, b) the ranks of b in the node's four neighbour lists (UU | UE << 8 | EU << 16 | EE << 24).
+// per (entry, b) the ranks of b in the node's displacement and eeq neighbour lists (U | E << 8). The eeq row of a node has the
+// length, block offsets and ranks of its displacement rows: the plan is made only where a displacement node and its eeq node
+// are the same local node of the same cells (RowsSupported), so they have the same neighbours in both fields.
 struct RowPlan
 {
-    int64_t rowU, rowE, first;                   // first values of the rows, first entry of the cell list
-    int32_t lenU, lenE, bUU, bUE, bEU, bEE, cells, pad0;
-    int64_t pad1; // 64 bytes: one record per two sectors
+    int64_t rowU, rowE, first; // first values of the rows, first entry of the cell list
+    int32_t len, bU, bE, cells; // values per row, offsets of the displacement and eeq columns
+    int64_t pad[3]; // 64 bytes: one record per two sectors
 };
 static_assert(sizeof(RowPlan) == 64, "one 64-byte record per node");
 struct RowPlanArgs
@@ -288,7 +290,6 @@ struct RowPlanArgs
     const uint32_t* packed;
     int64_t nodeFirst, nodeLast; // displacement nodes of the launch
     int64_t nEntries, nnz;
-    bool sameGraph; // the eeq row of every node has the positions of its displacement rows
 };
 
 // Element matrices in one arithmetic, scratch of its tangents. One buffer per arithmetic, sized at its first tangent: a captured
@@ -418,11 +419,13 @@ struct Ctx
 
     // geometry caches per integration point: planar [(q * S + k)][cell], S = 1 + nen_d * dim
     bool haveGeo = false;
-    DBuf<double> dGeo64;
+    DBuf<double> dGeo64; // geoCount values, then those of jac
+    size_t geoCount = 0;
     DBuf<float> dGeo32; // on first use of the FP32 element kernel
     // w det J and the inverse Jacobian (times SumFac::gradScale) per point, planar [(q * (1 + dim^2) + k)][cell]
-    // (Quad4 / Hex8 cells with the two-point rule)
-    DBuf<double> dJac;
+    // (Quad4 / Hex8 cells with the two-point rule, else nullptr)
+    double* jac = nullptr;
+    size_t jacCount = 0;
     int geoStride = 0;
 
     // row-gather tangent: integration-point records and the displacement-node -> eeq-node map
@@ -448,10 +451,11 @@ struct Ctx
     // element matrices of the last tangent in each arithmetic, and the plan of the row gather
     ElemMats<float> elemMats32;
     ElemMats<double> elemMats64;
-    DBuf<unsigned char> dRowPlan; // RowPlan per node, then slab numbers and packed ranks:
+    DBuf<unsigned char> dRowPlan; // where the element matrices were there before the plan
+    unsigned char* rowPlanRoom = nullptr; // room for the plan behind element matrices allocated without one
+    RowPlan* rowPlan = nullptr;
     uint32_t *rowSlab = nullptr, *packedRanks = nullptr;
     int rowPlanKey = 0; // slots the plan was built for (0: not built)
-    bool rowPlanSame = false;
     // device status word of kernels with bounded waits (0 = fine, else NUTO_GPU_ETIMEOUT), read after a stream
     // synchronisation; spinLimit bounds every wait loop (iterations)
     DBuf<int> dStatus;

@@ -8,8 +8,8 @@
 //
 // Bound by the latency of the chain node -> cells -> slab. It is kept to three dependent loads: the node's plan (rows,
 // block offsets, cell list: one 64-byte record), the slab numbers and packed ranks of a batch of 4 cells, their slabs.
-// The rows are kept interleaved where the eeq row has the positions of the displacement rows (every mesh whose DOF types share
-// one node graph): one vector access per column instead of one per row. FP32 Hex8 gradient damage at 48^3: 160 us with row
+// The rows are kept interleaved (the eeq row has the positions of the displacement rows): one vector access per column instead
+// of one per row. FP32 Hex8 gradient damage at 48^3: 160 us with row
 // pointers, cell indices and block offsets read one after the other, 139 us with the plan, 118 us interleaved (DRAM floor
 // 95 us; 81 % of the shared-memory wavefronts). Quad4 gradient damage (16 lanes per node) 70 -> 30 us for 71 k nodes.
 #pragma once
@@ -39,9 +39,8 @@ struct alignas(NR == 2 ? 2 * sizeof(T) : 16) RowVec
     T v[n];
 };
 
-// SAME: the eeq row has the same positions as the displacement rows (one node graph for both DOF types, and elastic cells
-// with their one): the rows are kept interleaved and updated with one vector access per column
-template <typename T, int DIM, int ND, bool GD, int W, bool SAME>
+// The rows of a node have the same positions and are kept interleaved: one vector access per column updates all of them
+template <typename T, int DIM, int ND, bool GD, int W>
 __global__ void __launch_bounds__(W * 32) k_rows_from_slabs(RowPlanArgs P, const T* __restrict__ em, T* __restrict__ vals)
 {
     using S = Slab<DIM, ND, GD>;
@@ -53,18 +52,11 @@ __global__ void __launch_bounds__(W * 32) k_rows_from_slabs(RowPlanArgs P, const
     PdlWait();
     const int64_t a = P.nodeFirst + (static_cast<int64_t>(blockIdx.x) * W + wid) * NPW + grp;
     V* sVec = sRowAll[wid * NPW + grp];
-    T* sRow = reinterpret_cast<T*>(sVec); // SAME = false: [row][kRowsCap]
     RowPlan p{};
     if (a < P.nodeLast)
         p = P.plan[a]; // p.cells = 0 beyond the last node: nothing to add or store
-    if constexpr (SAME)
-    {
-        for (int i = col; i < p.lenU; i += LPN)
-            sVec[i] = V{};
-    }
-    else
-        for (int i = col; i < NR * kRowsCap; i += LPN)
-            sRow[i] = T(0);
+    for (int i = col; i < p.len; i += LPN)
+        sVec[i] = V{};
     const bool ucol = col < ND * DIM;
     const int myB = col < NC ? (ucol ? col / DIM : col - ND * DIM) : 0;
     const int myL = ucol ? col % DIM : 0;
@@ -101,53 +93,25 @@ __global__ void __launch_bounds__(W * 32) k_rows_from_slabs(RowPlanArgs P, const
         {
             if (kb + c < p.cells && col < NC)
             {
-                const int r0 = word[c] & 0xff, r1 = (word[c] >> 8) & 0xff, r2 = (word[c] >> 16) & 0xff, r3 = word[c] >> 24;
-                const int posU = ucol ? p.bUU + DIM * r0 + myL : p.bUE + r1;
-                if constexpr (SAME)
-                {
-                    V& row = sVec[NG_IDX(posU, kRowsCap, 79)];
-                    V x = row;
+                const int rank = ucol ? word[c] & 0xff : word[c] >> 8;
+                V& row = sVec[NG_IDX(ucol ? p.bU + DIM * rank + myL : p.bE + rank, kRowsCap, 79)];
+                V x = row;
 #pragma unroll
-                    for (int k = 0; k < NR; ++k)
-                        x.v[k] += v[c][k];
-                    row = x;
-                }
-                else
-                {
-#pragma unroll
-                    for (int k = 0; k < DIM; ++k)
-                        sRow[k * kRowsCap + NG_IDX(posU, kRowsCap, 79)] += v[c][k];
-                    if (GD)
-                    {
-                        const int posE = ucol ? p.bEU + DIM * r2 + myL : p.bEE + r3;
-                        sRow[DIM * kRowsCap + NG_IDX(posE, kRowsCap, 79)] += v[c][DIM];
-                    }
-                }
+                for (int k = 0; k < NR; ++k)
+                    x.v[k] += v[c][k];
+                row = x;
             }
             __syncwarp();
         }
     }
-    if constexpr (SAME)
+    for (int i = col; i < p.len; i += LPN)
     {
-        for (int i = col; i < p.lenU; i += LPN)
-        {
-            const V x = sVec[i];
-#pragma unroll
-            for (int k = 0; k < DIM; ++k)
-                vals[NG_IDX(p.rowU + static_cast<int64_t>(k) * p.lenU + i, P.nnz, 75)] = x.v[k];
-            if (GD)
-                vals[NG_IDX(p.rowE + i, P.nnz, 75)] = x.v[DIM];
-        }
-    }
-    else
-    {
+        const V x = sVec[i];
 #pragma unroll
         for (int k = 0; k < DIM; ++k)
-            for (int i = col; i < p.lenU; i += LPN)
-                vals[NG_IDX(p.rowU + static_cast<int64_t>(k) * p.lenU + i, P.nnz, 75)] = sRow[k * kRowsCap + i];
+            vals[NG_IDX(p.rowU + static_cast<int64_t>(k) * p.len + i, P.nnz, 75)] = x.v[k];
         if (GD)
-            for (int i = col; i < p.lenE; i += LPN)
-                vals[NG_IDX(p.rowE + i, P.nnz, 75)] = sRow[DIM * kRowsCap + i];
+            vals[NG_IDX(p.rowE + i, P.nnz, 75)] = x.v[DIM];
     }
 }
 
@@ -171,7 +135,7 @@ __global__ void __launch_bounds__(W * 32) k_rows_from_wide_slabs(RowPlanArgs P, 
     if (a >= P.nodeLast)
         return; // the whole warp leaves; only warp-level synchronisation follows
     const RowPlan p = P.plan[a];
-    for (int i = lane; i < p.lenU; i += 32)
+    for (int i = lane; i < p.len; i += 32)
         row[i] = V{};
     const bool second = lane + 32 < NC;
     const int b0 = lane / 3, l0 = lane % 3, b1 = second ? (lane + 32) / 3 : 0, l1 = (lane + 32) % 3;
@@ -204,7 +168,7 @@ __global__ void __launch_bounds__(W * 32) k_rows_from_wide_slabs(RowPlanArgs P, 
         {
             if (kb + c < p.cells)
             {
-                V& x0 = row[NG_IDX(p.bUU + 3 * static_cast<int>(w0[c] & 0xff) + l0, kRowsCapWide, 79)];
+                V& x0 = row[NG_IDX(p.bU + 3 * static_cast<int>(w0[c] & 0xff) + l0, kRowsCapWide, 79)];
                 V t = x0;
 #pragma unroll
                 for (int r = 0; r < 3; ++r)
@@ -212,7 +176,7 @@ __global__ void __launch_bounds__(W * 32) k_rows_from_wide_slabs(RowPlanArgs P, 
                 x0 = t;
                 if (second)
                 {
-                    V& x1 = row[NG_IDX(p.bUU + 3 * static_cast<int>(w1[c] & 0xff) + l1, kRowsCapWide, 79)];
+                    V& x1 = row[NG_IDX(p.bU + 3 * static_cast<int>(w1[c] & 0xff) + l1, kRowsCapWide, 79)];
                     V s = x1;
 #pragma unroll
                     for (int r = 0; r < 3; ++r)
@@ -223,12 +187,12 @@ __global__ void __launch_bounds__(W * 32) k_rows_from_wide_slabs(RowPlanArgs P, 
             __syncwarp();
         }
     }
-    for (int i = lane; i < p.lenU; i += 32)
+    for (int i = lane; i < p.len; i += 32)
     {
         const V x = row[i];
 #pragma unroll
         for (int k = 0; k < 3; ++k)
-            vals[NG_IDX(p.rowU + static_cast<int64_t>(k) * p.lenU + i, P.nnz, 75)] = x.v[k];
+            vals[NG_IDX(p.rowU + static_cast<int64_t>(k) * p.len + i, P.nnz, 75)] = x.v[k];
     }
 }
 
@@ -258,12 +222,7 @@ inline void LaunchRows(Ctx& c, const RowPlanArgs& all, int64_t first, int64_t la
     if (last <= first)
         return;
     const dim3 grid(static_cast<unsigned>((last - first + perBlock - 1) / perBlock));
-    if (!GD || P.sameGraph)
-        NG_CUDA(LaunchEx(true, c.carveout, k_rows_from_slabs<T, DIM, ND, GD, W, true>, grid, dim3(W * 32), 0, c.stream, P, em,
-                         vals));
-    else if constexpr (GD)
-        NG_CUDA(LaunchEx(true, c.carveout, k_rows_from_slabs<T, DIM, ND, GD, W, false>, grid, dim3(W * 32), 0, c.stream, P,
-                         em, vals));
+    NG_CUDA(LaunchEx(true, c.carveout, k_rows_from_slabs<T, DIM, ND, GD, W>, grid, dim3(W * 32), 0, c.stream, P, em, vals));
     AfterLaunch(c, "k_rows_from_slabs");
     c.stats.kernel_launches += 1;
 }

@@ -598,8 +598,7 @@ namespace
 
 struct PlanArgs
 {
-    int64_t nNodes, nCells;
-    int dim;
+    int64_t nNodes, nCells, nEntries;
     const int64_t* gdofD;
     const int64_t* gdofE; // nullptr: no eeq rows
     const int32_t* eOf;
@@ -607,44 +606,33 @@ struct PlanArgs
     const int32_t* cellIdx;
     const uint8_t* cellLoc;
     const int64_t* rowPtr;
-    const uint8_t* rank[4]; // UU, UE, EU, EE
-    const int32_t* blk[4];
+    const uint8_t *rankU, *rankE;
+    const int32_t *blkU, *blkE;
 };
 
-// *differ becomes 1 where the eeq row of a node has other positions than its displacement rows
-__global__ void __launch_bounds__(256) k_row_plan(PlanArgs A, RowPlan* __restrict__ plan, int* __restrict__ differ)
-{
-    const int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (a >= A.nNodes)
-        return;
-    RowPlan p{};
-    const int64_t g = A.gdofD[a];
-    p.rowU = A.rowPtr[g];
-    p.lenU = static_cast<int32_t>(A.rowPtr[g + 1] - p.rowU); // the rows of a node's components have one length
-    p.first = A.cellPtr[a];
-    p.cells = static_cast<int32_t>(A.cellPtr[a + 1] - p.first);
-    p.bUU = A.blk[0][a];
-    if (A.gdofE)
-    {
-        const int32_t ae = A.eOf[a];
-        const int64_t ge = A.gdofE[ae];
-        p.rowE = A.rowPtr[ge];
-        p.lenE = static_cast<int32_t>(A.rowPtr[ge + 1] - p.rowE);
-        p.bUE = A.blk[1][a];
-        p.bEU = A.blk[2][ae];
-        p.bEE = A.blk[3][ae];
-        if (p.lenE != p.lenU || p.bEU != p.bUU || p.bEE != p.bUE)
-            *differ = 1;
-    }
-    plan[a] = p;
-}
-
+// thread it: the record of displacement node it, and slab and ranks of (entry, b) = (it / ND, it % ND) of the cell lists
 template <int ND>
-__global__ void __launch_bounds__(256) k_row_entries(PlanArgs A, int64_t nEntries, uint32_t* __restrict__ slab,
-                                                     uint32_t* __restrict__ packed, int* __restrict__ differ)
+__global__ void __launch_bounds__(256) k_row_plan(PlanArgs A, RowPlan* __restrict__ plan, uint32_t* __restrict__ slab,
+                                                  uint32_t* __restrict__ packed)
 {
     const int64_t it = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (it >= nEntries * ND)
+    if (it < A.nNodes)
+    {
+        RowPlan p{};
+        const int64_t g = A.gdofD[it];
+        p.rowU = A.rowPtr[g];
+        p.len = static_cast<int32_t>(A.rowPtr[g + 1] - p.rowU); // the rows of a node's components have one length
+        p.first = A.cellPtr[it];
+        p.cells = static_cast<int32_t>(A.cellPtr[it + 1] - p.first);
+        p.bU = A.blkU[it];
+        if (A.gdofE)
+        {
+            p.rowE = A.rowPtr[A.gdofE[A.eOf[it]]];
+            p.bE = A.blkE[it];
+        }
+        plan[it] = p;
+    }
+    if (it >= A.nEntries * ND)
         return;
     const int64_t kc = it / ND;
     const int b = static_cast<int>(it % ND);
@@ -653,10 +641,7 @@ __global__ void __launch_bounds__(256) k_row_entries(PlanArgs A, int64_t nEntrie
     if (b == 0)
         slab[kc] = static_cast<uint32_t>(e * ND + ia);
     const int64_t ridx = static_cast<int64_t>(ia * ND + b) * A.nCells + e;
-    const uint32_t r0 = A.rank[0][ridx], r1 = A.rank[1][ridx], r2 = A.rank[2][ridx], r3 = A.rank[3][ridx];
-    if (r0 != r2 || r1 != r3)
-        *differ = 1;
-    packed[it] = r0 | r1 << 8 | r2 << 16 | r3 << 24;
+    packed[it] = A.rankU[ridx] | static_cast<uint32_t>(A.rankE[ridx]) << 8;
 }
 
 } // namespace
@@ -672,29 +657,35 @@ bool RowPlanReady(const Ctx& c)
     return c.rowPlanKey == RowPlanKey(c);
 }
 
+// nodes' records, slab numbers, packed ranks
+static size_t RowPlanBytes(const Ctx& c)
+{
+    const Slot& D = c.slots[c.prm.disp_slot];
+    return static_cast<size_t>(D.nNodes) * sizeof(RowPlan) + static_cast<size_t>(c.nCells) * D.nen * (1 + D.nen) * sizeof(uint32_t);
+}
+
 RowPlanArgs EnsureRowPlan(Ctx& c)
 {
-    const int ns = static_cast<int>(c.slots.size());
-    const int dS = c.prm.disp_slot;
-    const bool gd = c.prm.kind == NUTO_GPU_GRADIENT_DAMAGE;
-    const int eS = gd ? c.prm.eeq_slot : dS;
-    const Slot& D = c.slots[dS];
+    const Slot& D = c.slots[c.prm.disp_slot];
     const int64_t entries = c.nCells * D.nen;
     if (!RowPlanReady(c))
     {
         c.cellChunkEnd.clear();
-        // one allocation: the nodes' records, slab numbers, packed ranks, and the flag that the kernels below may raise
-        const size_t plans = static_cast<size_t>(D.nNodes) * sizeof(RowPlan);
-        const size_t numbers = static_cast<size_t>(entries) * (1 + D.nen) + 1;
-        c.dRowPlan.alloc(plans + numbers * sizeof(uint32_t));
-        c.rowSlab = reinterpret_cast<uint32_t*>(c.dRowPlan.p + plans);
+        if (!c.rowPlanRoom)
+        {
+            c.dRowPlan.alloc(RowPlanBytes(c));
+            c.rowPlanRoom = c.dRowPlan.p;
+        }
+        c.rowPlan = reinterpret_cast<RowPlan*>(c.rowPlanRoom);
+        c.rowPlanRoom = nullptr;
+        c.rowSlab = reinterpret_cast<uint32_t*>(c.rowPlan + D.nNodes);
         c.packedRanks = c.rowSlab + entries;
-        RowPlan* plan = reinterpret_cast<RowPlan*>(c.dRowPlan.p);
-        int* differ = reinterpret_cast<int*>(c.packedRanks + entries * D.nen);
+        const bool gd = c.prm.kind == NUTO_GPU_GRADIENT_DAMAGE;
+        const int ns = static_cast<int>(c.slots.size()), dS = c.prm.disp_slot, eS = gd ? c.prm.eeq_slot : dS;
         PlanArgs A{};
         A.nNodes = D.nNodes;
         A.nCells = c.nCells;
-        A.dim = c.dim;
+        A.nEntries = entries;
         A.gdofD = D.dGdof.p;
         A.gdofE = gd ? c.slots[eS].dGdof.p : nullptr;
         A.eOf = gd ? c.dEOf.p : nullptr;
@@ -702,39 +693,22 @@ RowPlanArgs EnsureRowPlan(Ctx& c)
         A.cellIdx = D.dCellIdx.p;
         A.cellLoc = D.dCellLoc.p;
         A.rowPtr = c.dRowPtr.p;
-        const int pr[4] = {dS * ns + dS, dS * ns + eS, eS * ns + dS, eS * ns + eS};
-        for (int k = 0; k < 4; ++k)
-        {
-            A.rank[k] = c.pairs[pr[k]].rank;
-            A.blk[k] = c.pairs[pr[k]].dBlk.p;
-        }
-        NG_CUDA(cudaMemsetAsync(differ, 0, sizeof(int), c.stream));
-        k_row_plan<<<static_cast<unsigned>((D.nNodes + 255) / 256), 256, 0, c.stream>>>(A, plan, differ);
+        A.rankU = c.pairs[dS * ns + dS].rank;
+        A.rankE = c.pairs[dS * ns + eS].rank;
+        A.blkU = c.pairs[dS * ns + dS].dBlk.p;
+        A.blkE = c.pairs[dS * ns + eS].dBlk.p;
+        const int64_t items = std::max(D.nNodes, entries * D.nen);
+        auto kern = D.nen == 4 ? k_row_plan<4> : (D.nen == 20 ? k_row_plan<20> : k_row_plan<8>);
+        kern<<<static_cast<unsigned>((items + 255) / 256), 256, 0, c.stream>>>(A, c.rowPlan, c.rowSlab, c.packedRanks);
         AfterLaunch(c, "k_row_plan");
-        const unsigned blocks = static_cast<unsigned>((entries * D.nen + 255) / 256);
-        if (D.nen == 4)
-            k_row_entries<4><<<blocks, 256, 0, c.stream>>>(A, entries, c.rowSlab, c.packedRanks, differ);
-        else if (D.nen == 20)
-            k_row_entries<20><<<blocks, 256, 0, c.stream>>>(A, entries, c.rowSlab, c.packedRanks, differ);
-        else
-            k_row_entries<8><<<blocks, 256, 0, c.stream>>>(A, entries, c.rowSlab, c.packedRanks, differ);
-        AfterLaunch(c, "k_row_entries");
-        int h = 0; // without eeq rows there is nothing that could differ
-        if (gd)
-        {
-            NG_CUDA(cudaMemcpyAsync(&h, differ, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-            NG_CUDA(cudaStreamSynchronize(c.stream));
-        }
-        c.rowPlanSame = h == 0;
         c.rowPlanKey = RowPlanKey(c);
     }
     RowPlanArgs P{};
-    P.plan = reinterpret_cast<const RowPlan*>(c.dRowPlan.p);
+    P.plan = c.rowPlan;
     P.slab = c.rowSlab;
     P.packed = c.packedRanks;
     P.nEntries = entries;
     P.nnz = c.nnz;
-    P.sameGraph = c.rowPlanSame;
     return P;
 }
 
@@ -754,7 +728,10 @@ T* ElemMatsOrNull(Ctx& c, size_t count)
     NG_CUDA(cudaStreamIsCapturing(c.stream, &cs));
     if (cs != cudaStreamCaptureStatusNone)
         return nullptr;
-    const size_t bytes = count * sizeof(T);
+    // One allocation (20 to 80 us each) with the plan where that is still to be made; the plan keeps its place as long as the
+    // buffer: only a change of the pattern or of the integrand's slots, after which it is made anew, lets the buffer grow.
+    const size_t plan = RowPlanReady(c) ? 0 : RowPlanBytes(c), matrices = (count * sizeof(T) + 255) / 256 * 256;
+    const size_t bytes = matrices + plan;
     bool room = true;
     // The element kernel needs no scratch, so a large FP64 problem may have just the memory for its solver. Asking for the free
     // memory costs as much as a small assembly: below this size (1 GB of tangent at most) the attempt alone decides.
@@ -775,6 +752,7 @@ T* ElemMatsOrNull(Ctx& c, size_t count)
     E->buf.free();
     E->buf.p = p;
     E->buf.n = count;
+    c.rowPlanRoom = plan ? reinterpret_cast<unsigned char*>(p) + matrices : nullptr;
     return p;
 }
 template float* ElemMatsOrNull<float>(Ctx&, size_t);

@@ -768,7 +768,7 @@ bool LaunchTangentTc20(Ctx& c, const double* u, float* vals)
     A.nCells = n;
     A.nDofs = c.nDofs;
     A.nNodesD = D.nNodes;
-    A.geoSize = static_cast<int64_t>(c.dGeo64.n);
+    A.geoSize = static_cast<int64_t>(c.geoCount);
     A.connD = D.dConnT.p;
     A.gdofD = D.dGdof.p;
     A.relX = c.dRelX.p;

@@ -1,0 +1,124 @@
+"""The plan of the row gather: eeq nodes in another order than the displacement nodes, and one context whose integrand, pattern
+and arithmetic change from call to call."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+LAW = dict(E=30000.0, nu=0.2, kappa0=1e-4, beta=100.0, alpha=0.99, k=10.0, c=0.01)
+
+
+def _mesh(dim, order=None):
+    """(mesh, layers) with displacement and eeq nodes; order: the eeq layer's new number of each node"""
+    from nuto_gb300 import mesh as M
+
+    m = M.create_quads(6, 5) if dim == 2 else M.create_bricks(3, 4, 3)
+    layers = [M.add_dof_interpolation(m, dim), M.add_dof_interpolation(m, 1)]
+    if order is not None:
+        e = m.layers[layers[1]]
+        coords = np.empty_like(e.node_coords)
+        coords[order] = e.node_coords
+        m.layers[layers[1]] = M.DofLayer(1, e.interp, order[e.conn], coords)
+    return m, layers
+
+
+def _set(g, dim, kind, kappa):
+    g.set_integrand(kind=kind, dim=dim, disp_slot=0, eeq_slot=1 if kind == 2 else -1, **LAW)
+    if kind == 2:
+        g.history = kappa
+
+
+def _state(m, dim, rng):
+    n = m.layers[0].num_nodes
+    u = np.concatenate([rng.uniform(-2e-4, 2e-4, n * dim), rng.uniform(0.0, 4e-4, n)])
+    return u, rng.uniform(0.0, 4e-4, (m.num_cells, 2 ** dim))
+
+
+def _cuda():
+    import torch
+
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    return torch
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("precision", [32, 64])
+def test_eeq_nodes_in_another_order(dim, precision):
+    """The eeq row of a node has the neighbours of its displacement rows whatever the eeq numbering: every entry is the plain
+    mesh's, at the permuted place. FP64: to the rounding of a sum over the cells in another order; FP32 the same in its units."""
+    import scipy.sparse as sp
+    from nuto_gb300.assembly import GpuCellGroup
+
+    _cuda()
+    rng = np.random.default_rng(11)
+    n = _mesh(dim)[0].layers[0].num_nodes
+    order = rng.permutation(n)
+    K = []
+    for perm in (None, order):
+        m, layers = _mesh(dim, perm)
+        u, kappa = _state(m, dim, np.random.default_rng(13))
+        p = np.arange(n * (dim + 1))
+        if perm is not None:
+            p[n * dim:] = n * dim + perm
+            u[p] = u.copy()
+        g = GpuCellGroup(m, layers, 2)
+        g.build_pattern()
+        _set(g, dim, 2, kappa)
+        v = g.build_matrix(u, precision).double().cpu().numpy()
+        rp, ci = g.pattern()
+        K.append(sp.csr_matrix((v, ci, rp), shape=(len(u), len(u)))[p][:, p].toarray())
+    assert np.abs(K[0] - K[1]).max() <= (1e-6 if precision == 32 else 1e-14) * np.abs(K[0]).max()
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("steps", ["2f 2d 0d 0f 2f 2d", "0d 2d 2f 0f p2f 0d p2d", "2d p2d 0f 2f", "0f 2d p0d 2f"])
+def test_one_context_through_changes(dim, steps):
+    """Steps: p = pattern built again, 0 / 2 = elastic / gradient damage set, f / d = FP32 / FP64 tangent; after each the values
+    of a fresh context bit for bit."""
+    from nuto_gb300.assembly import GpuCellGroup
+
+    torch = _cuda()
+    m, layers = _mesh(dim)
+    u, kappa = _state(m, dim, np.random.default_rng(17))
+    g = GpuCellGroup(m, layers, 2)
+    g.build_pattern()
+    for step in steps.split():
+        if step[0] == "p":
+            g.build_pattern()
+        kind, precision = int(step[-2]), 32 if step[-1] == "f" else 64
+        _set(g, dim, kind, kappa)
+        fresh = GpuCellGroup(m, layers, 2)
+        fresh.build_pattern()
+        _set(fresh, dim, kind, kappa)
+        assert torch.equal(g.build_matrix(u, precision), fresh.build_matrix(u, precision)), step
+
+
+def test_first_fp64_tangent_of_a_context(monkeypatch):
+    """What the first FP64 tangent of a 200 x 200 mesh lays out (plan and element matrices, one allocation, no synchronisation)
+    costs about what its kernels save against the element kernel, which lays out nothing: at most 1.3 times that one's first
+    call (medians over 8 contexts; two allocations and a wait for the plan made it 1.5 times)."""
+    import time
+
+    torch = _cuda()
+    from nuto_gb300 import configs
+
+    s = configs.quad4_elastic(200)
+    u = torch.zeros(s.n_dofs, dtype=torch.float64, device="cuda")
+    first = {}
+    for form in ("", "atomic"):
+        monkeypatch.setenv("NUTO_GPU_TANGENT", form)
+        times = []
+        for _ in range(10):
+            g = s.build_gpu()
+            v = torch.empty(g.nnz, dtype=torch.float64, device="cuda")
+            g.build_vector(u)
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            g.build_matrix(u, 64, out=v)
+            torch.cuda.synchronize()
+            times.append(time.perf_counter() - t)
+            g.close()
+        first[form] = np.median(times[2:])
+    assert first[""] <= 1.3 * first["atomic"], first
