@@ -1475,8 +1475,7 @@ static RowArgs MakeRowArgs(Ctx& c)
     return r;
 }
 
-template <typename T>
-static void LaunchTangentRows(Ctx& c, const double* u, T* vals)
+static void LaunchTangentRows(Ctx& c, const double* u, float* vals)
 {
     CellArgs a = MakeCellArgs(c);
     ScatterArgs s = MakeScatterArgs(c);
@@ -1484,20 +1483,20 @@ static void LaunchTangentRows(Ctx& c, const double* u, T* vals)
     DispatchCfg(c, [&](auto cfg) {
         using C = decltype(cfg);
         using R = IpRecord<C::dim, C::nd, C::kind>;
-        using Sh = RowShape<T, C::dim, C::nd, C::nip, C::kind>;
-        const size_t recBytes = static_cast<size_t>(c.nCells) * C::nip * R::size * sizeof(T);
+        using Sh = RowShape<float, C::dim, C::nd, C::nip, C::kind>;
+        const size_t recBytes = static_cast<size_t>(c.nCells) * C::nip * R::size * sizeof(float);
         if (c.dRecords.n < recBytes)
             c.dRecords.alloc(recBytes);
-        T* recs = reinterpret_cast<T*>(c.dRecords.p);
+        float* recs = reinterpret_cast<float*>(c.dRecords.p);
         constexpr int CPB = TangentShape<C::nd, C::nip>::cpb;
         const int blocks = static_cast<int>((c.nCells + CPB - 1) / CPB);
         // the law is evaluated in FP64 and rounded into FP32 records: the loading/unloading and damage-threshold
-        // branches then agree with the FP64 residual's (an FP32 eeq or strain near kappa_h or kappa0 can take the
+        // branches then agree with the history update's (an FP32 eeq or strain near kappa_h or kappa0 can take the
         // other branch and change the coupling blocks of the tangent by far more than a rounding error)
-        k_tangent<double, C::dim, C::nd, C::nip, C::kind, true, T><<<blocks, TangentShape<C::nd, C::nip>::threads, 0,
+        k_tangent<double, C::dim, C::nd, C::nip, C::kind, true, float><<<blocks, TangentShape<C::nd, C::nip>::threads, 0,
                                                                      c.stream>>>(a, c.law, s, 0, 0, 0, 0, u, recs);
         AfterLaunch(c, "k_tangent (records)");
-        auto kern = k_tangent_rows<T, C::dim, C::nd, C::nip, C::kind>;
+        auto kern = k_tangent_rows<float, C::dim, C::nd, C::nip, C::kind>;
         if (Sh::smem > 48 * 1024)
             NG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(Sh::smem)));
@@ -1529,17 +1528,17 @@ static void LaunchTangentT(Ctx& c, const double* u, T* vals)
 {
     // FP32: row gather (no atomics). FP64: element matrices + row gather for linear cells, else the element kernel with
     // atomics.
-    if (sizeof(T) == 4 && RowsSupported(c) && !c.forceAtomicTangent)
-    {
-        // linear cells: element matrices + row gather; Hex20: the same with the element matrices from the tensor cores;
-        // otherwise, and without memory for them, FP64-law records + row gather
-        float* v = reinterpret_cast<float*>(vals);
-        if (c.forceRecordTangent || !((FusedTangentSupported(c) && LaunchTangentFused(c, u, v)) ||
-                                      (Tc20TangentSupported(c) && LaunchTangentTc20(c, u, v))))
-            LaunchTangentRows<T>(c, u, vals);
-        PrepareNoAlloc(c);
-        return;
-    }
+    if constexpr (sizeof(T) == 4)
+        if (RowsSupported(c) && !c.forceAtomicTangent)
+        {
+            // linear cells: element matrices + row gather; Hex20: the same with the element matrices from the tensor cores;
+            // otherwise, and without memory for them, FP64-law records + row gather
+            if (c.forceRecordTangent || !((FusedTangentSupported(c) && LaunchTangentFused(c, u, vals)) ||
+                                          (Tc20TangentSupported(c) && LaunchTangentTc20(c, u, vals))))
+                LaunchTangentRows(c, u, vals);
+            PrepareNoAlloc(c);
+            return;
+        }
     // FP64, linear cells with a constant ratio of the Lame parameters: element matrices + row gather (64^3 gradient
     // damage: 4.66 ms against 14.46 ms of the element kernel)
     if constexpr (sizeof(T) == 8)

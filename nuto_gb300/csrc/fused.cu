@@ -15,10 +15,11 @@
 //   kernels with one lane per node pair (each ordered pair with its own lambda and mu sums), 622 us now; 17^3 31 -> 19 us;
 //   200^2 Quad4 elastic 31 -> 15 us. Storing rows with 32-byte stores straight from the lanes: 687 us.
 //
-// Branch decisions of the law are the FP64 kernels' (residual, FP64 tangent): the nonlocal equivalent strain at a point is
-// formed in FP32 with an error bound, and where the bound does not separate it from the history kappa or from kappa0 it is
-// recomputed in FP64 exactly as the FP64 kernels form it. The loading/unloading and damage-threshold branches therefore
-// agree with the FP64 residual at every point; everything else is FP32.
+// Branch decisions of the law are those of the history update and the FP64 tangent: the nonlocal equivalent strain at a point
+// is formed in FP32 with an error bound, and where the bound does not separate it from the history kappa or from kappa0 it is
+// recomputed in FP64 in the order of k_history, so a converged loading point, whose kappa is that very value, is loading here.
+// (The residual forms it sum-factorised, with other last bits; it takes the larger of the two values, which has no branch.)
+// Everything else is FP32.
 #include "rows.cuh"
 #include "sumfac.cuh"
 
@@ -113,8 +114,8 @@ __device__ __forceinline__ F2 Add2(F2 a, F2 b)
 // Geometry, strain and law at integration point q of cell e from the cell's node data: X (coordinates relative to
 // the first node, eeq value in .w), U (displacements), E64 (eeq values in FP64, for the branch decisions); T the
 // (dN/dxi, N) table row of q and w its weight. Writes the point's record (CellShape). The loading/unloading and damage
-// branches are the FP64 kernels' (decided in FP32 where the error bound of eeq separates the operands, else in FP64 as the
-// FP64 tangent forms eeq: same order, FP64 shape values tabN).
+// branches are the FP64 tangent's (decided in FP32 where the error bound of eeq separates the operands, else in FP64 as that
+// tangent forms eeq: same order, FP64 shape values tabN).
 template <int DIM, int KIND>
 __device__ __forceinline__ void PointRecord(const FusedArgs& A, const LawParams& L, const float4* T, float w,
                                             const float4* X, const float4* U, const double* E64, int q, int64_t e,

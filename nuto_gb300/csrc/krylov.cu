@@ -973,10 +973,9 @@ __global__ void __launch_bounds__(kBS) k_gm_update_proj(int64_t n, const T* __re
     ProjFlush(sums, nv, acc2);
 }
 
-// w -= sum_i h_i V_i with h the second projection (gs + H2), |w|^2; the last block completes Arnoldi column j:
-// H(:, j) = h1 + h2, H(j+1, j) = |w|, earlier rotations applied, new rotation formed, residual estimate |g(j+1)|
-// tested. Row sums of |w|^2 are formed in T per thread and block, one FP64 atomic per block. zsrc (the sweep's output) is
-// kept as the preconditioned basis vector zdst.
+// w -= sum_i h_i V_i with h the second projection (gs + H2), and |w|^2, from which k_gm_normalize completes Arnoldi column j.
+// Row sums of |w|^2 are formed in T per thread and block, one FP64 atomic per block. zsrc (the sweep's output) is kept as the
+// preconditioned basis vector zdst.
 template <typename T>
 __global__ void __launch_bounds__(kBS) k_gm_update(int64_t n, const T* __restrict__ V, int nv, double* gs, T* w,
                                                     const T* __restrict__ zsrc, T* __restrict__ zdst, const int* st)
@@ -1264,7 +1263,7 @@ static int GmresSolve(Ctx& c, const TV* vals, const double* b, double* x64, bool
         const int cols = std::min(m, maxit - total);
         // The cycle is enqueued in chunks: after each chunk the host reads the state and the residual estimate and
         // sizes the next chunk from the observed convergence rate (the iterations still needed, 1 .. 16). Kernels
-        // of iterations enqueued after convergence return at once but still cost a launch each (about 140 per
+        // of iterations enqueued after convergence return at once but still cost a launch each (about 36 per
         // iteration with the multigrid sweep), so a cycle is never enqueued far past the expected convergence.
         int j = 0, chunk = kGmresFirstChunk, jCheck = 0;
         double resCheck = -1.;

@@ -9,7 +9,7 @@
 //                   node, strain, law, and a record of 6 float4: J^-1, lambda w, mu w, the Voigt vectors
 //                   s = dsigma/domega domega/dkappa w and t = deps_eq/deps (loading points only). The loading and
 //                   damage branches are the FP64 kernels' (decided in FP32 where an error bound separates the
-//                   operands, else from the FP64 strain formed exactly as k_residual forms it).
+//                   operands, else from the FP64 strain formed as k_residual and k_history form it).
 //   k_tangent_tc20  one block per SM walks the cells. Per cell it forms in shared memory the TF32 operands
 //                       A = [ lambda_q w_q g_qa,i | P_q(a,i) ]    rows (i, a)        q = 0..26 | 32 + q
 //                           [ mu_q w_q g_qa,i     | 0        ]    rows 64 + (i, a)
