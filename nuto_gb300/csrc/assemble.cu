@@ -1568,6 +1568,7 @@ static void LaunchTangentT(Ctx& c, const double* u, T* vals)
 void LaunchTangent(Ctx& c, const double* u, int precision, void* values)
 {
     c.valsVersion++;
+    c.solveFollows = precision != NUTO_GPU_FP64X;
     if (precision == NUTO_GPU_FP32)
         LaunchTangentT<float>(c, u, static_cast<float*>(values));
     else

@@ -449,6 +449,7 @@ struct Ctx
     bool forceTc20Off = false; // NUTO_GPU_TC20=off
     int tc20LawFp64 = 0;       // NUTO_GPU_TC20=fp64law: the law of every point in FP64
     // element matrices of the last tangent in each arithmetic, and the plan of the row gather
+    bool solveFollows = true; // the FP64 tangent is for an FP64 solve (not NUTO_GPU_FP64X): leave its memory
     ElemMats<float> elemMats32;
     ElemMats<double> elemMats64;
     DBuf<unsigned char> dRowPlan; // where the element matrices were there before the plan

@@ -1553,13 +1553,16 @@ int ResolveMethod(const Ctx& c, int method)
 
 // Device memory that a first FP64 solve of the context takes: the padded values, the multigrid's coarse levels (values in two
 // layouts; a fourth of the fine ones is on the safe side on lattices), its and the solver's vectors, and for GMRES both bases.
+// The tangent of the exact final phase (NUTO_GPU_FP64X) is not solved with: the padded values for its products.
 size_t SolverBytesToCome(const Ctx& c)
 {
     const size_t n = static_cast<size_t>(c.nDofs), nnz = static_cast<size_t>(c.nnz);
     const SolverWork* w = c.work;
-    size_t values = 0;
+    size_t values = c.nb.v64.n == 0 ? static_cast<size_t>(c.nb.total) : 0;
+    if (!c.solveFollows)
+        return values * sizeof(double);
     if (c.nb.v64.n == 0)
-        values += static_cast<size_t>(c.nb.total) + nnz / 2 + 20 * n;
+        values += nnz / 2 + 20 * n;
     if (!w || w->v64.n == 0)
         values += 21 * n;
     if (c.prm.kind != NUTO_GPU_MB_LINEAR_ELASTIC && (!w || w->g64.n == 0))

@@ -157,7 +157,7 @@ int DoStep(Ctx& c, double tNew, const nuto_gpu_step_options& o, int* itersOut)
         const int k = T.Begin();
         if (exactNow)
         {
-            LaunchTangent(c, x, NUTO_GPU_FP64, w.K64.p);
+            LaunchTangent(c, x, NUTO_GPU_FP64X, w.K64.p); // refines FP32 solves: products only
             k_round<<<static_cast<unsigned>((c.nnz + 255) / 256), 256, 0, c.stream>>>(c.nnz, w.K64.p, w.K32.p);
             c.valsVersion++;
             S.kernel_launches += 1;

@@ -62,6 +62,25 @@ def test_fp64_tangent_leaves_the_solve_its_memory(leave_free):
     assert (g.build_matrix(u, 64, out=values) - ref).abs().max() <= 1e-12 * ref.abs().max()
 
 
+def test_exact_phase_tangent_beside_the_fp32_solver(leave_free):
+    """The tangent of the exact final phase (precision 65) is multiplied with, not solved: in the same 1000 MB the element
+    matrices and the padded values fit, and the values are those of a context with all the memory bit for bit."""
+    import torch
+
+    full, u, _ = _group()
+    ref = full.build_matrix(u, 65).cpu()
+    del full
+    g, _, _ = _group()
+    values = torch.empty(g.nnz, dtype=torch.float64, device="cuda")
+    x = torch.ones(g.n_dofs, dtype=torch.float64, device="cuda")
+    leave_free(1000 << 20)
+    g.build_matrix(u, 65, out=values)
+    g.spmv(values, x)
+    torch.cuda.synchronize()
+    leave_free(None)
+    assert torch.equal(values.cpu(), ref)
+
+
 def test_fp32_tangent_without_room_for_element_matrices(leave_free):
     """In 200 MB the FP32 tangent comes from the point records (1e-6 of the largest entry from the element matrices, the bound
     of the no-alloc call, which has the same kernels); a new pattern asks for the memory again."""
